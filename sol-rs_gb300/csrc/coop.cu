@@ -523,12 +523,18 @@ __global__ void __launch_bounds__(kCoopBlock, (coop_min_blocks<KIND>())) k_batch
             for (uint32_t t = blockIdx.x * kCoopBlock + threadIdx.x; t < pp.pixels; t += gridDim.x * kCoopBlock)
                 accumulate_pixel<LdL2>(a.jobs, items, pp.item_count, t, a.rad);
         }
-        __syncthreads();  // every thread is done with pass c.p
-        if (threadIdx.x == 0) {
-            c.p = c.p + 1u;
-            c.b = 0u;
+        if constexpr (kNee) {
+            // generate zeroes the radiance slots of next-event-estimation
+            // paths, which other blocks may still be summing: meet first
+            if (!coop_barrier(a, c, kNextPass)) break;
+        } else {
+            __syncthreads();  // every thread is done with pass c.p
+            if (threadIdx.x == 0) {
+                c.p = c.p + 1u;
+                c.b = 0u;
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
     if (c.ok && coop_barrier(a, c, kStay))
         for (uint32_t t = blockIdx.x * kCoopBlock + threadIdx.x; t < a.total_pix; t += gridDim.x * kCoopBlock)
