@@ -494,12 +494,13 @@ solrt_status solrt_batch_info(solrt_batch* batch, uint32_t* passes, uint32_t* it
 
 /* ---- launch tuning ---------------------------------------------------------
  * No counterpart in the reference (its launch shape is the driver's). The
- * extend kernel's block size and the number of BVH2 traversal-stack slots
+ * extend kernel's block size and how much of the BVH2 traversal stack is
  * kept in shared memory, and the number of paths per batch pass, change
  * speed only: images are identical for every setting. */
 typedef struct solrt_tune_config {
     uint32_t block_size;   /* extend threads per block: 64, 128 or 256 */
-    uint32_t smem_stack;   /* BVH2 stack slots per thread in shared memory: 16 or 32 */
+    uint32_t smem_stack;   /* shared memory per thread for the BVH2 / BVH4 traversal stack: 16 or
+                              32 (12 or 16 entries; deeper ones in global memory) */
     uint32_t pass_paths;   /* paths per batch pass, <= the path capacity; 0 = the capacity */
     uint32_t reserved;
 } solrt_tune_config;

@@ -397,10 +397,14 @@ solrt_status solrt_context_create(const solrt_context_desc* desc, solrt_context*
     solrt_status s;
     if ((s = c->hits.alloc(16 * C)) != SOLRT_OK) return fail(s);
     if ((s = c->rad.alloc(16 * C)) != SOLRT_OK) return fail(s);
-    if ((s = c->ctl.alloc(sizeof(PassCtl))) != SOLRT_OK) return fail(s);
     if ((s = c->stats.alloc(2 * sizeof(DevStats))) != SOLRT_OK) return fail(s);
-    if ((s = c->trace_work.alloc(sizeof(unsigned int))) != SOLRT_OK) return fail(s);
-    if (cudaMemset(c->ctl.ptr, 0, sizeof(PassCtl)) != cudaSuccess ||
+    if ((s = c->trace_work.alloc(2 * sizeof(unsigned int))) != SOLRT_OK) return fail(s);
+    if ((s = c->queue_counts.alloc(2 * (SOLRT_MAX_BOUNCES + 2) * sizeof(unsigned int))) != SOLRT_OK) return fail(s);
+    if ((s = c->deep_stack.alloc(sizeof(int) * (SOLRT_BVH2_STACK + 1 - kMinStackSlots) * (size_t)c->sm_count *
+                                 kMaxThreadsPerSm)) != SOLRT_OK)
+        return fail(s);
+    if (cudaMemset(c->trace_work.ptr, 0, 2 * sizeof(unsigned int)) != cudaSuccess ||
+        cudaMemset(c->queue_counts.ptr, 0, c->queue_counts.bytes) != cudaSuccess ||
         cudaMemset(c->stats.ptr, 0, 2 * sizeof(DevStats)) != cudaSuccess ||
         cudaDeviceSynchronize() != cudaSuccess) {
         set_error("device initialisation failed");

@@ -38,56 +38,36 @@ SOLRT_D void instance_ray(const float4* inst, uint32_t k, float ox, float oy, fl
 // (ray transformed, marker pushed, BLAS root next), a parked triangle leaf
 // is tested before its lane leaves the instance, and the marker restores the
 // world ray (reloaded from the queue).
-template <class IO, bool kCount, int kBlock, int kSmem>
-SOLRT_D void extend_bvh2_2l_ww(const IO& io, uint32_t n, unsigned int* work, TraceCounters& cnt, uint32_t& ef) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lane_lt = (1u << lane) - 1u;
-    Bvh2Stack<kBlock, kSmem> stack;
-    __shared__ int s_stack[(kSmem > 0 ? kSmem : 1) * kBlock];
-    stack.sh = s_stack + threadIdx.x;
+template <class IO, bool kCount>
+SOLRT_D void extend_bvh2_2l_ww(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
+                               uint32_t& ef) {
+    Bvh2Stack stack;
+    stack.m = mem;
+    const RayMem rm = mem.ray_mem();
     int sp = 0;
     int node = kBvh2Sentinel;  // TLAS or BLAS node (>= 0), leaf (< 0), marker, or sentinel
     int leaf = 0;              // parked triangle leaf (< 0) or none (>= 0)
     int inst = -1;             // instance being traversed, -1 = the TLAS
     bool has = false;
     bool drained = false;
-    uint32_t idx = 0, budget = 0;
-    RayWT r;
-    TravScene ts{nullptr, nullptr, 0u, 0u};
-    float ix = 0.0f, iy = 0.0f, iz = 0.0f, nox = 0.0f, noy = 0.0f, noz = 0.0f;
-    float tmin = 0.0f;
-    HitRec best{0.0f, SOLRT_NO_HIT, 0.0f, 0.0f};
+    uint32_t budget = 0;
+    TravScene ts = io.first_scene();
+    RayBox<false> rb{};
+    float tmin = 0.0f, best_t = 0.0f;
     for (;;) {
         const bool idle = node == kBvh2Sentinel && leaf >= 0;
-        if (idle && has) {
-            io.store(idx, best);
-            has = false;
-        }
-        const uint32_t need = __ballot_sync(0xffffffffu, idle);
-        if (!drained && __popc(need) >= SOLRT_BVH2_REFILL) {
-            const int leader = __ffs(need) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(work, (unsigned int)__popc(need));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + (uint32_t)__popc(need) >= n) drained = true;
-            if (idle) {
-                const uint32_t i = base + (uint32_t)__popc(need & lane_lt);
-                if (i < n) {
-                    float4 o, d;
-                    io.load(i, o, d, ts);
-                    idx = i;
-                    has = true;
-                    tmin = o.w;
-                    bvh2_ray_consts<false>(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z, ix, iy, iz, nox, noy, noz);
-                    best = HitRec{d.w, SOLRT_NO_HIT, 0.0f, 0.0f};
-                    budget = 2u * (ts.node_count + ts.tri_count + ts.tlas_count + ts.inst_count) + 64u;
-                    stack.put(0, kBvh2Sentinel);
-                    sp = 1;
-                    inst = -1;
-                    node = (ts.tlas_count && ts.tri_count) ? 0 : kBvh2Sentinel;
-                    leaf = 0;
-                }
-            }
+        float4 o, d;
+        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH2_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+            rm.clear_hit();
+            tmin = o.w;
+            rb.set(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z);
+            best_t = d.w;
+            budget = 2u * (ts.node_count + ts.tri_count + ts.tlas_count + ts.inst_count) + 64u;
+            stack.put(0, kBvh2Sentinel);
+            sp = 1;
+            inst = -1;
+            node = (ts.tlas_count && ts.tri_count) ? 0 : kBvh2Sentinel;
+            leaf = 0;
         }
         if (!__any_sync(0xffffffffu, has)) {
             if (drained) break;
@@ -114,8 +94,8 @@ SOLRT_D void extend_bvh2_2l_ww(const IO& io, uint32_t n, unsigned int* work, Tra
             }
             if (leave) {  // back to the TLAS: world ray again
                 float4 o, d;
-                io.load_ray(idx, o, d);
-                bvh2_ray_consts<false>(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z, ix, iy, iz, nox, noy, noz);
+                io.load_ray(rm.get(kRayIdx), o, d);
+                rb.set(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z);
                 inst = -1;
                 node = stack.get(--sp);
                 continue;
@@ -125,12 +105,12 @@ SOLRT_D void extend_bvh2_2l_ww(const IO& io, uint32_t n, unsigned int* work, Tra
                 int root = -1;
                 if (k < ts.inst_count) {
                     float4 o, d;
-                    io.load_ray(idx, o, d);
+                    io.load_ray(rm.get(kRayIdx), o, d);
                     float px, py, pz, qx, qy, qz;
                     instance_ray(ts.inst, k, o.x, o.y, o.z, d.x, d.y, d.z, px, py, pz, qx, qy, qz, root);
                     if (root >= 0 && (uint32_t)root < ts.node_count && sp <= SOLRT_BVH2_STACK) {
-                        r = setup_ray(px, py, pz, qx, qy, qz, tmin);
-                        bvh2_ray_consts<false>(ts.nodes, px, py, pz, qx, qy, qz, ix, iy, iz, nox, noy, noz);
+                        rm.set_ray(px, py, pz, qx, qy, qz);
+                        rb.set(ts.nodes, px, py, pz, qx, qy, qz);
                         stack.put(sp++, kBvh2LeaveInstance);
                         inst = (int)k;
                         node = root;
@@ -141,7 +121,7 @@ SOLRT_D void extend_bvh2_2l_ww(const IO& io, uint32_t n, unsigned int* work, Tra
                 node = stack.get(--sp);
                 continue;
             }
-            // inner node of the current level
+            // inner nodes of the current level
             const float4* arr = inst < 0 ? ts.tlas : ts.nodes;
             const uint32_t cnt_nodes = inst < 0 ? ts.tlas_count : ts.node_count;
             if ((uint32_t)node >= cnt_nodes) {
@@ -150,27 +130,27 @@ SOLRT_D void extend_bvh2_2l_ww(const IO& io, uint32_t n, unsigned int* work, Tra
                 leaf = 0;
                 continue;
             }
-            if (kCount) ++cnt.nodes;
-            float t0, t1;
-            bool h0, h1;
-            int c0, c1;
-            bvh2_node_step<false>(arr, node, ix, iy, iz, nox, noy, noz, tmin, best.t, h0, t0, h1, t1, c0, c1);
-            h1 = h1 && c1 != c0;  // a node whose two children are the same (one instance, one triangle)
-            if (h0 && h1) {
-                const bool swap = t1 < t0;
-                if (sp <= SOLRT_BVH2_STACK) stack.put(sp++, swap ? c0 : c1);
-                else ef |= SOLRT_EFLAG_STACK;
-                node = swap ? c1 : c0;
-            } else if (h0) {
-                node = c0;
-            } else if (h1) {
-                node = c1;
-            } else {
-                node = stack.get(--sp);
-            }
-            if (inst >= 0 && node < 0 && leaf >= 0) {  // park a triangle, keep descending
-                leaf = node;
-                node = stack.get(--sp);
+#pragma unroll
+            for (int u = 0; u < SOLRT_BVH2_NODE_STEPS; ++u) {
+                if (u > 0 && (uint32_t)node >= cnt_nodes) break;
+                if (kCount) ++cnt.nodes;
+                float t0, t1;
+                bool h0, h1;
+                int c0, c1;
+                bvh2_node_step<false>(arr, node, rb, tmin, best_t, h0, t0, h1, t1, c0, c1);
+                h1 = h1 && c1 != c0;  // a node whose two children are the same (one instance, one triangle)
+                const bool first0 = h0 && (!h1 || !(t1 < t0));
+                node = first0 ? c0 : c1;
+                if (h0 && h1) {
+                    if (sp <= SOLRT_BVH2_STACK) stack.put(sp++, first0 ? c1 : c0);
+                    else ef |= SOLRT_EFLAG_STACK;
+                } else if (!h0 && !h1) {
+                    node = stack.get(--sp);
+                }
+                if (inst >= 0 && node < 0 && leaf >= 0) {  // park a triangle, keep descending
+                    leaf = node;
+                    node = stack.get(--sp);
+                }
             }
         }
         // leaf phase: triangles in the object space of the lane's instance
@@ -184,8 +164,8 @@ SOLRT_D void extend_bvh2_2l_ww(const IO& io, uint32_t n, unsigned int* work, Tra
                 } else {
                     const float4* tp = ts.tris + 3 * (size_t)k;
                     if (kCount) ++cnt.tris;
-                    cnt.fallbacks += intersect_tri(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best);
-                    if (io.any_hit && best.prim != SOLRT_NO_HIT) {  // occlusion query: done at the first hit
+                    if (intersect_tri(rm, tmin, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, cnt.fallbacks) &&
+                        io.any_hit) {  // occlusion query: done at the first hit
                         node = kBvh2Sentinel;
                         leaf = 0;
                     } else {
@@ -205,8 +185,8 @@ SOLRT_D void trace_bvh2_2l_ray(const TravScene& ts, float ox, float oy, float oz
     best = HitRec{tmax, SOLRT_NO_HIT, 0.0f, 0.0f};
     if (ts.tri_count == 0 || ts.tlas_count == 0) return;
     RayWT r;
-    float ix, iy, iz, nox, noy, noz;
-    bvh2_ray_consts<false>(ts.nodes, ox, oy, oz, dx, dy, dz, ix, iy, iz, nox, noy, noz);
+    RayBox<false> rb;
+    rb.set(ts.nodes, ox, oy, oz, dx, dy, dz);
     int stack[SOLRT_BVH2_STACK + 1];
     stack[0] = kBvh2Sentinel;
     int sp = 1;
@@ -219,7 +199,7 @@ SOLRT_D void trace_bvh2_2l_ray(const TravScene& ts, float ox, float oy, float oz
             return;
         }
         if (node == kBvh2LeaveInstance) {
-            bvh2_ray_consts<false>(ts.nodes, ox, oy, oz, dx, dy, dz, ix, iy, iz, nox, noy, noz);
+            rb.set(ts.nodes, ox, oy, oz, dx, dy, dz);
             inst = -1;
         } else if (node < 0 && inst < 0) {
             const uint32_t k = (uint32_t)(~node);
@@ -236,7 +216,7 @@ SOLRT_D void trace_bvh2_2l_ray(const TravScene& ts, float ox, float oy, float oz
                     return;
                 }
                 r = setup_ray(px, py, pz, qx, qy, qz, tmin);
-                bvh2_ray_consts<false>(ts.nodes, px, py, pz, qx, qy, qz, ix, iy, iz, nox, noy, noz);
+                rb.set(ts.nodes, px, py, pz, qx, qy, qz);
                 stack[sp++] = kBvh2LeaveInstance;
                 inst = (int)k;
                 node = root;
@@ -259,7 +239,7 @@ SOLRT_D void trace_bvh2_2l_ray(const TravScene& ts, float ox, float oy, float oz
             float t0, t1;
             bool h0, h1;
             int c0, c1;
-            bvh2_node_step<false>(arr, node, ix, iy, iz, nox, noy, noz, tmin, best.t, h0, t0, h1, t1, c0, c1);
+            bvh2_node_step<false>(arr, node, rb, tmin, best.t, h0, t0, h1, t1, c0, c1);
             h1 = h1 && c1 != c0;
             if (h0 && h1) {
                 const bool swap = t1 < t0;

@@ -5,9 +5,10 @@
 //   refill  lanes whose ray has finished take new rays from the global queue
 //           (one atomic per warp), once at least SOLRT_BVH2_REFILL lanes are
 //           free;
-//   nodes   lanes visit inner nodes until every lane has parked a leaf or has
-//           no inner node left, or until fewer than SOLRT_WW_NODE_MIN lanes
-//           still have inner nodes while others hold leaves; a lane that
+//   nodes   lanes visit inner nodes, up to SOLRT_BVH2_NODE_STEPS between two
+//           votes, until every lane has parked a leaf or has no inner node
+//           left, or until fewer than SOLRT_WW_NODE_MIN lanes still have
+//           inner nodes while others hold leaves; a lane that
 //           already parked a leaf keeps descending until it reaches a second
 //           one ("while-while" with speculative traversal, after Aila &
 //           Laine, HPG 2009);
@@ -31,18 +32,45 @@ constexpr int kBvh2Sentinel = 0x7fffffff;
 #ifndef SOLRT_WW_NODE_MIN
 #define SOLRT_WW_NODE_MIN 12
 #endif
-// 1: a lane that has parked a leaf keeps visiting inner nodes until it
-// reaches a second leaf; 0: it waits for the leaf phase.
-#ifndef SOLRT_WW_SPECULATE
-#define SOLRT_WW_SPECULATE 1
+// Inner nodes a lane may visit between two votes of its warp. The votes and
+// the phase tests are about a quarter of a step's instructions; 4.2M incoherent
+// rays through a 1M-triangle tree (32-byte nodes): 1 step 2.47 ms, 2 steps
+// 2.26, 3 steps 2.20, 4 steps 2.20; a 64-spp soup frame 121.4 / 117.7 / 116.2 ms
+// with 2 / 3 / 4.
+#ifndef SOLRT_BVH2_NODE_STEPS
+#define SOLRT_BVH2_NODE_STEPS 4
 #endif
-// Default traversal stack entries kept in shared memory (slot-major, one
-// column per thread, so lanes at different depths hit different banks);
-// deeper entries go to a local-memory array. The launch may pick 16 or 32
-// (solrt_context_set_tune / solrt_batch_autotune).
-#ifndef SOLRT_SMEM_STACK
-#define SOLRT_SMEM_STACK 32
-#endif
+// A thread's traversal-stack memory: entry k at shared address base + k *
+// stride for k < slots (stride = 4 x threads per block, so lanes at different
+// depths hit different banks), the rest at deep[k * deep_stride] in global
+// memory. A 1M-triangle tree's rays hold at most about 20 entries, so `deep` is
+// hardly ever touched; it is global and not local memory because a local load
+// cannot fault, so the compiler issues it for every pop, ahead of the test
+// (4.2M incoherent rays through a 1M-triangle tree: 4.12 ms with local memory
+// behind the shared slots, 3.19 with a ring of shared slots that spills,
+// 2.95 with global memory behind them).
+struct StackMem {
+    uint32_t base;
+    uint32_t stride;
+    int slots;
+    int* deep;
+    uint32_t deep_stride;
+    uint32_t ray;  // shared address of the thread's RayMem column (same stride)
+    SOLRT_D RayMem ray_mem() const { return RayMem{ray, stride}; }
+};
+
+// Per-thread traversal stack of SOLRT_BVH2_STACK + 1 entries.
+struct Bvh2Stack {
+    StackMem m;
+    SOLRT_D void put(int k, int v) {
+        if (k < m.slots) sts_u32(m.base + (uint32_t)k * m.stride, (uint32_t)v);
+        else m.deep[(size_t)((uint32_t)k * m.deep_stride)] = v;
+    }
+    SOLRT_D int get(int k) {
+        if (k < m.slots) return (int)lds_u32(m.base + (uint32_t)k * m.stride);
+        return m.deep[(size_t)((uint32_t)k * m.deep_stride)];
+    }
+};
 
 // The 4 float4 of BVH2 node `node` (64-byte aligned) in two 256-bit loads.
 SOLRT_D void load_bvh2_node(const float4* nodes, int node, float4& n0, float4& n1, float4& n2, int4& n3) {
@@ -53,114 +81,80 @@ SOLRT_D void load_bvh2_node(const float4* nodes, int node, float4& n0, float4& n
     n3 = make_int4(__float_as_int(r.x), __float_as_int(r.y), __float_as_int(r.z), __float_as_int(r.w));
 }
 
-// Per-thread traversal stack: slots [0, kSmem) in shared memory, the rest
-// in local memory; SOLRT_BVH2_STACK + 1 slots in all.
-template <int kBlock, int kSmem>
-struct Bvh2Stack {
-    int* sh;  // slot k at sh[k * kBlock]
-    int lo[SOLRT_BVH2_STACK + 1 - kSmem];
-    SOLRT_D void put(int k, int v) {
-        if (k < kSmem) sh[k * kBlock] = v;
-        else lo[k - kSmem] = v;
+// A ray's constants of the slab test: (1/d, -o/d) per axis for FP32 nodes,
+// (c/d, (G - o)/d - 2^23 c/d) for BVH2-q16 nodes (q16_ray).
+template <bool kQ16>
+struct RayBox {
+    float ix, iy, iz, nox, noy, noz;
+    SOLRT_D void set(const float4* nodes, float ox, float oy, float oz, float dx, float dy, float dz) {
+        if constexpr (kQ16) {
+            q16_ray(nodes, ox, oy, oz, dx, dy, dz, ix, iy, iz, nox, noy, noz);
+        } else {
+            ix = 1.0f / box_dir(dx);
+            iy = 1.0f / box_dir(dy);
+            iz = 1.0f / box_dir(dz);
+            nox = -(ox * ix);
+            noy = -(oy * iy);
+            noz = -(oz * iz);
+        }
     }
-    SOLRT_D int get(int k) const { return k < kSmem ? sh[k * kBlock] : lo[k - kSmem]; }
-};
-template <int kBlock>
-struct Bvh2Stack<kBlock, 0> {
-    int* sh;
-    int lo[SOLRT_BVH2_STACK + 1];
-    SOLRT_D void put(int k, int v) { lo[k] = v; }
-    SOLRT_D int get(int k) const { return lo[k]; }
 };
 
-// One node test in either node format (kQ16: 32-byte
-// BVH2-q16 nodes, one 256-bit load; else 64-byte FP32 nodes, two).
+// One node test in either node format (kQ16: 32-byte BVH2-q16 nodes, one
+// 256-bit load; else 64-byte FP32 nodes, two).
 template <bool kQ16>
-SOLRT_D void bvh2_node_step(const float4* nodes, int node, float ix, float iy, float iz, float nox, float noy,
-                            float noz, float tmin, float tmax, bool& h0, float& t0, bool& h1, float& t1, int& ref0,
-                            int& ref1) {
+SOLRT_D void bvh2_node_step(const float4* nodes, int node, const RayBox<kQ16>& r, float tmin, float tmax, bool& h0,
+                            float& t0, bool& h1, float& t1, int& ref0, int& ref1) {
     if constexpr (kQ16) {
         float4 a, b;
         ldg_2x4(nodes + 2 + 2 * (size_t)node, a, b);
-        slab2_q16(a, b, ix, iy, iz, nox, noy, noz, tmin, tmax, h0, t0, h1, t1);
+        slab2_q16(a, b, r.ix, r.iy, r.iz, r.nox, r.noy, r.noz, tmin, tmax, h0, t0, h1, t1);
         ref0 = __float_as_int(a.x);
         ref1 = __float_as_int(a.y);
     } else {
         float4 n0, n1, n2;
         int4 n3;
         load_bvh2_node(nodes, node, n0, n1, n2, n3);
-        slab2_fma(n0, n1, n2, ix, iy, iz, nox, noy, noz, tmin, tmax, h0, t0, h1, t1);
+        slab2_fma(n0, n1, n2, r.ix, r.iy, r.iz, r.nox, r.noy, r.noz, tmin, tmax, h0, t0, h1, t1);
         ref0 = n3.x;
         ref1 = n3.y;
     }
 }
 
-// Per-ray constants of the slab test: (1/d, -o/d) per axis for FP32 nodes,
-// (c/d, (G - o)/d - 2^23 c/d) for BVH2-q16 nodes (q16_ray).
-template <bool kQ16>
-SOLRT_D void bvh2_ray_consts(const float4* nodes, float ox, float oy, float oz, float dx, float dy, float dz,
-                             float& ix, float& iy, float& iz, float& nox, float& noy, float& noz) {
-    if constexpr (kQ16) {
-        q16_ray(nodes, ox, oy, oz, dx, dy, dz, ix, iy, iz, nox, noy, noz);
-    } else {
-        ix = 1.0f / box_dir(dx);
-        iy = 1.0f / box_dir(dy);
-        iz = 1.0f / box_dir(dz);
-        nox = -(ox * ix);
-        noy = -(oy * iy);
-        noz = -(oz * iz);
-    }
-}
-
-template <class IO, bool kCount, int kBlock, int kSmem, bool kQ16 = false>
-SOLRT_D void extend_bvh2_ww(const IO& io, uint32_t n, unsigned int* work, TraceCounters& cnt, uint32_t& ef) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lane_lt = (1u << lane) - 1u;
-    Bvh2Stack<kBlock, kSmem> stack;
-    __shared__ int s_stack[(kSmem > 0 ? kSmem : 1) * kBlock];
-    stack.sh = s_stack + threadIdx.x;
+template <class IO, bool kCount, bool kQ16 = false>
+SOLRT_D void extend_bvh2_ww(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
+                            uint32_t& ef) {
+    Bvh2Stack stack;
+    stack.m = mem;
+    const RayMem rm = mem.ray_mem();
     int sp = 0;
     int node = kBvh2Sentinel;  // >= 0 inner node, < 0 leaf ~k, sentinel = nothing left
     int leaf = 0;              // parked leaf (< 0) or none (>= 0)
     bool has = false;
     bool drained = false;      // the queue has no more rays for this warp
-    uint32_t idx = 0, budget = 0;
-    RayWT r;
-    TravScene ts{nullptr, nullptr, 0u, 0u};
-    float ix = 0.0f, iy = 0.0f, iz = 0.0f;     // 1 / box_dir(d)
-    float nox = 0.0f, noy = 0.0f, noz = 0.0f;  // -o / box_dir(d)
-    HitRec best{0.0f, SOLRT_NO_HIT, 0.0f, 0.0f};
+    uint32_t budget = 0;
+    TravScene ts = io.first_scene();
+    RayBox<kQ16> rb{};
+    float tmin = 0.0f, best_t = 0.0f;
     for (;;) {
-        const bool idle = node == kBvh2Sentinel && leaf >= 0;
-        if (idle && has) {
-            io.store(idx, best);
-            has = false;
+        // no inner node (an index past the last one counts as none) and no leaf
+        const bool idle = (unsigned)node >= ts.node_count && node >= 0 && leaf >= 0;
+        if (idle && node != kBvh2Sentinel) {
+            ef |= SOLRT_EFLAG_INDEX;
+            node = kBvh2Sentinel;
         }
-        const uint32_t need = __ballot_sync(0xffffffffu, idle);
-        if (!drained && __popc(need) >= SOLRT_BVH2_REFILL) {
-            const int leader = __ffs(need) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(work, (unsigned int)__popc(need));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + (uint32_t)__popc(need) >= n) drained = true;
-            if (idle) {
-                const uint32_t i = base + (uint32_t)__popc(need & lane_lt);
-                if (i < n) {
-                    float4 o, d;
-                    io.load(i, o, d, ts);
-                    idx = i;
-                    has = true;
-                    r = setup_ray(o.x, o.y, o.z, d.x, d.y, d.z, o.w);
-                    if (ts.tri_count)
-                        bvh2_ray_consts<kQ16>(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z, ix, iy, iz, nox, noy, noz);
-                    best = HitRec{d.w, SOLRT_NO_HIT, 0.0f, 0.0f};
-                    budget = 2u * (ts.node_count + ts.tri_count) + 64u;
-                    stack.put(0, kBvh2Sentinel);
-                    sp = 1;
-                    node = ts.tri_count ? 0 : kBvh2Sentinel;
-                    leaf = 0;
-                }
-            }
+        float4 o, d;
+        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH2_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+            rm.set_ray(o.x, o.y, o.z, d.x, d.y, d.z);
+            rm.clear_hit();
+            if (ts.tri_count) rb.set(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z);
+            tmin = o.w;
+            best_t = d.w;
+            budget = 2u * (ts.node_count + ts.tri_count) + 64u;
+            stack.put(0, kBvh2Sentinel);
+            sp = 1;
+            node = ts.tri_count ? 0 : kBvh2Sentinel;
+            leaf = 0;
         }
         if (!__any_sync(0xffffffffu, has)) {
             if (drained) break;
@@ -168,46 +162,42 @@ SOLRT_D void extend_bvh2_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
         }
         // node phase
         for (;;) {
-            const bool inner = (unsigned)node < (unsigned)kBvh2Sentinel;
             // two ballots decide the phase: stop when no lane without a
             // parked leaf has inner nodes, or when few lanes still have inner
             // nodes while others hold leaves (test the leaves first; the leaf
             // phase then has work, so this ends)
+            const bool inner = (unsigned)node < ts.node_count;
             const uint32_t b_inner = __ballot_sync(0xffffffffu, inner);
             const uint32_t b_leaf = __ballot_sync(0xffffffffu, leaf < 0);
-            const uint32_t b_free = b_inner & ~b_leaf;  // inner nodes, no parked leaf
-            if (b_free == 0u) break;
-#if SOLRT_WW_NODE_MIN > 0
-            if (__popc(SOLRT_WW_SPECULATE ? b_inner : b_free) < SOLRT_WW_NODE_MIN && b_leaf) break;
-#endif
-            if (inner && (SOLRT_WW_SPECULATE || leaf >= 0)) {
-                if (--budget == 0u || (uint32_t)node >= ts.node_count) {
-                    ef |= SOLRT_EFLAG_INDEX;
-                    node = kBvh2Sentinel;
-                    leaf = 0;
-                } else {
-                    if (kCount) ++cnt.nodes;
-                    float t0, t1;
-                    bool h0, h1;
-                    int c0, c1;
-                    bvh2_node_step<kQ16>(ts.nodes, node, ix, iy, iz, nox, noy, noz, r.tmin, best.t, h0, t0, h1, t1,
-                                         c0, c1);
-                    if (h0 && h1) {
-                        const bool swap = t1 < t0;
-                        if (sp <= SOLRT_BVH2_STACK) stack.put(sp++, swap ? c0 : c1);
-                        else ef |= SOLRT_EFLAG_STACK;
-                        node = swap ? c1 : c0;
-                    } else if (h0) {
-                        node = c0;
-                    } else if (h1) {
-                        node = c1;
-                    } else {
-                        node = stack.get(--sp);
-                    }
-                    if (node < 0 && leaf >= 0) {  // park the leaf, keep descending
-                        leaf = node;
-                        node = stack.get(--sp);
-                    }
+            if ((b_inner & ~b_leaf) == 0u) break;
+            if (__popc(b_inner) < SOLRT_WW_NODE_MIN && b_leaf) break;
+            if (!inner) continue;
+            if (--budget == 0u) {
+                ef |= SOLRT_EFLAG_INDEX;
+                node = kBvh2Sentinel;
+                leaf = 0;
+                continue;
+            }
+#pragma unroll
+            for (int u = 0; u < SOLRT_BVH2_NODE_STEPS; ++u) {
+                if (u > 0 && (unsigned)node >= ts.node_count) break;
+                if (kCount) ++cnt.nodes;
+                float t0, t1;
+                bool h0, h1;
+                int c0, c1;
+                bvh2_node_step<kQ16>(ts.nodes, node, rb, tmin, best_t, h0, t0, h1, t1, c0, c1);
+                // nearer child first; the other one, when hit too, is pushed
+                const bool first0 = h0 && (!h1 || !(t1 < t0));
+                node = first0 ? c0 : c1;
+                if (h0 && h1) {
+                    if (sp <= SOLRT_BVH2_STACK) stack.put(sp++, first0 ? c1 : c0);
+                    else ef |= SOLRT_EFLAG_STACK;
+                } else if (!h0 && !h1) {
+                    node = stack.get(--sp);
+                }
+                if (node < 0 && leaf >= 0) {  // park the leaf, keep descending
+                    leaf = node;
+                    node = stack.get(--sp);
                 }
             }
         }
@@ -222,8 +212,8 @@ SOLRT_D void extend_bvh2_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
                 } else {
                     const float4* tp = ts.tris + 3 * (size_t)k;
                     if (kCount) ++cnt.tris;
-                    cnt.fallbacks += intersect_tri(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best);
-                    if (io.any_hit && best.prim != SOLRT_NO_HIT) {  // occlusion query: done at the first hit
+                    if (intersect_tri(rm, tmin, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, cnt.fallbacks) &&
+                        io.any_hit) {  // occlusion query: done at the first hit
                         node = kBvh2Sentinel;
                         leaf = 0;
                     } else {
@@ -244,8 +234,8 @@ SOLRT_D void trace_bvh2_ray(const TravScene& ts, float ox, float oy, float oz, f
     best = HitRec{tmax, SOLRT_NO_HIT, 0.0f, 0.0f};
     if (ts.tri_count == 0) return;
     const RayWT r = setup_ray(ox, oy, oz, dx, dy, dz, tmin);
-    float ix, iy, iz, nox, noy, noz;
-    bvh2_ray_consts<kQ16>(ts.nodes, ox, oy, oz, dx, dy, dz, ix, iy, iz, nox, noy, noz);
+    RayBox<kQ16> rb;
+    rb.set(ts.nodes, ox, oy, oz, dx, dy, dz);
     int stack[SOLRT_BVH2_STACK + 1];
     stack[0] = kBvh2Sentinel;
     int sp = 1;
@@ -264,7 +254,7 @@ SOLRT_D void trace_bvh2_ray(const TravScene& ts, float ox, float oy, float oz, f
             float t0, t1;
             bool h0, h1;
             int c0, c1;
-            bvh2_node_step<kQ16>(ts.nodes, node, ix, iy, iz, nox, noy, noz, tmin, best.t, h0, t0, h1, t1, c0, c1);
+            bvh2_node_step<kQ16>(ts.nodes, node, rb, tmin, best.t, h0, t0, h1, t1, c0, c1);
             if (h0 && h1) {
                 const bool swap = t1 < t0;
                 if (sp <= SOLRT_BVH2_STACK) stack[sp++] = swap ? c0 : c1;

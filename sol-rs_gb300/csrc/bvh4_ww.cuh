@@ -68,60 +68,45 @@ SOLRT_D void sort4(uint32_t k[4]) {
     k[3] = h;
 }
 
-template <class IO, bool kCount, int kBlock, int kSmem>
-SOLRT_D void extend_bvh4_ww(const IO& io, uint32_t n, unsigned int* work, TraceCounters& cnt, uint32_t& ef) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lane_lt = (1u << lane) - 1u;
-    Bvh2Stack<kBlock, kSmem> stack;
-    __shared__ int s_stack[(kSmem > 0 ? kSmem : 1) * kBlock];
-    stack.sh = s_stack + threadIdx.x;
+template <class IO, bool kCount>
+SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
+                            uint32_t& ef) {
+    Bvh2Stack stack;
+    stack.m = mem;
     int sp = 0;
     int node = kBvh2Sentinel;            // next 4-wide node to visit, or none
     uint2 tgrp = make_uint2(0u, 0u);     // parked triangles: (triangle base, hit bits)
     bool has = false;
     bool drained = false;
-    uint32_t idx = 0, budget = 0;
+    uint32_t budget = 0;
     bool negx = false, negy = false, negz = false;
-    RayWT r;
-    TravScene ts{nullptr, nullptr, 0u, 0u};
+    const RayMem rm = mem.ray_mem();
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f, tmin = 0.0f, best_t = 0.0f;
+    TravScene ts = io.first_scene();
     float ix = 0.0f, iy = 0.0f, iz = 0.0f;
-    HitRec best{0.0f, SOLRT_NO_HIT, 0.0f, 0.0f};
     for (;;) {
         const bool idle = node == kBvh2Sentinel && tgrp.y == 0u;
-        if (idle && has) {
-            io.store(idx, best);
-            has = false;
-        }
-        const uint32_t need = __ballot_sync(0xffffffffu, idle);
-        if (!drained && __popc(need) >= SOLRT_BVH2_REFILL) {
-            const int leader = __ffs(need) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(work, (unsigned int)__popc(need));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + (uint32_t)__popc(need) >= n) drained = true;
-            if (idle) {
-                const uint32_t i = base + (uint32_t)__popc(need & lane_lt);
-                if (i < n) {
-                    float4 o, d;
-                    io.load(i, o, d, ts);
-                    idx = i;
-                    has = true;
-                    r = setup_ray(o.x, o.y, o.z, d.x, d.y, d.z, o.w);
-                    const float bx = box_dir(d.x), by = box_dir(d.y), bz = box_dir(d.z);
-                    ix = 1.0f / bx;
-                    iy = 1.0f / by;
-                    iz = 1.0f / bz;
-                    negx = signbit(bx);
-                    negy = signbit(by);
-                    negz = signbit(bz);
-                    best = HitRec{d.w, SOLRT_NO_HIT, 0.0f, 0.0f};
-                    budget = 2u * (ts.node_count + ts.tri_count) + 64u;
-                    stack.put(0, kBvh2Sentinel);
-                    sp = 1;
-                    tgrp = make_uint2(0u, 0u);
-                    node = ts.tri_count ? 0 : kBvh2Sentinel;
-                }
-            }
+        float4 o, d;
+        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH2_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+            rm.set_ray(o.x, o.y, o.z, d.x, d.y, d.z);
+            rm.clear_hit();
+            ox = o.x;
+            oy = o.y;
+            oz = o.z;
+            tmin = o.w;
+            best_t = d.w;
+            const float bx = box_dir(d.x), by = box_dir(d.y), bz = box_dir(d.z);
+            ix = 1.0f / bx;
+            iy = 1.0f / by;
+            iz = 1.0f / bz;
+            negx = signbit(bx);
+            negy = signbit(by);
+            negz = signbit(bz);
+            budget = 2u * (ts.node_count + ts.tri_count) + 64u;
+            stack.put(0, kBvh2Sentinel);
+            sp = 1;
+            tgrp = make_uint2(0u, 0u);
+            node = ts.tri_count ? 0 : kBvh2Sentinel;
         }
         if (!__any_sync(0xffffffffu, has)) {
             if (drained) break;
@@ -145,7 +130,7 @@ SOLRT_D void extend_bvh4_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
                     ldg_2x4(np + 2, w2, w3);
                     if (kCount) ++cnt.nodes;
                     uint32_t keys[4], ht = 0;
-                    bvh4_node_test(w0, w1, w2, w3, r.ox, r.oy, r.oz, ix, iy, iz, negx, negy, negz, r.tmin, best.t,
+                    bvh4_node_test(w0, w1, w2, w3, ox, oy, oz, ix, iy, iz, negx, negy, negz, tmin, best_t,
                                    keys, ht);
                     sort4(keys);
                     const uint32_t imask = __float_as_uint(w0.w) >> 24;
@@ -183,8 +168,8 @@ SOLRT_D void extend_bvh4_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
                 } else {
                     const float4* tp = ts.tris + 3 * (size_t)ti;
                     if (kCount) ++cnt.tris;
-                    cnt.fallbacks += intersect_tri(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best);
-                    if (io.any_hit && best.prim != SOLRT_NO_HIT) {  // occlusion query: done at the first hit
+                    if (intersect_tri(rm, tmin, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, cnt.fallbacks) &&
+                        io.any_hit) {  // occlusion query: done at the first hit
                         tgrp.y = 0u;
                         node = kBvh2Sentinel;
                         sp = 1;

@@ -15,6 +15,7 @@
 // that of the per-ray loop.
 #pragma once
 
+#include "bvh2_ww.cuh"
 #include "bvh8_traverse.cuh"
 
 namespace solrt {
@@ -26,87 +27,53 @@ namespace solrt {
 #define SOLRT_BVH8_NODE_MIN 12
 #endif
 
-// Per-thread stack of node groups: entries [0, kSmem) in shared memory
-// (slot-major, one column per thread), the rest in local memory.
-template <int kBlock, int kSmem>
-struct Bvh8Stack {
-    uint2* sh;  // entry k at sh[k * kBlock]
-    uint2 lo[SOLRT_BVH8_STACK - kSmem];
-    SOLRT_D void put(int k, uint2 v) {
-        if (k < kSmem) sh[k * kBlock] = v;
-        else lo[k - kSmem] = v;
-    }
-    SOLRT_D uint2 get(int k) const { return k < kSmem ? sh[k * kBlock] : lo[k - kSmem]; }
-};
-template <int kBlock>
-struct Bvh8Stack<kBlock, 0> {
-    uint2* sh;
-    uint2 lo[SOLRT_BVH8_STACK];
-    SOLRT_D void put(int k, uint2 v) { lo[k] = v; }
-    SOLRT_D uint2 get(int k) const { return lo[k]; }
-};
-
-template <class IO, bool kCount, bool kF32 = false, int kBlock = 128, int kSmem = 0>
-SOLRT_D void extend_bvh8_ww(const IO& io, uint32_t n, unsigned int* work, TraceCounters& cnt, uint32_t& ef) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lane_lt = (1u << lane) - 1u;
-    Bvh8Stack<kBlock, kSmem> stack;
-    __shared__ uint2 s_stack8[(kSmem > 0 ? kSmem : 1) * kBlock];
-    stack.sh = s_stack8 + threadIdx.x;
+// The stack of node groups is in local memory (kept in shared memory it
+// was 1-7 % slower: the groups are 8 bytes and rarely popped).
+template <class IO, bool kCount, bool kF32 = false>
+SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
+                            uint32_t& ef) {
+    uint2 stack[SOLRT_BVH8_STACK];
     int sp = 0;
     uint2 grp = make_uint2(0u, 0u);   // (child base, hit bits << 24 | internal mask)
     uint2 tgrp = make_uint2(0u, 0u);  // parked triangles: (triangle base, hit bits)
     bool has = false;
     bool drained = false;
-    uint32_t idx = 0, budget = 0, oct = 0;
+    uint32_t budget = 0, oct = 0;
     bool negx = false, negy = false, negz = false;
-    RayWT r;
-    TravScene ts{nullptr, nullptr, 0u, 0u};
+    const RayMem rm = mem.ray_mem();
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f, tmin = 0.0f, best_t = 0.0f;
+    TravScene ts = io.first_scene();
     float ix = 0.0f, iy = 0.0f, iz = 0.0f;
     float nox = 0.0f, noy = 0.0f, noz = 0.0f;  // -o / box_dir(d) (FP32 nodes)
-    HitRec best{0.0f, SOLRT_NO_HIT, 0.0f, 0.0f};
     const uint4* nodes = nullptr;
     for (;;) {
         const bool idle = (grp.y >> 24) == 0u && sp == 0 && tgrp.y == 0u;
-        if (idle && has) {
-            io.store(idx, best);
-            has = false;
-        }
-        const uint32_t need = __ballot_sync(0xffffffffu, idle);
-        if (!drained && __popc(need) >= SOLRT_BVH8_REFILL) {
-            const int leader = __ffs(need) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(work, (unsigned int)__popc(need));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + (uint32_t)__popc(need) >= n) drained = true;
-            if (idle) {
-                const uint32_t i = base + (uint32_t)__popc(need & lane_lt);
-                if (i < n) {
-                    float4 o, d;
-                    io.load(i, o, d, ts);
-                    idx = i;
-                    has = true;
-                    r = setup_ray(o.x, o.y, o.z, d.x, d.y, d.z, o.w);
-                    const float bx = box_dir(d.x), by = box_dir(d.y), bz = box_dir(d.z);
-                    ix = 1.0f / bx;
-                    iy = 1.0f / by;
-                    iz = 1.0f / bz;
-                    negx = signbit(bx);
-                    negy = signbit(by);
-                    negz = signbit(bz);
-                    nox = -(o.x * ix);
-                    noy = -(o.y * iy);
-                    noz = -(o.z * iz);
-                    oct = (negx ? 1u : 0u) | (negy ? 2u : 0u) | (negz ? 4u : 0u);
-                    best = HitRec{d.w, SOLRT_NO_HIT, 0.0f, 0.0f};
-                    budget = 2u * (ts.node_count + ts.tri_count) + 64u;
-                    nodes = reinterpret_cast<const uint4*>(ts.nodes);
-                    sp = 0;
-                    tgrp = make_uint2(0u, 0u);
-                    // the root as a group of one internal child in slot 0
-                    grp = ts.tri_count ? make_uint2(0u, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);
-                }
-            }
+        float4 o, d;
+        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH8_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+            rm.set_ray(o.x, o.y, o.z, d.x, d.y, d.z);
+            rm.clear_hit();
+            ox = o.x;
+            oy = o.y;
+            oz = o.z;
+            tmin = o.w;
+            best_t = d.w;
+            const float bx = box_dir(d.x), by = box_dir(d.y), bz = box_dir(d.z);
+            ix = 1.0f / bx;
+            iy = 1.0f / by;
+            iz = 1.0f / bz;
+            negx = signbit(bx);
+            negy = signbit(by);
+            negz = signbit(bz);
+            nox = -(o.x * ix);
+            noy = -(o.y * iy);
+            noz = -(o.z * iz);
+            oct = (negx ? 1u : 0u) | (negy ? 2u : 0u) | (negz ? 4u : 0u);
+            budget = 2u * (ts.node_count + ts.tri_count) + 64u;
+            nodes = reinterpret_cast<const uint4*>(ts.nodes);
+            sp = 0;
+            tgrp = make_uint2(0u, 0u);
+            // the root as a group of one internal child in slot 0
+            grp = ts.tri_count ? make_uint2(0u, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);
         }
         if (!__any_sync(0xffffffffu, has)) {
             if (drained) break;
@@ -119,13 +86,13 @@ SOLRT_D void extend_bvh8_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
             if (wb == 0u) break;
             if (__popc(wb) < SOLRT_BVH8_NODE_MIN && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
             if (want) {
-                if ((grp.y >> 24) == 0u) grp = stack.get(--sp);
+                if ((grp.y >> 24) == 0u) grp = stack[--sp];
                 const uint32_t j = (uint32_t)(__ffs(grp.y >> 24) - 1);
                 grp.y &= ~(1u << (24u + j));
                 const uint32_t s = j ^ oct;
                 const uint32_t node = grp.x + (uint32_t)__popc(grp.y & ((1u << s) - 1u) & 0xffu);
                 if (grp.y >> 24) {
-                    if (sp < SOLRT_BVH8_STACK) stack.put(sp++, grp);
+                    if (sp < SOLRT_BVH8_STACK) stack[sp++] = grp;
                     else ef |= SOLRT_EFLAG_STACK;
                 }
                 grp = make_uint2(0u, 0u);
@@ -137,7 +104,7 @@ SOLRT_D void extend_bvh8_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
                     uint32_t hi = 0, ht = 0;
                     if constexpr (kF32) {
                         uint32_t cbase = 0, tbase = 0, imask = 0;
-                        bvh8f_node_test(ts.nodes + 14 * (size_t)node, ix, iy, iz, nox, noy, noz, oct, r.tmin, best.t,
+                        bvh8f_node_test(ts.nodes + 14 * (size_t)node, ix, iy, iz, nox, noy, noz, oct, tmin, best_t,
                                         hi, ht, cbase, tbase, imask);
                         if (hi) grp = make_uint2(cbase, (hi << 24) | imask);
                         tgrp = make_uint2(tbase, ht);
@@ -145,8 +112,8 @@ SOLRT_D void extend_bvh8_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
                         const uint4* np = nodes + 5 * (size_t)node;
                         const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3),
                                     w4 = __ldg(np + 4);
-                        bvh8_node_test(w0, w1, w2, w3, w4, r.ox, r.oy, r.oz, ix, iy, iz, negx, negy, negz, oct,
-                                       r.tmin, best.t, hi, ht);
+                        bvh8_node_test(w0, w1, w2, w3, w4, ox, oy, oz, ix, iy, iz, negx, negy, negz, oct,
+                                       tmin, best_t, hi, ht);
                         if (hi) grp = make_uint2(w1.x, (hi << 24) | (w0.w >> 24));
                         tgrp = make_uint2(w1.y, ht);
                     }
@@ -167,8 +134,8 @@ SOLRT_D void extend_bvh8_ww(const IO& io, uint32_t n, unsigned int* work, TraceC
                 } else {
                     const float4* tp = ts.tris + 3 * (size_t)ti;
                     if (kCount) ++cnt.tris;
-                    cnt.fallbacks += intersect_tri(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best);
-                    if (io.any_hit && best.prim != SOLRT_NO_HIT) {  // occlusion query: done at the first hit
+                    if (intersect_tri(rm, tmin, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, cnt.fallbacks) &&
+                        io.any_hit) {  // occlusion query: done at the first hit
                         tgrp.y = 0u;
                         grp = make_uint2(0u, 0u);
                         sp = 0;

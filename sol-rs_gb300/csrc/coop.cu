@@ -30,11 +30,7 @@
 // rays' terms to their paths, as issue_pass does with separate launches.
 #include <algorithm>
 
-#include "bvh2_2l.cuh"
-#include "bvh2_ww.cuh"
-#include "bvh4_ww.cuh"
-#include "bvh8_ww.cuh"
-#include "internal.h"
+#include "extend.cuh"
 #include "path_ops.cuh"
 
 namespace solrt {
@@ -70,6 +66,7 @@ namespace {
 #define SOLRT_COOP_MINB 8
 #endif
 constexpr int kCoopBlock = SOLRT_COOP_BLOCK;
+constexpr uint32_t kCoopSlots = stack_slots(32);  // traversal-stack entries in shared memory
 
 // Barrier state at the start of the batch's cooperative buffer (zeroed
 // before every launch), followed by the per-pass queue counts and work
@@ -98,6 +95,7 @@ struct CoopArgs {
     unsigned int* ctr;    // per pass: count, work, shadow count, shadow work (ctr_stride each, by bounce)
     uint32_t ctr_stride;
     DevStats* stats;
+    int* deep;  // Context::deep_stack
     long long wait_cycles;  // budget of one barrier wait in SM clock cycles
 };
 
@@ -113,6 +111,8 @@ struct CoopIOT {
     const DevJob* jobs;
     float4* hits;
     bool any_hit;
+    static constexpr int lanes = 32;
+    SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
         o = __ldcg(o_tmin + i);
         d = __ldcg(d_tmax + i);
@@ -130,8 +130,9 @@ struct CoopIOT {
         o = __ldcg(o_tmin + i);
         d = __ldcg(d_tmax + i);
     }
-    SOLRT_D void store(uint32_t i, const HitRec& h) const {
+    SOLRT_D bool next(uint32_t i, float, const HitRec& h, float4&, float4&, const TraceCounters&, uint32_t&) const {
         hits[i] = make_float4(h.t, __uint_as_float(h.prim), h.u, h.v);
+        return false;
     }
 };
 template <>
@@ -143,6 +144,8 @@ struct CoopIOT<false> {
     float4* hits;
     bool unused;
     static constexpr bool any_hit = false;
+    static constexpr int lanes = 32;
+    SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
         CoopIOT<true>{o_tmin, d_tmax, meta, jobs, hits, false}.load(i, o, d, ts);
     }
@@ -150,8 +153,9 @@ struct CoopIOT<false> {
         o = __ldcg(o_tmin + i);
         d = __ldcg(d_tmax + i);
     }
-    SOLRT_D void store(uint32_t i, const HitRec& h) const {
+    SOLRT_D bool next(uint32_t i, float, const HitRec& h, float4&, float4&, const TraceCounters&, uint32_t&) const {
         hits[i] = make_float4(h.t, __uint_as_float(h.prim), h.u, h.v);
+        return false;
     }
 };
 
@@ -403,27 +407,25 @@ SOLRT_D uint32_t coop_resolve(const PathQueue& qs, const float4* hits, uint32_t 
     return reached;
 }
 
+// Traversal-stack memory of the calling thread (stack_mem with this kernel's
+// fixed shape).
+SOLRT_D StackMem coop_stack(const int* s_stack, int* deep) {
+    const uint32_t threads = gridDim.x * kCoopBlock;
+    return StackMem{smem_addr(s_stack + threadIdx.x), 4u * kCoopBlock, (int)kCoopSlots,
+                    deep + blockIdx.x * kCoopBlock + threadIdx.x - (size_t)kMinStackSlots * threads, threads,
+                    smem_addr(s_stack + kCoopSlots * kCoopBlock + threadIdx.x)};
+}
+
 // The closest hits of the n rays of queue q (the extend kernel's loop for
 // the kind, 32 shared-memory stack slots for the binary kinds). Returns
 // (FP64 fallbacks, error flags).
 template <int KIND, bool kNee>
-SOLRT_COOP_EXTEND_ATTR uint2 coop_extend(const CoopIOT<kNee>& io, uint32_t n, unsigned int* work) {
-    using CoopIO = CoopIOT<kNee>;
+SOLRT_COOP_EXTEND_ATTR uint2 coop_extend(const CoopIOT<kNee>& io, uint32_t n, unsigned int* work, int* deep) {
+    __shared__ int s_stack[(kCoopSlots + kRayWords) * kCoopBlock];
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
-    if constexpr (KIND == SOLRT_BVH2) {
-        extend_bvh2_ww<CoopIO, false, kCoopBlock, SOLRT_SMEM_STACK, false>(io, n, work, cnt, ef);
-    } else if constexpr (KIND == SOLRT_BVH2_Q16) {
-        extend_bvh2_ww<CoopIO, false, kCoopBlock, SOLRT_SMEM_STACK, true>(io, n, work, cnt, ef);
-    } else if constexpr (KIND == SOLRT_BVH2_TWO_LEVEL) {
-        extend_bvh2_2l_ww<CoopIO, false, kCoopBlock, SOLRT_SMEM_STACK>(io, n, work, cnt, ef);
-    } else if constexpr (KIND == SOLRT_BVH4_Q8) {
-        extend_bvh4_ww<CoopIO, false, kCoopBlock, SOLRT_SMEM_STACK>(io, n, work, cnt, ef);
-    } else if constexpr (KIND == SOLRT_BVH8_F32) {
-        extend_bvh8_ww<CoopIO, false, true, kCoopBlock, 0>(io, n, work, cnt, ef);
-    } else {
-        extend_bvh8_ww<CoopIO, false, false, kCoopBlock, 0>(io, n, work, cnt, ef);
-    }
+    CoopIOT<kNee> q = io;
+    extend_kind<KIND, false>(q, n, work, coop_stack(s_stack, deep), cnt, ef);
     return make_uint2(cnt.fallbacks, ef);
 }
 
@@ -475,7 +477,7 @@ __global__ void __launch_bounds__(kCoopBlock, (coop_min_blocks<KIND>())) k_batch
                 const PathQueue& qin = (b & 1u) ? a.q1 : a.q0;
                 const uint2 r = coop_extend<KIND, kNee>(
                     CoopIOT<kNee>{qin.o_tmin, qin.d_tmax, qin.meta, a.jobs, a.hits, false}, n,
-                    count + a.ctr_stride + b);
+                    count + a.ctr_stride + b, a.deep);
                 coop_flush(c, r.x, r.y);
             }
             if (!coop_barrier(a, c, kStay)) break;
@@ -506,7 +508,7 @@ __global__ void __launch_bounds__(kCoopBlock, (coop_min_blocks<KIND>())) k_batch
                         atomicAdd(&a.stats[1].segments, (unsigned long long)ns);
                     const uint2 r = coop_extend<KIND, kNee>(
                         CoopIOT<kNee>{a.qs.o_tmin, a.qs.d_tmax, a.qs.meta, a.jobs, a.hits, true}, ns,
-                        count + 3u * a.ctr_stride + b);
+                        count + 3u * a.ctr_stride + b, a.deep);
                     if (r.x) atomicAdd(const_cast<uint32_t*>(&c.sfb), r.x);
                     if (r.y) atomicOr(const_cast<uint32_t*>(&c.ef), r.y);
                     if (!coop_barrier(a, c, kStay)) break;
@@ -625,6 +627,7 @@ solrt_status launch_batch_coop(Context& ctx, uint32_t kind, const DevJob* jobs, 
     a.ctr = reinterpret_cast<unsigned int*>(static_cast<char*>(coop) + sizeof(CoopSync));
     a.ctr_stride = ctr_stride;
     a.stats = ctx.stats.as<DevStats>();
+    a.deep = ctx.deep_stack.as<int>();
     a.wait_cycles = wait_budget_cycles(ctx, 4.0);
     if (kind == SOLRT_BVH8_Q8) SOLRT_TRY(launch_kind<SOLRT_BVH8_Q8>(ctx, a, nee));
     else if (kind == SOLRT_BVH4_Q8) SOLRT_TRY(launch_kind<SOLRT_BVH4_Q8>(ctx, a, nee));

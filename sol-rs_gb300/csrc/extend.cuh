@@ -1,0 +1,123 @@
+// extend.cuh — the traversal loop of a BVH kind and the launch shape of the
+// kernels built around it (trace.cu, paths.cu, siblings.cu).
+#pragma once
+
+#include <algorithm>
+#include <atomic>
+
+#include "bvh2_2l.cuh"
+#include "bvh2_ww.cuh"
+#include "bvh4_ww.cuh"
+#include "bvh8_ww.cuh"
+#include "internal.h"
+
+namespace solrt {
+
+// Rays of `io` until the work counter passes n, with the kind's loop.
+template <int KIND, bool kCount, class IO>
+SOLRT_D void extend_kind(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
+                         uint32_t& ef) {
+    if constexpr (KIND == SOLRT_BVH2) extend_bvh2_ww<IO, kCount, false>(io, n, work, mem, cnt, ef);
+    else if constexpr (KIND == SOLRT_BVH2_Q16) extend_bvh2_ww<IO, kCount, true>(io, n, work, mem, cnt, ef);
+    else if constexpr (KIND == SOLRT_BVH2_TWO_LEVEL) extend_bvh2_2l_ww<IO, kCount>(io, n, work, mem, cnt, ef);
+    else if constexpr (KIND == SOLRT_BVH4_Q8) extend_bvh4_ww<IO, kCount>(io, n, work, mem, cnt, ef);
+    else if constexpr (KIND == SOLRT_BVH8_F32) extend_bvh8_ww<IO, kCount, true>(io, n, work, mem, cnt, ef);
+    else extend_bvh8_ww<IO, kCount, false>(io, n, work, mem, cnt, ef);
+}
+
+// Shared-memory stack slots of a launch: the context's choice for the kinds
+// with a node stack, none for the 8-wide kinds (group stack in local memory).
+template <int KIND>
+constexpr bool kind_has_smem_stack() {
+    return KIND != SOLRT_BVH8_Q8 && KIND != SOLRT_BVH8_F32;
+}
+
+extern __shared__ int s_dyn[];
+
+// Traversal memory of the calling thread: its stack column at the start of
+// the block's shared memory, its ray column (RayMem) behind the stacks, and its
+// entries of `deep` (Context::deep_stack).
+SOLRT_D StackMem stack_mem(uint32_t slots, int* deep) {
+    const uint32_t threads = gridDim.x * blockDim.x;
+    return StackMem{smem_addr(s_dyn + threadIdx.x), 4u * blockDim.x, (int)slots,
+                    deep + blockIdx.x * blockDim.x + threadIdx.x - (size_t)kMinStackSlots * threads, threads,
+                    smem_addr(s_dyn + slots * blockDim.x + threadIdx.x)};
+}
+// The thread's column of the block's program state (word w at address
+// column + 4 * w * blockDim.x), behind the stacks and the rays.
+SOLRT_D uint32_t state_column(uint32_t slots) {
+    return smem_addr(s_dyn + (slots + kRayWords) * blockDim.x + threadIdx.x);
+}
+
+// Zeroes the work counter for the next launch on the stream once every block
+// is done with it: `work` is (next ray, finished blocks), both 0 between
+// launches.
+SOLRT_D void release_work(unsigned int* work) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(work + 1, 1u) == gridDim.x - 1u) {
+            work[0] = 0u;
+            work[1] = 0u;
+        }
+    }
+}
+
+SOLRT_D void flush_traversal(DevStats* stats, const TraceCounters& cnt, uint32_t ef, bool count_nodes) {
+    const uint32_t fb = __reduce_add_sync(0xffffffffu, cnt.fallbacks);
+    const uint32_t e = __reduce_or_sync(0xffffffffu, ef);
+    uint32_t nn = 0, nt = 0;
+    if (count_nodes) {
+        nn = __reduce_add_sync(0xffffffffu, cnt.nodes);
+        nt = __reduce_add_sync(0xffffffffu, cnt.tris);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (fb) atomicAdd(&stats->fp64_fallbacks, (unsigned long long)fb);
+        if (e) atomicOr(&stats->eflags, e);
+        if (nn) atomicAdd(&stats->node_visits, (unsigned long long)nn);
+        if (nt) atomicAdd(&stats->tri_tests, (unsigned long long)nt);
+    }
+}
+
+// Blocks of 256 threads that an SM must hold, for the register allocator: 5
+// (48 registers, 1280 threads). 4 / 5 / 6: a 64-spp soup frame through FP32
+// nodes 132.9 / 131.9 / 134.0 ms, 4.2M incoherent rays 2.80 / 2.72 / 2.86 ms, the
+// 8-wide tree on a tunnel frame 68.3 / 67.3 / 69.3 ms, two-level scenes 9.41 /
+// 9.12 / 9.99 ms.
+constexpr int kTraverseMinBlocks = 5;
+
+// Shape of one launch of `kern`: the context's block size and stack slots,
+// state_words words of program state per thread, a grid of (SMs x resident
+// blocks) or fewer blocks when `units` rays or paths need fewer, and how many
+// lanes of each warp take work: 32, or as few as spread the units over all
+// warps of a full grid when there are not enough for every lane (a warp with
+// fewer rays steps faster, and otherwise most SMs would be idle).
+struct LaunchShape {
+    uint32_t grid = 0, block = 0, smem = 0, slots = 0, lanes = 32;
+};
+
+template <int KIND, auto kern>
+solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t units, LaunchShape& s) {
+    s.block = ctx.tune.block;
+    s.slots = kind_has_smem_stack<KIND>() ? stack_slots(ctx.tune.smem) : 0u;
+    s.smem = 4u * s.block * (s.slots + kRayWords + state_words);
+    // resident blocks per SM of this kernel for each of the six shapes: a
+    // property of the compiled kernel, looked up once (0 = not yet)
+    static std::atomic<int> resident[6];
+    std::atomic<int>& r = resident[(s.block == 64 ? 0 : s.block == 128 ? 2 : 4) + (ctx.tune.smem == 16 ? 0 : 1)];
+    int b = r.load(std::memory_order_relaxed);
+    if (b == 0) {
+        const uint32_t most = 4u * 256u * (32u + kRayWords + state_words);
+        SOLRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        SOLRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, (int)s.block, s.smem));
+        b = std::max(b, 1);
+        r.store(b, std::memory_order_relaxed);
+    }
+    const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;
+    const uint32_t warps = full * (s.block / 32u);
+    s.lanes = std::min(32u, std::max(1u, (units + warps - 1u) / warps));
+    s.grid = std::min(full, (units + s.lanes * (s.block / 32u) - 1u) / (s.lanes * (s.block / 32u)));
+    return SOLRT_OK;
+}
+
+}  // namespace solrt

@@ -82,14 +82,7 @@ struct DevStats {
     unsigned int pad;
 };
 
-// Per-pass control block: queue lengths and work counters per bounce.
 #define SOLRT_MAX_BOUNCES 1024
-struct PassCtl {
-    unsigned int count[SOLRT_MAX_BOUNCES + 2];
-    unsigned int work[SOLRT_MAX_BOUNCES + 2];
-    unsigned int scount[SOLRT_MAX_BOUNCES + 2];  // shadow queue per bounce
-    unsigned int swork[SOLRT_MAX_BOUNCES + 2];
-};
 
 // Structure-of-arrays path queue (one wavefront).
 struct PathQueue {
@@ -124,10 +117,17 @@ struct DevJob {
 // A work item of one pass: samples [s0, s0 + k) of pixels [pix0, pix0 + npix)
 // of one job. Its paths occupy slots [path_base, path_base + npix * k) of the
 // pass (pixel-major), its pixels [pix_base, pix_base + npix) of the pass's
-// pixel space.
+// pixel space, and its units of work (item_units) [unit_base, ...) of the
+// path kernel's.
 struct DevItem {
-    uint32_t job, pix0, npix, s0, k, path_base, pix_base, pad;
+    uint32_t job, pix0, npix, s0, k, path_base, pix_base, unit_base;
 };
+
+// Units of work of an item in the path kernel: its paths, or its pixels when
+// the samples of a pixel share one random stream and are traced in sequence.
+SOLRT_HD uint32_t item_units(const DevItem& it, uint32_t rng_mode) {
+    return rng_mode == SOLRT_RNG_REF_STREAM ? it.npix : it.npix * it.k;
+}
 
 // The depth field of a path's meta word also carries its job.
 constexpr uint32_t kDepthBits = 11;
@@ -136,8 +136,9 @@ constexpr uint32_t kDepthMask = (1u << kDepthBits) - 1u;
 struct PassPlan {
     uint32_t item_begin, item_count;
     uint32_t paths, pixels;
-    uint32_t bounces;  // extend/shade launches of the pass
+    uint32_t bounces;  // bounce levels of the pass (cooperative batches)
     uint32_t nee = 0;  // a job of the pass uses SOLRT_INTEGRATOR_PATH_NEE
+    uint32_t units = 0;  // units of work of the path kernel (item_units summed)
 };
 
 struct Context;
@@ -174,9 +175,20 @@ struct Batch {
 // solrt_context_set_tune or solrt_batch_autotune.
 struct TuneConfig {
     uint32_t block = 128;      // threads per extend block: 64, 128 or 256
-    uint32_t smem = 32;        // BVH2 traversal-stack slots in shared memory: 16 or 32
+    uint32_t smem = 32;        // shared-memory traversal stack: 16 or 32 (stack_slots entries)
     uint32_t pass_paths = 0;   // paths per batch pass (0 = the path capacity)
 };
+
+// Threads of the largest resident grid per SM, and the stack entries of each
+// kept in Context::deep_stack: those from the smallest number of shared slots
+// up.
+constexpr uint32_t kMaxThreadsPerSm = 2048;
+constexpr uint32_t kMinStackSlots = 12;
+
+// Traversal-stack entries per thread that a tuned shared-memory size keeps on
+// the SM. More than 16 buys nothing (rays of a 1M-triangle tree hold at most
+// about 20 entries, 99.98 % of them at most 16) and takes L1 cache away.
+constexpr uint32_t stack_slots(uint32_t smem) { return smem >= 32 ? 16u : kMinStackSlots; }
 
 struct Context {
     // The handle and every scene, image and batch created on the context hold
@@ -195,7 +207,13 @@ struct Context {
     // SOLRT_INTEGRATOR_PATH_NEE (allocated when a render first needs it)
     DeviceBuffer q_o[3], q_d[3], q_thr[3], q_meta[3];
     DeviceBuffer q_prev[2];  // per path of queues 0 and 1, next-event estimation only
-    DeviceBuffer hits, rad, ctl, stats, trace_work;
+    DeviceBuffer hits, rad, stats;
+    DeviceBuffer queue_counts;  // paths, then shadow rays, per bounce level of a pass; zero between passes
+    // next unit and finished blocks of the persistent kernels; both 0 between
+    // launches (release_work)
+    DeviceBuffer trace_work;
+    // traversal-stack entries beyond the shared-memory slots (StackMem::deep)
+    DeviceBuffer deep_stack;
     DeviceBuffer blue_noise;  // RGBA8 texels of SOLRT_INTEGRATOR_AO
     DeviceBuffer sibling_job;  // one-job table of DEBUG / AO launches
     uint32_t noise_w = 0, noise_h = 0;
@@ -330,12 +348,13 @@ solrt_status regenerate_scene(Context& ctx, Scene& sc, uint32_t mode);
 
 // trace.cu
 solrt_status launch_trace_rays(Context& ctx, const Scene& sc, const solrt_ray* rays, uint32_t n, solrt_hit* hits);
-// Extend for a batched queue: the scene of ray i is jobs[meta[i].y >> kDepthBits].sc.
-// Closest hits of the `*count` rays of queue `q` (any_hit: some hit in
-// (tmin, tmax), for occlusion queries); `st` (default: the context's first
-// stats block) receives their segment and visit counts.
-solrt_status launch_extend(Context& ctx, uint32_t kind, const DevJob* jobs, const PathQueue& q, float4* hits,
-                           const unsigned int* count, unsigned int* work, DevStats* st = nullptr,
+// Closest hits of the `*count` (at most `most`) rays of queue `q` (any_hit: some
+// hit in (tmin, tmax), for occlusion queries). The rays' scene is `scene`, or
+// with a null `scene` that of ray i's job, jobs[meta[i].y >> kDepthBits].sc.
+// `st` (default: the context's first stats block) receives their segment and
+// visit counts.
+solrt_status launch_extend(Context& ctx, uint32_t kind, const DevScene* scene, const DevJob* jobs, const PathQueue& q,
+                           float4* hits, const unsigned int* count, uint32_t most, DevStats* st = nullptr,
                            bool any_hit = false);
 // Whether an extend kernel exists for this block size / shared stack slots.
 bool extend_variant_ok(uint32_t block, uint32_t smem);

@@ -301,8 +301,8 @@ SOLRT_D void add_sample_kahan(f3& ks, f3& kc, float& kn, float4 c) {
 }
 
 // ---------------------------------------------------------------------------
-// Stage bodies shared by the one-stage-per-launch kernels (pathtrace.cu) and
-// the cooperative one-launch batch (coop.cu). `Ld` loads what an earlier
+// Stage bodies shared by the kernels of pathtrace.cu and the cooperative
+// one-launch batch (coop.cu). `Ld` loads what an earlier
 // stage wrote: plain loads when stages are separate launches, loads through
 // L2 (ld.global.cg) when they are phases of one launch, where this SM's L1
 // may still hold lines from before another SM's writes.
@@ -334,12 +334,10 @@ SOLRT_D void begin_pixel(const DevJob* jobs, const uint32_t* job_pix, uint32_t n
     if (J.accum_mode != SOLRT_ACCUM_KAHAN) J.fsum[t - job_pix[j]] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-// Camera ray of path slot i of a pass (rgen:47-61) into queue q.
+// Camera ray of path slot i of a pass (rgen:47-61), a path of work item `it`
+// of job J, into queue q.
 template <class Ld>
-SOLRT_D void generate_path(const DevJob* jobs, const DevItem* items, uint32_t nitems, uint32_t i, const PathQueue& q,
-                           float4* rad) {
-    const DevItem it = items[find_last_le(nitems, i, [&](uint32_t t) { return items[t].path_base; })];
-    const DevJob& J = jobs[it.job];
+SOLRT_D void generate_slot(const DevJob& J, const DevItem& it, uint32_t i, const PathQueue& q, float4* rad) {
     const uint32_t local = i - it.path_base;
     const uint32_t lp = local / it.k, j = local - lp * it.k;
     const uint32_t pix = it.pix0 + lp, s = it.s0 + j;
@@ -353,28 +351,27 @@ SOLRT_D void generate_path(const DevJob* jobs, const DevItem* items, uint32_t ni
     if (J.integrator == SOLRT_INTEGRATOR_PATH_NEE) rad[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // sums shadow terms
 }
 
-// Adds the pass's samples of pass pixel t to its pixel's sums, in sample
-// order (rgen:86).
+// generate_slot for a path of the tables `jobs` and `items`.
 template <class Ld>
-SOLRT_D void accumulate_pixel(const DevJob* jobs, const DevItem* items, uint32_t nitems, uint32_t t,
-                              const float4* rad) {
-    const DevItem it = items[find_last_le(nitems, t, [&](uint32_t i) { return items[i].pix_base; })];
-    const DevJob& J = jobs[it.job];
-    const uint32_t lp = t - it.pix_base;
-    const uint32_t pix = it.pix0 + lp;
-    const float4* r = rad + it.path_base + (size_t)lp * it.k;
+SOLRT_D void generate_path(const DevJob* jobs, const DevItem* items, uint32_t nitems, uint32_t i, const PathQueue& q,
+                           float4* rad) {
+    const DevItem it = items[find_last_le(nitems, i, [&](uint32_t t) { return items[t].path_base; })];
+    generate_slot<Ld>(jobs[it.job], it, i, q, rad);
+}
+
+// Sums of a pixel over its samples (rgen:86): plain, or compensated.
+struct PixelSum {
+    f3 s{0.0f, 0.0f, 0.0f}, c{0.0f, 0.0f, 0.0f};
+    float n = 0.0f;  // Kahan: finite samples
+};
+
+// Adds the samples r[0, it.k) of pixel pix, in sample order.
+template <class Ld>
+SOLRT_D void sum_samples(const DevJob& J, const DevItem& it, uint32_t pix, const float4* r, PixelSum& p) {
     if (J.accum_mode == SOLRT_ACCUM_KAHAN) {
-        const float4 s4 = Ld::ld(J.ksum + pix), c4 = Ld::ld(J.kcomp + pix);
-        f3 ks{s4.x, s4.y, s4.z}, kc{c4.x, c4.y, c4.z};
-        float kn = s4.w;
-        for (uint32_t j = 0; j < it.k; ++j) add_sample_kahan(ks, kc, kn, Ld::ld(r + j));
-        J.ksum[pix] = make_float4(ks.x, ks.y, ks.z, kn);
-        J.kcomp[pix] = make_float4(kc.x, kc.y, kc.z, 0.0f);
+        for (uint32_t j = 0; j < it.k; ++j) add_sample_kahan(p.s, p.c, p.n, Ld::ld(r + j));
     } else {
-        const float4 s4 = Ld::ld(J.fsum + pix);
-        f3 s{s4.x, s4.y, s4.z};
-        for (uint32_t j = 0; j < it.k; ++j) add_sample(s, Ld::ld(r + j));
-        J.fsum[pix] = make_float4(s.x, s.y, s.z, 0.0f);
+        for (uint32_t j = 0; j < it.k; ++j) add_sample(p.s, Ld::ld(r + j));
     }
     if (J.sq) {  // squared sample sums of the stopping rule (samples the sums above keep)
         float q = Ld::ld(J.sq + pix);
@@ -387,28 +384,60 @@ SOLRT_D void accumulate_pixel(const DevJob* jobs, const DevItem* items, uint32_t
     }
 }
 
+// The sums kept between passes: Kahan sums from launch to launch, plain
+// sums within one launch.
+template <class Ld>
+SOLRT_D PixelSum load_sum(const DevJob& J, uint32_t pix) {
+    PixelSum p;
+    if (J.accum_mode == SOLRT_ACCUM_KAHAN) {
+        const float4 s4 = Ld::ld(J.ksum + pix), c4 = Ld::ld(J.kcomp + pix);
+        p.s = f3{s4.x, s4.y, s4.z};
+        p.c = f3{c4.x, c4.y, c4.z};
+        p.n = s4.w;
+    } else {
+        const float4 s4 = Ld::ld(J.fsum + pix);
+        p.s = f3{s4.x, s4.y, s4.z};
+    }
+    return p;
+}
+SOLRT_D void store_sum(const DevJob& J, uint32_t pix, const PixelSum& p) {
+    if (J.accum_mode == SOLRT_ACCUM_KAHAN) {
+        J.ksum[pix] = make_float4(p.s.x, p.s.y, p.s.z, p.n);
+        J.kcomp[pix] = make_float4(p.c.x, p.c.y, p.c.z, 0.0f);
+    } else {
+        J.fsum[pix] = make_float4(p.s.x, p.s.y, p.s.z, 0.0f);
+    }
+}
+
+// Adds the pass's samples of pass pixel t to its pixel's sums, in sample
+// order (rgen:86).
+template <class Ld>
+SOLRT_D void accumulate_pixel(const DevJob* jobs, const DevItem* items, uint32_t nitems, uint32_t t,
+                              const float4* rad) {
+    const DevItem it = items[find_last_le(nitems, t, [&](uint32_t i) { return items[i].pix_base; })];
+    const DevJob& J = jobs[it.job];
+    const uint32_t lp = t - it.pix_base, pix = it.pix0 + lp;
+    PixelSum p = load_sum<Ld>(J, pix);
+    sum_samples<Ld>(J, it, pix, rad + it.path_base + (size_t)lp * it.k, p);
+    store_sum(J, pix, p);
+}
+
 SOLRT_D unsigned char to_unorm8(float c) {
     const float cl = glsl_min(glsl_max(c, 0.0f), 1.0f);
     return (unsigned char)(cl * 255.0f + 0.5f);
 }
 
-// rgen:88-103 (REF_MIX) or the Kahan mean, for pixel t of the batch's pixel
-// space.
-template <class Ld>
-SOLRT_D void finalize_pixel(const DevJob* jobs, const uint32_t* job_pix, uint32_t njobs, uint32_t t) {
-    const uint32_t j = find_last_le(njobs, t, [&](uint32_t i) { return job_pix[i]; });
-    const DevJob& J = jobs[j];
-    const uint32_t pix = t - job_pix[j];
+// rgen:88-103 (REF_MIX) or the Kahan mean: the images of pixel pix from its
+// sums.
+SOLRT_D void write_pixel(const DevJob& J, uint32_t pix, const PixelSum& p) {
     const float4 a = J.accum[pix];
     const f3 old{a.x, a.y, a.z};
     f3 out;
     if (J.accum_mode == SOLRT_ACCUM_KAHAN) {
-        const float4 s = Ld::ld(J.ksum + pix);
-        out = s.w > 0.0f ? f3{s.x / s.w, s.y / s.w, s.z / s.w} : old;
+        out = p.n > 0.0f ? f3{p.s.x / p.n, p.s.y / p.n, p.s.z / p.n} : old;
     } else {
-        const float4 s = Ld::ld(J.fsum + pix);
         const float inv = 1.0f / __uint2float_rn(J.spp);
-        const f3 mean = inv * f3{s.x, s.y, s.z};
+        const f3 mean = inv * p.s;
         const float alpha = 1.0f / __uint2float_rn(J.frame + 1u - J.start);
         out = mix(old, mean, alpha);
         if (isnan(out.x) || isnan(out.y) || isnan(out.z)) out = old;
@@ -417,6 +446,29 @@ SOLRT_D void finalize_pixel(const DevJob* jobs, const uint32_t* job_pix, uint32_
     J.accum[pix] = make_float4(out.x, out.y, out.z, 1.0f);
     const float g = 1.0f / 2.2f;
     J.rgba8[pix] = make_uchar4(to_unorm8(powf(out.x, g)), to_unorm8(powf(out.y, g)), to_unorm8(powf(out.z, g)), 255);
+}
+
+// write_pixel for pixel t of the batch's pixel space.
+template <class Ld>
+SOLRT_D void finalize_pixel(const DevJob* jobs, const uint32_t* job_pix, uint32_t njobs, uint32_t t) {
+    const uint32_t j = find_last_le(njobs, t, [&](uint32_t i) { return job_pix[i]; });
+    const DevJob& J = jobs[j];
+    const uint32_t pix = t - job_pix[j];
+    write_pixel(J, pix, load_sum<Ld>(J, pix));
+}
+
+// One pass's share of pixel lp of work item `it`: its samples added to the
+// sums of the passes before (none for plain sums at sample 0), then the
+// images once every sample is in, else the sums kept for the next pass.
+SOLRT_D void resolve_pixel(const DevJob& J, const DevItem& it, uint32_t lp, const float4* rad) {
+    const uint32_t pix = it.pix0 + lp;
+    const bool kahan = J.accum_mode == SOLRT_ACCUM_KAHAN;
+    PixelSum p;
+    if (kahan || it.s0 > 0u) p = load_sum<LdPlain>(J, pix);
+    sum_samples<LdPlain>(J, it, pix, rad + it.path_base + (size_t)lp * it.k, p);
+    const bool last = it.s0 + it.k >= J.spp;
+    if (kahan || !last) store_sum(J, pix, p);
+    if (last) write_pixel(J, pix, p);
 }
 
 }  // namespace solrt

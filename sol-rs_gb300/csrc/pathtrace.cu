@@ -23,27 +23,48 @@
 // bit.
 #include <algorithm>
 
-#include "bvh2_2l.cuh"
-#include "bvh2_ww.cuh"
-#include "bvh4_ww.cuh"
-#include "bvh8_traverse.cuh"
-#include "internal.h"
+#include "extend.cuh"
 #include "path_ops.cuh"
 
 namespace solrt {
 
 namespace {
 
-__global__ void k_generate(const DevJob* __restrict__ jobs, const DevItem* __restrict__ items, uint32_t nitems,
-                           uint32_t P, PathQueue q, unsigned int* __restrict__ count0, DevStats* stats,
-                           float4* __restrict__ rad) {
+// One pass of the wavefront: of one job and one work item (held in the
+// kernels' parameters), or of the tables `jobs` and `items`.
+struct PassArgs {
+    DevJob job;
+    DevItem item;
+    const DevJob* jobs;
+    const DevItem* items;
+    uint32_t nitems, paths, pixels, bounces, capacity;
+    unsigned int* count;   // paths of each bounce level's queue; zero between passes
+    unsigned int* scount;  // shadow rays of each bounce level
+    float4* hits;
+    float4* rad;
+    DevStats* stats;
+};
+
+template <bool kSingle>
+SOLRT_D const DevJob& pass_job(const PassArgs& a, uint32_t j) {
+    return kSingle ? a.job : a.jobs[j];
+}
+template <bool kSingle>
+SOLRT_D const DevItem& pass_item(const PassArgs& a, uint32_t slot) {
+    if (kSingle) return a.item;
+    return a.items[find_last_le(a.nitems, slot, [&](uint32_t t) { return a.items[t].path_base; })];
+}
+
+template <bool kSingle>
+__global__ void __launch_bounds__(256) k_generate(const __grid_constant__ PassArgs a, PathQueue q) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
-        *count0 = P;
-        atomicAdd(&stats->paths, (unsigned long long)P);
+        a.count[0] = a.paths;
+        atomicAdd(&a.stats->paths, (unsigned long long)a.paths);
     }
-    if (i >= P) return;
-    generate_path<LdPlain>(jobs, items, nitems, i, q, rad);
+    if (i >= a.paths) return;
+    const DevItem& it = pass_item<kSingle>(a, i);
+    generate_slot<LdPlain>(pass_job<kSingle>(a, it.job), it, i, q, a.rad);
 }
 
 // kNee: the variant for passes with SOLRT_INTEGRATOR_PATH_NEE jobs (shadow
@@ -67,29 +88,21 @@ __global__ void k_generate(const DevJob* __restrict__ jobs, const DevItem* __res
 #ifndef SOLRT_SHADE_BLOCK_COMPACT
 #define SOLRT_SHADE_BLOCK_COMPACT 1
 #endif
-// 1: with block compaction, a block's continuing paths are written grouped
-// by the octant of their new direction (octant-major, then warp and lane),
-// so that the extend kernel's warps, which take consecutive queue slots, get
-// rays of one or two octants; same images (queue order changes no result).
-// Measured: extend -0.4 / -0.5 %, shade +3 / +5 % (soup / tunnel frame), no
-// gain: the pixel-ordered queue is about as coherent.
-#ifndef SOLRT_SHADE_OCTANT_SORT
-#define SOLRT_SHADE_OCTANT_SORT 0
-#endif
-template <bool kNee>
+template <bool kSingle, bool kNee>
 __global__ void __launch_bounds__(256, SOLRT_SHADE_MINB)
-    k_shade(const DevJob* __restrict__ jobs, const DevItem* __restrict__ items, uint32_t nitems, PathQueue qin,
-            const float4* __restrict__ hits, const unsigned int* __restrict__ count_in, PathQueue qout,
-            unsigned int* __restrict__ count_out, uint32_t capacity, float4* __restrict__ rad, DevStats* stats,
-            PathQueue qs, unsigned int* __restrict__ count_s) {
-    const unsigned int n = *count_in;
+    k_shade(const __grid_constant__ PassArgs a, uint32_t bounce, PathQueue qin, PathQueue qout, PathQueue qs) {
+    const unsigned int n = a.count[bounce];
+    unsigned int* const count_out = a.count + bounce + 1;
+    unsigned int* const count_s = a.scount + bounce;
+    const float4* __restrict__ hits = a.hits;
+    float4* __restrict__ rad = a.rad;
+    const uint32_t capacity = a.capacity;
     const int lane = threadIdx.x & 31;
     const uint32_t lane_lt = (1u << lane) - 1u;
     constexpr bool kBlock = SOLRT_SHADE_BLOCK_COMPACT && !kNee;
     // kBlock: a block-uniform loop, slots [base, base + 256) per block and
     // step; else a warp-uniform one, 32 slots per warp and step
     __shared__ uint32_t s_cnt[8], s_pre[8], s_base;
-    __shared__ uint32_t s_cnt8[SOLRT_SHADE_OCTANT_SORT ? 64 : 1], s_pre8[SOLRT_SHADE_OCTANT_SORT ? 64 : 1];
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t start = kBlock ? blockIdx.x * blockDim.x : ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u;
     const uint32_t stride = kBlock ? gridDim.x * blockDim.x : ((gridDim.x * blockDim.x) >> 5) * 32u;
@@ -107,7 +120,7 @@ __global__ void __launch_bounds__(256, SOLRT_SHADE_MINB)
             const float4 o = qin.o_tmin[i], d = qin.d_tmax[i], tr = qin.thr_rng[i];
             m = qin.meta[i];
             const uint32_t job = m.y >> kDepthBits;
-            const DevJob& J = jobs[job];
+            const DevJob& J = pass_job<kSingle>(a, job);
             const bool nee = kNee && J.integrator == SOLRT_INTEGRATOR_PATH_NEE && qs.o_tmin != nullptr;
             uint32_t rng = __float_as_uint(tr.w);
             uint32_t depth = m.y & kDepthMask;
@@ -132,39 +145,14 @@ __global__ void __launch_bounds__(256, SOLRT_SHADE_MINB)
                     rad[m.x] = make_float4(acc.x, acc.y, acc.z, 0.0f);
                 }
                 if (J.rng_mode == SOLRT_RNG_REF_STREAM) {
-                    const DevItem it = items[find_last_le(nitems, m.x, [&](uint32_t t) { return items[t].path_base; })];
+                    const DevItem& it = pass_item<kSingle>(a, m.x);
                     J.rng_state[it.pix0 + (m.x - it.path_base) / it.k] = rng;
                 }
             }
         }
         const uint32_t mask = __ballot_sync(0xffffffffu, alive);
         const uint32_t smask = kNee ? __ballot_sync(0xffffffffu, shadow) : 0u;
-        uint32_t same = 0, oct = 0;  // octant sort: the lanes of this warp with this lane's octant
-        if constexpr (kBlock && SOLRT_SHADE_OCTANT_SORT) {
-            oct = (out_d.x < 0.0f ? 1u : 0u) | (out_d.y < 0.0f ? 2u : 0u) | (out_d.z < 0.0f ? 4u : 0u);
-#pragma unroll
-            for (uint32_t o = 0; o < 8u; ++o) {
-                const uint32_t bo = __ballot_sync(0xffffffffu, alive && oct == o);
-                if (lane == 0) s_cnt8[o * 8u + warp] = (uint32_t)__popc(bo);
-                if (oct == o) same = bo;
-            }
-            __syncthreads();
-            if (threadIdx.x < 32) {  // exclusive scan of the 64 counts (octant-major), two per lane
-                const uint32_t a0 = s_cnt8[2 * lane], a1 = s_cnt8[2 * lane + 1];
-                uint32_t x = a0 + a1;
-#pragma unroll
-                for (int dd = 1; dd < 32; dd <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, dd);
-                    if (lane >= dd) x += y;
-                }
-                const uint32_t excl = x - (a0 + a1);
-                s_pre8[2 * lane] = excl;
-                s_pre8[2 * lane + 1] = excl + a0;
-                const uint32_t total = __shfl_sync(0xffffffffu, x, 31);
-                if (lane == 0) s_base = total ? atomicAdd(count_out, total) : 0u;
-            }
-            __syncthreads();
-        } else if constexpr (kBlock) {
+        if constexpr (kBlock) {
             if (lane == 0) s_cnt[warp] = (uint32_t)__popc(mask);
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -187,9 +175,7 @@ __global__ void __launch_bounds__(256, SOLRT_SHADE_MINB)
                 pos0 = __shfl_sync(0xffffffffu, pos0, leader);
             }
             if (alive) {
-                const uint32_t pos = (kBlock && SOLRT_SHADE_OCTANT_SORT)
-                                         ? s_base + s_pre8[oct * 8u + warp] + (uint32_t)__popc(same & lane_lt)
-                                         : pos0 + __popc(mask & lane_lt);
+                const uint32_t pos = pos0 + __popc(mask & lane_lt);
                 if (pos < capacity) {
                     qout.o_tmin[pos] = out_o;
                     qout.d_tmax[pos] = out_d;
@@ -219,7 +205,7 @@ __global__ void __launch_bounds__(256, SOLRT_SHADE_MINB)
             }
         }
     }
-    if (ef) atomicOr(&stats->eflags, ef);
+    if (ef) atomicOr(&a.stats->eflags, ef);
 }
 
 // Adds the contribution of every shadow ray that reached its light to its
@@ -242,12 +228,30 @@ __global__ void __launch_bounds__(256) k_shadow_resolve(PathQueue qs, const floa
     if ((threadIdx.x & 31) == 0 && w) atomicAdd(&sstats->unoccluded, (unsigned long long)w);
 }
 
-// Per-pixel sums of one pass, samples in order (rgen:86).
-__global__ void k_accumulate(const DevJob* __restrict__ jobs, const DevItem* __restrict__ items, uint32_t nitems,
-                             uint32_t pixels, const float4* __restrict__ rad) {
+// The pixels of one pass: sums in sample order, images when a job's samples
+// are complete (rgen:86-103). Zeroes the queue counts for the next pass.
+template <bool kSingle>
+__global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ PassArgs a) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= pixels) return;
-    accumulate_pixel<LdPlain>(jobs, items, nitems, t, rad);
+    if (blockIdx.x == 0)
+        for (uint32_t b = threadIdx.x; b <= a.bounces; b += blockDim.x) a.count[b] = a.scount[b] = 0u;
+    if (t >= a.pixels) return;
+    if (kSingle) {
+        resolve_pixel(a.job, a.item, t, a.rad);
+    } else {
+        const DevItem it = a.items[find_last_le(a.nitems, t, [&](uint32_t i) { return a.items[i].pix_base; })];
+        resolve_pixel(a.jobs[it.job], it, t - it.pix_base, a.rad);
+    }
+}
+
+// Per-pixel sums of one pass of a served tick, samples in order (rgen:86).
+// Zeroes the queue counts for the next pass.
+__global__ void __launch_bounds__(256) k_accumulate(const __grid_constant__ PassArgs a) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0)
+        for (uint32_t b = threadIdx.x; b <= a.bounces; b += blockDim.x) a.count[b] = a.scount[b] = 0u;
+    if (t >= a.pixels) return;
+    accumulate_pixel<LdPlain>(a.jobs, a.items, a.nitems, t, a.rad);
 }
 
 // Per job, the sum over its pixels of the variance of the pixel mean summed
@@ -448,6 +452,7 @@ __global__ void __launch_bounds__(128, SOLRT_MEGA_MINB)
         __syncwarp();
     }
     flush_stats(stats, segs, paths, cnt.fallbacks, ef);
+    release_work(work);
 }
 
 // ---------------------------------------------------------------------------
@@ -594,14 +599,7 @@ __global__ void __launch_bounds__(128, SOLRT_MEGA_MINB)
         __syncwarp();
     }
     flush_mega_counts(stats, mc);
-}
-
-// Zeroes the per-frame sample sums of running-mix jobs.
-__global__ void k_begin(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ job_pix, uint32_t njobs,
-                        uint32_t pixels) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= pixels) return;
-    begin_pixel(jobs, job_pix, njobs, t);
+    release_work(work);
 }
 
 // ---------------------------------------------------------------------------
@@ -845,58 +843,89 @@ DevJob make_job(const Scene& sc, const Image& img, const solrt_camera& cam, cons
     return J;
 }
 
-// One pass: generate, (extend, shade) x bounces, accumulate.
-solrt_status issue_pass(Context& ctx, uint32_t kind, const DevJob* dj, const DevItem* items, const PassPlan& pp,
+// One pass on the context stream: generate, (extend, shade) x bounces, then
+// its pixels (`resolve`: sums and finished images; else, for served jobs, the
+// sums alone). `single`: of a.job and a.item, else of the tables.
+solrt_status issue_pass(Context& ctx, uint32_t kind, PassArgs a, bool single, bool nee, bool resolve,
                         bool record_timing) {
     cudaStream_t st = ctx.stream;
-    DevStats* stats = ctx.stats.as<DevStats>();
-    PassCtl* ctl = ctx.ctl.as<PassCtl>();
-    const size_t ctl_bytes = sizeof(unsigned int) * (pp.bounces + 1);
-    SOLRT_CUDA(cudaMemsetAsync(ctl->count, 0, ctl_bytes, st));
-    SOLRT_CUDA(cudaMemsetAsync(ctl->work, 0, ctl_bytes, st));
-    if (pp.nee) {
-        if (!ctx.q_o[2].ptr) { set_error("shadow queue not allocated"); return SOLRT_ERR_INVALID; }
-        SOLRT_CUDA(cudaMemsetAsync(ctl->scount, 0, ctl_bytes, st));
-        SOLRT_CUDA(cudaMemsetAsync(ctl->swork, 0, ctl_bytes, st));
-    }
+    if (nee && !ctx.q_o[2].ptr) { set_error("shadow queue not allocated"); return SOLRT_ERR_INVALID; }
+    a.capacity = ctx.capacity;
+    a.count = ctx.queue_counts.as<unsigned int>();
+    a.scount = a.count + SOLRT_MAX_BOUNCES + 2;
+    a.hits = ctx.hits.as<float4>();
+    a.rad = ctx.rad.as<float4>();
+    a.stats = ctx.stats.as<DevStats>();
     const int tg = record_timing ? ctx.timing_begin(2) : -1;
-    k_generate<<<cdiv(pp.paths, 256), 256, 0, st>>>(dj, items, pp.item_count, pp.paths, ctx.queue(0), ctl->count,
-                                                    stats, ctx.rad.as<float4>());
+    if (single) k_generate<true><<<cdiv(a.paths, 256), 256, 0, st>>>(a, ctx.queue(0));
+    else k_generate<false><<<cdiv(a.paths, 256), 256, 0, st>>>(a, ctx.queue(0));
     ctx.timing_end(tg);
     ++ctx.launches;
-    const int shade_grid = ctx.sm_count * 8;
-    for (uint32_t bnc = 0; bnc < pp.bounces; ++bnc) {
+    const uint32_t shade_grid = std::min<uint32_t>(ctx.sm_count * 8, cdiv(a.paths, 256));
+    const DevScene* scene = single ? &a.job.sc : nullptr;
+    for (uint32_t bnc = 0; bnc < a.bounces; ++bnc) {
         const PathQueue qin = ctx.queue(bnc & 1), qout = ctx.queue((bnc + 1) & 1);
         const int te = record_timing ? ctx.timing_begin(0) : -1;
-        SOLRT_TRY(launch_extend(ctx, kind, dj, qin, ctx.hits.as<float4>(), ctl->count + bnc, ctl->work + bnc));
+        SOLRT_TRY(launch_extend(ctx, kind, scene, a.jobs, qin, a.hits, a.count + bnc, a.paths));
         ctx.timing_end(te);
         const int ts = record_timing ? ctx.timing_begin(1) : -1;
-        if (pp.nee)
-            k_shade<true><<<shade_grid, 256, 0, st>>>(dj, items, pp.item_count, qin, ctx.hits.as<float4>(),
-                                                      ctl->count + bnc, qout, ctl->count + bnc + 1, ctx.capacity,
-                                                      ctx.rad.as<float4>(), stats, ctx.queue(2), ctl->scount + bnc);
-        else
-            k_shade<false><<<shade_grid, 256, 0, st>>>(dj, items, pp.item_count, qin, ctx.hits.as<float4>(),
-                                                       ctl->count + bnc, qout, ctl->count + bnc + 1, ctx.capacity,
-                                                       ctx.rad.as<float4>(), stats, PathQueue{}, ctl->scount + bnc);
+        const PathQueue qs = nee ? ctx.queue(2) : PathQueue{};
+        if (single && nee) k_shade<true, true><<<shade_grid, 256, 0, st>>>(a, bnc, qin, qout, qs);
+        else if (single) k_shade<true, false><<<shade_grid, 256, 0, st>>>(a, bnc, qin, qout, qs);
+        else if (nee) k_shade<false, true><<<shade_grid, 256, 0, st>>>(a, bnc, qin, qout, qs);
+        else k_shade<false, false><<<shade_grid, 256, 0, st>>>(a, bnc, qin, qout, qs);
         ctx.timing_end(ts);
         ++ctx.launches;
-        if (pp.nee && bnc + 1 < pp.bounces) {  // shadow rays of this bounce (none at the last: depth > max)
+        if (nee && bnc + 1 < a.bounces) {  // shadow rays of this bounce (none at the last: depth > max)
             const int tx = record_timing ? ctx.timing_begin(0) : -1;
-            SOLRT_TRY(launch_extend(ctx, kind, dj, ctx.queue(2), ctx.hits.as<float4>(), ctl->scount + bnc,
-                                    ctl->swork + bnc, stats + 1, true));
+            SOLRT_TRY(launch_extend(ctx, kind, scene, a.jobs, qs, a.hits, a.scount + bnc, a.paths, a.stats + 1, true));
             ctx.timing_end(tx);
             const int tr = record_timing ? ctx.timing_begin(1) : -1;
-            k_shadow_resolve<<<shade_grid, 256, 0, st>>>(ctx.queue(2), ctx.hits.as<float4>(), ctl->scount + bnc,
-                                                         ctx.rad.as<float4>(), stats + 1);
+            k_shadow_resolve<<<shade_grid, 256, 0, st>>>(qs, a.hits, a.scount + bnc, a.rad, a.stats + 1);
             ctx.timing_end(tr);
             ++ctx.launches;
         }
     }
     const int ta = record_timing ? ctx.timing_begin(3) : -1;
-    k_accumulate<<<cdiv(pp.pixels, 256), 256, 0, st>>>(dj, items, pp.item_count, pp.pixels, ctx.rad.as<float4>());
+    if (!resolve) k_accumulate<<<cdiv(a.pixels, 256), 256, 0, st>>>(a);
+    else if (single) k_resolve<true><<<cdiv(a.pixels, 256), 256, 0, st>>>(a);
+    else k_resolve<false><<<cdiv(a.pixels, 256), 256, 0, st>>>(a);
     ctx.timing_end(ta);
     ++ctx.launches;
+    SOLRT_CUDA(cudaGetLastError());
+    return SOLRT_OK;
+}
+
+PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp) {
+    PassArgs a{};
+    a.jobs = jobs;
+    a.items = items;
+    a.nitems = pp.item_count;
+    a.paths = pp.paths;
+    a.pixels = pp.pixels;
+    a.bounces = pp.bounces;
+    return a;
+}
+
+// One frame of one job: its samples in passes of at most the path capacity,
+// everything the kernels need in their parameters.
+solrt_status issue_frame(Context& ctx, uint32_t kind, const DevJob& J) {
+    const uint32_t np = J.width * J.height;
+    const uint32_t cap = ctx.tune.pass_paths ? std::min(ctx.tune.pass_paths, ctx.capacity) : ctx.capacity;
+    PassArgs a{};
+    a.job = J;
+    a.nitems = 1;
+    a.bounces = J.max_bounces + 1u;
+    for (uint32_t p0 = 0; p0 < np; p0 += std::min(cap, np - p0)) {
+        const uint32_t npix = std::min(cap, np - p0);
+        const uint32_t kmax = J.rng_mode == SOLRT_RNG_REF_STREAM ? 1u : std::max(1u, std::min(J.spp, cap / npix));
+        for (uint32_t s0 = 0; s0 < J.spp; s0 += std::min(kmax, J.spp - s0)) {
+            a.item = DevItem{0, p0, npix, s0, std::min(kmax, J.spp - s0), 0, 0, 0};
+            a.paths = npix * a.item.k;
+            a.pixels = npix;
+            SOLRT_TRY(issue_pass(ctx, kind, a, true, J.integrator == SOLRT_INTEGRATOR_PATH_NEE, true, true));
+        }
+    }
     return SOLRT_OK;
 }
 
@@ -924,7 +953,6 @@ solrt_status batch_issue(Batch& b, bool record_timing) {
     const uint32_t total_pix = b.job_pix_base[njobs];
     if (b.flags & SOLRT_BATCH_PERSISTENT) {
         unsigned int* work = ctx.trace_work.as<unsigned int>();
-        SOLRT_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned int), st));
         const int tm = record_timing ? ctx.timing_begin(0) : -1;  // traversal and shading in one launch
         bool nee = false;
         for (const DevJob& J : b.jobs) nee = nee || J.integrator == SOLRT_INTEGRATOR_PATH_NEE;
@@ -953,15 +981,9 @@ solrt_status batch_issue(Batch& b, bool record_timing) {
         SOLRT_CUDA(cudaGetLastError());
         return SOLRT_OK;
     }
-    const int tb = record_timing ? ctx.timing_begin(3) : -1;
-    k_begin<<<cdiv(total_pix, 256), 256, 0, st>>>(dj, jp, njobs, total_pix);
-    ctx.timing_end(tb);
-    ++ctx.launches;
-    for (const PassPlan& pp : b.passes) SOLRT_TRY(issue_pass(ctx, b.kind, dj, di + pp.item_begin, pp, record_timing));
-    const int tf = record_timing ? ctx.timing_begin(3) : -1;
-    k_finalize<<<cdiv(total_pix, 256), 256, 0, st>>>(dj, jp, njobs, total_pix);
-    ctx.timing_end(tf);
-    ++ctx.launches;
+    for (const PassPlan& pp : b.passes)
+        SOLRT_TRY(issue_pass(ctx, b.kind, table_pass(dj, di + pp.item_begin, pp), false, pp.nee != 0, true,
+                             record_timing));
     SOLRT_CUDA(cudaGetLastError());
     return SOLRT_OK;
 }
@@ -1017,6 +1039,9 @@ solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_
     for (uint32_t j = 0; j < n; ++j) {
         const DevJob& J = b.jobs[j];
         const uint32_t np = J.width * J.height;
+        // one sample of a REF_STREAM pixel per pass: the cooperative launch
+        // traces a pass's paths side by side, and plans are the same for
+        // every batch mode
         const uint32_t k = J.rng_mode == SOLRT_RNG_REF_STREAM ? 1u : std::max(1u, std::min(J.spp, cap / std::max(np, 1u)));
         for (uint32_t p0 = 0; p0 < np; p0 += cap) chunks.push_back(Chunk{j, p0, std::min(cap, np - p0), k, J.spp});
     }
@@ -1049,8 +1074,10 @@ solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_
             while (p < bins.size() && bins[p].plan.paths + paths > cap) ++p;
             if (p == bins.size()) bins.push_back(Bin{PassPlan{0, 0, 0, 0, 0}, {}});
             Bin& bn = bins[p];
-            DevItem it{ch.job, ch.pix0, ch.npix, s0, std::min(ch.k, ch.spp - s0), bn.plan.paths, bn.plan.pixels, 0};
+            DevItem it{ch.job, ch.pix0, ch.npix, s0, std::min(ch.k, ch.spp - s0), bn.plan.paths, bn.plan.pixels,
+                       bn.plan.units};
             bn.items.push_back(it);
+            bn.plan.units += item_units(it, b.jobs[it.job].rng_mode);
             bn.plan.item_count += 1;
             bn.plan.paths += (uint32_t)paths;
             bn.plan.pixels += it.npix;
@@ -1260,7 +1287,8 @@ solrt_status serve_tick(Context& ctx, TickBuffers& tb, uint32_t kind, const std:
     SOLRT_TRY(tb.items.alloc(sizeof(DevItem) * std::max<size_t>(items.size(), 1)));
     SOLRT_CUDA(cudaMemcpyAsync(tb.jobs.ptr, jobs.data(), sizeof(DevJob) * jobs.size(), cudaMemcpyHostToDevice, st));
     SOLRT_CUDA(cudaMemcpyAsync(tb.items.ptr, items.data(), sizeof(DevItem) * items.size(), cudaMemcpyHostToDevice, st));
-    if (pp.item_count) SOLRT_TRY(issue_pass(ctx, kind, tb.jobs.as<DevJob>(), tb.items.as<DevItem>(), pp, false));
+    if (pp.item_count) SOLRT_TRY(issue_pass(ctx, kind, table_pass(tb.jobs.as<DevJob>(), tb.items.as<DevItem>(), pp), false,
+                                            pp.nee != 0, false, false));
     if (!fin.empty()) {
         std::vector<uint32_t> pix(1, 0u);
         for (const DevJob& J : fin) pix.push_back(pix.back() + J.width * J.height);
@@ -1367,6 +1395,15 @@ solrt_status render_frame(Context& ctx, const Scene& sc, const solrt_camera& cam
                           Image& img) {
     if (p.integrator != SOLRT_INTEGRATOR_PATH && p.integrator != SOLRT_INTEGRATOR_PATH_NEE)
         return render_sibling(ctx, sc, cam, p, img);
+    if (p.kernel != SOLRT_KERNEL_MEGA) {
+        SOLRT_TRY(check_params(ctx, sc, img, p));
+        if (p.integrator == SOLRT_INTEGRATOR_PATH_NEE) SOLRT_TRY(ensure_shadow_queue(ctx));
+        cudaGetLastError();  // launch errors below must be this call's own
+        SOLRT_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
+        SOLRT_TRY(issue_frame(ctx, sc.info.kind, make_job(sc, img, cam, p)));
+        SOLRT_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
+        return SOLRT_OK;
+    }
     solrt_job jb;
     jb.scene = reinterpret_cast<solrt_scene*>(const_cast<Scene*>(&sc));
     jb.image = reinterpret_cast<solrt_image*>(&img);
@@ -1374,7 +1411,6 @@ solrt_status render_frame(Context& ctx, const Scene& sc, const solrt_camera& cam
     jb.params = p;
     jb.params.kernel = SOLRT_KERNEL_WAVEFRONT;
     SOLRT_TRY(batch_plan(ctx, &jb, 1, 0, ctx.single));
-    if (p.kernel != SOLRT_KERNEL_MEGA) return batch_launch(ctx.single);
     // per-pixel megakernel + the shared finalize
     Batch& b = ctx.single;
     cudaGetLastError();
