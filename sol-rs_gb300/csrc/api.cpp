@@ -680,7 +680,8 @@ solrt_status solrt_scene_bvh_export(solrt_scene* scene, void* nodes, size_t node
 solrt_status solrt_scene_bytes(solrt_scene* scene, uint64_t* out) {
     CHECK_ARG(scene && out, "null argument");
     *out = scene->vpos.bytes + scene->opos.bytes + scene->vnc.bytes + scene->tri_idx.bytes +
-           scene->materials.bytes + scene->sec_mat.bytes + scene->nodes.bytes + scene->tri_wt.bytes +
+           scene->materials.bytes + scene->sec_mat.bytes + scene->nodes.bytes + scene->qnodes.bytes +
+           scene->tri_wt.bytes +
            scene->vsec_start.bytes + scene->instances.bytes + scene->topo_order.bytes + scene->topo_child.bytes +
            scene->topo_par_int.bytes + scene->topo_par_leaf.bytes + scene->topo_range.bytes + scene->tlas.bytes +
            scene->inst_table.bytes + scene->lights.bytes + scene->tri_light.bytes;

@@ -429,17 +429,24 @@ solrt_status check_wide_depth(uint32_t width, uint32_t depth) {
 // the first two for ray origins within twice the scene's coordinate range,
 // and the relative 2^-16 widening of the far distance covers the rest (and
 // the case of farther origins, where |t| ~ |o| / |d|).
-__global__ void k_q16_grid(const float4* __restrict__ nbox, float4* __restrict__ header) {
+//
+// wide: an axis that does not fit such a grid (not finite, or too large) gets
+// one that covers every coordinate below 2^115, so that the nodes stay
+// conservative; without it the ok flag is cleared.
+__global__ void k_q16_grid(const float4* __restrict__ nbox, float4* __restrict__ header, bool wide,
+                           float* __restrict__ quality) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    if (quality) *quality = 0.0f;
     const float4 blo = nbox[0], bhi = nbox[1];
     const float lo[3] = {blo.x, blo.y, blo.z}, hi[3] = {bhi.x, bhi.y, bhi.z};
     float g[3], c[3];
     uint32_t ok = 1u;
     for (int a = 0; a < 3; ++a) {
-        if (!isfinite(lo[a]) || !isfinite(hi[a]) || lo[a] > hi[a]) {
+        const bool fits = isfinite(lo[a]) && isfinite(hi[a]) && lo[a] <= hi[a];
+        if (!fits) {
             ok = 0u;
-            g[a] = 0.0f;
-            c[a] = 1.0f;
+            g[a] = wide ? -0x1p115f : 0.0f;
+            c[a] = wide ? 0x1p100f : 1.0f;
             continue;
         }
         const double ext = (double)hi[a] - (double)lo[a];
@@ -447,7 +454,14 @@ __global__ void k_q16_grid(const float4* __restrict__ nbox, float4* __restrict__
         const double need = fmax(fmax(ext / 60000.0, m * 0x1p-20), 0x1p-60);
         int e = ilogb(need);
         if (ldexp(1.0, e) < need) ++e;
-        if (e > 23) ok = 0u;
+        if (e > 23) {
+            ok = 0u;
+            if (wide) {
+                g[a] = -0x1p115f;
+                c[a] = 0x1p100f;
+                continue;
+            }
+        }
         const double cd = ldexp(1.0, e);
         c[a] = (float)cd;
         g[a] = (float)(floor((double)lo[a] / cd) * cd - 4.0 * cd);
@@ -465,6 +479,62 @@ __device__ __forceinline__ uint32_t q16_pair(float lo, float hi, float g, float 
     const double qh = ceil(__dsub_ru((double)hi, (double)g) / dc) + 2.0;
     const uint32_t a = (uint32_t)fmin(fmax(ql, 0.0), 65535.0), b = (uint32_t)fmin(fmax(qh, 0.0), 65535.0);
     return a | (b << 16);
+}
+
+// q16_pair in FP32: the difference rounded outward by at most one unit in its
+// last place (a 256th of a cell), the scaling by the power of two exact; the
+// planes are those of q16_pair or one cell further out. (FP64 units are few on
+// this chip: 1M nodes take 15 us this way, 210 us through q16_pair.) An axis
+// of the covering grid (cell 2^100) gets its whole range.
+__device__ __forceinline__ uint32_t q16_pair_f32(float lo, float hi, float g, float c) {
+    if (c >= 0x1p100f) return 0xffff0000u;
+    const float ic = 1.0f / c;
+    const float ql = floorf(__fsub_rd(lo, g) * ic) - 2.0f, qh = ceilf(__fsub_ru(hi, g) * ic) + 2.0f;
+    const uint32_t a = (uint32_t)fminf(fmaxf(ql, 0.0f), 65535.0f), b = (uint32_t)fminf(fmaxf(qh, 0.0f), 65535.0f);
+    return a | (b << 16);
+}
+
+// How much larger the quantised box of one child is than the box itself, as
+// the ratio of their surface areas, at most 16.
+__device__ __forceinline__ float q16_growth(float lx, float hx, float ly, float hy, float lz, float hz, uint32_t qx,
+                                            uint32_t qy, uint32_t qz, const float c[3]) {
+    const float ex = hx - lx, ey = hy - ly, ez = hz - lz;
+    const float fx = (float)((qx >> 16) - (qx & 0xffffu)) * c[0], fy = (float)((qy >> 16) - (qy & 0xffffu)) * c[1],
+                fz = (float)((qz >> 16) - (qz & 0xffffu)) * c[2];
+    const float r = (fx * fy + fy * fz + fz * fx) / (ex * ey + ey * ez + ez * ex);
+    return r >= 1.0f ? fminf(r, 16.0f) : (r < 1.0f ? 1.0f : 16.0f);
+}
+
+// The traversal's 32-byte copy of BVH2 nodes; `quality` receives the sum of
+// every child's growth.
+__global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nodes, uint32_t ni,
+                                                  float4* __restrict__ out, float* __restrict__ quality) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    float grow = 0.0f;
+    if (i < ni) {
+        const float4 h0 = out[0], h1 = out[1];
+        const float g[3] = {h0.x, h0.y, h0.z}, c[3] = {h0.w, h1.x, h1.y};
+        const float4 n0 = nodes[4 * (size_t)i], n1 = nodes[4 * (size_t)i + 1], n2 = nodes[4 * (size_t)i + 2],
+                     n3 = nodes[4 * (size_t)i + 3];
+        const uint32_t x0 = q16_pair_f32(n0.x, n0.y, g[0], c[0]), y0 = q16_pair_f32(n0.z, n0.w, g[1], c[1]),
+                       z0 = q16_pair_f32(n2.x, n2.y, g[2], c[2]);
+        const uint32_t x1 = q16_pair_f32(n1.x, n1.y, g[0], c[0]), y1 = q16_pair_f32(n1.z, n1.w, g[1], c[1]),
+                       z1 = q16_pair_f32(n2.z, n2.w, g[2], c[2]);
+        uint4* o = reinterpret_cast<uint4*>(out + 2 + 2 * (size_t)i);
+        o[0] = make_uint4(__float_as_uint(n3.x), __float_as_uint(n3.y), x0, y0);
+        o[1] = make_uint4(z0, x1, y1, z1);
+        grow = q16_growth(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, x0, y0, z0, c) +
+               q16_growth(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, x1, y1, z1, c);
+    }
+    __shared__ float s_grow[8];
+    for (int off = 16; off > 0; off >>= 1) grow += __shfl_down_sync(0xffffffffu, grow, off);
+    if ((threadIdx.x & 31) == 0) s_grow[threadIdx.x >> 5] = grow;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.0f;
+        for (int w = 0; w < 8; ++w) t += s_grow[w];
+        atomicAdd(quality, t);
+    }
 }
 
 __global__ void k_q16_nodes(const float4* __restrict__ nodes, uint32_t ni, float4* __restrict__ out) {
@@ -489,7 +559,7 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
     cudaStream_t st = ctx.stream;
     DeviceBuffer q;
     SOLRT_TRY(q.alloc(32ull * ((size_t)ni + 1)));
-    k_q16_grid<<<1, 32, 0, st>>>(nbox, q.as<float4>());
+    k_q16_grid<<<1, 32, 0, st>>>(nbox, q.as<float4>(), false, nullptr);
     k_q16_nodes<<<blocks_for(ni, 256), 256, 0, st>>>(nodes.as<float4>(), ni, q.as<float4>());
     ctx.launches += 2;
     SOLRT_CUDA(cudaGetLastError());
@@ -501,6 +571,41 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
         return SOLRT_ERR_INVALID;
     }
     nodes.adopt(q);
+    return SOLRT_OK;
+}
+
+// The traversal's 32-byte copy of a BVH2 scene's nodes (Scene::qnodes), and
+// whether launches use it. It halves what a node visit loads, which is what
+// bounds the traversal once the nodes spill out of L1; it costs byte permutes
+// and, where the scene's grid is coarse for its triangles, larger boxes. 4M
+// incoherent rays, FP32 nodes / 32-byte nodes:
+//   soups: 100 triangles 0.38 / 0.39 ms, 300 0.57 / 0.58, 1000 0.89 / 0.81,
+//   8000 1.56 / 1.28, 100k 2.17 / 1.78, 1M (mean growth of the child boxes
+//   1.03) 2.63 / 2.18; tubes: 1M triangles (1.09) 1.18 / 1.11, 4M (1.21) 1.22 /
+//   1.25; a 1M soup in a box 7 times its size (1.14) 3.26 / 2.81, 21 times
+//   (1.61) 3.19 / 3.30, 61 times (4.2) 3.9 / 7.1.
+// So: from 512 triangles on, up to a mean growth of 1.18. The mean is over the
+// children, not weighted by area, so that a small detailed object in a large
+// scene counts. `nbox` holds the exact internal-node boxes (root first).
+// Synchronises.
+constexpr uint32_t kQ16MinTris = 512;
+constexpr float kQ16MaxGrowth = 1.18f;
+solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox) {
+    sc.use_qnodes = false;
+    if (sc.tri_count < kQ16MinTris) return SOLRT_OK;
+    cudaStream_t st = ctx.stream;
+    const uint32_t ni = sc.info.node_count;
+    SOLRT_TRY(sc.qnodes.alloc(32ull * ((size_t)ni + 1)));
+    SOLRT_TRY(ctx.build_word.alloc(sizeof(float)));
+    float* quality = ctx.build_word.as<float>();
+    k_q16_grid<<<1, 32, 0, st>>>(nbox, sc.qnodes.as<float4>(), true, quality);
+    k_q16_copy<<<blocks_for(ni, 256), 256, 0, st>>>(sc.nodes.as<float4>(), ni, sc.qnodes.as<float4>(), quality);
+    ctx.launches += 2;
+    SOLRT_CUDA(cudaGetLastError());
+    float sum = 0.0f;
+    SOLRT_CUDA(cudaMemcpyAsync(&sum, quality, sizeof(sum), cudaMemcpyDeviceToHost, st));
+    SOLRT_CUDA(cudaStreamSynchronize(st));
+    sc.use_qnodes = sum <= kQ16MaxGrowth * 2.0f * (float)ni;
     return SOLRT_OK;
 }
 
@@ -1212,6 +1317,8 @@ static solrt_status build_single_level(Context& ctx, Scene& sc, const solrt_bvh_
         if (desc.kind == SOLRT_BVH2_Q16) {
             SOLRT_TRY(quantize_bvh2(ctx, sc.nodes, L.nbox.as<float4>(), ni));
             sc.info.node_bytes = 32ull * ((uint64_t)ni + 1);
+        } else {
+            SOLRT_TRY(copy_nodes_q16(ctx, sc, L.nbox.as<float4>()));
         }
         sc.info.depth = L.depth;
     }
@@ -1236,6 +1343,8 @@ solrt_status build_bvh(Context& ctx, Scene& sc, const solrt_bvh_desc& desc) {
     sc.info.tri_count = n;
     sc.nodes.release();
     sc.tri_wt.release();
+    sc.use_qnodes = false;
+    if (desc.kind != SOLRT_BVH2) sc.qnodes.release();
     sc.desc = desc;
     if (n == 0) return SOLRT_OK;
     cudaGetLastError();  // launch errors below must be this call's own
@@ -1346,6 +1455,8 @@ solrt_status refit_bvh(Context& ctx, Scene& sc) {
     } else if (q16) {
         SOLRT_TRY(quantize_bvh2(ctx, nodes2, nbox.as<float4>(), ni));
         sc.nodes.adopt(nodes2);
+    } else {
+        SOLRT_TRY(copy_nodes_q16(ctx, sc, nbox.as<float4>()));
     }
     SOLRT_CUDA(cudaEventRecord(ctx.ev1, st));
     SOLRT_CUDA(cudaEventSynchronize(ctx.ev1));

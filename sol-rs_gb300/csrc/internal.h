@@ -147,7 +147,8 @@ struct Context;
 struct Batch {
     Context* ctx = nullptr;
     uint32_t flags = 0;
-    uint32_t kind = 0;
+    uint32_t kind = 0;       // of every job's scene
+    uint32_t trav_kind = 0;  // nodes its launches traverse
     std::vector<DevJob> jobs;
     std::vector<DevItem> items;
     std::vector<PassPlan> passes;
@@ -212,6 +213,7 @@ struct Context {
     // next unit and finished blocks of the persistent kernels; both 0 between
     // launches (release_work)
     DeviceBuffer trace_work;
+    DeviceBuffer build_word;  // one word that BVH builds read back
     // traversal-stack entries beyond the shared-memory slots (StackMem::deep)
     DeviceBuffer deep_stack;
     DeviceBuffer blue_noise;  // RGBA8 texels of SOLRT_INTEGRATOR_AO
@@ -275,6 +277,11 @@ struct Scene {
     // section its material index
     DeviceBuffer vpos, tri_idx, materials, sec_mat;
     DeviceBuffer nodes, tri_wt;
+    // SOLRT_BVH2: the nodes in the 32-byte format of SOLRT_BVH2_Q16, made by
+    // every build and refit, and whether launches traverse them (same hits;
+    // `nodes` is what solrt_scene_bvh_export gives)
+    DeviceBuffer qnodes;
+    bool use_qnodes = false;
     solrt_bvh_info info{};
     solrt_bvh_desc desc{};
     // Object-space positions / normals (float4 per vertex; shading reads
@@ -308,10 +315,15 @@ struct Scene {
     std::vector<uint32_t> light_sec_mat;
     std::vector<solrt_material> light_mats;
     uint32_t light_count = 0;
-    DevScene view() const {
+    // The kind of nodes that launches traverse.
+    uint32_t traversal_kind() const { return use_qnodes ? (uint32_t)SOLRT_BVH2_Q16 : info.kind; }
+    DevScene view() const { return view(traversal_kind()); }
+    // The scene with its nodes as launches for `kind` read them (a BVH2 scene's
+    // may be asked for as BVH2, too).
+    DevScene view(uint32_t kind) const {
         DevScene d;
         d.tri_count = tri_count;
-        d.bvh_kind = info.kind;
+        d.bvh_kind = kind;
         d.node_count = info.node_count;
         const bool two = info.kind == SOLRT_BVH2_TWO_LEVEL;
         d.tlas_count = two ? tlas_count : 0u;
@@ -325,7 +337,7 @@ struct Scene {
         d.sections = instances.as<float4>();
         d.sec_mat = sec_mat.as<uint32_t>();
         d.materials = materials.as<float4>();
-        d.nodes = nodes.as<float4>();
+        d.nodes = (info.kind == SOLRT_BVH2 && kind == SOLRT_BVH2_Q16 ? qnodes : nodes).as<float4>();
         d.tri_wt = tri_wt.as<float4>();
         d.lights = lights.as<float4>();
         d.tri_light = tri_light.as<uint32_t>();
@@ -395,7 +407,9 @@ solrt_status estimate_rmse(Context& ctx, TickBuffers& tb, const std::vector<DevJ
                            const std::vector<uint32_t>& n, std::vector<double>& out);
 solrt_status serve_tick(Context& ctx, TickBuffers& tb, uint32_t kind, const std::vector<DevJob>& jobs,
                         const std::vector<DevItem>& items, const PassPlan& pp, const std::vector<DevJob>& fin);
-DevJob job_for(const Scene& sc, const Image& img, const solrt_camera& cam, const solrt_render_params& p);
+// `kind`: the nodes that the launch traverses (Scene::view).
+DevJob job_for(const Scene& sc, uint32_t kind, const Image& img, const solrt_camera& cam,
+               const solrt_render_params& p);
 solrt_status check_job(const Context& ctx, const Scene& sc, const Image& img, const solrt_render_params& p);
 // Allocates the shadow-ray queue of SOLRT_INTEGRATOR_PATH_NEE (no-op once done).
 solrt_status ensure_shadow_queue(Context& ctx);

@@ -815,9 +815,11 @@ solrt_status check_params(const Context& ctx, const Scene& sc, const Image& img,
     return SOLRT_OK;
 }
 
-DevJob make_job(const Scene& sc, const Image& img, const solrt_camera& cam, const solrt_render_params& p) {
+// `kind`: the nodes that the launch traverses.
+DevJob make_job(const Scene& sc, uint32_t kind, const Image& img, const solrt_camera& cam,
+                const solrt_render_params& p) {
     DevJob J{};
-    J.sc = sc.view();
+    J.sc = sc.view(kind);
     std::copy(cam.view_inverse, cam.view_inverse + 16, J.vinv);
     std::copy(cam.projection_inverse, cam.projection_inverse + 16, J.pinv);
     J.width = p.width;
@@ -956,11 +958,11 @@ solrt_status batch_issue(Batch& b, bool record_timing) {
         const int tm = record_timing ? ctx.timing_begin(0) : -1;  // traversal and shading in one launch
         bool nee = false;
         for (const DevJob& J : b.jobs) nee = nee || J.integrator == SOLRT_INTEGRATOR_PATH_NEE;
-        if (b.kind == SOLRT_BVH8_Q8) launch_mega_batch<SOLRT_BVH8_Q8>(ctx, dj, jp, njobs, total_pix, work, nee);
-        else if (b.kind == SOLRT_BVH4_Q8) launch_mega_batch<SOLRT_BVH4_Q8>(ctx, dj, jp, njobs, total_pix, work, nee);
-        else if (b.kind == SOLRT_BVH8_F32) launch_mega_batch<SOLRT_BVH8_F32>(ctx, dj, jp, njobs, total_pix, work, nee);
-        else if (b.kind == SOLRT_BVH2_Q16) launch_mega_batch<SOLRT_BVH2_Q16>(ctx, dj, jp, njobs, total_pix, work, nee);
-        else if (b.kind == SOLRT_BVH2_TWO_LEVEL)
+        if (b.trav_kind == SOLRT_BVH8_Q8) launch_mega_batch<SOLRT_BVH8_Q8>(ctx, dj, jp, njobs, total_pix, work, nee);
+        else if (b.trav_kind == SOLRT_BVH4_Q8) launch_mega_batch<SOLRT_BVH4_Q8>(ctx, dj, jp, njobs, total_pix, work, nee);
+        else if (b.trav_kind == SOLRT_BVH8_F32) launch_mega_batch<SOLRT_BVH8_F32>(ctx, dj, jp, njobs, total_pix, work, nee);
+        else if (b.trav_kind == SOLRT_BVH2_Q16) launch_mega_batch<SOLRT_BVH2_Q16>(ctx, dj, jp, njobs, total_pix, work, nee);
+        else if (b.trav_kind == SOLRT_BVH2_TWO_LEVEL)
             launch_mega_batch<SOLRT_BVH2_TWO_LEVEL>(ctx, dj, jp, njobs, total_pix, work, nee);
         else launch_mega_batch<SOLRT_BVH2>(ctx, dj, jp, njobs, total_pix, work, nee);
         ctx.timing_end(tm);
@@ -975,17 +977,34 @@ solrt_status batch_issue(Batch& b, bool record_timing) {
         const int tm = record_timing ? ctx.timing_begin(0) : -1;  // every stage in one launch
         bool nee = false;
         for (const PassPlan& pp : b.passes) nee = nee || pp.nee;
-        SOLRT_TRY(launch_batch_coop(ctx, b.kind, dj, di, b.d_passes.as<PassPlan>(), (uint32_t)b.passes.size(),
+        SOLRT_TRY(launch_batch_coop(ctx, b.trav_kind, dj, di, b.d_passes.as<PassPlan>(), (uint32_t)b.passes.size(),
                                     b.coop_stride, jp, njobs, total_pix, b.d_coop.ptr, nee));
         ctx.timing_end(tm);
         SOLRT_CUDA(cudaGetLastError());
         return SOLRT_OK;
     }
     for (const PassPlan& pp : b.passes)
-        SOLRT_TRY(issue_pass(ctx, b.kind, table_pass(dj, di + pp.item_begin, pp), false, pp.nee != 0, true,
+        SOLRT_TRY(issue_pass(ctx, b.trav_kind, table_pass(dj, di + pp.item_begin, pp), false, pp.nee != 0, true,
                              record_timing));
     SOLRT_CUDA(cudaGetLastError());
     return SOLRT_OK;
+}
+
+// The nodes that one launch over all jobs traverses: the 32-byte copies when
+// every scene has them in use, else those of the kind. The per-pixel kernels
+// (SOLRT_BATCH_PERSISTENT) keep the 64-byte nodes: their per-ray loop waits on
+// latency, not on bytes, and the decoding only adds to it (an ambient-occlusion
+// frame 7.1 -> 7.6 ms).
+uint32_t batch_traversal_kind(uint32_t kind, uint32_t flags, const solrt_job* jobs, size_t n) {
+    if (kind != SOLRT_BVH2 || (flags & SOLRT_BATCH_PERSISTENT)) return kind;
+    for (size_t j = 0; j < n; ++j)
+        if (!static_cast<const Scene*>(reinterpret_cast<const void*>(jobs[j].scene))->use_qnodes) return kind;
+    return SOLRT_BVH2_Q16;
+}
+
+DevJob batch_job(uint32_t trav_kind, const solrt_job& jb) {
+    return make_job(*static_cast<const Scene*>(reinterpret_cast<const void*>(jb.scene)), trav_kind,
+                    *static_cast<const Image*>(reinterpret_cast<const void*>(jb.image)), jb.camera, jb.params);
 }
 
 }  // namespace
@@ -1017,11 +1036,12 @@ solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_
         if (jb.params.integrator == SOLRT_INTEGRATOR_PATH_NEE) SOLRT_TRY(ensure_shadow_queue(ctx));
         if (j == 0) b.kind = sc.info.kind;
         if (sc.info.kind != b.kind) { set_error("job %u: all scenes of a batch need the same BVH kind", j); return SOLRT_ERR_INVALID; }
-        b.jobs.push_back(make_job(sc, img, jb.camera, jb.params));
         const uint64_t np = (uint64_t)jb.params.width * jb.params.height;
         if (b.job_pix_base.back() + np >= (1ull << 31)) { set_error("batch has too many pixels"); return SOLRT_ERR_CAPACITY; }
         b.job_pix_base.push_back(b.job_pix_base.back() + (uint32_t)np);
     }
+    b.trav_kind = batch_traversal_kind(b.kind, flags, jobs, n);
+    for (uint32_t j = 0; j < n; ++j) b.jobs.push_back(batch_job(b.trav_kind, jobs[j]));
     if (flags & SOLRT_BATCH_PERSISTENT) {  // no passes: one launch over all pixels
         for (const DevJob& J : b.jobs) b.total_paths += (uint64_t)J.width * J.height * J.spp;
         SOLRT_TRY(b.d_jobs.alloc(sizeof(DevJob) * b.jobs.size()));
@@ -1116,12 +1136,13 @@ solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_
 
 // Replaces cameras / frames / seeds (the plan's structure must not change).
 solrt_status batch_set_jobs(Batch& b, const solrt_job* jobs) {
+    const uint32_t trav_kind = batch_traversal_kind(b.kind, b.flags, jobs, b.jobs.size());
     for (size_t j = 0; j < b.jobs.size(); ++j) {
         const solrt_job& jb = jobs[j];
         const Scene& sc = *static_cast<const Scene*>(reinterpret_cast<const void*>(jb.scene));
         const Image& img = *static_cast<const Image*>(reinterpret_cast<const void*>(jb.image));
         SOLRT_TRY(check_params(*b.ctx, sc, img, jb.params));
-        const DevJob nj = make_job(sc, img, jb.camera, jb.params);
+        const DevJob nj = batch_job(trav_kind, jb);
         const DevJob& oj = b.jobs[j];
         if (nj.width != oj.width || nj.height != oj.height || nj.spp != oj.spp || nj.max_bounces != oj.max_bounces ||
             nj.rng_mode != oj.rng_mode || nj.accum_mode != oj.accum_mode || sc.info.kind != b.kind) {
@@ -1130,6 +1151,13 @@ solrt_status batch_set_jobs(Batch& b, const solrt_job* jobs) {
         }
         b.jobs[j] = nj;
         b.src[j] = jb;
+    }
+    if (trav_kind != b.trav_kind) {  // a captured graph holds the other kind's kernels
+        if (b.exec) cudaGraphExecDestroy(b.exec);
+        if (b.graph) cudaGraphDestroy(b.graph);
+        b.exec = nullptr;
+        b.graph = nullptr;
+        b.trav_kind = trav_kind;
     }
     SOLRT_CUDA(cudaMemcpyAsync(b.d_jobs.ptr, b.jobs.data(), sizeof(DevJob) * b.jobs.size(), cudaMemcpyHostToDevice,
                                b.ctx->stream));
@@ -1330,8 +1358,9 @@ solrt_status estimate_rmse(Context& ctx, TickBuffers& tb, const std::vector<DevJ
     return SOLRT_OK;
 }
 
-DevJob job_for(const Scene& sc, const Image& img, const solrt_camera& cam, const solrt_render_params& p) {
-    return make_job(sc, img, cam, p);
+DevJob job_for(const Scene& sc, uint32_t kind, const Image& img, const solrt_camera& cam,
+               const solrt_render_params& p) {
+    return make_job(sc, kind, img, cam, p);
 }
 
 solrt_status check_job(const Context& ctx, const Scene& sc, const Image& img, const solrt_render_params& p) {
@@ -1357,7 +1386,8 @@ solrt_status ensure_shadow_queue(Context& ctx) {
 static solrt_status render_sibling(Context& ctx, const Scene& sc, const solrt_camera& cam,
                                    const solrt_render_params& p, Image& img) {
     SOLRT_TRY(check_params(ctx, sc, img, p));
-    DevJob J = make_job(sc, img, cam, p);
+    const uint32_t kind = sc.info.kind;
+    DevJob J = make_job(sc, kind, img, cam, p);
     J.integrator = p.integrator;
     J.noise = ctx.blue_noise.as<uchar4>();
     J.noise_w = ctx.noise_w;
@@ -1369,7 +1399,6 @@ static solrt_status render_sibling(Context& ctx, const Scene& sc, const solrt_ca
     const DevJob* dj = ctx.sibling_job.as<DevJob>();
     DevStats* stats = ctx.stats.as<DevStats>();
     SOLRT_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
-    const uint32_t kind = sc.info.kind;
     if (p.integrator == SOLRT_INTEGRATOR_DEBUG) {
         if (kind == SOLRT_BVH8_Q8) k_debug<SOLRT_BVH8_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
         else if (kind == SOLRT_BVH4_Q8) k_debug<SOLRT_BVH4_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
@@ -1400,7 +1429,7 @@ solrt_status render_frame(Context& ctx, const Scene& sc, const solrt_camera& cam
         if (p.integrator == SOLRT_INTEGRATOR_PATH_NEE) SOLRT_TRY(ensure_shadow_queue(ctx));
         cudaGetLastError();  // launch errors below must be this call's own
         SOLRT_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
-        SOLRT_TRY(issue_frame(ctx, sc.info.kind, make_job(sc, img, cam, p)));
+        SOLRT_TRY(issue_frame(ctx, sc.traversal_kind(), make_job(sc, sc.traversal_kind(), img, cam, p)));
         SOLRT_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
         return SOLRT_OK;
     }
@@ -1410,7 +1439,7 @@ solrt_status render_frame(Context& ctx, const Scene& sc, const solrt_camera& cam
     jb.camera = cam;
     jb.params = p;
     jb.params.kernel = SOLRT_KERNEL_WAVEFRONT;
-    SOLRT_TRY(batch_plan(ctx, &jb, 1, 0, ctx.single));
+    SOLRT_TRY(batch_plan(ctx, &jb, 1, SOLRT_BATCH_PERSISTENT, ctx.single));
     // per-pixel megakernel + the shared finalize
     Batch& b = ctx.single;
     cudaGetLastError();
@@ -1420,22 +1449,22 @@ solrt_status render_frame(Context& ctx, const Scene& sc, const solrt_camera& cam
     DevStats* dst = ctx.stats.as<DevStats>();
     const uint32_t g = cdiv(npix, 128);
     if (p.integrator == SOLRT_INTEGRATOR_PATH_NEE) {
-        if (b.kind == SOLRT_BVH8_Q8) k_megakernel_nee<SOLRT_BVH8_Q8><<<g, 128, 0, ctx.stream>>>(dj, dst);
-        else if (b.kind == SOLRT_BVH4_Q8) k_megakernel_nee<SOLRT_BVH4_Q8><<<g, 128, 0, ctx.stream>>>(dj, dst);
-        else if (b.kind == SOLRT_BVH8_F32) k_megakernel_nee<SOLRT_BVH8_F32><<<g, 128, 0, ctx.stream>>>(dj, dst);
-        else if (b.kind == SOLRT_BVH2_Q16) k_megakernel_nee<SOLRT_BVH2_Q16><<<g, 128, 0, ctx.stream>>>(dj, dst);
-        else if (b.kind == SOLRT_BVH2_TWO_LEVEL)
+        if (b.trav_kind == SOLRT_BVH8_Q8) k_megakernel_nee<SOLRT_BVH8_Q8><<<g, 128, 0, ctx.stream>>>(dj, dst);
+        else if (b.trav_kind == SOLRT_BVH4_Q8) k_megakernel_nee<SOLRT_BVH4_Q8><<<g, 128, 0, ctx.stream>>>(dj, dst);
+        else if (b.trav_kind == SOLRT_BVH8_F32) k_megakernel_nee<SOLRT_BVH8_F32><<<g, 128, 0, ctx.stream>>>(dj, dst);
+        else if (b.trav_kind == SOLRT_BVH2_Q16) k_megakernel_nee<SOLRT_BVH2_Q16><<<g, 128, 0, ctx.stream>>>(dj, dst);
+        else if (b.trav_kind == SOLRT_BVH2_TWO_LEVEL)
             k_megakernel_nee<SOLRT_BVH2_TWO_LEVEL><<<g, 128, 0, ctx.stream>>>(dj, dst);
         else k_megakernel_nee<SOLRT_BVH2><<<g, 128, 0, ctx.stream>>>(dj, dst);
-    } else if (b.kind == SOLRT_BVH8_Q8)
+    } else if (b.trav_kind == SOLRT_BVH8_Q8)
         k_megakernel<SOLRT_BVH8_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(b.d_jobs.as<DevJob>(), ctx.stats.as<DevStats>());
-    else if (b.kind == SOLRT_BVH4_Q8)
+    else if (b.trav_kind == SOLRT_BVH4_Q8)
         k_megakernel<SOLRT_BVH4_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(b.d_jobs.as<DevJob>(), ctx.stats.as<DevStats>());
-    else if (b.kind == SOLRT_BVH8_F32)
+    else if (b.trav_kind == SOLRT_BVH8_F32)
         k_megakernel<SOLRT_BVH8_F32><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(b.d_jobs.as<DevJob>(), ctx.stats.as<DevStats>());
-    else if (b.kind == SOLRT_BVH2_Q16)
+    else if (b.trav_kind == SOLRT_BVH2_Q16)
         k_megakernel<SOLRT_BVH2_Q16><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(b.d_jobs.as<DevJob>(), ctx.stats.as<DevStats>());
-    else if (b.kind == SOLRT_BVH2_TWO_LEVEL)
+    else if (b.trav_kind == SOLRT_BVH2_TWO_LEVEL)
         k_megakernel<SOLRT_BVH2_TWO_LEVEL><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(b.d_jobs.as<DevJob>(), ctx.stats.as<DevStats>());
     else
         k_megakernel<SOLRT_BVH2><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(b.d_jobs.as<DevJob>(), ctx.stats.as<DevStats>());

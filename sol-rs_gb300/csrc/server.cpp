@@ -219,6 +219,7 @@ void serve_loop(solrt_server* srv) {
     std::vector<double> est_sum;
     for (;;) {
         solrt::PassPlan pp{0, 0, 0, 0, 0};
+        uint32_t trav_kind = 0;
         {
             std::unique_lock<std::mutex> lock(srv->mu);
             srv->cv_work.wait_for(lock, std::chrono::milliseconds(20),
@@ -259,6 +260,12 @@ void serve_loop(solrt_server* srv) {
                     return wx != wy ? wx < wy : a < b;
                 });
             }
+            trav_kind = srv->kind;
+            if (trav_kind == SOLRT_BVH2) {  // the 32-byte nodes when every scene of the tick has them in use
+                bool q = true;
+                for (uint64_t t : srv->active) q = q && static_cast<solrt::Scene*>(srv->jobs[t].scene)->use_qnodes;
+                if (q) trav_kind = SOLRT_BVH2_Q16;
+            }
             const uint32_t share = std::max<uint32_t>(1u, srv->tick_paths / (uint32_t)srv->active.size());
             for (uint64_t t : srv->active) {
                 ServerJob& j = srv->jobs[t];
@@ -279,7 +286,7 @@ void serve_loop(solrt_server* srv) {
                 solrt::DevItem it{(uint32_t)jobs.size(), 0u, np, j.spp_done, k, pp.paths, pp.pixels, pp.units};
                 const solrt::Scene& sc = *static_cast<solrt::Scene*>(j.scene);
                 const solrt::Image& img = *static_cast<solrt::Image*>(j.image);
-                jobs.push_back(solrt::job_for(sc, img, j.cam, j.p));
+                jobs.push_back(solrt::job_for(sc, trav_kind, img, j.cam, j.p));
                 jobs.back().sq = j.sq;
                 items.push_back(it);
                 pp.item_count += 1;
@@ -298,7 +305,7 @@ void serve_loop(solrt_server* srv) {
         }
         // run the tick outside the lock
         cudaEventRecord(e0, ctx.stream);
-        const solrt_status s = solrt::serve_tick(ctx, srv->tb, srv->kind, jobs, items, pp, fin);
+        const solrt_status s = solrt::serve_tick(ctx, srv->tb, trav_kind, jobs, items, pp, fin);
         cudaEventRecord(e1, ctx.stream);
         const cudaError_t e = cudaEventSynchronize(e1);
         float ms = 0.0f;
@@ -361,7 +368,7 @@ void serve_loop(solrt_server* srv) {
                     q.spp = j.spp_done;
                     const solrt::Scene& sc = *static_cast<solrt::Scene*>(j.scene);
                     const solrt::Image& img = *static_cast<solrt::Image*>(j.image);
-                    fin.push_back(solrt::job_for(sc, img, j.cam, q));
+                    fin.push_back(solrt::job_for(sc, sc.traversal_kind(), img, j.cam, q));
                     fin_tickets.push_back(j.ticket);
                 }
             }

@@ -1,0 +1,102 @@
+"""BVH2 scenes traverse a 32-byte copy of their nodes when it pays (from 512
+triangles on, unless the scene's 16-bit grid is too coarse for them): hit
+records stay those of the oracle's brute force on both sides of each rule,
+through builds, refits and batches that mix both."""
+import numpy as np
+import pytest
+
+from helpers import S
+
+pytestmark = pytest.mark.gpu
+
+
+def _rays(rng, data, n):
+    pos = data.vertices["pos"][data.indices][:, :3].astype(np.float64)
+    tri = pos.reshape(-1, 3, 3)
+    k = rng.integers(0, len(tri), n)
+    b = rng.dirichlet((1, 1, 1), n)
+    target = (tri[k] * b[:, :, None]).sum(1)   # points on triangles, some on edges
+    target[: n // 8] = tri[k[: n // 8], 0]      # and some on vertices
+    d = rng.normal(size=(n, 3))
+    d[n // 2:: 16, 0] = 0.0                     # axis-parallel components
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    ext = np.linalg.norm(tri.max((0, 1)) - tri.min((0, 1)))
+    rays = np.zeros(n, [("origin", "<f4", 3), ("tmin", "<f4"), ("dir", "<f4", 3), ("tmax", "<f4")])
+    rays["origin"] = target - d * (rng.random((n, 1)) * 0.3 * ext)
+    rays["dir"] = d
+    rays["tmin"], rays["tmax"] = 1e-5 * ext, 1e4 * ext
+    return rays
+
+
+def _stretched(n, far):
+    """A soup of n triangles and two that stretch the scene's box to +-far."""
+    d = S.soup(n, seed=11, sigma=0.05)
+    v = d.vertices.copy()
+    v["pos"][0:3, :3] = [[far, far, far], [far + 0.1, far, far], [far, far + 0.1, far]]
+    v["pos"][3:6, :3] = [[-far, -far, -far], [0.1 - far, -far, -far], [-far, 0.1 - far, -far]]
+    return S.SceneData(v, d.indices, d.sections, d.materials, None, d.camera, "stretched")
+
+
+def _moved(n, offset, scale):
+    d = S.soup(n, seed=12, sigma=0.05)
+    v = d.vertices.copy()
+    v["pos"][:, :3] = v["pos"][:, :3] * np.float32(scale) + np.float32(offset)
+    return S.SceneData(v, d.indices, d.sections, d.materials, None, d.camera, "moved")
+
+
+@pytest.mark.parametrize("maker", [
+    lambda: S.soup(511, seed=1, sigma=0.05), lambda: S.soup(512, seed=1, sigma=0.05),
+    lambda: S.soup(513, seed=1, sigma=0.05), lambda: S.soup(3001, seed=2, sigma=0.03),
+    lambda: _stretched(2000, 3.0), lambda: _stretched(2000, 1e3), lambda: _stretched(2000, 1e7),
+    lambda: _moved(2000, 1000.0, 1.0), lambda: _moved(2000, 0.0, 1e-6), lambda: _moved(2000, -3e5, 1e4),
+    lambda: S.tunnel(n_ang=64, n_ax=32, length=300.0),
+], ids=["511", "512", "513", "3001", "far3", "far1e3", "far1e7", "off1000", "tiny", "off3e5", "tunnel"])
+@pytest.mark.parametrize("sah", [False, True])
+def test_hits_equal_brute_force(solrt, oracle, ctx, maker, sah):
+    d = maker()
+    rays = _rays(np.random.default_rng(5), d, 4096).view(solrt.RAY_DTYPE)
+    sc = solrt.SceneDescription(ctx, d, sah=sah)
+    got = sc.trace_rays(rays)
+    want, _ = oracle.OracleScene(d).trace(rays, brute=True)
+    for f in ("prim", "t", "u", "v"):
+        assert np.array_equal(got[f].view(np.uint32), want[f].view(np.uint32)), f
+    sc.close()
+
+
+def test_non_finite_vertices_do_not_hide_the_rest(solrt, oracle, ctx):
+    """A vertex at infinity leaves no finite grid: the scene still gives the
+    oracle's hits."""
+    d = S.soup(1000, seed=3, sigma=0.05)
+    v = d.vertices.copy()
+    v["pos"][7, 1] = np.inf
+    d = S.SceneData(v, d.indices, d.sections, d.materials, None, d.camera, "inf")
+    rays = _rays(np.random.default_rng(6), S.soup(1000, seed=3, sigma=0.05), 2048).view(solrt.RAY_DTYPE)
+    sc = solrt.SceneDescription(ctx, d)
+    got = sc.trace_rays(rays)
+    want, _ = oracle.OracleScene(d).trace(rays, brute=True)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    sc.close()
+
+
+def test_batch_mixing_both_node_formats(solrt, ctx):
+    """One batch over a scene below and one above the size rule, then updated
+    with cameras swapped: each image equals its own render."""
+    scenes = [solrt.SceneDescription(ctx, d) for d in (S.cornell(), S.soup(4000, seed=4, sigma=0.03))]
+    cams = [solrt.camera_look_at(sc.data.camera["eye"], sc.data.camera["center"], sc.data.camera["up"],
+                                 sc.data.camera["vfov"], 1.0) for sc in scenes]
+    p = solrt.render_params(40, 40, spp=3, max_bounces=4, seed=9, miss_mode=solrt.MISS_GRADIENT,
+                            material_mode=solrt.MATERIAL_LAMBERT, rng_mode=solrt.RNG_PER_SAMPLE)
+    for pick in ((0, 1), (1, 1)):
+        jobs = [(scenes[k], solrt.Image(ctx, 40, 40), cams[k], p) for k in pick]
+        b = solrt.Batch(ctx, jobs, graph=True)
+        for _ in range(2):
+            b.launch()
+            ctx.synchronize()
+            for sc, img, cam, q in jobs:
+                alone = solrt.Image(ctx, 40, 40)
+                solrt.Renderer(ctx).cmd_trace_rays(sc, cam, q, alone)
+                ctx.synchronize()
+                assert np.array_equal(img.read()[0].view(np.uint32), alone.read()[0].view(np.uint32))
+                alone.close()
+            b.update(jobs)
+        b.close()
