@@ -259,7 +259,9 @@ typedef enum solrt_integrator {
 } solrt_integrator;
 
 typedef enum solrt_kernel {
-    /* generate / extend / shade stages over queues shared by all paths */
+    /* generate / extend / shade stages over queues shared by all paths; frames
+     * with few rays per bounce level run the same steps in one launch whose
+     * warps keep their paths to the end (same image) */
     SOLRT_KERNEL_WAVEFRONT = 0,
     /* the reference's structure (pathtrace.rgen:39-104): one thread per pixel
      * loops over its samples and bounces; same image, the plain kernel that

@@ -57,7 +57,7 @@ SOLRT_D void extend_bvh2_2l_ww(IO& io, uint32_t n, unsigned int* work, const Sta
     for (;;) {
         const bool idle = node == kBvh2Sentinel && leaf >= 0;
         float4 o, d;
-        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH2_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+        if (warp_feed(io, idle, has, drained, rm, n, work, tmin, best_t, o, d, ts, cnt, ef)) {
             rm.clear_hit();
             tmin = o.w;
             rb.set(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z);

@@ -3,8 +3,7 @@
 // A warp keeps 32 rays in flight. Every step of its loop is warp-uniform
 // (full-warp votes decide the phases), so lanes re-converge at each step:
 //   refill  lanes whose ray has finished take new rays from the global queue
-//           (one atomic per warp), once at least SOLRT_BVH2_REFILL lanes are
-//           free;
+//           (one atomic per warp), once enough lanes are free (warp_feed);
 //   nodes   lanes visit inner nodes, up to SOLRT_BVH2_NODE_STEPS between two
 //           votes, until every lane has parked a leaf or has no inner node
 //           left, or until fewer than SOLRT_WW_NODE_MIN lanes still have
@@ -23,9 +22,6 @@
 namespace solrt {
 
 constexpr int kBvh2Sentinel = 0x7fffffff;
-#ifndef SOLRT_BVH2_REFILL
-#define SOLRT_BVH2_REFILL 16
-#endif
 // The node phase ends early when fewer than this many lanes have inner
 // nodes to visit and some lane holds a leaf (0 = only when no lane without
 // a parked leaf has inner nodes left).
@@ -90,9 +86,9 @@ struct RayBox {
         if constexpr (kQ16) {
             q16_ray(nodes, ox, oy, oz, dx, dy, dz, ix, iy, iz, nox, noy, noz);
         } else {
-            ix = 1.0f / box_dir(dx);
-            iy = 1.0f / box_dir(dy);
-            iz = 1.0f / box_dir(dz);
+            ix = box_rcp(box_dir(dx));
+            iy = box_rcp(box_dir(dy));
+            iz = box_rcp(box_dir(dz));
             nox = -(ox * ix);
             noy = -(oy * iy);
             noz = -(oz * iz);
@@ -144,7 +140,7 @@ SOLRT_D void extend_bvh2_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             node = kBvh2Sentinel;
         }
         float4 o, d;
-        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH2_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+        if (warp_feed(io, idle, has, drained, rm, n, work, tmin, best_t, o, d, ts, cnt, ef)) {
             rm.set_ray(o.x, o.y, o.z, d.x, d.y, d.z);
             rm.clear_hit();
             if (ts.tri_count) rb.set(ts.nodes, o.x, o.y, o.z, d.x, d.y, d.z);

@@ -87,7 +87,7 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
     for (;;) {
         const bool idle = node == kBvh2Sentinel && tgrp.y == 0u;
         float4 o, d;
-        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH2_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+        if (warp_feed(io, idle, has, drained, rm, n, work, tmin, best_t, o, d, ts, cnt, ef)) {
             rm.set_ray(o.x, o.y, o.z, d.x, d.y, d.z);
             rm.clear_hit();
             ox = o.x;
@@ -96,9 +96,9 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             tmin = o.w;
             best_t = d.w;
             const float bx = box_dir(d.x), by = box_dir(d.y), bz = box_dir(d.z);
-            ix = 1.0f / bx;
-            iy = 1.0f / by;
-            iz = 1.0f / bz;
+            ix = box_rcp(bx);
+            iy = box_rcp(by);
+            iz = box_rcp(bz);
             negx = signbit(bx);
             negy = signbit(by);
             negz = signbit(bz);
@@ -188,7 +188,7 @@ SOLRT_D void trace_bvh4_ray(const TravScene& ts, float ox, float oy, float oz, f
     if (ts.tri_count == 0) return;
     const RayWT r = setup_ray(ox, oy, oz, dx, dy, dz, tmin);
     const float bx = box_dir(dx), by = box_dir(dy), bz = box_dir(dz);
-    const float ix = 1.0f / bx, iy = 1.0f / by, iz = 1.0f / bz;
+    const float ix = box_rcp(bx), iy = box_rcp(by), iz = box_rcp(bz);
     const bool negx = signbit(bx), negy = signbit(by), negz = signbit(bz);
     int stack[SOLRT_BVH2_STACK + 1];
     stack[0] = kBvh2Sentinel;

@@ -187,7 +187,7 @@ SOLRT_D void trace_bvh8(const TravScene& sc, float ox, float oy, float oz, float
     if (sc.tri_count == 0) return;
     const RayWT r = setup_ray(ox, oy, oz, dx, dy, dz, tmin);
     const float bx = box_dir(dx), by = box_dir(dy), bz = box_dir(dz);
-    const float ix = 1.0f / bx, iy = 1.0f / by, iz = 1.0f / bz;
+    const float ix = box_rcp(bx), iy = box_rcp(by), iz = box_rcp(bz);
     const float nox = -(ox * ix), noy = -(oy * iy), noz = -(oz * iz);
     const bool negx = signbit(bx), negy = signbit(by), negz = signbit(bz);
     const uint32_t oct = (negx ? 1u : 0u) | (negy ? 2u : 0u) | (negz ? 4u : 0u);

@@ -2,7 +2,7 @@
 // like bvh2_ww.cuh: a warp keeps 32 rays in flight and every step of its loop
 // is warp-uniform.
 //   refill  lanes whose ray has finished take new rays from the global queue
-//           once at least SOLRT_BVH8_REFILL lanes are free;
+//           once enough lanes are free (warp_feed);
 //   nodes   lanes with no parked triangles visit one 8-wide node per step:
 //           the nearest remaining internal child of their current node group
 //           (octant order), pushing the rest of the group; the node's hit
@@ -20,9 +20,6 @@
 
 namespace solrt {
 
-#ifndef SOLRT_BVH8_REFILL
-#define SOLRT_BVH8_REFILL 16
-#endif
 #ifndef SOLRT_BVH8_NODE_MIN
 #define SOLRT_BVH8_NODE_MIN 12
 #endif
@@ -49,7 +46,7 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
     for (;;) {
         const bool idle = (grp.y >> 24) == 0u && sp == 0 && tgrp.y == 0u;
         float4 o, d;
-        if (warp_feed(io, idle, has, drained, rm, n, work, SOLRT_BVH8_REFILL, tmin, best_t, o, d, ts, cnt, ef)) {
+        if (warp_feed(io, idle, has, drained, rm, n, work, tmin, best_t, o, d, ts, cnt, ef)) {
             rm.set_ray(o.x, o.y, o.z, d.x, d.y, d.z);
             rm.clear_hit();
             ox = o.x;
@@ -58,9 +55,9 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             tmin = o.w;
             best_t = d.w;
             const float bx = box_dir(d.x), by = box_dir(d.y), bz = box_dir(d.z);
-            ix = 1.0f / bx;
-            iy = 1.0f / by;
-            iz = 1.0f / bz;
+            ix = box_rcp(bx);
+            iy = box_rcp(by);
+            iz = box_rcp(bz);
             negx = signbit(bx);
             negy = signbit(by);
             negz = signbit(bz);

@@ -584,15 +584,14 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
 //   1.03) 2.63 / 2.18; tubes: 1M triangles (1.09) 1.18 / 1.11, 4M (1.21) 1.22 /
 //   1.25; a 1M soup in a box 7 times its size (1.14) 3.26 / 2.81, 21 times
 //   (1.61) 3.19 / 3.30, 61 times (4.2) 3.9 / 7.1.
-// So: from 512 triangles on, up to a mean growth of 1.18. The mean is over the
+// So: from kSmallScene triangles on, up to a mean growth of 1.18. The mean is over the
 // children, not weighted by area, so that a small detailed object in a large
 // scene counts. `nbox` holds the exact internal-node boxes (root first).
 // Synchronises.
-constexpr uint32_t kQ16MinTris = 512;
 constexpr float kQ16MaxGrowth = 1.18f;
 solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox) {
     sc.use_qnodes = false;
-    if (sc.tri_count < kQ16MinTris) return SOLRT_OK;
+    if (sc.tri_count < kSmallScene) return SOLRT_OK;
     cudaStream_t st = ctx.stream;
     const uint32_t ni = sc.info.node_count;
     SOLRT_TRY(sc.qnodes.alloc(32ull * ((size_t)ni + 1)));

@@ -111,7 +111,7 @@ struct CoopIOT {
     const DevJob* jobs;
     float4* hits;
     bool any_hit;
-    static constexpr int lanes = 32;
+    static constexpr int lanes = 32, refill = kRefill;
     SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
         o = __ldcg(o_tmin + i);
@@ -144,7 +144,7 @@ struct CoopIOT<false> {
     float4* hits;
     bool unused;
     static constexpr bool any_hit = false;
-    static constexpr int lanes = 32;
+    static constexpr int lanes = 32, refill = kRefill;
     SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
         CoopIOT<true>{o_tmin, d_tmax, meta, jobs, hits, false}.load(i, o, d, ts);

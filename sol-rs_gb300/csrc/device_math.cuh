@@ -80,7 +80,9 @@ SOLRT_D float next_rand(uint32_t& rng) {
     rng = rng * 747796405u + 1u;
     uint32_t word = ((rng >> ((rng >> 28) + 4u)) ^ rng) * 277803737u;
     word = (word >> 22) ^ word;
-    return __fdiv_rn(__uint2float_rn(word), 4294967295.0f);
+    // sampling.glsl divides by 4294967295.0, which is 2^32 as a float: the
+    // product with 2^-32 is the same value, exactly
+    return __uint2float_rn(word) * 0x1p-32f;
 }
 
 // ---------------------------------------------------------------------------

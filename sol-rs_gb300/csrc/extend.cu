@@ -22,6 +22,7 @@ struct QueueIO {
     float4* __restrict__ hits;
     const TravScene& scene;
     int lanes;
+    static constexpr int refill = kRefill;
     bool any_hit;  // occlusion queries (shadow rays): any hit in (tmin, tmax)
     SOLRT_D TravScene first_scene() const { return kSingle ? scene : TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {

@@ -89,15 +89,16 @@ constexpr int kTraverseMinBlocks = 5;
 // Shape of one launch of `kern`: the context's block size and stack slots,
 // state_words words of program state per thread, a grid of (SMs x resident
 // blocks) or fewer blocks when `units` rays or paths need fewer, and how many
-// lanes of each warp take work: 32, or as few as spread the units over all
-// warps of a full grid when there are not enough for every lane (a warp with
-// fewer rays steps faster, and otherwise most SMs would be idle).
+// lanes of each warp take work: 32, or as few (but `least`) as spread the units
+// over all warps of a full grid when there are not enough for every lane (a
+// warp with fewer rays steps faster, and otherwise most SMs would be idle).
 struct LaunchShape {
     uint32_t grid = 0, block = 0, smem = 0, slots = 0, lanes = 32;
 };
 
 template <int KIND, auto kern>
-solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t units, LaunchShape& s) {
+solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t units, LaunchShape& s,
+                          uint32_t least = 1) {
     s.block = ctx.tune.block;
     s.slots = kind_has_smem_stack<KIND>() ? stack_slots(ctx.tune.smem) : 0u;
     s.smem = 4u * s.block * (s.slots + kRayWords + state_words);
@@ -115,7 +116,7 @@ solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t uni
     }
     const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;
     const uint32_t warps = full * (s.block / 32u);
-    s.lanes = std::min(32u, std::max(1u, (units + warps - 1u) / warps));
+    s.lanes = std::min(32u, std::max(least, (units + warps - 1u) / warps));
     s.grid = std::min(full, (units + s.lanes * (s.block / 32u) - 1u) / (s.lanes * (s.block / 32u)));
     return SOLRT_OK;
 }

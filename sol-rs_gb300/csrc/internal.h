@@ -117,17 +117,10 @@ struct DevJob {
 // A work item of one pass: samples [s0, s0 + k) of pixels [pix0, pix0 + npix)
 // of one job. Its paths occupy slots [path_base, path_base + npix * k) of the
 // pass (pixel-major), its pixels [pix_base, pix_base + npix) of the pass's
-// pixel space, and its units of work (item_units) [unit_base, ...) of the
-// path kernel's.
+// pixel space.
 struct DevItem {
-    uint32_t job, pix0, npix, s0, k, path_base, pix_base, unit_base;
+    uint32_t job, pix0, npix, s0, k, path_base, pix_base;
 };
-
-// Units of work of an item in the path kernel: its paths, or its pixels when
-// the samples of a pixel share one random stream and are traced in sequence.
-SOLRT_HD uint32_t item_units(const DevItem& it, uint32_t rng_mode) {
-    return rng_mode == SOLRT_RNG_REF_STREAM ? it.npix : it.npix * it.k;
-}
 
 // The depth field of a path's meta word also carries its job.
 constexpr uint32_t kDepthBits = 11;
@@ -138,7 +131,6 @@ struct PassPlan {
     uint32_t paths, pixels;
     uint32_t bounces;  // bounce levels of the pass (cooperative batches)
     uint32_t nee = 0;  // a job of the pass uses SOLRT_INTEGRATOR_PATH_NEE
-    uint32_t units = 0;  // units of work of the path kernel (item_units summed)
 };
 
 struct Context;
@@ -345,6 +337,10 @@ struct Scene {
         return d;
     }
 };
+
+// Scenes of fewer triangles are small: their nodes and triangles stay in an
+// SM's L1, and a ray visits a dozen nodes.
+constexpr uint32_t kSmallScene = 512;
 
 struct Image {
     Context* ctx = nullptr;

@@ -67,6 +67,17 @@ SOLRT_D void hit_frame(const DevScene& sc, uint4 ti, float b0, float b1, float b
     pos = mat4_xyz(inst + 1, p.x, p.y, p.z, 1.0f);
 }
 
+// sign(dot(normal, -normalize(dir))) (rchit:94-95) for a normal and a direction
+// of about unit length. Normalising scales the products by one factor up to
+// rounding, so the sign is that of dot(normal, -dir) unless the two are within
+// 1e-4 of perpendicular; only then is the direction normalised (a square root
+// and three divisions).
+SOLRT_D float facing_sign(f3 normal, f3 dir) {
+    const float c = dot(normal, -dir), l2 = dot(dir, dir);
+    if (fabsf(c) > 1e-4f && l2 > 0.5f && l2 < 2.0f && dot(normal, normal) < 2.0f) return glsl_sign(c);
+    return glsl_sign(dot(normal, -normalize(dir)));
+}
+
 // One closest-hit or miss step (pathtrace.rchit:56-113, pathtrace.rmiss:8-21
 // and pathtrace.rgen:77-84). h = (t, prim bits, u, v). Updates the path
 // throughput `acc`, the rng state and the depth; returns true when the path
@@ -122,8 +133,7 @@ SOLRT_D bool shade_step(const DevJob& J, float4 o, float4 d, float4 h, f3& acc, 
     const float b0 = (1.0f - b1) - b2;                                       // rchit:82
     f3 normal, pos, vcol;
     hit_frame(sc, ti, b0, b1, b2, normal, pos, &vcol);                       // rchit:82-90
-    const f3 wi = normalize(dir);                                            // rchit:94-95
-    const f3 n_o = normal * glsl_sign(dot(normal, -wi));
+    const f3 n_o = normal * facing_sign(normal, dir);                        // rchit:94-95
     const float alpha2 = m2.y * m2.y;
     const float xi0 = next_rand(rng);                                        // rchit:97-98
     const float xi1 = next_rand(rng);

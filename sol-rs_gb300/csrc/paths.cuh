@@ -1,0 +1,258 @@
+// paths.cuh — a frame of one job as one persistent launch: the path kernel.
+//
+// The reference runs one raygen invocation per pixel that loops over 8
+// samples and up to maxBounces+1 traceRayEXT calls, each resuming in the
+// closest-hit or miss shader (assets/glsl/pathtrace.rgen:39-104,
+// pathtrace.rchit:56-113, pathtrace.rmiss:8-21). Here a warp holds up to 32
+// paths in the traversal loop of the BVH kind; when at least half of its lanes
+// have finished their rays, those lanes shade their hits and go on with the
+// next ray of their path, or end it and take another one from the launch's
+// work counter (warp_feed). Path state that traversal does not touch waits in
+// shared memory.
+//
+// What it saves over the wavefront (pathtrace.cu) is the launches, two per
+// bounce level, and the end of each extend launch, which lasts as long as its
+// longest ray with few other rays left to trace. What it costs is shading with
+// part of a warp while the other lanes wait: on frames large enough to fill
+// the wavefront's launches it is a third slower (path_kernel_pays, below,
+// draws the line).
+//
+// A unit of work is a path, or, for jobs with one random stream per pixel
+// (SOLRT_RNG_REF_STREAM), a pixel whose samples the lane traces one after
+// the other. Every sample writes its radiance to its own slot and per-pixel
+// sums run in sample order, so the image equals a sequential per-pixel
+// evaluation, and the wavefront's, bit for bit.
+#pragma once
+
+#include "extend.cuh"
+#include "path_ops.cuh"
+
+#ifndef SOLRT_PATH_MINB
+#define SOLRT_PATH_MINB 4
+#endif
+
+namespace solrt {
+
+// One launch: the samples of one work item of one job, `units` units of work.
+struct PathArgs {
+    DevJob job;
+    DevItem item;
+    uint32_t units, slots;
+    int refill;  // warp_feed's threshold
+    unsigned int* work;
+    int* deep;
+    float4* rad;
+    DevStats* stats;
+};
+
+// Shared-memory words per thread.
+enum PathWord {
+    kWDir = 0,      // direction of the ray in flight (3)
+    kWThr = 3,      // throughput (3)
+    kWRng = 6,      // random stream
+    kWSlot = 7,     // radiance slot in the pass
+    kWDepth = 8,    // bounces so far
+    kWSegs = 9,     // rays traced by this thread, shadow rays apart
+    kWOrg = 10,     // origin of the ray in flight (3; two-level scenes and next-event estimation)
+    kWNext = 13,    // next-event estimation: direction after the shadow ray (3)
+    kWLight = 16,   // what the shadow ray adds when it is unoccluded (3)
+    kWSum = 19,     // sum of the path's light terms (3)
+    kWPrev = 22,    // normal of the vertex the ray left, pdf of its direction (4)
+    kWMark = 26,    // FP64 fallbacks when the last ray ended
+    kWShadow = 27,  // FP64 fallbacks of shadow rays
+    kWShadowSegs = 28,  // shadow rays traced, and those that reached their light (2)
+    kWNeeEnd = 30,
+};
+template <int KIND, bool kNee>
+constexpr uint32_t path_words() {
+    return kNee ? kWNeeEnd : KIND == SOLRT_BVH2_TWO_LEVEL ? kWNext : kWOrg;
+}
+
+// The any-hit switch of the traversal loops: a per-lane flag where shadow
+// rays are traced, a constant elsewhere.
+template <bool kNee> struct PathAnyHit { bool any_hit = false; };
+template <> struct PathAnyHit<false> { static constexpr bool any_hit = false; };
+
+template <int KIND, bool kNee>
+struct PathIO : PathAnyHit<kNee> {
+    const PathArgs& a;
+    uint32_t st;      // shared address of the thread's column of path state
+    uint32_t stride;  // bytes from word to word
+    const int refill;
+    static constexpr int lanes = 32;  // fewer make a lone small frame no faster and several at once slower
+    static constexpr bool kOrg = kNee || KIND == SOLRT_BVH2_TWO_LEVEL;
+
+    SOLRT_D PathIO(const PathArgs& args) : a(args), st(state_column(args.slots)), stride(4u * blockDim.x), refill(args.refill) {
+        put(kWSegs, 0u);
+        if (kNee)
+            for (int w = kWMark; w < kWNeeEnd; ++w) put(w, 0u);
+    }
+    SOLRT_D uint32_t get(uint32_t w) const { return lds_u32(st + w * stride); }
+    SOLRT_D void put(uint32_t w, uint32_t v) { sts_u32(st + w * stride, v); }
+    SOLRT_D void bump(uint32_t w) { put(w, get(w) + 1u); }
+    SOLRT_D float getf(uint32_t w) const { return __uint_as_float(get(w)); }
+    SOLRT_D f3 get3(uint32_t w) const { return f3{getf(w), getf(w + 1), getf(w + 2)}; }
+    SOLRT_D void put3(uint32_t w, float x, float y, float z) {
+        put(w, __float_as_uint(x));
+        put(w + 1, __float_as_uint(y));
+        put(w + 2, __float_as_uint(z));
+    }
+    SOLRT_D TravScene first_scene() const { return trav_scene(a.job.sc); }
+
+    // The camera ray of a sample of pixel pix (rgen:47-61).
+    SOLRT_D void start(uint32_t pix, uint32_t rng, uint32_t slot, float4& o, float4& d) {
+        camera_ray(a.job, pix, rng, o, d);
+        put3(kWDir, d.x, d.y, d.z);
+        put3(kWThr, 1.0f, 1.0f, 1.0f);
+        put(kWRng, rng);
+        put(kWSlot, slot);
+        put(kWDepth, 0u);
+        if (kOrg) put3(kWOrg, o.x, o.y, o.z);
+        if (kNee) put3(kWSum, 0.0f, 0.0f, 0.0f);
+        bump(kWSegs);
+    }
+    SOLRT_D void load(uint32_t unit, float4& o, float4& d, TravScene&) {
+        const DevItem& it = a.item;
+        const bool chain = a.job.rng_mode == SOLRT_RNG_REF_STREAM;
+        const uint32_t lp = chain ? unit : unit / it.k, j = chain ? 0u : unit - lp * it.k;
+        const uint32_t pix = it.pix0 + lp, s = it.s0 + j;
+        const uint32_t rng = sample_seed(a.job, pix, s, chain && s > 0 ? a.job.rng_state[pix] : 0u);
+        start(pix, rng, lp * it.k + j, o, d);
+    }
+    SOLRT_D void load_ray(uint32_t, float4& o, float4& d) const {
+        const f3 p = get3(kWOrg), q = get3(kWDir);
+        o = make_float4(p.x, p.y, p.z, 0.0f);
+        d = make_float4(q.x, q.y, q.z, 0.0f);
+    }
+    // The lane's ray is done: shades its hit. True with the path's next ray
+    // (or its pixel's next sample).
+    SOLRT_D bool next(uint32_t unit, float tmin, const HitRec& best, float4& o, float4& d, const TraceCounters& cnt,
+                      uint32_t& ef) {
+        const DevJob& J = a.job;
+        const f3 dir = get3(kWDir);
+        f3 org{0.0f, 0.0f, 0.0f};
+        if (kOrg) org = get3(kWOrg);
+        if constexpr (kNee) {
+            if (this->any_hit) put(kWShadow, get(kWShadow) + cnt.fallbacks - get(kWMark));
+            put(kWMark, cnt.fallbacks);
+            if (this->any_hit) {  // a shadow ray: its term, then the bounce ray from the same vertex
+                this->any_hit = false;
+                if (best.prim == SOLRT_NO_HIT) {
+                    const f3 c = get3(kWLight), s = get3(kWSum);
+                    put3(kWSum, s.x + c.x, s.y + c.y, s.z + c.z);
+                    bump(kWShadowSegs + 1);
+                }
+                const f3 q = get3(kWNext);
+                put3(kWDir, q.x, q.y, q.z);
+                o = make_float4(org.x, org.y, org.z, tmin);
+                d = make_float4(q.x, q.y, q.z, J.tmax);
+                bump(kWSegs);
+                return true;
+            }
+        }
+        f3 acc = get3(kWThr);
+        uint32_t rng = get(kWRng), depth = get(kWDepth);
+        const float4 h = make_float4(best.t, __uint_as_float(best.prim), best.u, best.v);
+        const bool nee = kNee && J.integrator == SOLRT_INTEGRATOR_PATH_NEE;
+        f3 n_o{0.0f, 0.0f, 0.0f};
+        float4 prev = make_float4(0.0f, 0.0f, 0.0f, 0.0f), prev_out = prev;
+        if (nee && depth > 0u) {
+            const f3 n = get3(kWPrev);
+            prev = make_float4(n.x, n.y, n.z, getf(kWPrev + 3));
+        }
+        if (shade_step<kNee>(J, make_float4(org.x, org.y, org.z, tmin), make_float4(dir.x, dir.y, dir.z, J.tmax), h, acc,
+                             rng, depth, o, d, ef, &n_o, prev, &prev_out)) {
+            put3(kWThr, acc.x, acc.y, acc.z);
+            put(kWDepth, depth);
+            if (kOrg) put3(kWOrg, o.x, o.y, o.z);
+            if constexpr (kNee) {
+                if (nee) {
+                    put3(kWPrev, prev_out.x, prev_out.y, prev_out.z);
+                    put(kWPrev + 3, __float_as_uint(prev_out.w));
+                    float4 so, sd;
+                    f3 c;
+                    if (nee_sample(J.sc, f3{o.x, o.y, o.z}, n_o, acc, tmin, rng, so, sd, c)) {
+                        put3(kWNext, d.x, d.y, d.z);
+                        put3(kWLight, c.x, c.y, c.z);
+                        d = sd;
+                        this->any_hit = true;
+                        bump(kWShadowSegs);
+                    }
+                }
+            }
+            put(kWRng, rng);
+            put3(kWDir, d.x, d.y, d.z);
+            if (!this->any_hit) bump(kWSegs);
+            return true;
+        }
+        if (nee) acc = get3(kWSum) + acc;  // light terms in bounce order, then the end term
+        const uint32_t slot = get(kWSlot);
+        a.rad[slot] = make_float4(acc.x, acc.y, acc.z, 0.0f);
+        if (J.rng_mode == SOLRT_RNG_REF_STREAM) {  // the pixel's next sample continues the stream
+            const uint32_t pix = a.item.pix0 + unit;
+            if (slot - unit * a.item.k + 1u < a.item.k) {
+                start(pix, rng, slot + 1u, o, d);
+                return true;
+            }
+            J.rng_state[pix] = rng;
+        }
+        return false;
+    }
+};
+
+// Registers capped at 64 (1024 threads per SM): shading holds more than
+// traversal does.
+template <int KIND, bool kNee>
+__global__ void __launch_bounds__(256, SOLRT_PATH_MINB) k_paths(const __grid_constant__ PathArgs a) {
+    PathIO<KIND, kNee> io(a);
+    TraceCounters cnt{0, 0, 0};
+    uint32_t ef = 0;
+    extend_kind<KIND, false>(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
+    if constexpr (kNee) {
+        const TraceCounters sc{0u, 0u, io.get(kWShadow)};
+        cnt.fallbacks -= sc.fallbacks;
+        flush_traversal(a.stats + 1, sc, 0u, false);
+        const uint32_t ws = __reduce_add_sync(0xffffffffu, io.get(kWShadowSegs));
+        const uint32_t wu = __reduce_add_sync(0xffffffffu, io.get(kWShadowSegs + 1));
+        if ((threadIdx.x & 31) == 0) {
+            if (ws) atomicAdd(&a.stats[1].segments, (unsigned long long)ws);
+            if (wu) atomicAdd(&a.stats[1].unoccluded, (unsigned long long)wu);
+        }
+    }
+    flush_traversal(a.stats, cnt, ef, false);
+    const uint32_t wsegs = __reduce_add_sync(0xffffffffu, io.get(kWSegs));
+    if ((threadIdx.x & 31) == 0 && wsegs) atomicAdd(&a.stats->segments, (unsigned long long)wsegs);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(&a.stats->paths, (unsigned long long)a.item.npix * a.item.k);
+    release_work(a.work);
+}
+
+template <int KIND, bool kNee>
+solrt_status launch_paths_kind(Context& ctx, PathArgs a) {
+    LaunchShape s;
+    SOLRT_TRY((launch_shape<KIND, k_paths<KIND, kNee>>(ctx, path_words<KIND, kNee>(), a.units, s, 32)));
+    a.slots = s.slots;
+    k_paths<KIND, kNee><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
+    ++ctx.launches;
+    SOLRT_CUDA(cudaGetLastError());
+    return SOLRT_OK;
+}
+
+template <bool kNee>
+solrt_status launch_paths_any(Context& ctx, uint32_t kind, const PathArgs& a) {
+    switch (kind) {
+        case SOLRT_BVH8_Q8: return launch_paths_kind<SOLRT_BVH8_Q8, kNee>(ctx, a);
+        case SOLRT_BVH4_Q8: return launch_paths_kind<SOLRT_BVH4_Q8, kNee>(ctx, a);
+        case SOLRT_BVH8_F32: return launch_paths_kind<SOLRT_BVH8_F32, kNee>(ctx, a);
+        case SOLRT_BVH2_Q16: return launch_paths_kind<SOLRT_BVH2_Q16, kNee>(ctx, a);
+        case SOLRT_BVH2_TWO_LEVEL: return launch_paths_kind<SOLRT_BVH2_TWO_LEVEL, kNee>(ctx, a);
+        default: return launch_paths_kind<SOLRT_BVH2, kNee>(ctx, a);
+    }
+}
+
+// Queues one launch of the path kernel on the context stream (paths.cu,
+// paths_nee.cu).
+solrt_status launch_paths(Context& ctx, uint32_t kind, const PathArgs& a);
+solrt_status launch_paths_nee(Context& ctx, uint32_t kind, const PathArgs& a);
+
+}  // namespace solrt

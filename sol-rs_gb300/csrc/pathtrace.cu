@@ -23,8 +23,7 @@
 // bit.
 #include <algorithm>
 
-#include "extend.cuh"
-#include "path_ops.cuh"
+#include "paths.cuh"
 
 namespace solrt {
 
@@ -909,23 +908,78 @@ PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp
     return a;
 }
 
+// Whether a frame whose wavefront passes hold `paths` paths runs through the
+// path kernel (paths.cuh) instead. The wavefront costs two launches per bounce
+// level, each as long as its longest ray; the path kernel has none of that but
+// shades with part of a warp, so it pays while a level has few rays. Their
+// number is taken as the pass's paths times 4 (a usual path length) over the
+// bounce levels. Measured with three frames in flight on three contexts
+// (microseconds, wavefront / path kernel; a lone frame gains more, 1.3-2.8x at
+// the same sizes):
+//   Cornell box, rays per level 26k: 113 / 92 (480x270, 6 levels), 170k: 154 /
+//   182; per-pixel streams 28k: 4632 / 2611, 111k: 7598 / 7908;
+//   meshes: 207k: 566 / 511, 410k: 910 / 947; per-pixel streams 16k: 6653 /
+//   1472 (2000 triangles), 63k: 23902 / 18836 (150k), 111k: 30251 / 26188;
+//   next-event estimation (its light-tree walks hold up the other lanes): 25k:
+//   1862 / 1121, 51k: 2219 / 2300;
+//   moving scenes, whose rebuild waits for the device before every frame, so
+//   that no other frame fills the ends of the launches: 415k: 2431 / 1998
+//   with the rebuild, 830k: 2786 / 2372.
+bool path_kernel_pays(const Context& ctx, const Scene& sc, const DevJob& J, uint64_t paths) {
+    if (ctx.counters) return false;  // node and triangle counts: wavefront only
+    const uint64_t levels = J.max_bounces + 1ull;
+    const uint64_t per_level = levels > 4 ? paths * 4 / levels : paths;
+    if (J.integrator == SOLRT_INTEGRATOR_PATH_NEE) return per_level <= 32768;
+    if (sc.dynamic && sc.info.kind != SOLRT_BVH2_TWO_LEVEL) return per_level <= 917504;
+    return per_level <= (J.sc.tri_count < kSmallScene ? 90112 : 229376);
+}
+
 // One frame of one job: its samples in passes of at most the path capacity,
 // everything the kernels need in their parameters.
-solrt_status issue_frame(Context& ctx, uint32_t kind, const DevJob& J) {
+solrt_status issue_frame(Context& ctx, const Scene& sc, uint32_t kind, const DevJob& J) {
     const uint32_t np = J.width * J.height;
     const uint32_t cap = ctx.tune.pass_paths ? std::min(ctx.tune.pass_paths, ctx.capacity) : ctx.capacity;
+    const bool nee = J.integrator == SOLRT_INTEGRATOR_PATH_NEE, stream = J.rng_mode == SOLRT_RNG_REF_STREAM;
     PassArgs a{};
     a.job = J;
     a.nitems = 1;
     a.bounces = J.max_bounces + 1u;
     for (uint32_t p0 = 0; p0 < np; p0 += std::min(cap, np - p0)) {
         const uint32_t npix = std::min(cap, np - p0);
-        const uint32_t kmax = J.rng_mode == SOLRT_RNG_REF_STREAM ? 1u : std::max(1u, std::min(J.spp, cap / npix));
+        const uint32_t kmost = std::max(1u, std::min(J.spp, cap / npix));
+        // the wavefront traces one sample of a REF_STREAM pixel per pass
+        const bool fused = path_kernel_pays(ctx, sc, J, stream ? (uint64_t)npix : (uint64_t)npix * kmost);
+        const uint32_t kmax = stream && !fused ? 1u : kmost;
         for (uint32_t s0 = 0; s0 < J.spp; s0 += std::min(kmax, J.spp - s0)) {
-            a.item = DevItem{0, p0, npix, s0, std::min(kmax, J.spp - s0), 0, 0, 0};
+            a.item = DevItem{0, p0, npix, s0, std::min(kmax, J.spp - s0), 0, 0};
             a.paths = npix * a.item.k;
             a.pixels = npix;
-            SOLRT_TRY(issue_pass(ctx, kind, a, true, J.integrator == SOLRT_INTEGRATOR_PATH_NEE, true, true));
+            if (!fused) {
+                SOLRT_TRY(issue_pass(ctx, kind, a, true, nee, true, true));
+                continue;
+            }
+            PathArgs pa{};
+            pa.job = J;
+            pa.item = a.item;
+            pa.units = stream ? npix : a.paths;
+            // fuller warps to shade where traversal is short or shading long
+            pa.refill = nee || J.sc.tri_count < kSmallScene ? 24 : kRefill;
+            pa.work = ctx.trace_work.as<unsigned int>();
+            pa.deep = ctx.deep_stack.as<int>();
+            pa.rad = ctx.rad.as<float4>();
+            pa.stats = ctx.stats.as<DevStats>();
+            const int te = ctx.timing_begin(0);
+            SOLRT_TRY(nee ? launch_paths_nee(ctx, kind, pa) : launch_paths(ctx, kind, pa));
+            ctx.timing_end(te);
+            a.rad = pa.rad;
+            a.count = a.scount = ctx.queue_counts.as<unsigned int>();
+            PassArgs r = a;
+            r.bounces = 0;
+            const int ta = ctx.timing_begin(3);
+            k_resolve<true><<<cdiv(npix, 256), 256, 0, ctx.stream>>>(r);
+            ctx.timing_end(ta);
+            ++ctx.launches;
+            SOLRT_CUDA(cudaGetLastError());
         }
     }
     return SOLRT_OK;
@@ -1094,10 +1148,8 @@ solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_
             while (p < bins.size() && bins[p].plan.paths + paths > cap) ++p;
             if (p == bins.size()) bins.push_back(Bin{PassPlan{0, 0, 0, 0, 0}, {}});
             Bin& bn = bins[p];
-            DevItem it{ch.job, ch.pix0, ch.npix, s0, std::min(ch.k, ch.spp - s0), bn.plan.paths, bn.plan.pixels,
-                       bn.plan.units};
+            DevItem it{ch.job, ch.pix0, ch.npix, s0, std::min(ch.k, ch.spp - s0), bn.plan.paths, bn.plan.pixels};
             bn.items.push_back(it);
-            bn.plan.units += item_units(it, b.jobs[it.job].rng_mode);
             bn.plan.item_count += 1;
             bn.plan.paths += (uint32_t)paths;
             bn.plan.pixels += it.npix;
@@ -1429,7 +1481,7 @@ solrt_status render_frame(Context& ctx, const Scene& sc, const solrt_camera& cam
         if (p.integrator == SOLRT_INTEGRATOR_PATH_NEE) SOLRT_TRY(ensure_shadow_queue(ctx));
         cudaGetLastError();  // launch errors below must be this call's own
         SOLRT_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
-        SOLRT_TRY(issue_frame(ctx, sc.traversal_kind(), make_job(sc, sc.traversal_kind(), img, cam, p)));
+        SOLRT_TRY(issue_frame(ctx, sc, sc.traversal_kind(), make_job(sc, sc.traversal_kind(), img, cam, p)));
         SOLRT_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
         return SOLRT_OK;
     }

@@ -283,7 +283,7 @@ void serve_loop(solrt_server* srv) {
                     if (pp.paths + np > ctx.capacity) continue;  // next tick
                     k = 1;
                 }
-                solrt::DevItem it{(uint32_t)jobs.size(), 0u, np, j.spp_done, k, pp.paths, pp.pixels, pp.units};
+                solrt::DevItem it{(uint32_t)jobs.size(), 0u, np, j.spp_done, k, pp.paths, pp.pixels};
                 const solrt::Scene& sc = *static_cast<solrt::Scene*>(j.scene);
                 const solrt::Image& img = *static_cast<solrt::Image*>(j.image);
                 jobs.push_back(solrt::job_for(sc, trav_kind, img, j.cam, j.p));
@@ -291,7 +291,6 @@ void serve_loop(solrt_server* srv) {
                 items.push_back(it);
                 pp.item_count += 1;
                 pp.paths += np * k;
-                pp.units += solrt::item_units(it, j.p.rng_mode);
                 pp.pixels += np;
                 pp.bounces = std::max(pp.bounces, j.p.max_bounces + 1u);
                 if (j.p.integrator == SOLRT_INTEGRATOR_PATH_NEE) pp.nee = 1u;

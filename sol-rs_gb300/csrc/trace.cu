@@ -18,6 +18,7 @@ struct RayFileIO {
     float4* __restrict__ hits;
     const TravScene& scene;
     int lanes;
+    static constexpr int refill = kRefill;
     static constexpr bool any_hit = false;
     SOLRT_D TravScene first_scene() const { return scene; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene&) const { load_ray(i, o, d); }

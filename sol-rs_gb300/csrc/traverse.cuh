@@ -239,6 +239,16 @@ SOLRT_D float min3(float a, float b, float c) {
 // inside the slab.
 SOLRT_D float box_dir(float v) { return fabsf(v) < 0x1p-100f ? copysignf(0x1p-100f, v) : v; }
 
+// 1 / v of a box-test direction component, to one unit in the last place: it
+// scales both plane distances of an axis alike, so its error is relative in t,
+// 2^-23 against the 2^-16 by which the far distance is widened. (An IEEE
+// division here is about ten instructions, three per ray.)
+SOLRT_D float box_rcp(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // Slab test in the form t = fma(plane, 1/d, -o/d) (one instruction per
 // plane). Its rounding error relative to |o/d| is covered by the widening of
 // every BVH2 child box by a relative 2^-21 at build time (widen_lo /
@@ -314,7 +324,7 @@ SOLRT_D void q16_ray(const float4* header, float ox, float oy, float oz, float d
                      float& sy, float& sz, float& ax, float& ay, float& az) {
     float4 g0, g1;
     ldg_2x4(header, g0, g1);
-    const float jx = 1.0f / box_dir_q16(dx), jy = 1.0f / box_dir_q16(dy), jz = 1.0f / box_dir_q16(dz);
+    const float jx = box_rcp(box_dir_q16(dx)), jy = box_rcp(box_dir_q16(dy)), jz = box_rcp(box_dir_q16(dz));
     sx = g0.w * jx;
     sy = g1.x * jy;
     sz = g1.y * jz;
@@ -364,19 +374,25 @@ struct TraceCounters {
 #define SOLRT_BVH2_STACK 64
 #endif
 
-// The queue end of the warp-organised traversal loops: once at least `refill`
-// lanes are idle, idle lanes hand in the ray they finished (IO::next, which
-// may answer with the same path's next ray) and lanes left without a path
-// take new ones from the global counter `work` (one atomic per warp; IO::load).
-// A lane that gets a ray returns true with it in (o, d). Called by all 32
-// lanes; lanes at or above `lanes` never take one.
+constexpr int kRefill = 16;
+
+// The queue end of the warp-organised traversal loops: once io.refill / 32 of
+// the lanes in play are idle (half of them, kRefill, unless the IO's next ray
+// costs so much that fuller warps pay), idle lanes hand in the ray they finished
+// (IO::next, which may answer with the same path's next ray) and lanes left
+// without a path take new ones from the global counter `work` (one atomic per
+// warp; IO::load). In play are the lanes that hold a path and, while there are
+// new ones, the first `io.lanes`. A lane that gets a ray returns true with it in
+// (o, d). Called by all 32 lanes.
 template <class IO>
 SOLRT_D bool warp_feed(IO& io, bool idle, bool& has, bool& drained, const RayMem& rm, uint32_t n, unsigned int* work,
-                       int refill, float tmin, float best_t, float4& o, float4& d, TravScene& ts,
+                       float tmin, float best_t, float4& o, float4& d, TravScene& ts,
                        const TraceCounters& cnt, uint32_t& ef) {
     const int lane = threadIdx.x & 31;
     bool fresh = false;
-    if (__popc(__ballot_sync(0xffffffffu, idle)) < refill) return false;
+    const uint32_t play = __ballot_sync(0xffffffffu, has || (!drained && lane < io.lanes));
+    const uint32_t wait = __ballot_sync(0xffffffffu, idle) & play;
+    if (wait == 0u || 32 * __popc(wait) < io.refill * __popc(play)) return false;
     if (idle && has) {
         fresh = io.next(rm.get(kRayIdx), tmin, rm.hit(best_t), o, d, cnt, ef);
         has = fresh;

@@ -1,0 +1,108 @@
+"""Frames with few rays per bounce level run through the one-launch path
+kernel, larger ones and all batches through the wavefront's launches: the
+images and ray counts of a render must equal those of a batch of that one
+job, for every BVH kind and mode and on both sides of the rule's sizes."""
+import numpy as np
+import pytest
+
+from helpers import S
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ["BVH2", "BVH8_Q8", "BVH4_Q8", "BVH8_F32", "BVH2_Q16", "BVH2_TWO_LEVEL"]
+MODES = {
+    "lambert": dict(material_mode="MATERIAL_LAMBERT", rng_mode="RNG_PER_SAMPLE", max_bounces=5),
+    "stream": dict(material_mode="MATERIAL_REF", rng_mode="RNG_REF_STREAM", max_bounces=9),
+    "kahan": dict(material_mode="MATERIAL_REF", rng_mode="RNG_PER_SAMPLE", max_bounces=3, accum_mode="ACCUM_KAHAN"),
+    "kahan_stream": dict(material_mode="MATERIAL_REF", rng_mode="RNG_REF_STREAM", max_bounces=4,
+                         accum_mode="ACCUM_KAHAN"),
+    "one_ray": dict(material_mode="MATERIAL_LAMBERT", rng_mode="RNG_PER_SAMPLE", max_bounces=0),
+    "nee": dict(material_mode="MATERIAL_LAMBERT", rng_mode="RNG_PER_SAMPLE", max_bounces=5,
+                integrator="INTEGRATOR_PATH_NEE"),
+    "nee_stream": dict(material_mode="MATERIAL_LAMBERT", rng_mode="RNG_REF_STREAM", max_bounces=4,
+                       integrator="INTEGRATOR_PATH_NEE"),
+}
+
+
+def _both(solrt, ctx, sc, data, w, h, spp, mode, frames=2):
+    kw = {k: getattr(solrt, v) if isinstance(v, str) else v for k, v in MODES[mode].items()}
+    c = data.camera
+    cam = solrt.camera_look_at(c["eye"], c["center"], c["up"], c["vfov"], w / h)
+    out = []
+    for batch in (False, True):
+        img = solrt.Image(ctx, w, h, kw.get("accum_mode", solrt.ACCUM_REF_MIX))
+        ctx.reset_stats()
+        for f in range(frames):
+            p = solrt.render_params(w, h, spp=spp, frame=f, seed=5, miss_mode=solrt.MISS_GRADIENT, **kw)
+            if batch:
+                b = solrt.Batch(ctx, [(sc, img, cam, p)])
+                b.launch()
+                ctx.synchronize()
+                b.close()
+            else:
+                solrt.Renderer(ctx).cmd_trace_rays(sc, cam, p, img)
+        ctx.synchronize()
+        st = ctx.stats()
+        assert st.error_flags == 0
+        a, r8 = img.read()
+        out.append((a.view(np.uint32).copy(), r8.copy(), st.segments, st.paths, st.shadow_segments,
+                    st.shadow_unoccluded, st.fp64_fallbacks))
+        img.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("mode", list(MODES))
+@pytest.mark.parametrize("kind", KINDS)
+def test_render_equals_batch(solrt, ctx, kind, mode):
+    for data in (S.cornell(), S.mixed_scene(1, max_tris=1200)[0]):
+        sc = solrt.SceneDescription(ctx, data, bvh=getattr(solrt, kind))
+        for w, h, spp in ((1, 1, 1), (61, 47, 3)):
+            _both(solrt, ctx, sc, data, w, h, spp, mode)
+        sc.close()
+
+
+@pytest.mark.parametrize("mode", ["lambert", "stream", "kahan", "nee"])
+def test_render_in_several_passes(solrt, mode):
+    """A capacity below the frame's pixels, and one below its samples."""
+    data = S.cornell()
+    for cap in (1000, 3000, 7000):
+        c = solrt.Context(0, path_capacity=cap)
+        sc = solrt.SceneDescription(c, data)
+        big = solrt.Context(0, path_capacity=1 << 16)
+        scb = solrt.SceneDescription(big, data)
+        imgs = []
+        for cx, s in ((c, sc), (big, scb)):
+            kw = {k: getattr(solrt, v) if isinstance(v, str) else v for k, v in MODES[mode].items()}
+            cam = solrt.camera_look_at(*(data.camera[k] for k in ("eye", "center", "up", "vfov")), 1.0)
+            img = solrt.Image(cx, 50, 50, kw.get("accum_mode", solrt.ACCUM_REF_MIX))
+            p = solrt.render_params(50, 50, spp=5, seed=3, **kw)
+            solrt.Renderer(cx).cmd_trace_rays(s, cam, p, img)
+            cx.synchronize()
+            imgs.append(img.read()[0].view(np.uint32).copy())
+            img.close()
+            s.close()
+            cx.close()
+        assert np.array_equal(*imgs)
+
+
+@pytest.mark.parametrize("w,h,spp,mode,tris", [
+    (300, 300, 1, "kahan", 0), (301, 301, 1, "kahan", 0),               # 90,000 and 90,601 rays per level
+    (479, 478, 1, "kahan", 3000), (479, 479, 1, "kahan", 3000),         # 228,962 and 229,441
+    (221, 222, 1, "nee", 3000), (222, 222, 1, "nee", 3000),             # 32,708 and 32,856
+    (412, 491, 2, "stream", 0),                                         # 80,916 of 202,292 pixels
+])
+def test_both_sides_of_the_rule(solrt, ctx, w, h, spp, mode, tris):
+    data = S.mixed_scene(2, min_tris=tris, max_tris=tris + 1)[0] if tris else S.cornell()
+    sc = solrt.SceneDescription(ctx, data)
+    _both(solrt, ctx, sc, data, w, h, spp, mode, frames=1)
+    sc.close()
+
+
+def test_moving_scene(solrt, ctx):
+    """The larger limit of dynamic scenes: 230,400 rays per level."""
+    data = S.soup(2000, seed=3, sigma=0.03)
+    sc = solrt.SceneDescription(ctx, data, dynamic=True)
+    sc.tlas_regenerate()
+    _both(solrt, ctx, sc, data, 480, 480, 1, "kahan", frames=1)
+    sc.close()
