@@ -352,16 +352,18 @@ solrt_status solrt_context_create(const solrt_context_desc* desc, solrt_context*
     }
     CHECK_ARG(d.device >= 0 && d.device < ndev, "device ordinal out of range");
     SOLRT_CUDA(cudaSetDevice(d.device));
-    cudaDeviceProp prop;
-    SOLRT_CUDA(cudaGetDeviceProperties(&prop, d.device));
-    if (prop.major * 10 + prop.minor != 103) {
-        set_error("solrt is built for sm_103a (GB300); device %d is sm_%d%d", d.device, prop.major, prop.minor);
+    int major = 0, minor = 0, sms = 0;
+    SOLRT_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, d.device));
+    SOLRT_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, d.device));
+    SOLRT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device));
+    if (major * 10 + minor != 103) {
+        set_error("solrt is built for sm_103a (GB300); device %d is sm_%d%d", d.device, major, minor);
         return SOLRT_ERR_DEVICE;
     }
     solrt_context* c = new (std::nothrow) solrt_context();
     if (!c) return SOLRT_ERR_OOM;
     c->device = d.device;
-    c->sm_count = prop.multiProcessorCount;
+    c->sm_count = sms;
     c->capacity = d.path_capacity ? d.path_capacity : (32u << 20);
     c->counters = d.enable_counters != 0;
     c->block_size = d.block_size;
@@ -403,9 +405,9 @@ solrt_status solrt_context_create(const solrt_context_desc* desc, solrt_context*
     if ((s = c->deep_stack.alloc(sizeof(int) * (SOLRT_BVH2_STACK + 1 - kMinStackSlots) * (size_t)c->sm_count *
                                  kMaxThreadsPerSm)) != SOLRT_OK)
         return fail(s);
-    if (cudaMemset(c->trace_work.ptr, 0, 2 * sizeof(unsigned int)) != cudaSuccess ||
-        cudaMemset(c->queue_counts.ptr, 0, c->queue_counts.bytes) != cudaSuccess ||
-        cudaMemset(c->stats.ptr, 0, 2 * sizeof(DevStats)) != cudaSuccess ||
+    if (cudaMemsetAsync(c->trace_work.ptr, 0, 2 * sizeof(unsigned int), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->queue_counts.ptr, 0, c->queue_counts.bytes, c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->stats.ptr, 0, 2 * sizeof(DevStats), c->stream) != cudaSuccess ||
         cudaDeviceSynchronize() != cudaSuccess) {
         set_error("device initialisation failed");
         return fail(SOLRT_ERR_DEVICE);

@@ -130,8 +130,9 @@ SOLRT_D void extend_bvh2_2l_ww(IO& io, uint32_t n, unsigned int* work, const Sta
                 leaf = 0;
                 continue;
             }
-#pragma unroll
-            for (int u = 0; u < SOLRT_BVH2_NODE_STEPS; ++u) {
+            constexpr int kUnroll = IO::kNodeUnroll;
+#pragma unroll kUnroll
+            for (int u = 0; u < IO::kNodeSteps; ++u) {
                 if (u > 0 && (uint32_t)node >= cnt_nodes) break;
                 if (kCount) ++cnt.nodes;
                 float t0, t1;

@@ -4,7 +4,7 @@
 // (full-warp votes decide the phases), so lanes re-converge at each step:
 //   refill  lanes whose ray has finished take new rays from the global queue
 //           (one atomic per warp), once enough lanes are free (warp_feed);
-//   nodes   lanes visit inner nodes, up to SOLRT_BVH2_NODE_STEPS between two
+//   nodes   lanes visit inner nodes, up to IO::kNodeSteps between two
 //           votes, until every lane has parked a leaf or has no inner node
 //           left, or until fewer than SOLRT_WW_NODE_MIN lanes still have
 //           inner nodes while others hold leaves; a lane that
@@ -28,14 +28,22 @@ constexpr int kBvh2Sentinel = 0x7fffffff;
 #ifndef SOLRT_WW_NODE_MIN
 #define SOLRT_WW_NODE_MIN 12
 #endif
-// Inner nodes a lane may visit between two votes of its warp. The votes and
-// the phase tests are about a quarter of a step's instructions; 4.2M incoherent
-// rays through a 1M-triangle tree (32-byte nodes): 1 step 2.47 ms, 2 steps
-// 2.26, 3 steps 2.20, 4 steps 2.20; a 64-spp soup frame 121.4 / 117.7 / 116.2 ms
-// with 2 / 3 / 4.
-#ifndef SOLRT_BVH2_NODE_STEPS
-#define SOLRT_BVH2_NODE_STEPS 4
-#endif
+// Inner nodes a lane may visit between two votes of its warp (IO::kNodeSteps,
+// unrolled IO::kNodeUnroll times). The votes and the phase tests are about a
+// quarter of a step's instructions: 4.2M incoherent rays through a 1M-triangle
+// tree (32-byte nodes) take 2.47 / 2.26 / 2.20 / 2.20 ms with 1 / 2 / 3 / 4 steps,
+// a 64-spp soup frame 121.4 / 117.7 / 116.2 ms with 2 / 3 / 4. Kernels that shade
+// between traversals roll the loop: unrolled, the two no longer fit the
+// instruction cache together (640x360 Cornell frame with per-pixel streams
+// 2.62 ms unrolled, 2.31 as a loop of 8 steps; next-event estimation in a
+// tunnel 1105 / 907 us).
+struct UnrolledSteps {
+    static constexpr int kNodeSteps = 4, kNodeUnroll = 4;
+};
+struct RolledSteps {
+    static constexpr int kNodeSteps = 8, kNodeUnroll = 1;
+};
+
 // A thread's traversal-stack memory: entry k at shared address base + k *
 // stride for k < slots (stride = 4 x threads per block, so lanes at different
 // depths hit different banks), the rest at deep[k * deep_stride] in global
@@ -174,8 +182,9 @@ SOLRT_D void extend_bvh2_ww(IO& io, uint32_t n, unsigned int* work, const StackM
                 leaf = 0;
                 continue;
             }
-#pragma unroll
-            for (int u = 0; u < SOLRT_BVH2_NODE_STEPS; ++u) {
+            constexpr int kUnroll = IO::kNodeUnroll;
+#pragma unroll kUnroll
+            for (int u = 0; u < IO::kNodeSteps; ++u) {
                 if (u > 0 && (unsigned)node >= ts.node_count) break;
                 if (kCount) ++cnt.nodes;
                 float t0, t1;
@@ -270,6 +279,38 @@ SOLRT_D void trace_bvh2_ray(const TravScene& ts, float ox, float oy, float oz, f
             cnt.fallbacks += intersect_tri(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best);
         }
         node = stack[--sp];
+    }
+}
+
+// The queue loop for small scenes: every lane of a warp traces its ray to the
+// end with trace_bvh2_ray, then all of them go on together (warp_feed). A ray
+// visits a dozen nodes there and the lanes differ little, so votes and parked
+// leaves cost more than they save.
+template <class IO>
+SOLRT_D void extend_bvh2_plain(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
+                               uint32_t& ef) {
+    const RayMem rm = mem.ray_mem();
+    const TravScene scene = io.first_scene();
+    bool has = false, drained = false;
+    float tmin = 0.0f, best_t = 0.0f;
+    for (;;) {
+        float4 o, d;
+        TravScene ts = scene;
+        const bool fresh = warp_feed(io, true, has, drained, rm, n, work, tmin, best_t, o, d, ts, cnt, ef);
+        if (!__any_sync(0xffffffffu, has)) {
+            if (drained) break;
+            continue;
+        }
+        if (fresh) {
+            HitRec best;
+            trace_bvh2_ray(scene, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, best, cnt, ef);
+            tmin = o.w;
+            best_t = best.t;
+            rm.put(kRayPrim, best.prim);
+            rm.putf(kRayU, best.u);
+            rm.putf(kRayV, best.v);
+        }
+        __syncwarp();
     }
 }
 

@@ -104,7 +104,7 @@ struct CoopArgs {
 // (any-hit) phases share one instantiation of the traversal loop and its
 // shared-memory stack.
 template <bool kNee>
-struct CoopIOT {
+struct CoopIOT : UnrolledSteps {
     const float4* o_tmin;
     const float4* d_tmax;
     const uint2* meta;
@@ -136,7 +136,7 @@ struct CoopIOT {
     }
 };
 template <>
-struct CoopIOT<false> {
+struct CoopIOT<false> : UnrolledSteps {
     const float4* o_tmin;
     const float4* d_tmax;
     const uint2* meta;
@@ -147,7 +147,7 @@ struct CoopIOT<false> {
     static constexpr int lanes = 32, refill = kRefill;
     SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
-        CoopIOT<true>{o_tmin, d_tmax, meta, jobs, hits, false}.load(i, o, d, ts);
+        CoopIOT<true>{{}, o_tmin, d_tmax, meta, jobs, hits, false}.load(i, o, d, ts);
     }
     SOLRT_D void load_ray(uint32_t i, float4& o, float4& d) const {
         o = __ldcg(o_tmin + i);
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kCoopBlock, (coop_min_blocks<KIND>())) k_batch
                 if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats->segments, (unsigned long long)n);
                 const PathQueue& qin = (b & 1u) ? a.q1 : a.q0;
                 const uint2 r = coop_extend<KIND, kNee>(
-                    CoopIOT<kNee>{qin.o_tmin, qin.d_tmax, qin.meta, a.jobs, a.hits, false}, n,
+                    CoopIOT<kNee>{{}, qin.o_tmin, qin.d_tmax, qin.meta, a.jobs, a.hits, false}, n,
                     count + a.ctr_stride + b, a.deep);
                 coop_flush(c, r.x, r.y);
             }
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kCoopBlock, (coop_min_blocks<KIND>())) k_batch
                     if (blockIdx.x == 0 && threadIdx.x == 0)
                         atomicAdd(&a.stats[1].segments, (unsigned long long)ns);
                     const uint2 r = coop_extend<KIND, kNee>(
-                        CoopIOT<kNee>{a.qs.o_tmin, a.qs.d_tmax, a.qs.meta, a.jobs, a.hits, true}, ns,
+                        CoopIOT<kNee>{{}, a.qs.o_tmin, a.qs.d_tmax, a.qs.meta, a.jobs, a.hits, true}, ns,
                         count + 3u * a.ctr_stride + b, a.deep);
                     if (r.x) atomicAdd(const_cast<uint32_t*>(&c.sfb), r.x);
                     if (r.y) atomicOr(const_cast<uint32_t*>(&c.ef), r.y);

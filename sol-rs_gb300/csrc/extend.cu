@@ -14,7 +14,7 @@ namespace {
 // rays in `scene`, else ray i in the scene of its job (meta[i].y >> kDepthBits),
 // or in `scene` when there is no job table.
 template <bool kSingle>
-struct QueueIO {
+struct QueueIO : UnrolledSteps {
     const float4* __restrict__ o_tmin;
     const float4* __restrict__ d_tmax;
     const uint2* __restrict__ meta;
@@ -57,7 +57,7 @@ template <int KIND, bool kSingle, bool kCount>
 __global__ void __launch_bounds__(256, kTraverseMinBlocks) k_extend(const __grid_constant__ ExtendArgs a) {
     const uint32_t n = *a.count;
     if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(&a.stats->segments, (unsigned long long)n);
-    QueueIO<kSingle> io{a.q.o_tmin, a.q.d_tmax, a.q.meta, a.jobs, a.hits, a.scene, a.lanes, a.any_hit};
+    QueueIO<kSingle> io{{}, a.q.o_tmin, a.q.d_tmax, a.q.meta, a.jobs, a.hits, a.scene, a.lanes, a.any_hit};
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
     extend_kind<KIND, kCount>(io, n, a.work, stack_mem(a.slots, a.deep), cnt, ef);

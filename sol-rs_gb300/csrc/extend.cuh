@@ -63,6 +63,23 @@ SOLRT_D void release_work(unsigned int* work) {
     }
 }
 
+// A thread's words of program state in shared memory (state_column).
+struct StateMem {
+    uint32_t base, stride;
+    SOLRT_D explicit StateMem(uint32_t slots) : base(state_column(slots)), stride(4u * blockDim.x) {}
+    SOLRT_D uint32_t get(uint32_t w) const { return lds_u32(base + w * stride); }
+    SOLRT_D void put(uint32_t w, uint32_t v) const { sts_u32(base + w * stride, v); }
+    SOLRT_D void bump(uint32_t w) const { put(w, get(w) + 1u); }
+    SOLRT_D float getf(uint32_t w) const { return __uint_as_float(get(w)); }
+    SOLRT_D void putf(uint32_t w, float v) const { put(w, __float_as_uint(v)); }
+    SOLRT_D f3 get3(uint32_t w) const { return f3{getf(w), getf(w + 1), getf(w + 2)}; }
+    SOLRT_D void put3(uint32_t w, float x, float y, float z) const {
+        putf(w, x);
+        putf(w + 1, y);
+        putf(w + 2, z);
+    }
+};
+
 SOLRT_D void flush_traversal(DevStats* stats, const TraceCounters& cnt, uint32_t ef, bool count_nodes) {
     const uint32_t fb = __reduce_add_sync(0xffffffffu, cnt.fallbacks);
     const uint32_t e = __reduce_or_sync(0xffffffffu, ef);
@@ -111,7 +128,8 @@ solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t uni
         const uint32_t most = 4u * 256u * (32u + kRayWords + state_words);
         SOLRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         SOLRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, (int)s.block, s.smem));
-        b = std::max(b, 1);
+        // (the stack memory of a context is for kMaxThreadsPerSm)
+        b = std::min(std::max(b, 1), (int)(kMaxThreadsPerSm / s.block));
         r.store(b, std::memory_order_relaxed);
     }
     const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;

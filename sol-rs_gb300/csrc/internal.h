@@ -175,7 +175,7 @@ struct TuneConfig {
 // Threads of the largest resident grid per SM, and the stack entries of each
 // kept in Context::deep_stack: those from the smallest number of shared slots
 // up.
-constexpr uint32_t kMaxThreadsPerSm = 2048;
+constexpr uint32_t kMaxThreadsPerSm = 1536;
 constexpr uint32_t kMinStackSlots = 12;
 
 // Traversal-stack entries per thread that a tuned shared-memory size keeps on
@@ -209,7 +209,6 @@ struct Context {
     // traversal-stack entries beyond the shared-memory slots (StackMem::deep)
     DeviceBuffer deep_stack;
     DeviceBuffer blue_noise;  // RGBA8 texels of SOLRT_INTEGRATOR_AO
-    DeviceBuffer sibling_job;  // one-job table of DEBUG / AO launches
     uint32_t noise_w = 0, noise_h = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint64_t launches = 0;
@@ -379,6 +378,9 @@ solrt_status launch_batch_coop(Context& ctx, uint32_t kind, const DevJob* jobs, 
 // at, each wait bounded by `seconds`; returns the error flags it raised
 // (SOLRT_EFLAG_TIMEOUT expected). Synchronises.
 solrt_status coop_wait_test(Context& ctx, double seconds, uint32_t* eflags);
+
+// siblings.cu: one launch of the DEBUG or AO integrator over J's pixels.
+solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J);
 
 // pathtrace.cu
 solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_t flags, Batch& b);

@@ -74,42 +74,31 @@ template <bool kNee> struct PathAnyHit { bool any_hit = false; };
 template <> struct PathAnyHit<false> { static constexpr bool any_hit = false; };
 
 template <int KIND, bool kNee>
-struct PathIO : PathAnyHit<kNee> {
+struct PathIO : PathAnyHit<kNee>, RolledSteps {
     const PathArgs& a;
-    uint32_t st;      // shared address of the thread's column of path state
-    uint32_t stride;  // bytes from word to word
+    const StateMem st;
     const int refill;
     static constexpr int lanes = 32;  // fewer make a lone small frame no faster and several at once slower
     static constexpr bool kOrg = kNee || KIND == SOLRT_BVH2_TWO_LEVEL;
 
-    SOLRT_D PathIO(const PathArgs& args) : a(args), st(state_column(args.slots)), stride(4u * blockDim.x), refill(args.refill) {
-        put(kWSegs, 0u);
+    SOLRT_D PathIO(const PathArgs& args) : a(args), st(args.slots), refill(args.refill) {
+        st.put(kWSegs, 0u);
         if (kNee)
-            for (int w = kWMark; w < kWNeeEnd; ++w) put(w, 0u);
-    }
-    SOLRT_D uint32_t get(uint32_t w) const { return lds_u32(st + w * stride); }
-    SOLRT_D void put(uint32_t w, uint32_t v) { sts_u32(st + w * stride, v); }
-    SOLRT_D void bump(uint32_t w) { put(w, get(w) + 1u); }
-    SOLRT_D float getf(uint32_t w) const { return __uint_as_float(get(w)); }
-    SOLRT_D f3 get3(uint32_t w) const { return f3{getf(w), getf(w + 1), getf(w + 2)}; }
-    SOLRT_D void put3(uint32_t w, float x, float y, float z) {
-        put(w, __float_as_uint(x));
-        put(w + 1, __float_as_uint(y));
-        put(w + 2, __float_as_uint(z));
+            for (int w = kWMark; w < kWNeeEnd; ++w) st.put(w, 0u);
     }
     SOLRT_D TravScene first_scene() const { return trav_scene(a.job.sc); }
 
     // The camera ray of a sample of pixel pix (rgen:47-61).
     SOLRT_D void start(uint32_t pix, uint32_t rng, uint32_t slot, float4& o, float4& d) {
         camera_ray(a.job, pix, rng, o, d);
-        put3(kWDir, d.x, d.y, d.z);
-        put3(kWThr, 1.0f, 1.0f, 1.0f);
-        put(kWRng, rng);
-        put(kWSlot, slot);
-        put(kWDepth, 0u);
-        if (kOrg) put3(kWOrg, o.x, o.y, o.z);
-        if (kNee) put3(kWSum, 0.0f, 0.0f, 0.0f);
-        bump(kWSegs);
+        st.put3(kWDir, d.x, d.y, d.z);
+        st.put3(kWThr, 1.0f, 1.0f, 1.0f);
+        st.put(kWRng, rng);
+        st.put(kWSlot, slot);
+        st.put(kWDepth, 0u);
+        if (kOrg) st.put3(kWOrg, o.x, o.y, o.z);
+        if (kNee) st.put3(kWSum, 0.0f, 0.0f, 0.0f);
+        st.bump(kWSegs);
     }
     SOLRT_D void load(uint32_t unit, float4& o, float4& d, TravScene&) {
         const DevItem& it = a.item;
@@ -120,7 +109,7 @@ struct PathIO : PathAnyHit<kNee> {
         start(pix, rng, lp * it.k + j, o, d);
     }
     SOLRT_D void load_ray(uint32_t, float4& o, float4& d) const {
-        const f3 p = get3(kWOrg), q = get3(kWDir);
+        const f3 p = st.get3(kWOrg), q = st.get3(kWDir);
         o = make_float4(p.x, p.y, p.z, 0.0f);
         d = make_float4(q.x, q.y, q.z, 0.0f);
     }
@@ -129,64 +118,64 @@ struct PathIO : PathAnyHit<kNee> {
     SOLRT_D bool next(uint32_t unit, float tmin, const HitRec& best, float4& o, float4& d, const TraceCounters& cnt,
                       uint32_t& ef) {
         const DevJob& J = a.job;
-        const f3 dir = get3(kWDir);
+        const f3 dir = st.get3(kWDir);
         f3 org{0.0f, 0.0f, 0.0f};
-        if (kOrg) org = get3(kWOrg);
+        if (kOrg) org = st.get3(kWOrg);
         if constexpr (kNee) {
-            if (this->any_hit) put(kWShadow, get(kWShadow) + cnt.fallbacks - get(kWMark));
-            put(kWMark, cnt.fallbacks);
+            if (this->any_hit) st.put(kWShadow, st.get(kWShadow) + cnt.fallbacks - st.get(kWMark));
+            st.put(kWMark, cnt.fallbacks);
             if (this->any_hit) {  // a shadow ray: its term, then the bounce ray from the same vertex
                 this->any_hit = false;
                 if (best.prim == SOLRT_NO_HIT) {
-                    const f3 c = get3(kWLight), s = get3(kWSum);
-                    put3(kWSum, s.x + c.x, s.y + c.y, s.z + c.z);
-                    bump(kWShadowSegs + 1);
+                    const f3 c = st.get3(kWLight), s = st.get3(kWSum);
+                    st.put3(kWSum, s.x + c.x, s.y + c.y, s.z + c.z);
+                    st.bump(kWShadowSegs + 1);
                 }
-                const f3 q = get3(kWNext);
-                put3(kWDir, q.x, q.y, q.z);
+                const f3 q = st.get3(kWNext);
+                st.put3(kWDir, q.x, q.y, q.z);
                 o = make_float4(org.x, org.y, org.z, tmin);
                 d = make_float4(q.x, q.y, q.z, J.tmax);
-                bump(kWSegs);
+                st.bump(kWSegs);
                 return true;
             }
         }
-        f3 acc = get3(kWThr);
-        uint32_t rng = get(kWRng), depth = get(kWDepth);
+        f3 acc = st.get3(kWThr);
+        uint32_t rng = st.get(kWRng), depth = st.get(kWDepth);
         const float4 h = make_float4(best.t, __uint_as_float(best.prim), best.u, best.v);
         const bool nee = kNee && J.integrator == SOLRT_INTEGRATOR_PATH_NEE;
         f3 n_o{0.0f, 0.0f, 0.0f};
         float4 prev = make_float4(0.0f, 0.0f, 0.0f, 0.0f), prev_out = prev;
         if (nee && depth > 0u) {
-            const f3 n = get3(kWPrev);
-            prev = make_float4(n.x, n.y, n.z, getf(kWPrev + 3));
+            const f3 n = st.get3(kWPrev);
+            prev = make_float4(n.x, n.y, n.z, st.getf(kWPrev + 3));
         }
         if (shade_step<kNee>(J, make_float4(org.x, org.y, org.z, tmin), make_float4(dir.x, dir.y, dir.z, J.tmax), h, acc,
                              rng, depth, o, d, ef, &n_o, prev, &prev_out)) {
-            put3(kWThr, acc.x, acc.y, acc.z);
-            put(kWDepth, depth);
-            if (kOrg) put3(kWOrg, o.x, o.y, o.z);
+            st.put3(kWThr, acc.x, acc.y, acc.z);
+            st.put(kWDepth, depth);
+            if (kOrg) st.put3(kWOrg, o.x, o.y, o.z);
             if constexpr (kNee) {
                 if (nee) {
-                    put3(kWPrev, prev_out.x, prev_out.y, prev_out.z);
-                    put(kWPrev + 3, __float_as_uint(prev_out.w));
+                    st.put3(kWPrev, prev_out.x, prev_out.y, prev_out.z);
+                    st.putf(kWPrev + 3, prev_out.w);
                     float4 so, sd;
                     f3 c;
                     if (nee_sample(J.sc, f3{o.x, o.y, o.z}, n_o, acc, tmin, rng, so, sd, c)) {
-                        put3(kWNext, d.x, d.y, d.z);
-                        put3(kWLight, c.x, c.y, c.z);
+                        st.put3(kWNext, d.x, d.y, d.z);
+                        st.put3(kWLight, c.x, c.y, c.z);
                         d = sd;
                         this->any_hit = true;
-                        bump(kWShadowSegs);
+                        st.bump(kWShadowSegs);
                     }
                 }
             }
-            put(kWRng, rng);
-            put3(kWDir, d.x, d.y, d.z);
-            if (!this->any_hit) bump(kWSegs);
+            st.put(kWRng, rng);
+            st.put3(kWDir, d.x, d.y, d.z);
+            if (!this->any_hit) st.bump(kWSegs);
             return true;
         }
-        if (nee) acc = get3(kWSum) + acc;  // light terms in bounce order, then the end term
-        const uint32_t slot = get(kWSlot);
+        if (nee) acc = st.get3(kWSum) + acc;  // light terms in bounce order, then the end term
+        const uint32_t slot = st.get(kWSlot);
         a.rad[slot] = make_float4(acc.x, acc.y, acc.z, 0.0f);
         if (J.rng_mode == SOLRT_RNG_REF_STREAM) {  // the pixel's next sample continues the stream
             const uint32_t pix = a.item.pix0 + unit;
@@ -202,37 +191,39 @@ struct PathIO : PathAnyHit<kNee> {
 
 // Registers capped at 64 (1024 threads per SM): shading holds more than
 // traversal does.
-template <int KIND, bool kNee>
+// kPlain: the small-scene loop (extend_bvh2_plain).
+template <int KIND, bool kNee, bool kPlain>
 __global__ void __launch_bounds__(256, SOLRT_PATH_MINB) k_paths(const __grid_constant__ PathArgs a) {
     PathIO<KIND, kNee> io(a);
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
-    extend_kind<KIND, false>(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
+    if constexpr (kPlain) extend_bvh2_plain(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
+    else extend_kind<KIND, false>(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
     if constexpr (kNee) {
-        const TraceCounters sc{0u, 0u, io.get(kWShadow)};
+        const TraceCounters sc{0u, 0u, io.st.get(kWShadow)};
         cnt.fallbacks -= sc.fallbacks;
         flush_traversal(a.stats + 1, sc, 0u, false);
-        const uint32_t ws = __reduce_add_sync(0xffffffffu, io.get(kWShadowSegs));
-        const uint32_t wu = __reduce_add_sync(0xffffffffu, io.get(kWShadowSegs + 1));
+        const uint32_t ws = __reduce_add_sync(0xffffffffu, io.st.get(kWShadowSegs));
+        const uint32_t wu = __reduce_add_sync(0xffffffffu, io.st.get(kWShadowSegs + 1));
         if ((threadIdx.x & 31) == 0) {
             if (ws) atomicAdd(&a.stats[1].segments, (unsigned long long)ws);
             if (wu) atomicAdd(&a.stats[1].unoccluded, (unsigned long long)wu);
         }
     }
     flush_traversal(a.stats, cnt, ef, false);
-    const uint32_t wsegs = __reduce_add_sync(0xffffffffu, io.get(kWSegs));
+    const uint32_t wsegs = __reduce_add_sync(0xffffffffu, io.st.get(kWSegs));
     if ((threadIdx.x & 31) == 0 && wsegs) atomicAdd(&a.stats->segments, (unsigned long long)wsegs);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(&a.stats->paths, (unsigned long long)a.item.npix * a.item.k);
     release_work(a.work);
 }
 
-template <int KIND, bool kNee>
+template <int KIND, bool kNee, bool kPlain = false>
 solrt_status launch_paths_kind(Context& ctx, PathArgs a) {
     LaunchShape s;
-    SOLRT_TRY((launch_shape<KIND, k_paths<KIND, kNee>>(ctx, path_words<KIND, kNee>(), a.units, s, 32)));
+    SOLRT_TRY((launch_shape<KIND, k_paths<KIND, kNee, kPlain>>(ctx, path_words<KIND, kNee>(), a.units, s, 32)));
     a.slots = s.slots;
-    k_paths<KIND, kNee><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
+    k_paths<KIND, kNee, kPlain><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
     ++ctx.launches;
     SOLRT_CUDA(cudaGetLastError());
     return SOLRT_OK;
@@ -246,7 +237,9 @@ solrt_status launch_paths_any(Context& ctx, uint32_t kind, const PathArgs& a) {
         case SOLRT_BVH8_F32: return launch_paths_kind<SOLRT_BVH8_F32, kNee>(ctx, a);
         case SOLRT_BVH2_Q16: return launch_paths_kind<SOLRT_BVH2_Q16, kNee>(ctx, a);
         case SOLRT_BVH2_TWO_LEVEL: return launch_paths_kind<SOLRT_BVH2_TWO_LEVEL, kNee>(ctx, a);
-        default: return launch_paths_kind<SOLRT_BVH2, kNee>(ctx, a);
+        default:
+            return a.job.sc.tri_count < kSmallScene ? launch_paths_kind<SOLRT_BVH2, kNee, true>(ctx, a)
+                                                    : launch_paths_kind<SOLRT_BVH2, kNee>(ctx, a);
     }
 }
 

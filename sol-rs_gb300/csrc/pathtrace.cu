@@ -601,144 +601,6 @@ __global__ void __launch_bounds__(128, SOLRT_MEGA_MINB)
     release_work(work);
 }
 
-// ---------------------------------------------------------------------------
-// Sibling integrators over the same traversal (one thread per pixel, the
-// structure of their ray-generation shaders).
-// ---------------------------------------------------------------------------
-
-// Primary direction of debug.rgen:20-27 / ao.rgen:56-61 for pixel position
-// (px, py): origin and direction through the inverse matrices.
-__device__ __forceinline__ void pixel_ray(const DevJob& J, float px, float py, float org[4], float dir[4]) {
-    const float ux = px / __uint2float_rn(J.width), uy = py / __uint2float_rn(J.height);
-    const float dx = ux * 2.0f - 1.0f, dy = uy * 2.0f - 1.0f;
-    float tgt[4];
-    mat4_mul(J.vinv, 0.0f, 0.0f, 0.0f, 1.0f, org);
-    mat4_mul(J.pinv, dx, dy, 1.0f, 1.0f, tgt);
-    const f3 tn = normalize(f3{tgt[0], tgt[1], tgt[2]});
-    mat4_mul(J.vinv, tn.x, tn.y, tn.z, 0.0f, dir);
-}
-
-template <int KIND>
-__device__ __forceinline__ void trace_one(const TravScene& ts, float ox, float oy, float oz, float dx, float dy,
-                                          float dz, float tmin, float tmax, HitRec& h, TraceCounters& cnt,
-                                          uint32_t& ef) {
-    if (KIND == SOLRT_BVH8_Q8) trace_bvh8<false>(ts, ox, oy, oz, dx, dy, dz, tmin, tmax, h, cnt, ef);
-    else if (KIND == SOLRT_BVH8_F32) trace_bvh8<false, true>(ts, ox, oy, oz, dx, dy, dz, tmin, tmax, h, cnt, ef);
-    else if (KIND == SOLRT_BVH4_Q8) trace_bvh4_ray(ts, ox, oy, oz, dx, dy, dz, tmin, tmax, h, cnt, ef);
-    else if (KIND == SOLRT_BVH2_Q16) trace_bvh2_ray<true>(ts, ox, oy, oz, dx, dy, dz, tmin, tmax, h, cnt, ef);
-    else if (KIND == SOLRT_BVH2_TWO_LEVEL) trace_bvh2_2l_ray(ts, ox, oy, oz, dx, dy, dz, tmin, tmax, h, cnt, ef);
-    else trace_bvh2_ray(ts, ox, oy, oz, dx, dy, dz, tmin, tmax, h, cnt, ef);
-}
-
-// debug.rgen:18-36, debug.rchit:9-13, debug.rmiss: barycentrics of the
-// primary hit through the pixel centre, else the ray direction; stored
-// without accumulation (imageStore of vec4(hitValue, 0)).
-template <int KIND>
-__global__ void __launch_bounds__(128) k_debug(const DevJob* __restrict__ job, DevStats* stats) {
-    const DevJob& J = *job;
-    const uint32_t npix = J.width * J.height;
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t segs = 0, ef = 0;
-    TraceCounters cnt{0, 0, 0};
-    if (pix < npix) {
-        const TravScene ts = trav_scene(J.sc);
-        const uint32_t x = pix % J.width, y = pix / J.width;
-        float org[4], dir[4];
-        pixel_ray(J, __uint2float_rn(x) + 0.5f, __uint2float_rn(y) + 0.5f, org, dir);
-        HitRec h;
-        trace_one<KIND>(ts, org[0], org[1], org[2], dir[0], dir[1], dir[2], 0.001f, 1000.0f, h, cnt, ef);
-        ++segs;
-        float4 v = make_float4(dir[0], dir[1], dir[2], 0.0f);
-        if (h.prim != SOLRT_NO_HIT) v = make_float4((1.0f - h.u) - h.v, h.u, h.v, 0.0f);
-        J.accum[pix] = v;
-        J.rgba8[pix] = make_uchar4(to_unorm8(v.x), to_unorm8(v.y), to_unorm8(v.z), 0);
-    }
-    flush_stats(stats, segs, pix < npix ? 1u : 0u, cnt.fallbacks, ef);
-}
-
-// ao.rgen:37-83, ao.rchit:53-88, ao.rmiss: `spp` jittered samples; each
-// follows cosine-weighted rays (directions from the blue-noise texture)
-// until a miss or max_bounces + 1 hits, counting every hit after the first.
-// Minimum resident 128-thread AO blocks per SM asked of the register
-// allocator: 8 (64 registers) against the unconstrained 96: 1083 vs 801
-// Mrays/s for the AO pipeline on the 1M-triangle soup at 1920x1080 (same
-// image), latency-bound like the megakernel.
-#ifndef SOLRT_AO_MINB
-#define SOLRT_AO_MINB 8
-#endif
-template <int KIND>
-__global__ void __launch_bounds__(128, SOLRT_AO_MINB) k_ao(const DevJob* __restrict__ job, DevStats* stats) {
-    const DevJob& J = *job;
-    const uint32_t npix = J.width * J.height;
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t segs = 0, ef = 0;
-    TraceCounters cnt{0, 0, 0};
-    if (pix < npix) {
-        const DevScene& sc = J.sc;
-        const TravScene ts = trav_scene(sc);
-        const uint32_t x = pix % J.width, y = pix / J.width;
-        uint32_t rng = tea(pix, J.frame);                                     // ao.rgen:49
-        const float max_samples = __uint2float_rn(J.max_bounces);
-        const float tw = __uint2float_rn(J.noise_w), th = __uint2float_rn(J.noise_h);
-        f3 ao{0.0f, 0.0f, 0.0f};
-        for (uint32_t i = 0; i < J.spp; ++i) {
-            const float j0 = next_rand(rng);                                  // nextRand2 (ao.rgen:53)
-            const float j1 = next_rand(rng);
-            float org[4], dir[4];
-            pixel_ray(J, __uint2float_rn(x) + j0, __uint2float_rn(y) + j1, org, dir);
-            f3 o{org[0], org[1], org[2]}, d{dir[0], dir[1], dir[2]};
-            float tmin = glsl_max(1.0f, length(o)) * 1e-3f, tmax = 10000.0f;  // preparePayload
-            float hv = 0.0f;
-            uint32_t depth = 0;
-            for (;;) {
-                HitRec h;
-                trace_one<KIND>(ts, o.x, o.y, o.z, d.x, d.y, d.z, tmin, tmax, h, cnt, ef);
-                ++segs;
-                if (h.prim == SOLRT_NO_HIT) break;                            // ao.rmiss
-                if (h.prim >= sc.tri_count) {
-                    ef |= SOLRT_EFLAG_INDEX;
-                    break;
-                }
-                const uint4 ti = __ldg(sc.tri_idx + h.prim);
-                const float b1 = h.u, b2 = h.v;
-                const float b0 = (1.0f - b1) - b2;
-                f3 normal, pos;
-                hit_frame(sc, ti, b0, b1, b2, normal, pos);                   // ao.rchit:66-75
-                const f3 no = pos + 0.00001f * d;                             // ao.rchit:78
-                // getBlueRand2(depth + depth * sampleId) (ao.rchit:43-49)
-                const uint32_t bi = depth + depth * i;
-                const float r0 = next_rand(rng);
-                const float r1 = next_rand(rng);
-                float cx = __uint2float_rn(x) + r0 * tw, cy = __uint2float_rn(y) + r1 * th;
-                cx = cx - tw * floorf(cx / tw);                               // GLSL mod
-                cy = cy - th * floorf(cy / th);
-                const int ix = min(max((int)cx, 0), (int)J.noise_w - 1);
-                const int iy = min(max((int)cy, 0), (int)J.noise_h - 1);
-                const uchar4 t = __ldg(J.noise + (size_t)iy * J.noise_w + ix);
-                const float blue[4] = {__uint2float_rn(t.x) / 255.0f, __uint2float_rn(t.y) / 255.0f,
-                                       __uint2float_rn(t.z) / 255.0f, __uint2float_rn(t.w) / 255.0f};
-                const f3 hit_n = normal * glsl_sign(dot(-d, normal));
-                d = sample_cosine(hit_n, blue[bi % 4], blue[(bi + 1) % 4]);
-                o = no;
-                tmin = 0.001f;
-                tmax = 10.0f;
-                if (depth > 0) hv = hv + 1.0f;
-                ++depth;
-                if (depth > J.max_bounces) break;                             // ao.rgen:75
-            }
-            ao = ao + (1.0f / max_samples) * f3{hv, hv, hv};                  // ao.rgen:77
-        }
-        const float n = __uint2float_rn(J.spp);
-        f3 color{1.0f - ao.x / n, 1.0f - ao.y / n, 1.0f - ao.z / n};
-        const float a = 1.0f / __uint2float_rn(J.frame - J.start + 1u);      // ao.rgen:79-82
-        const float4 old = J.accum[pix];
-        color = mix(f3{old.x, old.y, old.z}, color, a);
-        J.accum[pix] = make_float4(color.x, color.y, color.z, 1.0f);
-        J.rgba8[pix] = make_uchar4(to_unorm8(color.x), to_unorm8(color.y), to_unorm8(color.z), 255);
-    }
-    flush_stats(stats, segs, pix < npix ? J.spp : 0u, cnt.fallbacks, ef);
-}
-
 // rgen:88-103 (REF_MIX) or the Kahan mean, for every pixel of every job.
 __global__ void k_finalize(const DevJob* __restrict__ jobs, const uint32_t* __restrict__ job_pix, uint32_t njobs,
                            uint32_t pixels) {
@@ -916,12 +778,13 @@ PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp
 // bounce levels. Measured with three frames in flight on three contexts
 // (microseconds, wavefront / path kernel; a lone frame gains more, 1.3-2.8x at
 // the same sizes):
-//   Cornell box, rays per level 26k: 113 / 92 (480x270, 6 levels), 170k: 154 /
-//   182; per-pixel streams 28k: 4632 / 2611, 111k: 7598 / 7908;
+//   Cornell box, rays per level 86k: 114 / 76 (480x270), 170k: 154 / 151, 345k:
+//   236 / 273; per-pixel streams 28k: 4636 / 2074, 111k: 7614 / 6795;
+//   next-event estimation 77k: 243 / 238, 102k: 259 / 334;
 //   meshes: 207k: 566 / 511, 410k: 910 / 947; per-pixel streams 16k: 6653 /
 //   1472 (2000 triangles), 63k: 23902 / 18836 (150k), 111k: 30251 / 26188;
 //   next-event estimation (its light-tree walks hold up the other lanes): 25k:
-//   1862 / 1121, 51k: 2219 / 2300;
+//   1853 / 907, 40k: 2086 / 1393;
 //   moving scenes, whose rebuild waits for the device before every frame, so
 //   that no other frame fills the ends of the launches: 415k: 2431 / 1998
 //   with the rebuild, 830k: 2786 / 2372.
@@ -929,9 +792,10 @@ bool path_kernel_pays(const Context& ctx, const Scene& sc, const DevJob& J, uint
     if (ctx.counters) return false;  // node and triangle counts: wavefront only
     const uint64_t levels = J.max_bounces + 1ull;
     const uint64_t per_level = levels > 4 ? paths * 4 / levels : paths;
-    if (J.integrator == SOLRT_INTEGRATOR_PATH_NEE) return per_level <= 32768;
+    const bool small = J.sc.tri_count < kSmallScene;
+    if (J.integrator == SOLRT_INTEGRATOR_PATH_NEE) return per_level <= (small ? 73728 : 57344);
     if (sc.dynamic && sc.info.kind != SOLRT_BVH2_TWO_LEVEL) return per_level <= 917504;
-    return per_level <= (J.sc.tri_count < kSmallScene ? 90112 : 229376);
+    return per_level <= (small ? 180224 : 229376);
 }
 
 // One frame of one job: its samples in passes of at most the path capacity,
@@ -1434,40 +1298,18 @@ solrt_status ensure_shadow_queue(Context& ctx) {
     return SOLRT_OK;
 }
 
-// DEBUG / AO: one per-pixel launch over a one-job table.
+// DEBUG / AO: one launch over the frame's pixels.
 static solrt_status render_sibling(Context& ctx, const Scene& sc, const solrt_camera& cam,
                                    const solrt_render_params& p, Image& img) {
     SOLRT_TRY(check_params(ctx, sc, img, p));
-    const uint32_t kind = sc.info.kind;
+    const uint32_t kind = sc.traversal_kind();
     DevJob J = make_job(sc, kind, img, cam, p);
-    J.integrator = p.integrator;
     J.noise = ctx.blue_noise.as<uchar4>();
     J.noise_w = ctx.noise_w;
     J.noise_h = ctx.noise_h;
-    cudaGetLastError();
-    SOLRT_TRY(ctx.sibling_job.alloc(sizeof(DevJob)));
-    SOLRT_CUDA(cudaMemcpyAsync(ctx.sibling_job.ptr, &J, sizeof(DevJob), cudaMemcpyHostToDevice, ctx.stream));
-    const uint32_t npix = p.width * p.height;
-    const DevJob* dj = ctx.sibling_job.as<DevJob>();
-    DevStats* stats = ctx.stats.as<DevStats>();
+    cudaGetLastError();  // launch errors below must be this call's own
     SOLRT_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
-    if (p.integrator == SOLRT_INTEGRATOR_DEBUG) {
-        if (kind == SOLRT_BVH8_Q8) k_debug<SOLRT_BVH8_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH4_Q8) k_debug<SOLRT_BVH4_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH8_F32) k_debug<SOLRT_BVH8_F32><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH2_Q16) k_debug<SOLRT_BVH2_Q16><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH2_TWO_LEVEL) k_debug<SOLRT_BVH2_TWO_LEVEL><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else k_debug<SOLRT_BVH2><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-    } else {
-        if (kind == SOLRT_BVH8_Q8) k_ao<SOLRT_BVH8_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH4_Q8) k_ao<SOLRT_BVH4_Q8><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH8_F32) k_ao<SOLRT_BVH8_F32><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH2_Q16) k_ao<SOLRT_BVH2_Q16><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else if (kind == SOLRT_BVH2_TWO_LEVEL) k_ao<SOLRT_BVH2_TWO_LEVEL><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-        else k_ao<SOLRT_BVH2><<<cdiv(npix, 128), 128, 0, ctx.stream>>>(dj, stats);
-    }
-    ++ctx.launches;
-    SOLRT_CUDA(cudaGetLastError());
+    SOLRT_TRY(launch_sibling(ctx, kind, J));
     SOLRT_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
     return SOLRT_OK;
 }

@@ -13,7 +13,7 @@ namespace solrt {
 namespace {
 
 // AoS solrt_ray (2 float4) -> solrt_hit (float4), one scene.
-struct RayFileIO {
+struct RayFileIO : UnrolledSteps {
     const float4* __restrict__ rays;
     float4* __restrict__ hits;
     const TravScene& scene;
@@ -45,7 +45,7 @@ struct TraceArgs {
 
 template <int KIND, bool kCount>
 __global__ void __launch_bounds__(256, kTraverseMinBlocks) k_trace(const __grid_constant__ TraceArgs a) {
-    RayFileIO io{a.rays, a.hits, a.scene, a.lanes};
+    RayFileIO io{{}, a.rays, a.hits, a.scene, a.lanes};
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
     extend_kind<KIND, kCount>(io, a.n, a.work, stack_mem(a.slots, a.deep), cnt, ef);

@@ -87,9 +87,10 @@ def test_render_in_several_passes(solrt, mode):
 
 
 @pytest.mark.parametrize("w,h,spp,mode,tris", [
-    (300, 300, 1, "kahan", 0), (301, 301, 1, "kahan", 0),               # 90,000 and 90,601 rays per level
+    (424, 425, 1, "kahan", 0), (425, 425, 1, "kahan", 0),               # 180,200 and 180,625 rays per level
     (479, 478, 1, "kahan", 3000), (479, 479, 1, "kahan", 3000),         # 228,962 and 229,441
-    (221, 222, 1, "nee", 3000), (222, 222, 1, "nee", 3000),             # 32,708 and 32,856
+    (293, 293, 1, "nee", 3000), (294, 293, 1, "nee", 3000),             # 57,232 and 57,428
+    (332, 333, 1, "nee", 0), (333, 333, 1, "nee", 0),                   # 73,704 and 73,926
     (412, 491, 2, "stream", 0),                                         # 80,916 of 202,292 pixels
 ])
 def test_both_sides_of_the_rule(solrt, ctx, w, h, spp, mode, tris):
