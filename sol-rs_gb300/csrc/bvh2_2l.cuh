@@ -82,9 +82,7 @@ SOLRT_D void extend_bvh2_2l_ww(IO& io, uint32_t n, unsigned int* work, const Sta
             const uint32_t b_act = __ballot_sync(0xffffffffu, act);
             const uint32_t b_leaf = __ballot_sync(0xffffffffu, leaf < 0);
             if ((b_act & ~b_leaf) == 0u) break;
-#if SOLRT_WW_NODE_MIN > 0
-            if (__popc(b_act) < SOLRT_WW_NODE_MIN && b_leaf) break;
-#endif
+            if (__popc(b_act) < IO::kNodeMin && b_leaf) break;
             if (!act) continue;
             if (--budget == 0u) {
                 ef |= SOLRT_EFLAG_INDEX;

@@ -6,7 +6,7 @@
 //           (one atomic per warp), once enough lanes are free (warp_feed);
 //   nodes   lanes visit inner nodes, up to IO::kNodeSteps between two
 //           votes, until every lane has parked a leaf or has no inner node
-//           left, or until fewer than SOLRT_WW_NODE_MIN lanes still have
+//           left, or until fewer than IO::kNodeMin lanes still have
 //           inner nodes while others hold leaves; a lane that
 //           already parked a leaf keeps descending until it reaches a second
 //           one ("while-while" with speculative traversal, after Aila &
@@ -22,12 +22,6 @@
 namespace solrt {
 
 constexpr int kBvh2Sentinel = 0x7fffffff;
-// The node phase ends early when fewer than this many lanes have inner
-// nodes to visit and some lane holds a leaf (0 = only when no lane without
-// a parked leaf has inner nodes left).
-#ifndef SOLRT_WW_NODE_MIN
-#define SOLRT_WW_NODE_MIN 12
-#endif
 // Inner nodes a lane may visit between two votes of its warp (IO::kNodeSteps,
 // unrolled IO::kNodeUnroll times). The votes and the phase tests are about a
 // quarter of a step's instructions: 4.2M incoherent rays through a 1M-triangle
@@ -37,12 +31,24 @@ constexpr int kBvh2Sentinel = 0x7fffffff;
 // instruction cache together (640x360 Cornell frame with per-pixel streams
 // 2.62 ms unrolled, 2.31 as a loop of 8 steps; next-event estimation in a
 // tunnel 1105 / 907 us).
-struct UnrolledSteps {
-    static constexpr int kNodeSteps = 4, kNodeUnroll = 4;
+//
+// kNodeMin (kWideMin: the 8-wide kinds): the node phase ends early when fewer
+// lanes have inner nodes to visit and some lane holds a leaf. refill: see
+// warp_feed; a lane that only fetches its next ray should not wait long for
+// it, one that shades in between should have company. 4.2M incoherent rays /
+// a soup frame (16 spp) / a batch of 24 jobs: refill 16, kNodeMin 12 2160 us /
+// 30.5 ms / 6.61 ms, 8 and 12 2075 / 30.1 / 6.48, 8 and 18 2023 / 29.6 / 6.22,
+// 6 and 16 2013 / 29.5 / 6.27, 2 and 16 2018 / 29.8 / 6.30; the 8-wide tree on
+// a tunnel frame 67.7 ms with 16 and 12, 64.6 with 6 and 14. Shading programs:
+// an AO frame 4.66 ms with 16 and 12, 4.58 with 12 and 16.
+struct FetchLoop {
+    static constexpr int kNodeSteps = 4, kNodeUnroll = 4, kNodeMin = 18, kWideMin = 14;
+    static constexpr int refill = 6;
 };
-struct RolledSteps {
-    static constexpr int kNodeSteps = 8, kNodeUnroll = 1;
+struct ShadeLoop {
+    static constexpr int kNodeSteps = 8, kNodeUnroll = 1, kNodeMin = 16, kWideMin = 12;
 };
+constexpr int kShadeRefill = 12;
 
 // A thread's traversal-stack memory: entry k at shared address base + k *
 // stride for k < slots (stride = 4 x threads per block, so lanes at different
@@ -174,7 +180,7 @@ SOLRT_D void extend_bvh2_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             const uint32_t b_inner = __ballot_sync(0xffffffffu, inner);
             const uint32_t b_leaf = __ballot_sync(0xffffffffu, leaf < 0);
             if ((b_inner & ~b_leaf) == 0u) break;
-            if (__popc(b_inner) < SOLRT_WW_NODE_MIN && b_leaf) break;
+            if (__popc(b_inner) < IO::kNodeMin && b_leaf) break;
             if (!inner) continue;
             if (--budget == 0u) {
                 ef |= SOLRT_EFLAG_INDEX;

@@ -117,7 +117,7 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             const bool want = node != kBvh2Sentinel && tgrp.y == 0u;
             const uint32_t wb = __ballot_sync(0xffffffffu, want);
             if (wb == 0u) break;
-            if (__popc(wb) < SOLRT_WW_NODE_MIN && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
+            if (__popc(wb) < IO::kNodeMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
             if (want) {
                 if (--budget == 0u || (uint32_t)node >= ts.node_count) {
                     ef |= SOLRT_EFLAG_INDEX;

@@ -8,7 +8,7 @@
 //           (octant order), pushing the rest of the group; the node's hit
 //           internal children become the new group and its hit triangles are
 //           parked. The phase ends when no lane can step, or when fewer than
-//           SOLRT_BVH8_NODE_MIN lanes can while others hold triangles;
+//           IO::kWideMin lanes can while others hold triangles;
 //   leaves  lanes test their parked triangles, one per step.
 // The child-box tests are those of trace_bvh8 (bvh8_traverse.cuh: quantised
 // or, for SOLRT_BVH8_F32, full-precision nodes), so the closest hit equals
@@ -20,9 +20,6 @@
 
 namespace solrt {
 
-#ifndef SOLRT_BVH8_NODE_MIN
-#define SOLRT_BVH8_NODE_MIN 12
-#endif
 
 // The stack of node groups is in local memory (kept in shared memory it
 // was 1-7 % slower: the groups are 8 bytes and rarely popped).
@@ -81,7 +78,7 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             const bool want = tgrp.y == 0u && ((grp.y >> 24) != 0u || sp > 0);
             const uint32_t wb = __ballot_sync(0xffffffffu, want);
             if (wb == 0u) break;
-            if (__popc(wb) < SOLRT_BVH8_NODE_MIN && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
+            if (__popc(wb) < IO::kWideMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
             if (want) {
                 if ((grp.y >> 24) == 0u) grp = stack[--sp];
                 const uint32_t j = (uint32_t)(__ffs(grp.y >> 24) - 1);

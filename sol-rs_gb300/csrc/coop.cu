@@ -104,14 +104,14 @@ struct CoopArgs {
 // (any-hit) phases share one instantiation of the traversal loop and its
 // shared-memory stack.
 template <bool kNee>
-struct CoopIOT : UnrolledSteps {
+struct CoopIOT : FetchLoop {
     const float4* o_tmin;
     const float4* d_tmax;
     const uint2* meta;
     const DevJob* jobs;
     float4* hits;
     bool any_hit;
-    static constexpr int lanes = 32, refill = kRefill;
+    static constexpr int lanes = 32;
     SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
         o = __ldcg(o_tmin + i);
@@ -136,7 +136,7 @@ struct CoopIOT : UnrolledSteps {
     }
 };
 template <>
-struct CoopIOT<false> : UnrolledSteps {
+struct CoopIOT<false> : FetchLoop {
     const float4* o_tmin;
     const float4* d_tmax;
     const uint2* meta;
@@ -144,7 +144,7 @@ struct CoopIOT<false> : UnrolledSteps {
     float4* hits;
     bool unused;
     static constexpr bool any_hit = false;
-    static constexpr int lanes = 32, refill = kRefill;
+    static constexpr int lanes = 32;
     SOLRT_D TravScene first_scene() const { return TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {
         CoopIOT<true>{{}, o_tmin, d_tmax, meta, jobs, hits, false}.load(i, o, d, ts);

@@ -14,7 +14,7 @@ namespace {
 // rays in `scene`, else ray i in the scene of its job (meta[i].y >> kDepthBits),
 // or in `scene` when there is no job table.
 template <bool kSingle>
-struct QueueIO : UnrolledSteps {
+struct QueueIO : FetchLoop {
     const float4* __restrict__ o_tmin;
     const float4* __restrict__ d_tmax;
     const uint2* __restrict__ meta;
@@ -22,7 +22,6 @@ struct QueueIO : UnrolledSteps {
     float4* __restrict__ hits;
     const TravScene& scene;
     int lanes;
-    static constexpr int refill = kRefill;
     bool any_hit;  // occlusion queries (shadow rays): any hit in (tmin, tmax)
     SOLRT_D TravScene first_scene() const { return kSingle ? scene : TravScene{}; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene& ts) const {

@@ -74,7 +74,7 @@ template <bool kNee> struct PathAnyHit { bool any_hit = false; };
 template <> struct PathAnyHit<false> { static constexpr bool any_hit = false; };
 
 template <int KIND, bool kNee>
-struct PathIO : PathAnyHit<kNee>, RolledSteps {
+struct PathIO : PathAnyHit<kNee>, ShadeLoop {
     const PathArgs& a;
     const StateMem st;
     const int refill;

@@ -827,7 +827,7 @@ solrt_status issue_frame(Context& ctx, const Scene& sc, uint32_t kind, const Dev
             pa.item = a.item;
             pa.units = stream ? npix : a.paths;
             // fuller warps to shade where traversal is short or shading long
-            pa.refill = nee || J.sc.tri_count < kSmallScene ? 24 : kRefill;
+            pa.refill = nee || J.sc.tri_count < kSmallScene ? 24 : kShadeRefill;
             pa.work = ctx.trace_work.as<unsigned int>();
             pa.deep = ctx.deep_stack.as<int>();
             pa.rad = ctx.rad.as<float4>();

@@ -53,7 +53,7 @@ enum SiblingWord {
     kSWords = 12,
 };
 
-struct SiblingIO : RolledSteps {
+struct SiblingIO : ShadeLoop {
     const SiblingArgs& a;
     const StateMem st;
     const int refill;
@@ -274,7 +274,7 @@ solrt_status launch_kind(Context& ctx, const SiblingArgs& a) {
 }  // namespace
 
 solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J) {
-    const SiblingArgs a{J, J.width * J.height, 0, kRefill, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
+    const SiblingArgs a{J, J.width * J.height, 0, kShadeRefill, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
                         ctx.stats.as<DevStats>()};
     switch (kind) {
         case SOLRT_BVH8_Q8: return launch_kind<SOLRT_BVH8_Q8>(ctx, a);

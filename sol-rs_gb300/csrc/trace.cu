@@ -13,12 +13,11 @@ namespace solrt {
 namespace {
 
 // AoS solrt_ray (2 float4) -> solrt_hit (float4), one scene.
-struct RayFileIO : UnrolledSteps {
+struct RayFileIO : FetchLoop {
     const float4* __restrict__ rays;
     float4* __restrict__ hits;
     const TravScene& scene;
     int lanes;
-    static constexpr int refill = kRefill;
     static constexpr bool any_hit = false;
     SOLRT_D TravScene first_scene() const { return scene; }
     SOLRT_D void load(uint32_t i, float4& o, float4& d, TravScene&) const { load_ray(i, o, d); }

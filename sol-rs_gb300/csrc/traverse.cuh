@@ -374,11 +374,9 @@ struct TraceCounters {
 #define SOLRT_BVH2_STACK 64
 #endif
 
-constexpr int kRefill = 16;
 
 // The queue end of the warp-organised traversal loops: once io.refill / 32 of
-// the lanes in play are idle (half of them, kRefill, unless the IO's next ray
-// costs so much that fuller warps pay), idle lanes hand in the ray they finished
+// the lanes in play are idle, idle lanes hand in the ray they finished
 // (IO::next, which may answer with the same path's next ray) and lanes left
 // without a path take new ones from the global counter `work` (one atomic per
 // warp; IO::load). In play are the lanes that hold a path and, while there are
