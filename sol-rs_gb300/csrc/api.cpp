@@ -388,23 +388,31 @@ solrt_status solrt_context_create(const solrt_context_desc* desc, solrt_context*
         set_error("cudaEventCreate failed");
         return fail(SOLRT_ERR_DEVICE);
     }
+    // everything a context needs from the start, in one allocation
     const size_t C = c->capacity;
-    for (int i = 0; i < 2; ++i) {
-        solrt_status s;
-        if ((s = c->q_o[i].alloc(16 * C)) != SOLRT_OK) return fail(s);
-        if ((s = c->q_d[i].alloc(16 * C)) != SOLRT_OK) return fail(s);
-        if ((s = c->q_thr[i].alloc(16 * C)) != SOLRT_OK) return fail(s);
-        if ((s = c->q_meta[i].alloc(8 * C)) != SOLRT_OK) return fail(s);
+    char* at = nullptr;
+    size_t used = 0;
+    for (int round = 0; round < 2; ++round) {
+        used = 0;
+        for (int i = 0; i < 2; ++i) {
+            c->q_o[i].carve(at, used, 16 * C);
+            c->q_d[i].carve(at, used, 16 * C);
+            c->q_thr[i].carve(at, used, 16 * C);
+            c->q_meta[i].carve(at, used, 8 * C);
+        }
+        c->hits.carve(at, used, 16 * C);
+        c->rad.carve(at, used, 16 * C);
+        c->stats.carve(at, used, 2 * sizeof(DevStats));
+        c->trace_work.carve(at, used, 2 * sizeof(unsigned int));
+        c->queue_counts.carve(at, used, 2 * (SOLRT_MAX_BOUNCES + 2) * sizeof(unsigned int));
+        c->deep_stack.carve(at, used, sizeof(int) * (SOLRT_BVH2_STACK + 1 - kMinStackSlots) * (size_t)c->sm_count *
+                                          kMaxThreadsPerSm);
+        if (round == 0) {
+            const solrt_status s = c->slab.alloc(used);
+            if (s != SOLRT_OK) return fail(s);
+            at = c->slab.as<char>();
+        }
     }
-    solrt_status s;
-    if ((s = c->hits.alloc(16 * C)) != SOLRT_OK) return fail(s);
-    if ((s = c->rad.alloc(16 * C)) != SOLRT_OK) return fail(s);
-    if ((s = c->stats.alloc(2 * sizeof(DevStats))) != SOLRT_OK) return fail(s);
-    if ((s = c->trace_work.alloc(2 * sizeof(unsigned int))) != SOLRT_OK) return fail(s);
-    if ((s = c->queue_counts.alloc(2 * (SOLRT_MAX_BOUNCES + 2) * sizeof(unsigned int))) != SOLRT_OK) return fail(s);
-    if ((s = c->deep_stack.alloc(sizeof(int) * (SOLRT_BVH2_STACK + 1 - kMinStackSlots) * (size_t)c->sm_count *
-                                 kMaxThreadsPerSm)) != SOLRT_OK)
-        return fail(s);
     if (cudaMemsetAsync(c->trace_work.ptr, 0, 2 * sizeof(unsigned int), c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->queue_counts.ptr, 0, c->queue_counts.bytes, c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->stats.ptr, 0, 2 * sizeof(DevStats), c->stream) != cudaSuccess ||

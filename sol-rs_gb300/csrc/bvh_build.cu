@@ -43,6 +43,13 @@ __device__ __forceinline__ float ordered_to_float(unsigned int o) {
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
 
+// Bounds accumulators of k_centroids before its first atomic, and the words
+// that a build reads back (BuildOut).
+__global__ void k_build_init(unsigned int* __restrict__ cb, BuildOut* out) {
+    if (threadIdx.x < 6) cb[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+    if (out && threadIdx.x == 0) *out = BuildOut{0u, 0.0f};
+}
+
 // centroid = ((p0 + p1) + p2) / 3 per axis; bounds as ordered ints.
 __global__ void k_centroids(const float4* __restrict__ vpos, const uint4* __restrict__ tri_idx, uint32_t n,
                             float4* __restrict__ cen, unsigned int* __restrict__ cb) {
@@ -105,10 +112,17 @@ __device__ __forceinline__ uint32_t quantise10(float c, float lo, float ext) {
     return (uint32_t)f;
 }
 
+// Also clears what the hierarchy and refit start from: parent links and
+// arrival flags.
 __global__ void k_morton(const float4* __restrict__ cen, const unsigned int* __restrict__ cb, uint32_t n,
-                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                         uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ parent_int,
+                         unsigned int* __restrict__ flags) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i + 1 < n || n == 1) {
+        parent_int[i] = 0xffffffffu;
+        flags[i] = 0u;
+    }
     const float lo[3] = {ordered_to_float(cb[0]), ordered_to_float(cb[1]), ordered_to_float(cb[2])};
     const float hi[3] = {ordered_to_float(cb[3]), ordered_to_float(cb[4]), ordered_to_float(cb[5])};
     const float4 c = cen[i];
@@ -319,12 +333,15 @@ __device__ __forceinline__ int bvh2_ref(uint32_t r) {
 // arrive at a node computes its box from both children and continues upward.
 // Exact boxes of internal nodes go to `nbox` (lo.xyz, hi.xyz as 2 float4);
 // the child slots of each BVH2 node end up holding the children's boxes
-// widened by widen_lo / widen_hi (traverse.cuh).
+// widened by widen_lo / widen_hi (traverse.cuh). The arrival flag carries the
+// height of the subtree that arrived first, so the second arrival knows both:
+// `depth` (optional) receives the root's, the levels on the longest path.
 __global__ void k_refit(const float4* __restrict__ vpos, const uint4* __restrict__ tri_idx,
                         const uint32_t* __restrict__ order, const uint32_t* __restrict__ child,
                         const uint32_t* __restrict__ parent_int, const uint32_t* __restrict__ parent_leaf,
                         uint32_t n, unsigned int* __restrict__ flags, float4* __restrict__ nbox,
-                        float4* __restrict__ nodes, float4* __restrict__ tri_wt, uint32_t prim_base = 0) {
+                        float4* __restrict__ nodes, float4* __restrict__ tri_wt, uint32_t prim_base,
+                        unsigned int* depth) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t prim = order[k];
@@ -345,8 +362,10 @@ __global__ void k_refit(const float4* __restrict__ vpos, const uint4* __restrict
         nodes[3] = make_float4(__int_as_float(~0), __int_as_float(~0), 0.0f, 0.0f);
         nbox[0] = make_float4(lo[0], lo[1], lo[2], 0.0f);
         nbox[1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        if (depth) *depth = 1u;
         return;
     }
+    uint32_t height = 1u;
     uint32_t cur = 0x80000000u | k;
     uint32_t p = parent_leaf[k];
     for (uint32_t steps = 0; steps < n; ++steps) {
@@ -361,7 +380,9 @@ __global__ void k_refit(const float4* __restrict__ vpos, const uint4* __restrict
             reinterpret_cast<float2*>(np + 2)[1] = make_float2(lo[2], hi[2]);
         }
         __threadfence();
-        if (atomicAdd(flags + p, 1u) == 0u) return;
+        const uint32_t sibling = atomicExch(flags + p, height);
+        if (sibling == 0u) return;
+        height = max(height, sibling) + 1u;
         __threadfence();
         const float4 s0 = __ldcg(np + 0), s1 = __ldcg(np + 1), s2 = __ldcg(np + 2);
         lo[0] = fminf(s0.x, s1.x); hi[0] = fmaxf(s0.y, s1.y);
@@ -376,24 +397,13 @@ __global__ void k_refit(const float4* __restrict__ vpos, const uint4* __restrict
                             0.0f, 0.0f);
         nbox[2 * (size_t)p + 0] = make_float4(lo[0], lo[1], lo[2], 0.0f);
         nbox[2 * (size_t)p + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
-        if (p == 0) return;
+        if (p == 0) {
+            if (depth) *depth = height;
+            return;
+        }
         cur = p;
         p = parent_int[p];
     }
-}
-
-// Depth of every leaf (ancestors + 1), reduced with atomicMax.
-__global__ void k_depth(const uint32_t* __restrict__ parent_int, const uint32_t* __restrict__ parent_leaf,
-                        uint32_t n, unsigned int* __restrict__ depth) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n || n < 2) return;
-    uint32_t d = 1;
-    uint32_t p = parent_leaf[k];
-    while (p != 0 && p < n - 1 && d < n) {
-        p = parent_int[p];
-        ++d;
-    }
-    atomicMax(depth, d + 1);
 }
 
 inline uint32_t blocks_for(uint64_t n, uint32_t b) { return (uint32_t)((n + b - 1) / b); }
@@ -432,40 +442,38 @@ solrt_status check_wide_depth(uint32_t width, uint32_t depth) {
 //
 // wide: an axis that does not fit such a grid (not finite, or too large) gets
 // one that covers every coordinate below 2^115, so that the nodes stay
-// conservative; without it the ok flag is cleared.
-__global__ void k_q16_grid(const float4* __restrict__ nbox, float4* __restrict__ header, bool wide,
-                           float* __restrict__ quality) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    if (quality) *quality = 0.0f;
+// conservative; without it the grid is refused (false).
+__device__ bool q16_grid(const float4* nbox, bool wide, float g[3], float c[3]) {
     const float4 blo = nbox[0], bhi = nbox[1];
     const float lo[3] = {blo.x, blo.y, blo.z}, hi[3] = {bhi.x, bhi.y, bhi.z};
-    float g[3], c[3];
-    uint32_t ok = 1u;
+    bool ok = true;
     for (int a = 0; a < 3; ++a) {
         const bool fits = isfinite(lo[a]) && isfinite(hi[a]) && lo[a] <= hi[a];
-        if (!fits) {
-            ok = 0u;
+        int e = 0;
+        if (fits) {
+            const double ext = (double)hi[a] - (double)lo[a];
+            const double m = fmax(fabs((double)lo[a]), fabs((double)hi[a]));
+            const double need = fmax(fmax(ext / 60000.0, m * 0x1p-20), 0x1p-60);
+            e = ilogb(need);
+            if (ldexp(1.0, e) < need) ++e;
+        }
+        if (!fits || e > 23) ok = false;
+        if (!fits || (e > 23 && wide)) {
             g[a] = wide ? -0x1p115f : 0.0f;
             c[a] = wide ? 0x1p100f : 1.0f;
             continue;
-        }
-        const double ext = (double)hi[a] - (double)lo[a];
-        const double m = fmax(fabs((double)lo[a]), fabs((double)hi[a]));
-        const double need = fmax(fmax(ext / 60000.0, m * 0x1p-20), 0x1p-60);
-        int e = ilogb(need);
-        if (ldexp(1.0, e) < need) ++e;
-        if (e > 23) {
-            ok = 0u;
-            if (wide) {
-                g[a] = -0x1p115f;
-                c[a] = 0x1p100f;
-                continue;
-            }
         }
         const double cd = ldexp(1.0, e);
         c[a] = (float)cd;
         g[a] = (float)(floor((double)lo[a] / cd) * cd - 4.0 * cd);
     }
+    return ok;
+}
+
+__global__ void k_q16_grid(const float4* __restrict__ nbox, float4* __restrict__ header) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    float g[3], c[3];
+    const uint32_t ok = q16_grid(nbox, false, g, c) ? 1u : 0u;
     header[0] = make_float4(g[0], g[1], g[2], c[0]);
     header[1] = make_float4(c[1], c[2], __uint_as_float(ok), 0.0f);
 }
@@ -505,15 +513,23 @@ __device__ __forceinline__ float q16_growth(float lx, float hx, float ly, float 
     return r >= 1.0f ? fminf(r, 16.0f) : (r < 1.0f ? 1.0f : 16.0f);
 }
 
-// The traversal's 32-byte copy of BVH2 nodes; `quality` receives the sum of
-// every child's growth.
-__global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nodes, uint32_t ni,
-                                                  float4* __restrict__ out, float* __restrict__ quality) {
+// The traversal's 32-byte copy of BVH2 nodes and its header (the grid of the
+// root box nbox[0..1]); `growth` receives the sum of every child's.
+__global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nodes, const float4* __restrict__ nbox,
+                                                  uint32_t ni, float4* __restrict__ out, float* __restrict__ growth) {
+    __shared__ float s_g[3], s_c[3];
+    if (threadIdx.x == 0) {
+        const bool ok = q16_grid(nbox, true, s_g, s_c);
+        if (blockIdx.x == 0) {
+            out[0] = make_float4(s_g[0], s_g[1], s_g[2], s_c[0]);
+            out[1] = make_float4(s_c[1], s_c[2], __uint_as_float(ok ? 1u : 0u), 0.0f);
+        }
+    }
+    __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float grow = 0.0f;
     if (i < ni) {
-        const float4 h0 = out[0], h1 = out[1];
-        const float g[3] = {h0.x, h0.y, h0.z}, c[3] = {h0.w, h1.x, h1.y};
+        const float g[3] = {s_g[0], s_g[1], s_g[2]}, c[3] = {s_c[0], s_c[1], s_c[2]};
         const float4 n0 = nodes[4 * (size_t)i], n1 = nodes[4 * (size_t)i + 1], n2 = nodes[4 * (size_t)i + 2],
                      n3 = nodes[4 * (size_t)i + 3];
         const uint32_t x0 = q16_pair_f32(n0.x, n0.y, g[0], c[0]), y0 = q16_pair_f32(n0.z, n0.w, g[1], c[1]),
@@ -533,7 +549,7 @@ __global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nod
     if (threadIdx.x == 0) {
         float t = 0.0f;
         for (int w = 0; w < 8; ++w) t += s_grow[w];
-        atomicAdd(quality, t);
+        atomicAdd(growth, t);
     }
 }
 
@@ -559,7 +575,7 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
     cudaStream_t st = ctx.stream;
     DeviceBuffer q;
     SOLRT_TRY(q.alloc(32ull * ((size_t)ni + 1)));
-    k_q16_grid<<<1, 32, 0, st>>>(nbox, q.as<float4>(), false, nullptr);
+    k_q16_grid<<<1, 32, 0, st>>>(nbox, q.as<float4>());
     k_q16_nodes<<<blocks_for(ni, 256), 256, 0, st>>>(nodes.as<float4>(), ni, q.as<float4>());
     ctx.launches += 2;
     SOLRT_CUDA(cudaGetLastError());
@@ -586,25 +602,31 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
 //   (1.61) 3.19 / 3.30, 61 times (4.2) 3.9 / 7.1.
 // So: from kSmallScene triangles on, up to a mean growth of 1.18. The mean is over the
 // children, not weighted by area, so that a small detailed object in a large
-// scene counts. `nbox` holds the exact internal-node boxes (root first).
-// Synchronises.
+// scene counts. `nbox` holds the exact internal-node boxes (root first); the
+// growth goes to `out` (which must start at 0), read by finish_nodes_q16.
 constexpr float kQ16MaxGrowth = 1.18f;
-solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox) {
+solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox, BuildOut* out) {
     sc.use_qnodes = false;
     if (sc.tri_count < kSmallScene) return SOLRT_OK;
-    cudaStream_t st = ctx.stream;
     const uint32_t ni = sc.info.node_count;
     SOLRT_TRY(sc.qnodes.alloc(32ull * ((size_t)ni + 1)));
-    SOLRT_TRY(ctx.build_word.alloc(sizeof(float)));
-    float* quality = ctx.build_word.as<float>();
-    k_q16_grid<<<1, 32, 0, st>>>(nbox, sc.qnodes.as<float4>(), true, quality);
-    k_q16_copy<<<blocks_for(ni, 256), 256, 0, st>>>(sc.nodes.as<float4>(), ni, sc.qnodes.as<float4>(), quality);
-    ctx.launches += 2;
+    k_q16_copy<<<blocks_for(ni, 256), 256, 0, ctx.stream>>>(sc.nodes.as<float4>(), nbox, ni, sc.qnodes.as<float4>(),
+                                                           &out->growth);
+    ++ctx.launches;
     SOLRT_CUDA(cudaGetLastError());
-    float sum = 0.0f;
-    SOLRT_CUDA(cudaMemcpyAsync(&sum, quality, sizeof(sum), cudaMemcpyDeviceToHost, st));
-    SOLRT_CUDA(cudaStreamSynchronize(st));
-    sc.use_qnodes = sum <= kQ16MaxGrowth * 2.0f * (float)ni;
+    return SOLRT_OK;
+}
+
+void finish_nodes_q16(Scene& sc, const BuildOut& out) {
+    sc.use_qnodes = sc.info.kind == SOLRT_BVH2 && sc.tri_count >= kSmallScene &&
+                    out.growth <= kQ16MaxGrowth * 2.0f * (float)sc.info.node_count;
+}
+
+// The words that the builds of a context write, copied to the host.
+// Synchronises.
+solrt_status read_build_out(Context& ctx, const BuildOut* dev, BuildOut* host, uint32_t n = 1) {
+    SOLRT_CUDA(cudaMemcpyAsync(host, dev, sizeof(BuildOut) * (size_t)n, cudaMemcpyDeviceToHost, ctx.stream));
+    SOLRT_CUDA(cudaStreamSynchronize(ctx.stream));
     return SOLRT_OK;
 }
 
@@ -650,78 +672,63 @@ __global__ void k_offset_refs(float4* __restrict__ nodes, uint32_t ni, uint32_t 
 // One binary LBVH over triangles tri_idx[0, n) of positions vpos: the
 // 64-byte BVH2 nodes, the triangles in leaf order (prim = prim_base + index
 // into tri_idx), and the topology and exact boxes the wide collapse and the
-// refit reuse. Synchronises (reads the depth back).
+// refit reuse. Its depth goes to out->depth (read_build_out).
 struct Lbvh {
     uint32_t n = 0, ni = 0, depth = 0;
     DeviceBuffer nodes, tri_wt, child, par_int, par_leaf, range, nbox, order;
 };
 
 static solrt_status lbvh_build(Context& ctx, const float4* vpos, const uint4* tri_idx, uint32_t n, uint32_t prim_base,
-                               Lbvh& L) {
+                               Lbvh& L, BuildOut* out) {
     cudaStream_t st = ctx.stream;
     L.n = n;
     L.ni = n > 1 ? n - 1 : 1;  // internal nodes (one for a single triangle)
     const uint32_t ni = L.ni;
-    DeviceBuffer cen, cb, keys[2], vals[2], hist, flags, depth;
-    SOLRT_TRY(cen.alloc(sizeof(float4) * (size_t)n));
-    SOLRT_TRY(cb.alloc(6 * sizeof(unsigned int)));
-    for (int i = 0; i < 2; ++i) {
-        SOLRT_TRY(keys[i].alloc(sizeof(uint32_t) * (size_t)n));
-        SOLRT_TRY(vals[i].alloc(sizeof(uint32_t) * (size_t)n));
-    }
     const uint32_t nblocks = blocks_for(n, kSortTile);
-    SOLRT_TRY(hist.alloc(sizeof(uint32_t) * 256 * (size_t)nblocks));
-    DeviceBuffer scan_sums;
-    SOLRT_TRY(scan_sums.alloc(sizeof(uint32_t) * scan_tiles(256 * nblocks)));
+    BuildSpace& w = ctx.build;
+    SOLRT_TRY(w.cen.alloc(sizeof(float4) * (size_t)n));
+    SOLRT_TRY(w.cb.alloc(6 * sizeof(unsigned int)));
+    for (int i = 0; i < 2; ++i) SOLRT_TRY(w.keys[i].alloc(sizeof(uint32_t) * (size_t)n));
+    SOLRT_TRY(w.vals.alloc(sizeof(uint32_t) * (size_t)n));
+    SOLRT_TRY(w.hist.alloc(sizeof(uint32_t) * 256 * (size_t)nblocks));
+    SOLRT_TRY(w.scan_sums.alloc(sizeof(uint32_t) * scan_tiles(256 * nblocks)));
+    SOLRT_TRY(w.flags.alloc(sizeof(unsigned int) * (size_t)ni));
+    SOLRT_TRY(L.order.alloc(sizeof(uint32_t) * (size_t)n));
     SOLRT_TRY(L.child.alloc(sizeof(uint32_t) * 2 * (size_t)ni));
     SOLRT_TRY(L.par_int.alloc(sizeof(uint32_t) * (size_t)ni));
     SOLRT_TRY(L.par_leaf.alloc(sizeof(uint32_t) * (size_t)n));
-    SOLRT_TRY(flags.alloc(sizeof(unsigned int) * (size_t)ni));
     SOLRT_TRY(L.nbox.alloc(2 * sizeof(float4) * (size_t)ni));
-    SOLRT_TRY(depth.alloc(sizeof(unsigned int)));
     SOLRT_TRY(L.range.alloc(sizeof(uint2) * (size_t)ni));
     SOLRT_TRY(L.nodes.alloc(4 * sizeof(float4) * (size_t)ni));
     SOLRT_TRY(L.tri_wt.alloc(3 * sizeof(float4) * (size_t)n));
+    uint32_t* keys[2] = {w.keys[0].as<uint32_t>(), w.keys[1].as<uint32_t>()};
+    uint32_t* vals[2] = {L.order.as<uint32_t>(), w.vals.as<uint32_t>()};  // an even number of passes ends in `order`
 
-    const unsigned int cb_init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    SOLRT_CUDA(cudaMemcpyAsync(cb.ptr, cb_init, sizeof(cb_init), cudaMemcpyHostToDevice, st));
-    SOLRT_CUDA(cudaMemsetAsync(flags.ptr, 0, flags.bytes, st));
-    SOLRT_CUDA(cudaMemsetAsync(depth.ptr, 0, depth.bytes, st));
-    SOLRT_CUDA(cudaMemsetAsync(L.par_int.ptr, 0xff, L.par_int.bytes, st));
-
-    k_centroids<<<blocks_for(n, 256), 256, 0, st>>>(vpos, tri_idx, n, cen.as<float4>(), cb.as<unsigned int>());
-    k_morton<<<blocks_for(n, 256), 256, 0, st>>>(cen.as<float4>(), cb.as<unsigned int>(), n, keys[0].as<uint32_t>(),
-                                                 vals[0].as<uint32_t>());
+    k_build_init<<<1, 32, 0, st>>>(w.cb.as<unsigned int>(), out);
+    k_centroids<<<blocks_for(n, 256), 256, 0, st>>>(vpos, tri_idx, n, w.cen.as<float4>(), w.cb.as<unsigned int>());
+    k_morton<<<blocks_for(n, 256), 256, 0, st>>>(w.cen.as<float4>(), w.cb.as<unsigned int>(), n, keys[0], vals[0],
+                                                 L.par_int.as<uint32_t>(), w.flags.as<unsigned int>());
     int cur = 0;
     for (int shift = 0; shift < 30; shift += 8) {
-        k_radix_hist<<<nblocks, kSortThreads, 0, st>>>(keys[cur].as<uint32_t>(), n, shift, nblocks,
-                                                       hist.as<uint32_t>());
-        scan_exclusive_tiled(hist.as<uint32_t>(), 256 * nblocks, scan_sums.as<uint32_t>(), st);
-        k_radix_scatter<<<nblocks, kSortThreads, 0, st>>>(keys[cur].as<uint32_t>(), vals[cur].as<uint32_t>(),
-                                                          keys[cur ^ 1].as<uint32_t>(), vals[cur ^ 1].as<uint32_t>(),
-                                                          hist.as<uint32_t>(), n, shift, nblocks);
+        k_radix_hist<<<nblocks, kSortThreads, 0, st>>>(keys[cur], n, shift, nblocks, w.hist.as<uint32_t>());
+        scan_exclusive_tiled(w.hist.as<uint32_t>(), 256 * nblocks, w.scan_sums.as<uint32_t>(), st);
+        k_radix_scatter<<<nblocks, kSortThreads, 0, st>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1],
+                                                          w.hist.as<uint32_t>(), n, shift, nblocks);
         cur ^= 1;
         ctx.launches += 3;
     }
     if (n > 1) {
-        k_karras<<<blocks_for(n - 1, 256), 256, 0, st>>>(keys[cur].as<uint32_t>(), n, L.child.as<uint32_t>(),
+        k_karras<<<blocks_for(n - 1, 256), 256, 0, st>>>(keys[cur], n, L.child.as<uint32_t>(),
                                                          L.par_int.as<uint32_t>(), L.par_leaf.as<uint32_t>(),
                                                          L.range.as<uint2>());
         ++ctx.launches;
     }
-    k_refit<<<blocks_for(n, 256), 256, 0, st>>>(vpos, tri_idx, vals[cur].as<uint32_t>(), L.child.as<uint32_t>(),
+    k_refit<<<blocks_for(n, 256), 256, 0, st>>>(vpos, tri_idx, L.order.as<uint32_t>(), L.child.as<uint32_t>(),
                                                 L.par_int.as<uint32_t>(), L.par_leaf.as<uint32_t>(), n,
-                                                flags.as<unsigned int>(), L.nbox.as<float4>(), L.nodes.as<float4>(),
-                                                L.tri_wt.as<float4>(), prim_base);
-    k_depth<<<blocks_for(n, 256), 256, 0, st>>>(L.par_int.as<uint32_t>(), L.par_leaf.as<uint32_t>(), n,
-                                                depth.as<unsigned int>());
-    ctx.launches += 5;
+                                                w.flags.as<unsigned int>(), L.nbox.as<float4>(), L.nodes.as<float4>(),
+                                                L.tri_wt.as<float4>(), prim_base, &out->depth);
+    ctx.launches += 4;
     SOLRT_CUDA(cudaGetLastError());
-    L.order.adopt(vals[cur]);
-    unsigned int dh = 0;
-    SOLRT_CUDA(cudaMemcpyAsync(&dh, depth.ptr, sizeof(dh), cudaMemcpyDeviceToHost, st));
-    SOLRT_CUDA(cudaStreamSynchronize(st));
-    L.depth = n > 1 ? dh : 1;
     return SOLRT_OK;
 }
 
@@ -885,6 +892,7 @@ struct TreeletInput {
     const uint4* tri_idx;
     uint32_t prim_base;
     Lbvh* L;
+    BuildOut* out;
 };
 static solrt_status treelet_restructure(Context& ctx, const std::vector<TreeletInput>& in, int rounds);
 constexpr int kTreeletRoundsTwoLevel = 3;
@@ -908,12 +916,15 @@ static solrt_status build_two_level(Context& ctx, Scene& sc) {
     // together, one k_treelet launch per round
     std::unique_ptr<Lbvh[]> Ls(new (std::nothrow) Lbvh[S]);
     if (!Ls) return SOLRT_ERR_OOM;
+    SOLRT_TRY(ctx.build.out.alloc(sizeof(BuildOut) * std::max<size_t>(S, 1)));
+    BuildOut* out = ctx.build.out.as<BuildOut>();
     std::vector<TreeletInput> tin;
     for (uint32_t s = 0; s < S; ++s) {
         const uint32_t cnt = sc.sec_tri_count[s], first = sc.sec_tri_first[s];
         if (cnt == 0) continue;
-        SOLRT_TRY(lbvh_build(ctx, sc.opos.as<float4>(), sc.tri_idx.as<uint4>() + first, cnt, first, Ls[s]));
-        tin.push_back(TreeletInput{sc.opos.as<float4>(), sc.tri_idx.as<uint4>() + first, first, &Ls[s]});
+        SOLRT_TRY(lbvh_build(ctx, sc.opos.as<float4>(), sc.tri_idx.as<uint4>() + first, cnt, first, Ls[s],
+                             out + s));
+        tin.push_back(TreeletInput{sc.opos.as<float4>(), sc.tri_idx.as<uint4>() + first, first, &Ls[s], out + s});
     }
     if (sc.desc.flags & SOLRT_BVH_SAH) SOLRT_TRY(treelet_restructure(ctx, tin, kTreeletRoundsTwoLevel));
     std::vector<float4> boxes(2 * (size_t)S);
@@ -934,9 +945,11 @@ static solrt_status build_two_level(Context& ctx, Scene& sc) {
                                    cudaMemcpyDeviceToHost, st));
         sc.blas_root[s] = (int32_t)node_off;
         node_off += L.ni;
-        sc.blas_depth = std::max(sc.blas_depth, L.depth);
     }
-    SOLRT_CUDA(cudaStreamSynchronize(st));
+    std::vector<BuildOut> outs(S);
+    if (S) SOLRT_TRY(read_build_out(ctx, out, outs.data(), S));
+    for (uint32_t s = 0; s < S; ++s)
+        if (sc.sec_tri_count[s]) sc.blas_depth = std::max(sc.blas_depth, outs[s].depth);
     for (uint32_t s = 0; s < S; ++s) {
         if (sc.sec_tri_count[s] == 0) continue;
         const float4 lo = boxes[2 * (size_t)s], hi = boxes[2 * (size_t)s + 1];
@@ -1215,8 +1228,8 @@ __global__ void __launch_bounds__(32 * kTreeletWarps) k_treelet(const TreeletTre
 }  // namespace
 
 // Restructures the binary LBVHs of `in` in place (rounds of k_treelet, each
-// one launch over all of them), then writes each one's nodes again (k_refit)
-// and its depth. Synchronises.
+// one launch over all of them), then writes each one's nodes and depth again
+// (k_refit). Synchronises (the tree table is uploaded from the stack).
 static solrt_status treelet_restructure(Context& ctx, const std::vector<TreeletInput>& in, int rounds) {
     cudaStream_t st = ctx.stream;
     std::vector<TreeletTree> trees;
@@ -1234,10 +1247,9 @@ static solrt_status treelet_restructure(Context& ctx, const std::vector<TreeletI
     }
     if (trees.empty()) return SOLRT_OK;
     const uint32_t nt = (uint32_t)trees.size();
-    DeviceBuffer flags, cost, depth, table;
+    DeviceBuffer flags, cost, table;
     SOLRT_TRY(flags.alloc(sizeof(unsigned int) * total));
     SOLRT_TRY(cost.alloc(sizeof(float) * total));
-    SOLRT_TRY(depth.alloc(sizeof(unsigned int) * (size_t)nt));
     SOLRT_TRY(table.alloc(sizeof(TreeletTree) * (size_t)nt));
     for (uint32_t i = 0; i < nt; ++i) {
         trees[i].flags = flags.as<unsigned int>() + off[i];
@@ -1250,7 +1262,6 @@ static solrt_status treelet_restructure(Context& ctx, const std::vector<TreeletI
         ++ctx.launches;
     }
     SOLRT_CUDA(cudaMemsetAsync(flags.ptr, 0, flags.bytes, st));
-    SOLRT_CUDA(cudaMemsetAsync(depth.ptr, 0, depth.bytes, st));
     uint32_t i = 0;
     for (const TreeletInput& t : in) {
         Lbvh& L = *t.L;
@@ -1258,33 +1269,43 @@ static solrt_status treelet_restructure(Context& ctx, const std::vector<TreeletI
         k_refit<<<blocks_for(L.n, 256), 256, 0, st>>>(t.vpos, t.tri_idx, L.order.as<uint32_t>(), L.child.as<uint32_t>(),
                                                       L.par_int.as<uint32_t>(), L.par_leaf.as<uint32_t>(), L.n,
                                                       flags.as<unsigned int>() + off[i], L.nbox.as<float4>(),
-                                                      L.nodes.as<float4>(), L.tri_wt.as<float4>(), t.prim_base);
-        k_depth<<<blocks_for(L.n, 256), 256, 0, st>>>(L.par_int.as<uint32_t>(), L.par_leaf.as<uint32_t>(), L.n,
-                                                      depth.as<unsigned int>() + i);
-        ctx.launches += 2;
+                                                      L.nodes.as<float4>(), L.tri_wt.as<float4>(), t.prim_base,
+                                                      &t.out->depth);
+        ++ctx.launches;
         ++i;
     }
     SOLRT_CUDA(cudaGetLastError());
-    std::vector<unsigned int> dh(nt);
-    SOLRT_CUDA(cudaMemcpyAsync(dh.data(), depth.ptr, sizeof(unsigned int) * (size_t)nt, cudaMemcpyDeviceToHost, st));
     SOLRT_CUDA(cudaStreamSynchronize(st));
-    i = 0;
-    for (const TreeletInput& t : in)
-        if (t.L->n >= 3) t.L->depth = dh[i++];
     return SOLRT_OK;
 }
 
 static solrt_status build_single_level(Context& ctx, Scene& sc, const solrt_bvh_desc& desc) {
     const uint32_t n = sc.tri_count;
+    // A rebuild writes into what the last build left: the scene's own nodes,
+    // triangles and (dynamic scenes) topology, and the context's workspace for
+    // the rest.
+    BuildSpace& w = ctx.build;
     Lbvh L;
-    SOLRT_TRY(lbvh_build(ctx, sc.vpos.as<float4>(), sc.tri_idx.as<uint4>(), n, 0u, L));
+    if (sc.info.kind != SOLRT_BVH2_TWO_LEVEL) {
+        L.nodes.adopt(sc.nodes);
+        L.tri_wt.adopt(sc.tri_wt);
+    }
+    L.nbox.adopt(w.nbox);
+    L.order.adopt(sc.dynamic ? sc.topo_order : w.order);
+    L.child.adopt(sc.dynamic ? sc.topo_child : w.child);
+    L.par_int.adopt(sc.dynamic ? sc.topo_par_int : w.par_int);
+    L.par_leaf.adopt(sc.dynamic ? sc.topo_par_leaf : w.par_leaf);
+    L.range.adopt(sc.dynamic ? sc.topo_range : w.range);
+    SOLRT_TRY(w.out.alloc(sizeof(BuildOut)));
+    BuildOut* out = w.out.as<BuildOut>();
+    SOLRT_TRY(lbvh_build(ctx, sc.vpos.as<float4>(), sc.tri_idx.as<uint4>(), n, 0u, L, out));
     // Treelets for the binary kinds, and for the wide kinds when every leaf
     // slot holds one triangle: their collapse then reads a node's leaf range
     // only as "more than one triangle", which restructuring keeps true (a
     // restructured node's leaves need not be contiguous any more).
     const bool wide = desc.kind == SOLRT_BVH8_Q8 || desc.kind == SOLRT_BVH4_Q8 || desc.kind == SOLRT_BVH8_F32;
     if ((desc.flags & SOLRT_BVH_SAH) && (!wide || desc.leaf_max <= 1u))
-        SOLRT_TRY(treelet_restructure(ctx, {TreeletInput{sc.vpos.as<float4>(), sc.tri_idx.as<uint4>(), 0u, &L}},
+        SOLRT_TRY(treelet_restructure(ctx, {TreeletInput{sc.vpos.as<float4>(), sc.tri_idx.as<uint4>(), 0u, &L, out}},
                                       kTreeletRounds));
     const uint32_t ni = L.ni;
     if (desc.kind == SOLRT_BVH8_Q8 || desc.kind == SOLRT_BVH4_Q8 || desc.kind == SOLRT_BVH8_F32) {
@@ -1317,9 +1338,12 @@ static solrt_status build_single_level(Context& ctx, Scene& sc, const solrt_bvh_
             SOLRT_TRY(quantize_bvh2(ctx, sc.nodes, L.nbox.as<float4>(), ni));
             sc.info.node_bytes = 32ull * ((uint64_t)ni + 1);
         } else {
-            SOLRT_TRY(copy_nodes_q16(ctx, sc, L.nbox.as<float4>()));
+            SOLRT_TRY(copy_nodes_q16(ctx, sc, L.nbox.as<float4>(), out));
         }
-        sc.info.depth = L.depth;
+        BuildOut host{};
+        SOLRT_TRY(read_build_out(ctx, out, &host));
+        sc.info.depth = host.depth;
+        finish_nodes_q16(sc, host);
     }
     if (sc.dynamic) {  // the topology stays for solrt_scene_regenerate(REFIT)
         sc.topo_order.adopt(L.order);
@@ -1328,20 +1352,31 @@ static solrt_status build_single_level(Context& ctx, Scene& sc, const solrt_bvh_
         sc.topo_par_leaf.adopt(L.par_leaf);
         sc.topo_range.adopt(L.range);
     }
+    if (n <= kKeepBuildTris) {
+        w.nbox.adopt(L.nbox);
+        if (!sc.dynamic) {
+            w.order.adopt(L.order);
+            w.child.adopt(L.child);
+            w.par_int.adopt(L.par_int);
+            w.par_leaf.adopt(L.par_leaf);
+            w.range.adopt(L.range);
+        }
+    }
     return SOLRT_OK;
 }
 
 // Builds the LBVH of `sc` (and the wide collapse or the 16-bit quantisation
-// when asked). Scratch is allocated for the duration of the build.
-// Synchronises.
+// when asked). Synchronises.
 solrt_status build_bvh(Context& ctx, Scene& sc, const solrt_bvh_desc& desc) {
     const uint32_t n = sc.tri_count;
     cudaStream_t st = ctx.stream;
+    if (desc.kind != sc.info.kind || n == 0) {  // else the build writes into them
+        sc.nodes.release();
+        sc.tri_wt.release();
+    }
     sc.info = solrt_bvh_info{};
     sc.info.kind = desc.kind;
     sc.info.tri_count = n;
-    sc.nodes.release();
-    sc.tri_wt.release();
     sc.use_qnodes = false;
     if (desc.kind != SOLRT_BVH2) sc.qnodes.release();
     sc.desc = desc;
@@ -1351,6 +1386,7 @@ solrt_status build_bvh(Context& ctx, Scene& sc, const solrt_bvh_desc& desc) {
     SOLRT_CUDA(cudaEventRecord(ctx.ev0, st));
     if (desc.kind == SOLRT_BVH2_TWO_LEVEL) SOLRT_TRY(build_two_level(ctx, sc));
     else SOLRT_TRY(build_single_level(ctx, sc, desc));
+    if (n > kKeepBuildTris) ctx.build.release();
     sc.info.tri_bytes = sc.tri_wt.bytes;
     sc.info.shade_bytes = sc.opos.bytes + sc.vnc.bytes + sc.tri_idx.bytes + sc.materials.bytes +
                           sc.instances.bytes + sc.sec_mat.bytes;
@@ -1409,9 +1445,12 @@ solrt_status refit_bvh(Context& ctx, Scene& sc) {
     const uint32_t width = sc.info.kind == SOLRT_BVH4_Q8 ? 4u : 8u;
     const bool f32 = sc.info.kind == SOLRT_BVH8_F32;
     const bool q16 = sc.info.kind == SOLRT_BVH2_Q16;
-    DeviceBuffer flags, nbox, nodes2, tri2;
+    DeviceBuffer nodes2, tri2;
+    DeviceBuffer &flags = ctx.build.flags, &nbox = ctx.build.nbox;
     SOLRT_TRY(flags.alloc(sizeof(unsigned int) * (size_t)ni));
     SOLRT_TRY(nbox.alloc(2 * sizeof(float4) * (size_t)ni));
+    SOLRT_TRY(ctx.build.out.alloc(sizeof(BuildOut)));
+    BuildOut* out = ctx.build.out.as<BuildOut>();
     float4* nodes_out = sc.nodes.as<float4>();
     float4* tri_out = sc.tri_wt.as<float4>();
     if (b8) {
@@ -1423,11 +1462,12 @@ solrt_status refit_bvh(Context& ctx, Scene& sc) {
         SOLRT_TRY(nodes2.alloc(4 * sizeof(float4) * (size_t)ni));
         nodes_out = nodes2.as<float4>();
     }
-    SOLRT_CUDA(cudaMemsetAsync(flags.ptr, 0, flags.bytes, st));
+    SOLRT_CUDA(cudaMemsetAsync(flags.ptr, 0, sizeof(unsigned int) * (size_t)ni, st));
+    SOLRT_CUDA(cudaMemsetAsync(out, 0, sizeof(BuildOut), st));
     k_refit<<<blocks_for(n, 256), 256, 0, st>>>(sc.vpos.as<float4>(), sc.tri_idx.as<uint4>(),
                                                 sc.topo_order.as<uint32_t>(), sc.topo_child.as<uint32_t>(),
                                                 sc.topo_par_int.as<uint32_t>(), sc.topo_par_leaf.as<uint32_t>(), n,
-                                                flags.as<unsigned int>(), nbox.as<float4>(), nodes_out, tri_out);
+                                                flags.as<unsigned int>(), nbox.as<float4>(), nodes_out, tri_out, 0u, nullptr);
     ++ctx.launches;
     SOLRT_CUDA(cudaGetLastError());
     if (b8) {
@@ -1455,8 +1495,12 @@ solrt_status refit_bvh(Context& ctx, Scene& sc) {
         SOLRT_TRY(quantize_bvh2(ctx, nodes2, nbox.as<float4>(), ni));
         sc.nodes.adopt(nodes2);
     } else {
-        SOLRT_TRY(copy_nodes_q16(ctx, sc, nbox.as<float4>()));
+        SOLRT_TRY(copy_nodes_q16(ctx, sc, nbox.as<float4>(), out));
+        BuildOut host{};
+        SOLRT_TRY(read_build_out(ctx, out, &host));
+        finish_nodes_q16(sc, host);
     }
+    if (n > kKeepBuildTris) ctx.build.release();
     SOLRT_CUDA(cudaEventRecord(ctx.ev1, st));
     SOLRT_CUDA(cudaEventSynchronize(ctx.ev1));
     float ms = 0.0f;
@@ -1586,18 +1630,15 @@ extern "C" solrt_status solrt_bvh2_build_noalloc(const void* vpos, const void* t
     float4* nbox = reinterpret_cast<float4*>(s + kOffNbox);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    // The scratch keeps the previous call's contents: reset what must start
-    // at a known value (bounds accumulators, arrival flags, parent links).
-    SOLRT_CUDA(cudaMemsetAsync(cb, 0xff, 3 * sizeof(unsigned int), st));
-    SOLRT_CUDA(cudaMemsetAsync(cb + 3, 0, 3 * sizeof(unsigned int), st));
-    SOLRT_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned int) * ni, st));
-    SOLRT_CUDA(cudaMemsetAsync(par_int, 0xff, sizeof(uint32_t) * ni, st));
-
+    // The scratch keeps the previous call's contents: k_build_init and k_morton
+    // reset what must start at a known value (bounds accumulators, arrival
+    // flags, parent links).
+    k_build_init<<<1, 32, 0, st>>>(cb, nullptr);
     const float4* vp = static_cast<const float4*>(vpos);
     const uint4* ti = static_cast<const uint4*>(tri_idx);
     const uint32_t nblocks = blocks_for(n, kSortTile);
     k_centroids<<<blocks_for(n, 256), 256, 0, st>>>(vp, ti, n, cen, cb);
-    k_morton<<<blocks_for(n, 256), 256, 0, st>>>(cen, cb, n, keys[0], vals[0]);
+    k_morton<<<blocks_for(n, 256), 256, 0, st>>>(cen, cb, n, keys[0], vals[0], par_int, flags);
     int cur = 0;
     for (int shift = 0; shift < 30; shift += 8) {
         k_radix_hist<<<nblocks, kSortThreads, 0, st>>>(keys[cur], n, shift, nblocks, hist);
@@ -1608,7 +1649,7 @@ extern "C" solrt_status solrt_bvh2_build_noalloc(const void* vpos, const void* t
     }
     if (n > 1) k_karras<<<blocks_for(n - 1, 256), 256, 0, st>>>(keys[cur], n, child, par_int, par_leaf, nullptr);
     k_refit<<<blocks_for(n, 256), 256, 0, st>>>(vp, ti, vals[cur], child, par_int, par_leaf, n, flags, nbox,
-                                                static_cast<float4*>(nodes), static_cast<float4*>(tris));
+                                                static_cast<float4*>(nodes), static_cast<float4*>(tris), 0u, nullptr);
     SOLRT_CUDA(cudaGetLastError());
     return SOLRT_OK;
 }

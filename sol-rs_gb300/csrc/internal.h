@@ -36,14 +36,27 @@ void set_error(const char* fmt, ...);
 struct DeviceBuffer {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool borrowed = false;  // part of another allocation (carve), not freed here
     DeviceBuffer() = default;
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
     ~DeviceBuffer() { release(); }
     void release() {
-        if (ptr) cudaFree(ptr);
+        if (ptr && !borrowed) cudaFree(ptr);
         ptr = nullptr;
         bytes = 0;
+        borrowed = false;
+    }
+    // This buffer becomes the n bytes at at + used; `used` moves past them, to
+    // the next multiple of 256. A null `at` only counts the bytes.
+    void carve(char* at, size_t& used, size_t n) {
+        if (at) {
+            release();
+            ptr = at + used;
+            bytes = n;
+            borrowed = true;
+        }
+        used += (n + 255) & ~size_t(255);
     }
     solrt_status alloc(size_t n) {
         if (n <= bytes && ptr) return SOLRT_OK;
@@ -65,8 +78,10 @@ struct DeviceBuffer {
         release();
         ptr = o.ptr;
         bytes = o.bytes;
+        borrowed = o.borrowed;
         o.ptr = nullptr;
         o.bytes = 0;
+        o.borrowed = false;
     }
 };
 
@@ -91,6 +106,26 @@ struct PathQueue {
     float4* thr_rng;  // throughput, rng state (bits)
     uint2* meta;      // slot within the pass, job << kDepthBits | depth
     float4* prev;     // SOLRT_INTEGRATOR_PATH_NEE: normal of the vertex the ray left, pdf of its BSDF sample
+};
+
+// What a binary BVH build tells the host.
+struct BuildOut {
+    unsigned int depth;  // levels on the longest root-to-leaf path
+    float growth;        // of the child boxes in the 32-byte nodes, summed
+};
+
+// Temporary arrays of BVH builds, kept by a context from one build to the next
+// (allocating and freeing them took longer than a 262k-triangle rebuild's
+// kernels), up to builds of kKeepBuildTris triangles (about 110 bytes each).
+constexpr uint32_t kKeepBuildTris = 2u << 20;
+struct BuildSpace {
+    DeviceBuffer cen, cb, keys[2], vals, hist, scan_sums, flags, out;
+    DeviceBuffer nbox, order, child, par_int, par_leaf, range;  // for the duration of a build its Lbvh's
+    void release() {
+        for (DeviceBuffer* b : {&cen, &cb, &keys[0], &keys[1], &vals, &hist, &scan_sums, &flags, &out, &nbox, &order,
+                                &child, &par_int, &par_leaf, &range})
+            b->release();
+    }
 };
 
 // One job of a wavefront batch, as the device sees it.
@@ -196,6 +231,7 @@ struct Context {
     uint32_t capacity = 0;
     bool counters = false;
     uint32_t block_size = 0;
+    DeviceBuffer slab;  // holds the buffers that a context is created with
     // queues 0 and 1: paths of alternate bounces; queue 2: shadow rays of
     // SOLRT_INTEGRATOR_PATH_NEE (allocated when a render first needs it)
     DeviceBuffer q_o[3], q_d[3], q_thr[3], q_meta[3];
@@ -205,7 +241,7 @@ struct Context {
     // next unit and finished blocks of the persistent kernels; both 0 between
     // launches (release_work)
     DeviceBuffer trace_work;
-    DeviceBuffer build_word;  // one word that BVH builds read back
+    BuildSpace build;
     // traversal-stack entries beyond the shared-memory slots (StackMem::deep)
     DeviceBuffer deep_stack;
     DeviceBuffer blue_noise;  // RGBA8 texels of SOLRT_INTEGRATOR_AO
