@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256, kTraverseMinBlocks) k_extend(const __grid
 template <int KIND, bool kSingle, bool kCount>
 solrt_status launch_extend_variant(Context& ctx, ExtendArgs a, uint32_t most) {
     LaunchShape s;
-    SOLRT_TRY((launch_shape<KIND, k_extend<KIND, kSingle, kCount>>(ctx, 0, most, s)));
+    SOLRT_TRY((launch_shape<KIND, k_extend<KIND, kSingle, kCount>>(ctx, 0, most, true, s)));
     a.slots = s.slots;
     a.lanes = (int)s.lanes;
     k_extend<KIND, kSingle, kCount><<<s.grid, s.block, s.smem, ctx.stream>>>(a);

@@ -25,6 +25,18 @@ SOLRT_D void extend_kind(IO& io, uint32_t n, unsigned int* work, const StackMem&
     else extend_bvh8_ww<IO, kCount, false>(io, n, work, mem, cnt, ef);
 }
 
+// Closest hit of one ray with the kind's per-ray loop.
+template <int KIND>
+SOLRT_D void trace_one(const TravScene& ts, const float4& o, const float4& d, HitRec& h, TraceCounters& cnt,
+                       uint32_t& ef) {
+    if (KIND == SOLRT_BVH8_Q8) trace_bvh8<false>(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+    else if (KIND == SOLRT_BVH8_F32) trace_bvh8<false, true>(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+    else if (KIND == SOLRT_BVH4_Q8) trace_bvh4_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+    else if (KIND == SOLRT_BVH2_Q16) trace_bvh2_ray<true>(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+    else if (KIND == SOLRT_BVH2_TWO_LEVEL) trace_bvh2_2l_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+    else trace_bvh2_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+}
+
 // Shared-memory stack slots of a launch: the context's choice for the kinds
 // with a node stack, none for the 8-wide kinds (group stack in local memory).
 template <int KIND>
@@ -106,16 +118,19 @@ constexpr int kTraverseMinBlocks = 5;
 // Shape of one launch of `kern`: the context's block size and stack slots,
 // state_words words of program state per thread, a grid of (SMs x resident
 // blocks) or fewer blocks when `units` rays or paths need fewer, and how many
-// lanes of each warp take work: 32, or as few (but `least`) as spread the units
-// over all warps of a full grid when there are not enough for every lane (a
-// warp with fewer rays steps faster, and otherwise most SMs would be idle).
+// lanes of each warp take work: 32, or, for up to kSpreadUnits units with
+// `spread`, as few as spread them over all warps of a full grid. A warp with
+// fewer rays steps faster, but beyond that its idle lanes cost more than the
+// shorter steps gain (microseconds for one call, few lanes / 32: 2000 rays
+// through 20k triangles 94 / 134, 8000 117 / 143, 30k 159 / 152, 100k 214 / 194;
+// with three calls in flight 34 / 47, 43 / 47, 68 / 56, 98 / 74).
+constexpr uint32_t kSpreadUnits = 8192;
 struct LaunchShape {
     uint32_t grid = 0, block = 0, smem = 0, slots = 0, lanes = 32;
 };
 
 template <int KIND, auto kern>
-solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t units, LaunchShape& s,
-                          uint32_t least = 1) {
+solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t units, bool spread, LaunchShape& s) {
     s.block = ctx.tune.block;
     s.slots = kind_has_smem_stack<KIND>() ? stack_slots(ctx.tune.smem) : 0u;
     s.smem = 4u * s.block * (s.slots + kRayWords + state_words);
@@ -134,7 +149,7 @@ solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t uni
     }
     const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;
     const uint32_t warps = full * (s.block / 32u);
-    s.lanes = std::min(32u, std::max(least, (units + warps - 1u) / warps));
+    s.lanes = spread && units <= kSpreadUnits ? std::min(32u, std::max(1u, (units + warps - 1u) / warps)) : 32u;
     s.grid = std::min(full, (units + s.lanes * (s.block / 32u) - 1u) / (s.lanes * (s.block / 32u)));
     return SOLRT_OK;
 }

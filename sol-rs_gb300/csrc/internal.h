@@ -415,8 +415,11 @@ solrt_status launch_batch_coop(Context& ctx, uint32_t kind, const DevJob* jobs, 
 // (SOLRT_EFLAG_TIMEOUT expected). Synchronises.
 solrt_status coop_wait_test(Context& ctx, double seconds, uint32_t* eflags);
 
-// siblings.cu: one launch of the DEBUG or AO integrator over J's pixels.
-solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J);
+// siblings.cu: one launch of the DEBUG or AO integrator over J's pixels;
+// `plain` (sibling_plain; J then holds the nodes of the scene's own kind): one
+// thread per pixel.
+bool sibling_plain(const Scene& sc, const solrt_render_params& p);
+solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J, bool plain);
 
 // pathtrace.cu
 solrt_status batch_plan(Context& ctx, const solrt_job* jobs, uint32_t n, uint32_t flags, Batch& b);

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256, SOLRT_PATH_MINB) k_paths(const __grid_con
 template <int KIND, bool kNee, bool kPlain = false>
 solrt_status launch_paths_kind(Context& ctx, PathArgs a) {
     LaunchShape s;
-    SOLRT_TRY((launch_shape<KIND, k_paths<KIND, kNee, kPlain>>(ctx, path_words<KIND, kNee>(), a.units, s, 32)));
+    SOLRT_TRY((launch_shape<KIND, k_paths<KIND, kNee, kPlain>>(ctx, path_words<KIND, kNee>(), a.units, false, s)));
     a.slots = s.slots;
     k_paths<KIND, kNee, kPlain><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
     ++ctx.launches;

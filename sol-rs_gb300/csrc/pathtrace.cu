@@ -460,18 +460,6 @@ __global__ void __launch_bounds__(128, SOLRT_MEGA_MINB)
 // same estimator as the wavefront's shadow queue, one path at a time.
 // ---------------------------------------------------------------------------
 
-// Closest hit of one ray with the kind's per-ray loop.
-template <int KIND>
-SOLRT_D void trace_one(const TravScene& ts, const float4& o, const float4& d, HitRec& h, TraceCounters& cnt,
-                       uint32_t& ef) {
-    if (KIND == SOLRT_BVH8_Q8) trace_bvh8<false>(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
-    else if (KIND == SOLRT_BVH8_F32) trace_bvh8<false, true>(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
-    else if (KIND == SOLRT_BVH4_Q8) trace_bvh4_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
-    else if (KIND == SOLRT_BVH2_Q16) trace_bvh2_ray<true>(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
-    else if (KIND == SOLRT_BVH2_TWO_LEVEL) trace_bvh2_2l_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
-    else trace_bvh2_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
-}
-
 // Per-thread counts of the per-pixel NEE kernels.
 struct MegaCounts {
     uint32_t segs = 0, paths = 0, shadow = 0, unoccluded = 0, ef = 0;
@@ -1302,14 +1290,15 @@ solrt_status ensure_shadow_queue(Context& ctx) {
 static solrt_status render_sibling(Context& ctx, const Scene& sc, const solrt_camera& cam,
                                    const solrt_render_params& p, Image& img) {
     SOLRT_TRY(check_params(ctx, sc, img, p));
-    const uint32_t kind = sc.traversal_kind();
+    const bool plain = sibling_plain(sc, p);
+    const uint32_t kind = plain ? sc.info.kind : sc.traversal_kind();
     DevJob J = make_job(sc, kind, img, cam, p);
     J.noise = ctx.blue_noise.as<uchar4>();
     J.noise_w = ctx.noise_w;
     J.noise_h = ctx.noise_h;
     cudaGetLastError();  // launch errors below must be this call's own
     SOLRT_CUDA(cudaEventRecord(ctx.ev0, ctx.stream));
-    SOLRT_TRY(launch_sibling(ctx, kind, J));
+    SOLRT_TRY(launch_sibling(ctx, kind, J, plain));
     SOLRT_CUDA(cudaEventRecord(ctx.ev1, ctx.stream));
     return SOLRT_OK;
 }

@@ -5,9 +5,9 @@
 // Their shaders run one invocation per pixel. Here a persistent launch holds
 // 32 pixels per warp in the traversal loop of the BVH kind (warp_feed): lanes
 // whose ray is done shade and go on with their pixel's next ray or sample, or
-// take another pixel. A thread per pixel that follows its rays to the end,
-// which this replaced but for AO in small scenes, leaves a warp's lanes waiting
-// for its longest chain: an AO frame of a 300k-triangle soup (1280x720, 4
+// take another pixel. A thread per pixel that follows its rays to the end
+// (k_debug_plain, k_ao_plain; kept for small scenes and frames) leaves a warp's
+// lanes waiting for its longest chain: an AO frame of a 300k-triangle soup (1280x720, 4
 // samples) 7.1 -> 4.7 ms, a 1920x1080 DEBUG frame of it 597 -> 497 us.
 #include "extend.cuh"
 #include "path_ops.cuh"
@@ -19,7 +19,7 @@ namespace {
 struct SiblingArgs {
     DevJob job;
     uint32_t units, slots;
-    int refill;  // warp_feed's threshold
+    int lanes;
     unsigned int* work;
     int* deep;
     DevStats* stats;
@@ -53,13 +53,13 @@ enum SiblingWord {
     kSWords = 12,
 };
 
-struct SiblingIO : ShadeLoop {
+template <class Loop>
+struct SiblingIO : Loop {
     const SiblingArgs& a;
     const StateMem st;
-    const int refill;
-    static constexpr int lanes = 32;
+    const int lanes;
     static constexpr bool any_hit = false;
-    SOLRT_D explicit SiblingIO(const SiblingArgs& args) : a(args), st(args.slots), refill(args.refill) { st.put(kSSegs, 0u); }
+    SOLRT_D explicit SiblingIO(const SiblingArgs& args) : a(args), st(args.slots), lanes(args.lanes) { st.put(kSSegs, 0u); }
     SOLRT_D TravScene first_scene() const { return trav_scene(a.job.sc); }
     SOLRT_D void load_ray(uint32_t, float4& o, float4& d) const {
         const f3 p = st.get3(kSOrg), q = st.get3(kSDir);
@@ -76,21 +76,26 @@ struct SiblingIO : ShadeLoop {
 // debug.rgen:18-36, debug.rchit:9-13, debug.rmiss: barycentrics of the
 // primary hit through the pixel centre, else the ray direction; stored
 // without accumulation (imageStore of vec4(hitValue, 0)).
-struct DebugIO : SiblingIO {
-    using SiblingIO::SiblingIO;
+SOLRT_D void debug_ray(const DevJob& J, uint32_t pix, float4& o, float4& d) {
+    const uint32_t x = pix % J.width, y = pix / J.width;
+    pixel_ray(J, __uint2float_rn(x) + 0.5f, __uint2float_rn(y) + 0.5f, o, d);
+    o.w = 0.001f;
+    d.w = 1000.0f;
+}
+SOLRT_D void debug_write_pixel(const DevJob& J, uint32_t pix, const HitRec& h, f3 dir) {
+    float4 v = make_float4(dir.x, dir.y, dir.z, 0.0f);
+    if (h.prim != SOLRT_NO_HIT) v = make_float4((1.0f - h.u) - h.v, h.u, h.v, 0.0f);
+    J.accum[pix] = v;
+    J.rgba8[pix] = make_uchar4(to_unorm8(v.x), to_unorm8(v.y), to_unorm8(v.z), 0);
+}
+struct DebugIO : SiblingIO<FetchLoop> {
+    using SiblingIO<FetchLoop>::SiblingIO;
     SOLRT_D void load(uint32_t pix, float4& o, float4& d, TravScene&) const {
-        const uint32_t x = pix % a.job.width, y = pix / a.job.width;
-        pixel_ray(a.job, __uint2float_rn(x) + 0.5f, __uint2float_rn(y) + 0.5f, o, d);
-        o.w = 0.001f;
-        d.w = 1000.0f;
+        debug_ray(a.job, pix, o, d);
         keep_ray(o, d);
     }
     SOLRT_D bool next(uint32_t pix, float, const HitRec& h, float4&, float4&, const TraceCounters&, uint32_t&) const {
-        const f3 dir = st.get3(kSDir);
-        float4 v = make_float4(dir.x, dir.y, dir.z, 0.0f);
-        if (h.prim != SOLRT_NO_HIT) v = make_float4((1.0f - h.u) - h.v, h.u, h.v, 0.0f);
-        a.job.accum[pix] = v;
-        a.job.rgba8[pix] = make_uchar4(to_unorm8(v.x), to_unorm8(v.y), to_unorm8(v.z), 0);
+        debug_write_pixel(a.job, pix, h, st.get3(kSDir));
         return false;
     }
 };
@@ -162,8 +167,9 @@ SOLRT_D void ao_write_pixel(const DevJob& J, uint32_t pix, float sum) {
     J.rgba8[pix] = make_uchar4(to_unorm8(color.x), to_unorm8(color.y), to_unorm8(color.z), 255);
 }
 
-struct AoIO : SiblingIO {
-    using SiblingIO::SiblingIO;
+struct AoIO : SiblingIO<ShadeLoop> {
+    using SiblingIO<ShadeLoop>::SiblingIO;
+    static constexpr int refill = kShadeRefill;
     SOLRT_D void start(uint32_t pix, uint32_t sample, uint32_t rng, float4& o, float4& d) const {
         ao_camera_ray(a.job, pix, rng, o, d);
         st.put(kSRng, rng);
@@ -202,11 +208,34 @@ struct AoIO : SiblingIO {
     }
 };
 
-// AO of small scenes, one thread per pixel as in the shader: the lanes start
-// every sample together, and in scenes of a few dozen triangles that coherence
-// is worth more than full lanes (Cornell box, 1280x720, 4 samples: 1.06 ms,
-// through AoIO 1.26 ms; a 2000-triangle soup 2.56 / 2.19 ms).
-__global__ void __launch_bounds__(128, 8) k_ao_small(const __grid_constant__ SiblingArgs a) {
+// The same frames with one thread per pixel, as in the shaders: for small
+// scenes, where lanes that start every sample together are worth more than full
+// lanes (Cornell box, 1280x720, 4 samples: AO 1.06 ms, through AoIO 1.26 ms; a
+// 2000-triangle soup 2.56 / 2.19 ms), and for small frames (sibling_plain).
+SOLRT_D void flush_plain(const SiblingArgs& a, const TraceCounters& cnt, uint32_t ef, uint32_t segs, uint32_t paths) {
+    flush_traversal(a.stats, cnt, ef, false);
+    const uint32_t ws = __reduce_add_sync(0xffffffffu, segs);
+    if ((threadIdx.x & 31) == 0 && ws) atomicAdd(&a.stats->segments, (unsigned long long)ws);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats->paths, (unsigned long long)a.units * paths);
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(128) k_debug_plain(const __grid_constant__ SiblingArgs a) {
+    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t ef = 0;
+    TraceCounters cnt{0, 0, 0};
+    if (pix < a.units) {
+        float4 o, d;
+        debug_ray(a.job, pix, o, d);
+        HitRec h;
+        trace_one<KIND>(trav_scene(a.job.sc), o, d, h, cnt, ef);
+        debug_write_pixel(a.job, pix, h, f3{d.x, d.y, d.z});
+    }
+    flush_plain(a, cnt, ef, pix < a.units ? 1u : 0u, 1u);
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(128, 8) k_ao_plain(const __grid_constant__ SiblingArgs a) {
     const DevJob& J = a.job;
     const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t segs = 0, ef = 0;
@@ -221,7 +250,7 @@ __global__ void __launch_bounds__(128, 8) k_ao_small(const __grid_constant__ Sib
             float hits = 0.0f;
             for (uint32_t depth = 0; depth <= J.max_bounces; ++depth) {       // ao.rgen:75
                 HitRec h;
-                trace_bvh2_ray(ts, o.x, o.y, o.z, d.x, d.y, d.z, o.w, d.w, h, cnt, ef);
+                trace_one<KIND>(ts, o, d, h, cnt, ef);
                 ++segs;
                 if (!ao_bounce(J, pix, i, depth, h, f3{d.x, d.y, d.z}, rng, o, d, ef)) break;
                 if (depth > 0) hits = hits + 1.0f;
@@ -230,20 +259,15 @@ __global__ void __launch_bounds__(128, 8) k_ao_small(const __grid_constant__ Sib
         }
         ao_write_pixel(J, pix, sum);
     }
-    flush_traversal(a.stats, cnt, ef, false);
-    const uint32_t ws = __reduce_add_sync(0xffffffffu, segs);
-    if ((threadIdx.x & 31) == 0 && ws) atomicAdd(&a.stats->segments, (unsigned long long)ws);
-    if (pix == 0) atomicAdd(&a.stats->paths, (unsigned long long)a.units * J.spp);
+    flush_plain(a, cnt, ef, segs, J.spp);
 }
 
-// kPlain: the small-scene loop (extend_bvh2_plain).
-template <int KIND, class IO, bool kPlain>
+template <int KIND, class IO>
 __global__ void __launch_bounds__(256, 4) k_sibling(const __grid_constant__ SiblingArgs a) {
     IO io(a);
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
-    if constexpr (kPlain) extend_bvh2_plain(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
-    else extend_kind<KIND, false>(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
+    extend_kind<KIND, false>(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
     flush_traversal(a.stats, cnt, ef, false);
     const uint32_t segs = __reduce_add_sync(0xffffffffu, io.st.get(kSSegs));
     if ((threadIdx.x & 31) == 0 && segs) atomicAdd(&a.stats->segments, (unsigned long long)segs);
@@ -254,42 +278,57 @@ __global__ void __launch_bounds__(256, 4) k_sibling(const __grid_constant__ Sibl
     release_work(a.work);
 }
 
-template <int KIND, class IO, bool kPlain>
-solrt_status launch_io(Context& ctx, SiblingArgs a) {
+template <int KIND, class IO>
+solrt_status launch_io(const Context& ctx, SiblingArgs a) {
     LaunchShape s;
-    SOLRT_TRY((launch_shape<KIND, k_sibling<KIND, IO, kPlain>>(ctx, kSWords, a.units, s, 32)));
+    SOLRT_TRY((launch_shape<KIND, k_sibling<KIND, IO>>(ctx, kSWords, a.units, true, s)));
     a.slots = s.slots;
-    k_sibling<KIND, IO, kPlain><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
-    ++ctx.launches;
-    SOLRT_CUDA(cudaGetLastError());
+    a.lanes = (int)s.lanes;
+    k_sibling<KIND, IO><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
     return SOLRT_OK;
 }
 
 template <int KIND>
-solrt_status launch_kind(Context& ctx, const SiblingArgs& a) {
-    return a.job.integrator == SOLRT_INTEGRATOR_AO ? launch_io<KIND, AoIO, false>(ctx, a)
-                                                   : launch_io<KIND, DebugIO, false>(ctx, a);
+solrt_status launch_kind(const Context& ctx, const SiblingArgs& a, bool plain) {
+    const bool ao = a.job.integrator == SOLRT_INTEGRATOR_AO;
+    if (!plain) return ao ? launch_io<KIND, AoIO>(ctx, a) : launch_io<KIND, DebugIO>(ctx, a);
+    const uint32_t blocks = (a.units + 127) / 128;
+    if (ao) k_ao_plain<KIND><<<blocks, 128, 0, ctx.stream>>>(a);
+    else k_debug_plain<KIND><<<blocks, 128, 0, ctx.stream>>>(a);
+    return SOLRT_OK;
 }
 
 }  // namespace
 
-solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J) {
-    const SiblingArgs a{J, J.width * J.height, 0, kShadeRefill, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
+// One thread per pixel: small scenes (see k_ao_plain), and frames of so few
+// pixels that most of the GPU is idle anyway and the shorter steps of a plain
+// loop decide. Three frames in flight, a thread per pixel / persistent (us): AO
+// 64x48 of a 2000-triangle tube 134 / 160, 320x180 of a 300k soup 924 / 713;
+// DEBUG 640x48 of a 20k tube 17.3 / 19.8, 320x180 of the soup 65.5 / 65.6,
+// 1920x1080 597 / 497. The smallest DEBUG frames of BVH2 scenes go to the
+// persistent launch, which spreads them over all warps (launch_shape): 64x48 of
+// the soup 45.5 / 40.5, of a 2000-triangle soup 22.9 / 19.2.
+bool sibling_plain(const Scene& sc, const solrt_render_params& p) {
+    const uint64_t pixels = (uint64_t)p.width * p.height;
+    if (sc.info.kind == SOLRT_BVH2 && sc.tri_count < kSmallScene) return true;
+    if (p.integrator == SOLRT_INTEGRATOR_AO) return pixels <= 16384u;
+    return pixels <= 49152u && !(sc.info.kind == SOLRT_BVH2 && pixels <= kSpreadUnits);
+}
+
+solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J, bool plain) {
+    const SiblingArgs a{J, J.width * J.height, 0, 32, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
                         ctx.stats.as<DevStats>()};
     switch (kind) {
-        case SOLRT_BVH8_Q8: return launch_kind<SOLRT_BVH8_Q8>(ctx, a);
-        case SOLRT_BVH4_Q8: return launch_kind<SOLRT_BVH4_Q8>(ctx, a);
-        case SOLRT_BVH8_F32: return launch_kind<SOLRT_BVH8_F32>(ctx, a);
-        case SOLRT_BVH2_Q16: return launch_kind<SOLRT_BVH2_Q16>(ctx, a);
-        case SOLRT_BVH2_TWO_LEVEL: return launch_kind<SOLRT_BVH2_TWO_LEVEL>(ctx, a);
-        default:
-            if (J.sc.tri_count >= kSmallScene) return launch_kind<SOLRT_BVH2>(ctx, a);
-            if (J.integrator != SOLRT_INTEGRATOR_AO) return launch_io<SOLRT_BVH2, DebugIO, true>(ctx, a);
-            k_ao_small<<<(a.units + 127) / 128, 128, 0, ctx.stream>>>(a);
-            ++ctx.launches;
-            SOLRT_CUDA(cudaGetLastError());
-            return SOLRT_OK;
+        case SOLRT_BVH8_Q8: SOLRT_TRY(launch_kind<SOLRT_BVH8_Q8>(ctx, a, plain)); break;
+        case SOLRT_BVH4_Q8: SOLRT_TRY(launch_kind<SOLRT_BVH4_Q8>(ctx, a, plain)); break;
+        case SOLRT_BVH8_F32: SOLRT_TRY(launch_kind<SOLRT_BVH8_F32>(ctx, a, plain)); break;
+        case SOLRT_BVH2_Q16: SOLRT_TRY(launch_kind<SOLRT_BVH2_Q16>(ctx, a, plain)); break;
+        case SOLRT_BVH2_TWO_LEVEL: SOLRT_TRY(launch_kind<SOLRT_BVH2_TWO_LEVEL>(ctx, a, plain)); break;
+        default: SOLRT_TRY(launch_kind<SOLRT_BVH2>(ctx, a, plain)); break;
     }
+    ++ctx.launches;
+    SOLRT_CUDA(cudaGetLastError());
+    return SOLRT_OK;
 }
 
 }  // namespace solrt

@@ -56,8 +56,8 @@ template <int KIND>
 solrt_status launch_kind(Context& ctx, TraceArgs a) {
     auto kern = ctx.counters ? k_trace<KIND, true> : k_trace<KIND, false>;
     LaunchShape s;
-    if (ctx.counters) SOLRT_TRY((launch_shape<KIND, k_trace<KIND, true>>(ctx, 0, a.n, s)));
-    else SOLRT_TRY((launch_shape<KIND, k_trace<KIND, false>>(ctx, 0, a.n, s)));
+    if (ctx.counters) SOLRT_TRY((launch_shape<KIND, k_trace<KIND, true>>(ctx, 0, a.n, true, s)));
+    else SOLRT_TRY((launch_shape<KIND, k_trace<KIND, false>>(ctx, 0, a.n, true, s)));
     a.slots = s.slots;
     a.lanes = (int)s.lanes;
     kern<<<s.grid, s.block, s.smem, ctx.stream>>>(a);

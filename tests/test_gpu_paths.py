@@ -5,7 +5,7 @@ job, for every BVH kind and mode and on both sides of the rule's sizes."""
 import numpy as np
 import pytest
 
-from helpers import S
+from helpers import S, bvh_args, random_rays
 
 pytestmark = pytest.mark.gpu
 
@@ -106,4 +106,39 @@ def test_moving_scene(solrt, ctx):
     sc = solrt.SceneDescription(ctx, data, dynamic=True)
     sc.tlas_regenerate()
     _both(solrt, ctx, sc, data, 480, 480, 1, "kahan", frames=1)
+    sc.close()
+
+
+@pytest.mark.parametrize("integrator", ["INTEGRATOR_AO", "INTEGRATOR_DEBUG"])
+@pytest.mark.parametrize("w,h", [(128, 64), (128, 65), (128, 128), (129, 128), (256, 192), (257, 192)])
+def test_ao_and_debug_on_both_sides_of_the_pixel_limits(solrt, oracle, ctx, integrator, w, h):
+    """AO changes loops above 16,384 pixels, DEBUG above 8,192 and 49,152: both equal the
+    oracle, in a scene large enough for either loop."""
+    data = S.soup(1500, seed=6, sigma=0.04)
+    noise = np.random.default_rng(1).integers(0, 256, (64, 64, 4), dtype=np.uint8)
+    ctx.set_blue_noise(noise)
+    c = data.camera
+    cam = solrt.camera_look_at(c["eye"], c["center"], c["up"], c["vfov"], w / h)
+    p = solrt.render_params(w, h, spp=2, max_bounces=3, integrator=getattr(solrt, integrator))
+    sc = solrt.SceneDescription(ctx, data)
+    img = solrt.Image(ctx, w, h)
+    solrt.Renderer(ctx).cmd_trace_rays(sc, cam, p, img)
+    ctx.synchronize()
+    want, _, _ = oracle.OracleScene(data).render(cam, p, blue_noise=noise)
+    assert np.array_equal(img.read()[0].view(np.uint32), want.view(np.uint32))
+    img.close()
+    sc.close()
+
+
+@pytest.mark.parametrize("n", [8192, 8193])
+@pytest.mark.parametrize("bvh", ["bvh2", "bvh8", "bvh2t"])
+def test_rays_on_both_sides_of_the_spread_limit(solrt, oracle, ctx, bvh, n):
+    """Up to 8,192 rays are spread over all warps, from there on warps take 32."""
+    data = S.soup(600, seed=3, sigma=0.05)
+    args = bvh_args(solrt, bvh)
+    rays = random_rays(n, -1.0, 1.0, seed=5)
+    sc = solrt.SceneDescription(ctx, data, **args)
+    got = sc.trace_rays(rays)
+    want, _ = oracle.OracleScene(data, two_level=bvh == "bvh2t").trace(rays, brute=True)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
     sc.close()
