@@ -32,21 +32,21 @@ constexpr int kBvh2Sentinel = 0x7fffffff;
 // 2.62 ms unrolled, 2.31 as a loop of 8 steps; next-event estimation in a
 // tunnel 1105 / 907 us).
 //
-// kNodeMin (kWideMin: the 8-wide kinds): the node phase ends early when fewer
+// kNodeMin (kWideMin, kWideTriMin: the 8-wide kinds, see bvh8_ww.cuh): the node phase ends early when fewer
 // lanes have inner nodes to visit and some lane holds a leaf. refill: see
 // warp_feed; a lane that only fetches its next ray should not wait long for
 // it, one that shades in between should have company. 4.2M incoherent rays /
 // a soup frame (16 spp) / a batch of 24 jobs: refill 16, kNodeMin 12 2160 us /
 // 30.5 ms / 6.61 ms, 8 and 12 2075 / 30.1 / 6.48, 8 and 18 2023 / 29.6 / 6.22,
-// 6 and 16 2013 / 29.5 / 6.27, 2 and 16 2018 / 29.8 / 6.30; the 8-wide tree on
-// a tunnel frame 67.7 ms with 16 and 12, 64.6 with 6 and 14. Shading programs:
-// an AO frame 4.66 ms with 16 and 12, 4.58 with 12 and 16.
+// 6 and 16 2013 / 29.5 / 6.27, 2 and 16 2018 / 29.8 / 6.30. Shading programs:
+// an AO frame 4.66 ms with 16 and 12, 4.58 with 12 and 16; kWideMin 10 / 12 / 16
+// a 64x48 preview through 8-wide nodes 53.8 / 54.8 / 56.9 us.
 struct FetchLoop {
-    static constexpr int kNodeSteps = 4, kNodeUnroll = 4, kNodeMin = 18, kWideMin = 14;
+    static constexpr int kNodeSteps = 4, kNodeUnroll = 4, kNodeMin = 18, kWideMin = 16, kWideTriMin = 8;
     static constexpr int refill = 6;
 };
 struct ShadeLoop {
-    static constexpr int kNodeSteps = 8, kNodeUnroll = 1, kNodeMin = 16, kWideMin = 12;
+    static constexpr int kNodeSteps = 8, kNodeUnroll = 1, kNodeMin = 16, kWideMin = 10, kWideTriMin = 8;
 };
 constexpr int kShadeRefill = 12;
 

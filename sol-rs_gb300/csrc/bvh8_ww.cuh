@@ -3,13 +3,22 @@
 // is warp-uniform.
 //   refill  lanes whose ray has finished take new rays from the global queue
 //           once enough lanes are free (warp_feed);
-//   nodes   lanes with no parked triangles visit one 8-wide node per step:
-//           the nearest remaining internal child of their current node group
-//           (octant order), pushing the rest of the group; the node's hit
-//           internal children become the new group and its hit triangles are
-//           parked. The phase ends when no lane can step, or when fewer than
-//           IO::kWideMin lanes can while others hold triangles;
-//   leaves  lanes test their parked triangles, one per step.
+//   nodes   lanes visit one 8-wide node per step: the nearest remaining
+//           internal child of their current node group (octant order), pushing
+//           the rest of the group; the node's hit internal children become the
+//           new group and its hit triangles are parked. A lane goes on until it
+//           holds the triangles of two nodes. The phase ends when no lane can
+//           step, or when fewer than IO::kWideMin lanes can while others hold
+//           triangles;
+//   leaves  lanes test their parked triangles, one per step, until none has any
+//           left, or fewer than IO::kWideTriMin have while kWideMin lanes could
+//           step again.
+// Every other node visit finds triangles (tunnel scene: 14 nodes and 8 triangles
+// per ray), so with one parked node and leaf phases that ran to their end 13 of
+// 32 lanes were active on average. A 1366x768 tunnel frame (16 spp): 64.8 ms so,
+// 60.7 with the threshold in the leaf phase, 58.0 with a second parked node as
+// well, 55.3 at 64 registers a thread (traverse_min_blocks); 4.2M incoherent
+// rays 2.79 / 2.66 / 2.77 / 2.56 ms.
 // The child-box tests are those of trace_bvh8 (bvh8_traverse.cuh: quantised
 // or, for SOLRT_BVH8_F32, full-precision nodes), so the closest hit equals
 // that of the per-ray loop.
@@ -30,6 +39,7 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
     int sp = 0;
     uint2 grp = make_uint2(0u, 0u);   // (child base, hit bits << 24 | internal mask)
     uint2 tgrp = make_uint2(0u, 0u);  // parked triangles: (triangle base, hit bits)
+    uint2 tmore = make_uint2(0u, 0u); // those of a second node (only beside the first)
     bool has = false;
     bool drained = false;
     uint32_t budget = 0, oct = 0;
@@ -65,7 +75,7 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             budget = 2u * (ts.node_count + ts.tri_count) + 64u;
             nodes = reinterpret_cast<const uint4*>(ts.nodes);
             sp = 0;
-            tgrp = make_uint2(0u, 0u);
+            tgrp = tmore = make_uint2(0u, 0u);
             // the root as a group of one internal child in slot 0
             grp = ts.tri_count ? make_uint2(0u, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);
         }
@@ -75,7 +85,7 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
         }
         // node phase
         for (;;) {
-            const bool want = tgrp.y == 0u && ((grp.y >> 24) != 0u || sp > 0);
+            const bool want = tmore.y == 0u && ((grp.y >> 24) != 0u || sp > 0);
             const uint32_t wb = __ballot_sync(0xffffffffu, want);
             if (wb == 0u) break;
             if (__popc(wb) < IO::kWideMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
@@ -95,13 +105,12 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
                     sp = 0;
                 } else {
                     if (kCount) ++cnt.nodes;
-                    uint32_t hi = 0, ht = 0;
+                    uint32_t hi = 0, ht = 0, tbase = 0;
                     if constexpr (kF32) {
-                        uint32_t cbase = 0, tbase = 0, imask = 0;
+                        uint32_t cbase = 0, imask = 0;
                         bvh8f_node_test(ts.nodes + 14 * (size_t)node, ix, iy, iz, nox, noy, noz, oct, tmin, best_t,
                                         hi, ht, cbase, tbase, imask);
                         if (hi) grp = make_uint2(cbase, (hi << 24) | imask);
-                        tgrp = make_uint2(tbase, ht);
                     } else {
                         const uint4* np = nodes + 5 * (size_t)node;
                         const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3),
@@ -109,20 +118,30 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
                         bvh8_node_test(w0, w1, w2, w3, w4, ox, oy, oz, ix, iy, iz, negx, negy, negz, oct,
                                        tmin, best_t, hi, ht);
                         if (hi) grp = make_uint2(w1.x, (hi << 24) | (w0.w >> 24));
-                        tgrp = make_uint2(w1.y, ht);
+                        tbase = w1.y;
+                    }
+                    if (ht) {
+                        if (tgrp.y) tmore = make_uint2(tbase, ht);
+                        else tgrp = make_uint2(tbase, ht);
                     }
                 }
             }
         }
         // leaf phase
-        while (__any_sync(0xffffffffu, tgrp.y != 0u)) {
+        for (;;) {
+            const uint32_t tb = __ballot_sync(0xffffffffu, tgrp.y != 0u);
+            if (tb == 0u) break;
+            // (the node phase then has kWideMin lanes and takes a step)
+            if (__popc(tb) < IO::kWideTriMin &&
+                __popc(__ballot_sync(0xffffffffu, tmore.y == 0u && ((grp.y >> 24) != 0u || sp > 0))) >= IO::kWideMin)
+                break;
             if (tgrp.y) {
                 const uint32_t k = (uint32_t)(__ffs(tgrp.y) - 1);
                 tgrp.y &= tgrp.y - 1u;
                 const uint32_t ti = tgrp.x + k;
                 if (--budget == 0u || ti >= ts.tri_count) {
                     ef |= SOLRT_EFLAG_INDEX;
-                    tgrp.y = 0u;
+                    tgrp.y = tmore.y = 0u;
                     grp = make_uint2(0u, 0u);
                     sp = 0;
                 } else {
@@ -130,10 +149,14 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
                     if (kCount) ++cnt.tris;
                     if (intersect_tri(rm, tmin, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, cnt.fallbacks) &&
                         io.any_hit) {  // occlusion query: done at the first hit
-                        tgrp.y = 0u;
+                        tgrp.y = tmore.y = 0u;
                         grp = make_uint2(0u, 0u);
                         sp = 0;
                     }
+                }
+                if (tgrp.y == 0u) {
+                    tgrp = tmore;
+                    tmore.y = 0u;
                 }
             }
         }

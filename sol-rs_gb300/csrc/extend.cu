@@ -53,7 +53,7 @@ struct ExtendArgs {
 };
 
 template <int KIND, bool kSingle, bool kCount>
-__global__ void __launch_bounds__(256, kTraverseMinBlocks) k_extend(const __grid_constant__ ExtendArgs a) {
+__global__ void __launch_bounds__(256, traverse_min_blocks<KIND>()) k_extend(const __grid_constant__ ExtendArgs a) {
     const uint32_t n = *a.count;
     if (blockIdx.x == 0 && threadIdx.x == 0 && n) atomicAdd(&a.stats->segments, (unsigned long long)n);
     QueueIO<kSingle> io{{}, a.q.o_tmin, a.q.d_tmax, a.q.meta, a.jobs, a.hits, a.scene, a.lanes, a.any_hit};

@@ -43,7 +43,7 @@ struct TraceArgs {
 };
 
 template <int KIND, bool kCount>
-__global__ void __launch_bounds__(256, kTraverseMinBlocks) k_trace(const __grid_constant__ TraceArgs a) {
+__global__ void __launch_bounds__(256, traverse_min_blocks<KIND>()) k_trace(const __grid_constant__ TraceArgs a) {
     RayFileIO io{{}, a.rays, a.hits, a.scene, a.lanes};
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
