@@ -32,21 +32,30 @@ constexpr int kBvh2Sentinel = 0x7fffffff;
 // 2.62 ms unrolled, 2.31 as a loop of 8 steps; next-event estimation in a
 // tunnel 1105 / 907 us).
 //
-// kNodeMin (kWideMin, kWideTriMin: the 8-wide kinds, see bvh8_ww.cuh): the node phase ends early when fewer
-// lanes have inner nodes to visit and some lane holds a leaf. refill: see
-// warp_feed; a lane that only fetches its next ray should not wait long for
-// it, one that shades in between should have company. 4.2M incoherent rays /
+// kNodeMin (kWideMin and kWideTriMin: the wide kinds, see bvh8_ww.cuh): the
+// node phase ends early when fewer lanes have inner nodes to visit and some lane
+// holds a leaf. refill: see warp_feed; a lane that only fetches its next ray
+// should not wait long for it, one that shades in between should have company. 4.2M incoherent rays /
 // a soup frame (16 spp) / a batch of 24 jobs: refill 16, kNodeMin 12 2160 us /
 // 30.5 ms / 6.61 ms, 8 and 12 2075 / 30.1 / 6.48, 8 and 18 2023 / 29.6 / 6.22,
 // 6 and 16 2013 / 29.5 / 6.27, 2 and 16 2018 / 29.8 / 6.30. Shading programs:
 // an AO frame 4.66 ms with 16 and 12, 4.58 with 12 and 16; kWideMin 10 / 12 / 16
 // a 64x48 preview through 8-wide nodes 53.8 / 54.8 / 56.9 us.
+//
+// kLeafMin: the leaf phase ends early when fewer lanes still hold a leaf and
+// kNodeMin lanes have inner nodes (the rays with two or three leaves in a row
+// then wait for the next leaf phase; below kNodeMin, so that the node phase has
+// work). 1 / 4 / 8 / 13: 4.2M incoherent rays 1928 / 1865 / 1853 / 1854 us, a
+// 64-spp soup frame 111.6 / 108.6 / 108.0 / 108.3 ms, next-event estimation in a
+// tunnel 12.78 / 12.57 / 12.54 / 12.64 ms.
 struct FetchLoop {
-    static constexpr int kNodeSteps = 4, kNodeUnroll = 4, kNodeMin = 18, kWideMin = 16, kWideTriMin = 8;
+    static constexpr int kNodeSteps = 4, kNodeUnroll = 4, kNodeMin = 18, kLeafMin = 8;
+    static constexpr int kWideMin = 16, kWideTriMin = 8;
     static constexpr int refill = 6;
 };
 struct ShadeLoop {
-    static constexpr int kNodeSteps = 8, kNodeUnroll = 1, kNodeMin = 16, kWideMin = 10, kWideTriMin = 8;
+    static constexpr int kNodeSteps = 8, kNodeUnroll = 1, kNodeMin = 16, kLeafMin = 8;
+    static constexpr int kWideMin = 10, kWideTriMin = 8;
 };
 constexpr int kShadeRefill = 12;
 
@@ -213,7 +222,14 @@ SOLRT_D void extend_bvh2_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             }
         }
         // leaf phase
-        while (__any_sync(0xffffffffu, leaf < 0)) {
+        for (;;) {
+            const uint32_t b_leaf = __ballot_sync(0xffffffffu, leaf < 0);
+            if (b_leaf == 0u) break;
+            // (the node phase then has kNodeMin lanes, most of them without a
+            // leaf, and takes a step)
+            if (__popc(b_leaf) < IO::kLeafMin &&
+                __popc(__ballot_sync(0xffffffffu, (unsigned)node < ts.node_count)) >= IO::kNodeMin)
+                break;
             if (leaf < 0) {
                 const uint32_t k = (uint32_t)(~leaf);
                 if (--budget == 0u || k >= ts.tri_count) {
