@@ -38,6 +38,14 @@ SOLRT_D void instance_ray(const float4* inst, uint32_t k, float ox, float oy, fl
 // (ray transformed, marker pushed, BLAS root next), a parked triangle leaf
 // is tested before its lane leaves the instance, and the marker restores the
 // world ray (reloaded from the queue).
+//
+// A step between the levels (a ray to transform, a box set up) costs a warp
+// more than a node, and few lanes share it: while kLevelInner lanes have nodes
+// to visit, fewer than kLevelMin lanes wait with it. kLevelNodeMin: kNodeMin of
+// this loop. A 1280x720 frame of 64 moving sections (1M triangles, 4 spp): 7.68
+// ms without the wait (and 18), 7.55 / 7.60 / 7.66 with (8, 16, 20) / (10, 18,
+// 18) / (8, 16, 16).
+constexpr int kLevelMin = 8, kLevelInner = 16, kLevelNodeMin = 20;
 template <class IO, bool kCount>
 SOLRT_D void extend_bvh2_2l_ww(IO& io, uint32_t n, unsigned int* work, const StackMem& mem, TraceCounters& cnt,
                                uint32_t& ef) {
@@ -82,8 +90,12 @@ SOLRT_D void extend_bvh2_2l_ww(IO& io, uint32_t n, unsigned int* work, const Sta
             const uint32_t b_act = __ballot_sync(0xffffffffu, act);
             const uint32_t b_leaf = __ballot_sync(0xffffffffu, leaf < 0);
             if ((b_act & ~b_leaf) == 0u) break;
-            if (__popc(b_act) < IO::kNodeMin && b_leaf) break;
-            if (!act) continue;
+            if (__popc(b_act) < kLevelNodeMin && b_leaf) break;
+            // a step between the levels costs a warp as much as several nodes:
+            // few lanes wait with it until more have one, or too few have nodes
+            const uint32_t b_inner = __ballot_sync(0xffffffffu, inner);
+            const bool inner_only = __popc(b_act & ~b_inner) < kLevelMin && __popc(b_inner) >= kLevelInner;
+            if (!(inner_only ? inner : act)) continue;
             if (--budget == 0u) {
                 ef |= SOLRT_EFLAG_INDEX;
                 node = kBvh2Sentinel;
