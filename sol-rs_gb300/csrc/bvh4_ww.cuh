@@ -9,8 +9,10 @@
 // margin on every face); hit internal children are sorted by entry distance,
 // the nearest is visited next and the others are pushed far to near; hit leaf
 // triangles are parked and tested in the leaf phase. The warp organisation
-// (refill, node phase ended early when few lanes still have nodes, leaf
-// phase) is that of bvh2_ww.cuh.
+// is that of bvh8_ww.cuh: a lane holds the triangles of up to two nodes, and
+// both phases end early when few lanes are left in them (a 1366x768 tunnel frame,
+// 16 spp: 63.5 ms with one parked node, leaf phases that run to their end and 48
+// registers, now 57.4).
 #pragma once
 
 #include "bvh2_ww.cuh"
@@ -76,6 +78,7 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
     int sp = 0;
     int node = kBvh2Sentinel;            // next 4-wide node to visit, or none
     uint2 tgrp = make_uint2(0u, 0u);     // parked triangles: (triangle base, hit bits)
+    uint2 tmore = make_uint2(0u, 0u);    // those of a second node (only beside the first)
     bool has = false;
     bool drained = false;
     uint32_t budget = 0;
@@ -105,7 +108,7 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             budget = 2u * (ts.node_count + ts.tri_count) + 64u;
             stack.put(0, kBvh2Sentinel);
             sp = 1;
-            tgrp = make_uint2(0u, 0u);
+            tgrp = tmore = make_uint2(0u, 0u);
             node = ts.tri_count ? 0 : kBvh2Sentinel;
         }
         if (!__any_sync(0xffffffffu, has)) {
@@ -114,10 +117,10 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
         }
         // node phase
         for (;;) {
-            const bool want = node != kBvh2Sentinel && tgrp.y == 0u;
+            const bool want = node != kBvh2Sentinel && tmore.y == 0u;
             const uint32_t wb = __ballot_sync(0xffffffffu, want);
             if (wb == 0u) break;
-            if (__popc(wb) < IO::kNodeMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
+            if (__popc(wb) < IO::kWideMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
             if (want) {
                 if (--budget == 0u || (uint32_t)node >= ts.node_count) {
                     ef |= SOLRT_EFLAG_INDEX;
@@ -150,19 +153,29 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
                     } else {
                         node = stack.get(--sp);
                     }
-                    tgrp = make_uint2(__float_as_uint(w1.y), ht);
+                    if (ht) {
+                        const uint2 t = make_uint2(__float_as_uint(w1.y), ht);
+                        if (tgrp.y) tmore = t;
+                        else tgrp = t;
+                    }
                 }
             }
         }
         // leaf phase
-        while (__any_sync(0xffffffffu, tgrp.y != 0u)) {
+        for (;;) {
+            const uint32_t tb = __ballot_sync(0xffffffffu, tgrp.y != 0u);
+            if (tb == 0u) break;
+            // (the node phase then has kWideMin lanes and takes a step)
+            if (__popc(tb) < IO::kWideTriMin &&
+                __popc(__ballot_sync(0xffffffffu, node != kBvh2Sentinel && tmore.y == 0u)) >= IO::kWideMin)
+                break;
             if (tgrp.y) {
                 const uint32_t k = (uint32_t)(__ffs(tgrp.y) - 1);
                 tgrp.y &= tgrp.y - 1u;
                 const uint32_t ti = tgrp.x + k;
                 if (--budget == 0u || ti >= ts.tri_count) {
                     ef |= SOLRT_EFLAG_INDEX;
-                    tgrp.y = 0u;
+                    tgrp.y = tmore.y = 0u;
                     node = kBvh2Sentinel;
                     sp = 1;
                 } else {
@@ -170,10 +183,14 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
                     if (kCount) ++cnt.tris;
                     if (intersect_tri(rm, tmin, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), best_t, cnt.fallbacks) &&
                         io.any_hit) {  // occlusion query: done at the first hit
-                        tgrp.y = 0u;
+                        tgrp.y = tmore.y = 0u;
                         node = kBvh2Sentinel;
                         sp = 1;
                     }
+                }
+                if (tgrp.y == 0u) {
+                    tgrp = tmore;
+                    tmore.y = 0u;
                 }
             }
         }

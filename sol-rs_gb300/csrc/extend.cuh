@@ -109,14 +109,15 @@ SOLRT_D void flush_traversal(DevStats* stats, const TraceCounters& cnt, uint32_t
 }
 
 // Blocks of 256 threads that an SM must hold, for the register allocator: 5
-// (48 registers, 1280 threads), for the 8-wide kinds 4 (64 registers: their
-// node test holds more). 4 / 5 / 6: a 64-spp soup frame through FP32 binary
+// (48 registers, 1280 threads), for the wide kinds 4 (64 registers: their node
+// tests hold more). 4 / 5 / 6: a 64-spp soup frame through FP32 binary
 // nodes 132.9 / 131.9 / 134.0 ms, 4.2M incoherent rays 2.80 / 2.72 / 2.86 ms,
 // two-level scenes 9.41 / 9.12 / 9.99 ms; the 8-wide tree on a tunnel frame
-// 60.3 / 55.3 / 58.0 ms with 3 / 4 / 5.
+// 60.3 / 55.3 / 58.0 ms with 3 / 4 / 5, the 4-wide one 57.4 / 57.6 with 4 / 5
+// (next-event estimation through it 15.3 / 15.9 ms).
 template <int KIND>
 constexpr int traverse_min_blocks() {
-    return KIND == SOLRT_BVH8_Q8 || KIND == SOLRT_BVH8_F32 ? 4 : 5;
+    return KIND == SOLRT_BVH4_Q8 || KIND == SOLRT_BVH8_Q8 || KIND == SOLRT_BVH8_F32 ? 4 : 5;
 }
 
 // Shape of one launch of `kern`: the context's block size and stack slots,
