@@ -389,7 +389,7 @@ __global__ void k_refit(const float4* __restrict__ vpos, const uint4* __restrict
         lo[1] = fminf(s0.z, s1.z); hi[1] = fmaxf(s0.w, s1.w);
         lo[2] = fminf(s2.x, s2.z); hi[2] = fmaxf(s2.y, s2.w);
         // the union above used the exact child boxes; the traversal reads
-        // them widened (see slab_fma)
+        // them widened (see slab2_fma)
         np[0] = make_float4(widen_lo(s0.x), widen_hi(s0.y), widen_lo(s0.z), widen_hi(s0.w));
         np[1] = make_float4(widen_lo(s1.x), widen_hi(s1.y), widen_lo(s1.z), widen_hi(s1.w));
         np[2] = make_float4(widen_lo(s2.x), widen_hi(s2.y), widen_lo(s2.z), widen_hi(s2.w));

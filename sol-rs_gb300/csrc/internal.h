@@ -248,8 +248,6 @@ struct Context {
     uint32_t noise_w = 0, noise_h = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint64_t launches = 0;
-    double last_render_ms = 0.0;
-    int extend_blocks_per_sm = 0;
     // stage timing (enable_timing): event pairs recorded around launches
     bool timing = false;
     struct TimedLaunch {

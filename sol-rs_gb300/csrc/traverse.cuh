@@ -249,26 +249,14 @@ SOLRT_D float box_rcp(float v) {
     return r;
 }
 
-// Slab test in the form t = fma(plane, 1/d, -o/d) (one instruction per
-// plane). Its rounding error relative to |o/d| is covered by the widening of
-// every BVH2 child box by a relative 2^-21 at build time (widen_lo /
-// widen_hi) plus the relative 2^-16 widening of the far distance.
-SOLRT_D bool slab_fma(float lox, float hix, float loy, float hiy, float loz, float hiz, float ix, float iy,
-                      float iz, float nox, float noy, float noz, float tmin, float tmax, float& tnear) {
-    const float x0 = fmaf(lox, ix, nox), x1 = fmaf(hix, ix, nox);
-    const float y0 = fmaf(loy, iy, noy), y1 = fmaf(hiy, iy, noy);
-    const float z0 = fmaf(loz, iz, noz), z1 = fmaf(hiz, iz, noz);
-    const float tn = fmaxf(max3(fminf(x0, x1), fminf(y0, y1), fminf(z0, z1)), tmin);
-    const float tf = fminf(min3(fmaxf(x0, x1), fmaxf(y0, y1), fmaxf(z0, z1)), tmax);
-    tnear = tn;
-    return tn <= tf * 1.0000153f;
-}
-
 // Both child boxes of a BVH2 node (n0: child 0 x/y planes, n1: child 1 x/y
-// planes, n2: z planes of both) against one ray: the same arithmetic as two
-// slab_fma calls. With SOLRT_SLAB_F32X2 the 12 plane distances are six
-// packed two-lane FMAs (PTX fma.rn.f32x2, sm_100 and later; each lane is an
-// ordinary correctly rounded fma).
+// planes, n2: z planes of both) against one ray, in the form t = fma(plane,
+// 1/d, -o/d). Its rounding error relative to |o/d| is covered by the widening
+// of every BVH2 child box by a relative 2^-21 at build time (widen_lo /
+// widen_hi) plus the relative 2^-16 widening of the far distance. With
+// SOLRT_SLAB_F32X2 the 12 plane distances are six packed two-lane FMAs (PTX
+// fma.rn.f32x2, sm_100 and later; each lane is an ordinary correctly rounded
+// fma).
 #ifndef SOLRT_SLAB_F32X2
 #define SOLRT_SLAB_F32X2 1
 #endif
