@@ -50,12 +50,12 @@ constexpr int kBvh2Sentinel = 0x7fffffff;
 // tunnel 12.78 / 12.57 / 12.54 / 12.64 ms.
 struct FetchLoop {
     static constexpr int kNodeSteps = 4, kNodeUnroll = 4, kNodeMin = 18, kLeafMin = 8;
-    static constexpr int kWideMin = 16, kWideTriMin = 8;
+    static constexpr int kWideMin = 16, kWideEnd = 6, kWideTriMin = 8;
     static constexpr int refill = 6;
 };
 struct ShadeLoop {
     static constexpr int kNodeSteps = 8, kNodeUnroll = 1, kNodeMin = 16, kLeafMin = 8;
-    static constexpr int kWideMin = 10, kWideTriMin = 8;
+    static constexpr int kWideMin = 10, kWideEnd = 6, kWideTriMin = 8;
 };
 constexpr int kShadeRefill = 12;
 

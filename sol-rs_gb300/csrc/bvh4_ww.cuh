@@ -115,12 +115,13 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             if (drained) break;
             continue;
         }
+        const int node_min = drained ? IO::kWideEnd : IO::kWideMin;
         // node phase
         for (;;) {
             const bool want = node != kBvh2Sentinel && tmore.y == 0u;
             const uint32_t wb = __ballot_sync(0xffffffffu, want);
             if (wb == 0u) break;
-            if (__popc(wb) < IO::kWideMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
+            if (__popc(wb) < node_min && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
             if (want) {
                 if (--budget == 0u || (uint32_t)node >= ts.node_count) {
                     ef |= SOLRT_EFLAG_INDEX;
@@ -165,9 +166,9 @@ SOLRT_D void extend_bvh4_ww(IO& io, uint32_t n, unsigned int* work, const StackM
         for (;;) {
             const uint32_t tb = __ballot_sync(0xffffffffu, tgrp.y != 0u);
             if (tb == 0u) break;
-            // (the node phase then has kWideMin lanes and takes a step)
+            // (the node phase then has node_min lanes and takes a step)
             if (__popc(tb) < IO::kWideTriMin &&
-                __popc(__ballot_sync(0xffffffffu, node != kBvh2Sentinel && tmore.y == 0u)) >= IO::kWideMin)
+                __popc(__ballot_sync(0xffffffffu, node != kBvh2Sentinel && tmore.y == 0u)) >= node_min)
                 break;
             if (tgrp.y) {
                 const uint32_t k = (uint32_t)(__ffs(tgrp.y) - 1);

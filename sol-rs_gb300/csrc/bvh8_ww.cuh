@@ -18,7 +18,9 @@
 // 32 lanes were active on average. A 1366x768 tunnel frame (16 spp): 64.8 ms so,
 // 60.7 with the threshold in the leaf phase, 58.0 with a second parked node as
 // well, 55.3 at 64 registers a thread (traverse_min_blocks); 4.2M incoherent
-// rays 2.79 / 2.66 / 2.77 / 2.56 ms.
+// rays 2.79 / 2.66 / 2.77 / 2.56 ms. Once the queue is empty kWideEnd takes the
+// place of kWideMin, which few warps reach any more: calls of 20k and 80k rays
+// 43.7 -> 42.6 and 24.5 -> 22.9 us (three in flight; 4.2M rays 2.56 -> 2.59 ms).
 // The child-box tests are those of trace_bvh8 (bvh8_traverse.cuh: quantised
 // or, for SOLRT_BVH8_F32, full-precision nodes), so the closest hit equals
 // that of the per-ray loop.
@@ -83,12 +85,13 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
             if (drained) break;
             continue;
         }
+        const int node_min = drained ? IO::kWideEnd : IO::kWideMin;
         // node phase
         for (;;) {
             const bool want = tmore.y == 0u && ((grp.y >> 24) != 0u || sp > 0);
             const uint32_t wb = __ballot_sync(0xffffffffu, want);
             if (wb == 0u) break;
-            if (__popc(wb) < IO::kWideMin && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
+            if (__popc(wb) < node_min && __any_sync(0xffffffffu, tgrp.y != 0u)) break;
             if (want) {
                 if ((grp.y >> 24) == 0u) grp = stack[--sp];
                 const uint32_t j = (uint32_t)(__ffs(grp.y >> 24) - 1);
@@ -131,9 +134,9 @@ SOLRT_D void extend_bvh8_ww(IO& io, uint32_t n, unsigned int* work, const StackM
         for (;;) {
             const uint32_t tb = __ballot_sync(0xffffffffu, tgrp.y != 0u);
             if (tb == 0u) break;
-            // (the node phase then has kWideMin lanes and takes a step)
+            // (the node phase then has node_min lanes and takes a step)
             if (__popc(tb) < IO::kWideTriMin &&
-                __popc(__ballot_sync(0xffffffffu, tmore.y == 0u && ((grp.y >> 24) != 0u || sp > 0))) >= IO::kWideMin)
+                __popc(__ballot_sync(0xffffffffu, tmore.y == 0u && ((grp.y >> 24) != 0u || sp > 0))) >= node_min)
                 break;
             if (tgrp.y) {
                 const uint32_t k = (uint32_t)(__ffs(tgrp.y) - 1);

@@ -123,13 +123,17 @@ constexpr int traverse_min_blocks() {
 // Shape of one launch of `kern`: the context's block size and stack slots,
 // state_words words of program state per thread, a grid of (SMs x resident
 // blocks) or fewer blocks when `units` rays or paths need fewer, and how many
-// lanes of each warp take work: 32, or, for up to kSpreadUnits units with
+// lanes of each warp take work: 32, or, for up to spread_units units with
 // `spread`, as few as spread them over all warps of a full grid. A warp with
 // fewer rays steps faster, but beyond that its idle lanes cost more than the
 // shorter steps gain (microseconds for one call, few lanes / 32: 2000 rays
 // through 20k triangles 94 / 134, 8000 117 / 143, 30k 159 / 152, 100k 214 / 194;
-// with three calls in flight 34 / 47, 43 / 47, 68 / 56, 98 / 74).
-constexpr uint32_t kSpreadUnits = 8192;
+// with three calls in flight 34 / 47, 43 / 47, 68 / 56, 98 / 74; the 8-wide tree
+// 7400 rays 88 / 92 and 30.9 / 29.9, 4000 97 / 117 and 37.1 / 39.1).
+template <int KIND>
+constexpr uint32_t spread_units() {
+    return KIND == SOLRT_BVH8_Q8 || KIND == SOLRT_BVH8_F32 ? 4096 : 8192;
+}
 struct LaunchShape {
     uint32_t grid = 0, block = 0, smem = 0, slots = 0, lanes = 32;
 };
@@ -154,7 +158,7 @@ solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t uni
     }
     const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;
     const uint32_t warps = full * (s.block / 32u);
-    s.lanes = spread && units <= kSpreadUnits ? std::min(32u, std::max(1u, (units + warps - 1u) / warps)) : 32u;
+    s.lanes = spread && units <= spread_units<KIND>() ? std::min(32u, std::max(1u, (units + warps - 1u) / warps)) : 32u;
     s.grid = std::min(full, (units + s.lanes * (s.block / 32u) - 1u) / (s.lanes * (s.block / 32u)));
     return SOLRT_OK;
 }

@@ -775,7 +775,10 @@ PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp
 //   1853 / 907, 40k: 2086 / 1393;
 //   moving scenes, whose rebuild waits for the device before every frame, so
 //   that no other frame fills the ends of the launches: 415k: 2431 / 1998
-//   with the rebuild, 830k: 2786 / 2372.
+//   with the rebuild, 830k: 2786 / 2372;
+//   the wide kinds, whose refills find fewer lanes idle: Cornell box 68k: 102 /
+//   89, 102k: 136 / 153, 160k: 184 / 231; meshes 102k: 236 / 212, 160k: 282 /
+//   299 and 536 / 601.
 bool path_kernel_pays(const Context& ctx, const Scene& sc, const DevJob& J, uint64_t paths) {
     if (ctx.counters) return false;  // node and triangle counts: wavefront only
     const uint64_t levels = J.max_bounces + 1ull;
@@ -783,6 +786,8 @@ bool path_kernel_pays(const Context& ctx, const Scene& sc, const DevJob& J, uint
     const bool small = J.sc.tri_count < kSmallScene;
     if (J.integrator == SOLRT_INTEGRATOR_PATH_NEE) return per_level <= (small ? 73728 : 57344);
     if (sc.dynamic && sc.info.kind != SOLRT_BVH2_TWO_LEVEL) return per_level <= 917504;
+    const uint32_t k = sc.info.kind;
+    if (k == SOLRT_BVH8_Q8 || k == SOLRT_BVH8_F32 || k == SOLRT_BVH4_Q8) return per_level <= (small ? 73728 : 114688);
     return per_level <= (small ? 180224 : 229376);
 }
 

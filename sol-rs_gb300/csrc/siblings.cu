@@ -2,13 +2,13 @@
 // traversal: DEBUG (debug.rgen / .rchit / .rmiss) and AO (ao.rgen / .rchit /
 // .rmiss).
 //
-// Their shaders run one invocation per pixel. Here a persistent launch holds
-// 32 pixels per warp in the traversal loop of the BVH kind (warp_feed): lanes
-// whose ray is done shade and go on with their pixel's next ray or sample, or
-// take another pixel. A thread per pixel that follows its rays to the end
-// (k_debug_plain, k_ao_plain; kept for small scenes and frames) leaves a warp's
-// lanes waiting for its longest chain: an AO frame of a 300k-triangle soup (1280x720, 4
-// samples) 7.1 -> 4.7 ms, a 1920x1080 DEBUG frame of it 597 -> 497 us.
+// Their shaders run one invocation per pixel, and so do k_debug and k_ao_plain.
+// AO frames of large scenes run k_ao instead (ao_plain, below): a persistent
+// launch that holds 32 pixels per warp in the traversal loop of the BVH kind
+// (warp_feed), where lanes whose ray is done shade and go on with their pixel's
+// next ray or sample, or take another pixel, instead of waiting for the warp's
+// longest chain: a 1280x720 frame (4 samples) of a 300k-triangle soup 7.1 -> 4.4
+// ms.
 #include "extend.cuh"
 #include "path_ops.cuh"
 
@@ -19,7 +19,6 @@ namespace {
 struct SiblingArgs {
     DevJob job;
     uint32_t units, slots;
-    int lanes;
     unsigned int* work;
     int* deep;
     DevStats* stats;
@@ -53,25 +52,13 @@ enum SiblingWord {
     kSWords = 12,
 };
 
-template <class Loop>
-struct SiblingIO : Loop {
-    const SiblingArgs& a;
-    const StateMem st;
-    const int lanes;
-    static constexpr bool any_hit = false;
-    SOLRT_D explicit SiblingIO(const SiblingArgs& args) : a(args), st(args.slots), lanes(args.lanes) { st.put(kSSegs, 0u); }
-    SOLRT_D TravScene first_scene() const { return trav_scene(a.job.sc); }
-    SOLRT_D void load_ray(uint32_t, float4& o, float4& d) const {
-        const f3 p = st.get3(kSOrg), q = st.get3(kSDir);
-        o = make_float4(p.x, p.y, p.z, 0.0f);
-        d = make_float4(q.x, q.y, q.z, 0.0f);
-    }
-    SOLRT_D void keep_ray(const float4& o, const float4& d) const {
-        st.put3(kSOrg, o.x, o.y, o.z);
-        st.put3(kSDir, d.x, d.y, d.z);
-        st.bump(kSSegs);
-    }
-};
+// Statistics of a thread that traced `segs` rays of its pixel.
+SOLRT_D void flush_plain(const SiblingArgs& a, const TraceCounters& cnt, uint32_t ef, uint32_t segs, uint32_t paths) {
+    flush_traversal(a.stats, cnt, ef, false);
+    const uint32_t ws = __reduce_add_sync(0xffffffffu, segs);
+    if ((threadIdx.x & 31) == 0 && ws) atomicAdd(&a.stats->segments, (unsigned long long)ws);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats->paths, (unsigned long long)a.units * paths);
+}
 
 // debug.rgen:18-36, debug.rchit:9-13, debug.rmiss: barycentrics of the
 // primary hit through the pixel centre, else the ray direction; stored
@@ -88,17 +75,21 @@ SOLRT_D void debug_write_pixel(const DevJob& J, uint32_t pix, const HitRec& h, f
     J.accum[pix] = v;
     J.rgba8[pix] = make_uchar4(to_unorm8(v.x), to_unorm8(v.y), to_unorm8(v.z), 0);
 }
-struct DebugIO : SiblingIO<FetchLoop> {
-    using SiblingIO<FetchLoop>::SiblingIO;
-    SOLRT_D void load(uint32_t pix, float4& o, float4& d, TravScene&) const {
+
+template <int KIND>
+__global__ void __launch_bounds__(128, 1) k_debug(const __grid_constant__ SiblingArgs a) {
+    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t ef = 0;
+    TraceCounters cnt{0, 0, 0};
+    if (pix < a.units) {
+        float4 o, d;
         debug_ray(a.job, pix, o, d);
-        keep_ray(o, d);
+        HitRec h;
+        trace_one<KIND>(trav_scene(a.job.sc), o, d, h, cnt, ef);
+        debug_write_pixel(a.job, pix, h, f3{d.x, d.y, d.z});
     }
-    SOLRT_D bool next(uint32_t pix, float, const HitRec& h, float4&, float4&, const TraceCounters&, uint32_t&) const {
-        debug_write_pixel(a.job, pix, h, st.get3(kSDir));
-        return false;
-    }
-};
+    flush_plain(a, cnt, ef, pix < a.units ? 1u : 0u, 1u);
+}
 
 // ao.rgen:37-83, ao.rchit:53-88, ao.rmiss: `spp` jittered samples; each
 // follows cosine-weighted rays (directions from the blue-noise texture)
@@ -167,9 +158,23 @@ SOLRT_D void ao_write_pixel(const DevJob& J, uint32_t pix, float sum) {
     J.rgba8[pix] = make_uchar4(to_unorm8(color.x), to_unorm8(color.y), to_unorm8(color.z), 255);
 }
 
-struct AoIO : SiblingIO<ShadeLoop> {
-    using SiblingIO<ShadeLoop>::SiblingIO;
-    static constexpr int refill = kShadeRefill;
+struct AoIO : ShadeLoop {
+    const SiblingArgs& a;
+    const StateMem st;
+    static constexpr int lanes = 32, refill = kShadeRefill;
+    static constexpr bool any_hit = false;
+    SOLRT_D explicit AoIO(const SiblingArgs& args) : a(args), st(args.slots) { st.put(kSSegs, 0u); }
+    SOLRT_D TravScene first_scene() const { return trav_scene(a.job.sc); }
+    SOLRT_D void load_ray(uint32_t, float4& o, float4& d) const {
+        const f3 p = st.get3(kSOrg), q = st.get3(kSDir);
+        o = make_float4(p.x, p.y, p.z, 0.0f);
+        d = make_float4(q.x, q.y, q.z, 0.0f);
+    }
+    SOLRT_D void keep_ray(const float4& o, const float4& d) const {
+        st.put3(kSOrg, o.x, o.y, o.z);
+        st.put3(kSDir, d.x, d.y, d.z);
+        st.bump(kSSegs);
+    }
     SOLRT_D void start(uint32_t pix, uint32_t sample, uint32_t rng, float4& o, float4& d) const {
         ao_camera_ray(a.job, pix, rng, o, d);
         st.put(kSRng, rng);
@@ -208,32 +213,7 @@ struct AoIO : SiblingIO<ShadeLoop> {
     }
 };
 
-// The same frames with one thread per pixel, as in the shaders: for small
-// scenes, where lanes that start every sample together are worth more than full
-// lanes (Cornell box, 1280x720, 4 samples: AO 1.06 ms, through AoIO 1.26 ms; a
-// 2000-triangle soup 2.56 / 2.19 ms), and for small frames (sibling_plain).
-SOLRT_D void flush_plain(const SiblingArgs& a, const TraceCounters& cnt, uint32_t ef, uint32_t segs, uint32_t paths) {
-    flush_traversal(a.stats, cnt, ef, false);
-    const uint32_t ws = __reduce_add_sync(0xffffffffu, segs);
-    if ((threadIdx.x & 31) == 0 && ws) atomicAdd(&a.stats->segments, (unsigned long long)ws);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats->paths, (unsigned long long)a.units * paths);
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(128) k_debug_plain(const __grid_constant__ SiblingArgs a) {
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t ef = 0;
-    TraceCounters cnt{0, 0, 0};
-    if (pix < a.units) {
-        float4 o, d;
-        debug_ray(a.job, pix, o, d);
-        HitRec h;
-        trace_one<KIND>(trav_scene(a.job.sc), o, d, h, cnt, ef);
-        debug_write_pixel(a.job, pix, h, f3{d.x, d.y, d.z});
-    }
-    flush_plain(a, cnt, ef, pix < a.units ? 1u : 0u, 1u);
-}
-
+// AO with one thread per pixel, 8 blocks per SM (64 registers).
 template <int KIND>
 __global__ void __launch_bounds__(128, 8) k_ao_plain(const __grid_constant__ SiblingArgs a) {
     const DevJob& J = a.job;
@@ -262,61 +242,54 @@ __global__ void __launch_bounds__(128, 8) k_ao_plain(const __grid_constant__ Sib
     flush_plain(a, cnt, ef, segs, J.spp);
 }
 
-template <int KIND, class IO>
-__global__ void __launch_bounds__(256, 4) k_sibling(const __grid_constant__ SiblingArgs a) {
-    IO io(a);
+template <int KIND>
+__global__ void __launch_bounds__(256, 4) k_ao(const __grid_constant__ SiblingArgs a) {
+    AoIO io(a);
     TraceCounters cnt{0, 0, 0};
     uint32_t ef = 0;
     extend_kind<KIND, false>(io, a.units, a.work, stack_mem(a.slots, a.deep), cnt, ef);
     flush_traversal(a.stats, cnt, ef, false);
     const uint32_t segs = __reduce_add_sync(0xffffffffu, io.st.get(kSSegs));
     if ((threadIdx.x & 31) == 0 && segs) atomicAdd(&a.stats->segments, (unsigned long long)segs);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const uint64_t per = a.job.integrator == SOLRT_INTEGRATOR_AO ? a.job.spp : 1u;
-        atomicAdd(&a.stats->paths, (unsigned long long)a.units * per);
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.stats->paths, (unsigned long long)a.units * a.job.spp);
     release_work(a.work);
 }
 
-template <int KIND, class IO>
-solrt_status launch_io(const Context& ctx, SiblingArgs a) {
-    LaunchShape s;
-    SOLRT_TRY((launch_shape<KIND, k_sibling<KIND, IO>>(ctx, kSWords, a.units, true, s)));
-    a.slots = s.slots;
-    a.lanes = (int)s.lanes;
-    k_sibling<KIND, IO><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
-    return SOLRT_OK;
-}
-
 template <int KIND>
-solrt_status launch_kind(const Context& ctx, const SiblingArgs& a, bool plain) {
-    const bool ao = a.job.integrator == SOLRT_INTEGRATOR_AO;
-    if (!plain) return ao ? launch_io<KIND, AoIO>(ctx, a) : launch_io<KIND, DebugIO>(ctx, a);
+solrt_status launch_kind(const Context& ctx, SiblingArgs a, bool plain) {
     const uint32_t blocks = (a.units + 127) / 128;
-    if (ao) k_ao_plain<KIND><<<blocks, 128, 0, ctx.stream>>>(a);
-    else k_debug_plain<KIND><<<blocks, 128, 0, ctx.stream>>>(a);
+    if (a.job.integrator != SOLRT_INTEGRATOR_AO) {
+        k_debug<KIND><<<blocks, 128, 0, ctx.stream>>>(a);
+    } else if (plain) {
+        k_ao_plain<KIND><<<blocks, 128, 0, ctx.stream>>>(a);
+    } else {
+        LaunchShape s;
+        SOLRT_TRY((launch_shape<KIND, k_ao<KIND>>(ctx, kSWords, a.units, false, s)));
+        a.slots = s.slots;
+        k_ao<KIND><<<s.grid, s.block, s.smem, ctx.stream>>>(a);
+    }
     return SOLRT_OK;
 }
 
 }  // namespace
 
-// One thread per pixel: small scenes (see k_ao_plain), and frames of so few
-// pixels that most of the GPU is idle anyway and the shorter steps of a plain
-// loop decide. Three frames in flight, a thread per pixel / persistent (us): AO
-// 64x48 of a 2000-triangle tube 134 / 160, 320x180 of a 300k soup 924 / 713;
-// DEBUG 640x48 of a 20k tube 17.3 / 19.8, 320x180 of the soup 65.5 / 65.6,
-// 1920x1080 597 / 497. The smallest DEBUG frames of BVH2 scenes go to the
-// persistent launch, which spreads them over all warps (launch_shape): 64x48 of
-// the soup 45.5 / 40.5, of a 2000-triangle soup 22.9 / 19.2.
+// Whether a frame runs one thread per pixel. Always for DEBUG: its one ray per
+// pixel leaves no chain to wait for, and neighbouring camera rays stay together
+// in a plain loop (1280x720, three frames in flight, per pixel / persistent: a
+// 300k-triangle tube 112 / 147 us, a 300k soup 297 / 251). For AO the
+// persistent launch pays once traversals are long: a soup ends its chains at
+// many lengths, a tube hardly, and what its refills cost in coherence there
+// shrinks with the size of the tree (640x360, 4 samples, us: tubes of 5k
+// triangles 830 / 1088, 50k 1294 / 1584, 300k 2105 / 2179, 1M 2571 / 2629;
+// soups 1007 / 802, 1584 / 1187, 1927 / 1430, 2140 / 1560; 320x180 of the 300k
+// tube 653 / 577). Frames of few pixels leave the GPU idle either way and take
+// the shorter steps of the plain loop (64x48 of a tube 134 / 160).
 bool sibling_plain(const Scene& sc, const solrt_render_params& p) {
-    const uint64_t pixels = (uint64_t)p.width * p.height;
-    if (sc.info.kind == SOLRT_BVH2 && sc.tri_count < kSmallScene) return true;
-    if (p.integrator == SOLRT_INTEGRATOR_AO) return pixels <= 16384u;
-    return pixels <= 49152u && !(sc.info.kind == SOLRT_BVH2 && pixels <= kSpreadUnits);
+    return p.integrator != SOLRT_INTEGRATOR_AO || sc.tri_count < 196608u || (uint64_t)p.width * p.height <= 16384u;
 }
 
 solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J, bool plain) {
-    const SiblingArgs a{J, J.width * J.height, 0, 32, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
+    const SiblingArgs a{J, J.width * J.height, 0, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
                         ctx.stats.as<DevStats>()};
     switch (kind) {
         case SOLRT_BVH8_Q8: SOLRT_TRY(launch_kind<SOLRT_BVH8_Q8>(ctx, a, plain)); break;

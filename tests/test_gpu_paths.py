@@ -109,17 +109,17 @@ def test_moving_scene(solrt, ctx):
     sc.close()
 
 
-@pytest.mark.parametrize("integrator", ["INTEGRATOR_AO", "INTEGRATOR_DEBUG"])
-@pytest.mark.parametrize("w,h", [(128, 64), (128, 65), (128, 128), (129, 128), (256, 192), (257, 192)])
-def test_ao_and_debug_on_both_sides_of_the_pixel_limits(solrt, oracle, ctx, integrator, w, h):
-    """AO changes loops above 16,384 pixels, DEBUG above 8,192 and 49,152: both equal the
-    oracle, in a scene large enough for either loop."""
-    data = S.soup(1500, seed=6, sigma=0.04)
+@pytest.mark.parametrize("tris", [196607, 196608])
+@pytest.mark.parametrize("w,h", [(128, 128), (129, 128)])
+def test_ao_on_both_sides_of_its_limits(solrt, oracle, ctx, tris, w, h):
+    """AO frames change loops from 196,608 triangles on, above 16,384 pixels:
+    all equal the oracle."""
+    data = S.soup(tris, seed=6, sigma=0.004)
     noise = np.random.default_rng(1).integers(0, 256, (64, 64, 4), dtype=np.uint8)
     ctx.set_blue_noise(noise)
     c = data.camera
     cam = solrt.camera_look_at(c["eye"], c["center"], c["up"], c["vfov"], w / h)
-    p = solrt.render_params(w, h, spp=2, max_bounces=3, integrator=getattr(solrt, integrator))
+    p = solrt.render_params(w, h, spp=2, max_bounces=3, integrator=solrt.INTEGRATOR_AO)
     sc = solrt.SceneDescription(ctx, data)
     img = solrt.Image(ctx, w, h)
     solrt.Renderer(ctx).cmd_trace_rays(sc, cam, p, img)
@@ -130,10 +130,11 @@ def test_ao_and_debug_on_both_sides_of_the_pixel_limits(solrt, oracle, ctx, inte
     sc.close()
 
 
-@pytest.mark.parametrize("n", [8192, 8193])
+@pytest.mark.parametrize("n", [4096, 4097, 8192, 8193])
 @pytest.mark.parametrize("bvh", ["bvh2", "bvh8", "bvh2t"])
 def test_rays_on_both_sides_of_the_spread_limit(solrt, oracle, ctx, bvh, n):
-    """Up to 8,192 rays are spread over all warps, from there on warps take 32."""
+    """Up to 8,192 rays (8-wide trees: 4,096) are spread over all warps, from
+    there on warps take 32."""
     data = S.soup(600, seed=3, sigma=0.05)
     args = bvh_args(solrt, bvh)
     rays = random_rays(n, -1.0, 1.0, seed=5)
