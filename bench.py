@@ -47,6 +47,8 @@ NODE_BYTES = {0: 64, 1: 80, 2: 64, 3: 224, 4: 32, 5: 64}
 # the pass traced (profiles/extend_dram_soup1M_tunnel4M.md). limiter: the
 # counters of one `ncu --set full` launch (profiles/extend_soup1M_bvh2_full.md,
 # profiles/extend_soup1M_treelet_full.md, profiles/extend_tunnel_640x360_full.md).
+# All were captured with the 64-byte nodes, before the traversal's 32-byte
+# copies of them.
 # Keys: (workload, "lbvh" or "treelet" BVH2).
 EXTEND_CAPTURES = {
     ("soup", "lbvh"): {"dram_bytes_per_segment": 62.4, "dram_source": "profiles/extend_dram_soup1M_tunnel4M.md",
@@ -1026,7 +1028,8 @@ def main():
                 "frac": round(achieved / peak, 4), "traffic": traffic,
                 "frac_note": "achieved counts algorithmic bytes (node, triangle, ray and hit bytes of every visit) "
                              "with no cache reuse; L1 / L2 serve nearly all of them, so frac > 1 is not HBM "
-                             "traffic: dram is what reaches HBM, limiter what binds" if cap else None,
+                             "traffic; BVH2 nodes count 64 bytes each, also where the traversal reads its 32-byte "
+                             "copy of them; dram and limiter were captured before those copies" if cap else None,
                 "dram": dram, "limiter": cap["limiter"] if (cap and dram) else None,
                 "peak_source": peak_kind + " (MEASURED_PEAKS hbm_gbs)",
                 "kernel": "k_megakernel (traversal + shading, whole render time)" if args.kernel == "mega"
