@@ -598,13 +598,14 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
 //   soups: 100 triangles 0.38 / 0.39 ms, 300 0.57 / 0.58, 1000 0.89 / 0.81,
 //   8000 1.56 / 1.28, 100k 2.17 / 1.78, 1M (mean growth of the child boxes
 //   1.03) 2.63 / 2.18; tubes: 1M triangles (1.09) 1.18 / 1.11, 4M (1.21) 1.22 /
-//   1.25; a 1M soup in a box 7 times its size (1.14) 3.26 / 2.81, 21 times
+//   1.25 (a 1366x768 frame of it, 16 spp, with today's loop 62.5 / 58.0 ms); a 1M
+//   soup in a box 7 times its size (1.14) 3.26 / 2.81, 21 times
 //   (1.61) 3.19 / 3.30, 61 times (4.2) 3.9 / 7.1.
-// So: from kSmallScene triangles on, up to a mean growth of 1.18. The mean is over the
-// children, not weighted by area, so that a small detailed object in a large
-// scene counts. `nbox` holds the exact internal-node boxes (root first); the
+// So: from kSmallScene triangles on, up to a mean growth of 1.25. The mean is
+// over the children, not weighted by area, so that a small detailed object in a
+// large scene counts. `nbox` holds the exact internal-node boxes (root first); the
 // growth goes to `out` (which must start at 0), read by finish_nodes_q16.
-constexpr float kQ16MaxGrowth = 1.18f;
+constexpr float kQ16MaxGrowth = 1.25f;
 solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox, BuildOut* out) {
     sc.use_qnodes = false;
     if (sc.tri_count < kSmallScene) return SOLRT_OK;
