@@ -440,10 +440,12 @@ solrt_status check_wide_depth(uint32_t width, uint32_t depth) {
 // and the relative 2^-16 widening of the far distance covers the rest (and
 // the case of farther origins, where |t| ~ |o| / |d|).
 //
-// wide: an axis that does not fit such a grid (not finite, or too large) gets
-// one that covers every coordinate below 2^115, so that the nodes stay
-// conservative; without it the grid is refused (false).
-__device__ bool q16_grid(const float4* nbox, bool wide, float g[3], float c[3]) {
+// False when an axis does not fit such a grid (not finite, or too large).
+// skip: that axis then gets the origin NaN and the cell 0, which make its
+// plane distances NaN, so that the slab test, whose minima and maxima pass
+// over NaN, decides by the other axes and the nodes stay conservative (a grid
+// wide enough for every coordinate would overflow 2^23 c / d).
+__device__ bool q16_grid(const float4* nbox, bool skip, float g[3], float c[3]) {
     const float4 blo = nbox[0], bhi = nbox[1];
     const float lo[3] = {blo.x, blo.y, blo.z}, hi[3] = {bhi.x, bhi.y, bhi.z};
     bool ok = true;
@@ -458,9 +460,9 @@ __device__ bool q16_grid(const float4* nbox, bool wide, float g[3], float c[3]) 
             if (ldexp(1.0, e) < need) ++e;
         }
         if (!fits || e > 23) ok = false;
-        if (!fits || (e > 23 && wide)) {
-            g[a] = wide ? -0x1p115f : 0.0f;
-            c[a] = wide ? 0x1p100f : 1.0f;
+        if (!fits || (e > 23 && skip)) {
+            g[a] = skip ? __int_as_float(0x7fffffff) : 0.0f;
+            c[a] = skip ? 0.0f : 1.0f;
             continue;
         }
         const double cd = ldexp(1.0, e);
@@ -492,10 +494,10 @@ __device__ __forceinline__ uint32_t q16_pair(float lo, float hi, float g, float 
 // q16_pair in FP32: the difference rounded outward by at most one unit in its
 // last place (a 256th of a cell), the scaling by the power of two exact; the
 // planes are those of q16_pair or one cell further out. (FP64 units are few on
-// this chip: 1M nodes take 15 us this way, 210 us through q16_pair.) An axis
-// of the covering grid (cell 2^100) gets its whole range.
+// this chip: 1M nodes take 15 us this way, 210 us through q16_pair.) An
+// axis without a grid (cell 0) gets the whole range.
 __device__ __forceinline__ uint32_t q16_pair_f32(float lo, float hi, float g, float c) {
-    if (c >= 0x1p100f) return 0xffff0000u;
+    if (c == 0.0f) return 0xffff0000u;
     const float ic = 1.0f / c;
     const float ql = floorf(__fsub_rd(lo, g) * ic) - 2.0f, qh = ceilf(__fsub_ru(hi, g) * ic) + 2.0f;
     const uint32_t a = (uint32_t)fminf(fmaxf(ql, 0.0f), 65535.0f), b = (uint32_t)fminf(fmaxf(qh, 0.0f), 65535.0f);
@@ -503,26 +505,29 @@ __device__ __forceinline__ uint32_t q16_pair_f32(float lo, float hi, float g, fl
 }
 
 // How much larger the quantised box of one child is than the box itself, as
-// the ratio of their surface areas, at most 16.
+// the ratio of their surface areas, at most kQ16MostGrowth.
+constexpr float kQ16MostGrowth = 16.0f;
 __device__ __forceinline__ float q16_growth(float lx, float hx, float ly, float hy, float lz, float hz, uint32_t qx,
                                             uint32_t qy, uint32_t qz, const float c[3]) {
     const float ex = hx - lx, ey = hy - ly, ez = hz - lz;
     const float fx = (float)((qx >> 16) - (qx & 0xffffu)) * c[0], fy = (float)((qy >> 16) - (qy & 0xffffu)) * c[1],
                 fz = (float)((qz >> 16) - (qz & 0xffffu)) * c[2];
     const float r = (fx * fy + fy * fz + fz * fx) / (ex * ey + ey * ez + ez * ex);
-    return r >= 1.0f ? fminf(r, 16.0f) : (r < 1.0f ? 1.0f : 16.0f);
+    return r >= 1.0f ? fminf(r, kQ16MostGrowth) : (r < 1.0f ? 1.0f : kQ16MostGrowth);
 }
 
 // The traversal's 32-byte copy of BVH2 nodes and its header (the grid of the
-// root box nbox[0..1]); `growth` receives the sum of every child's.
+// root box nbox[0..1]); `growth` receives the sum of every child's, the most
+// each where an axis has no grid.
 __global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nodes, const float4* __restrict__ nbox,
                                                   uint32_t ni, float4* __restrict__ out, float* __restrict__ growth) {
     __shared__ float s_g[3], s_c[3];
+    __shared__ bool s_ok;
     if (threadIdx.x == 0) {
-        const bool ok = q16_grid(nbox, true, s_g, s_c);
+        s_ok = q16_grid(nbox, true, s_g, s_c);
         if (blockIdx.x == 0) {
             out[0] = make_float4(s_g[0], s_g[1], s_g[2], s_c[0]);
-            out[1] = make_float4(s_c[1], s_c[2], __uint_as_float(ok ? 1u : 0u), 0.0f);
+            out[1] = make_float4(s_c[1], s_c[2], __uint_as_float(s_ok ? 1u : 0u), 0.0f);
         }
     }
     __syncthreads();
@@ -539,8 +544,9 @@ __global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nod
         uint4* o = reinterpret_cast<uint4*>(out + 2 + 2 * (size_t)i);
         o[0] = make_uint4(__float_as_uint(n3.x), __float_as_uint(n3.y), x0, y0);
         o[1] = make_uint4(z0, x1, y1, z1);
-        grow = q16_growth(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, x0, y0, z0, c) +
-               q16_growth(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, x1, y1, z1, c);
+        grow = s_ok ? q16_growth(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, x0, y0, z0, c) +
+                          q16_growth(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, x1, y1, z1, c)
+                    : 2.0f * kQ16MostGrowth;
     }
     __shared__ float s_grow[8];
     for (int off = 16; off > 0; off >>= 1) grow += __shfl_down_sync(0xffffffffu, grow, off);

@@ -100,3 +100,51 @@ def test_batch_mixing_both_node_formats(solrt, ctx):
                 alone.close()
             b.update(jobs)
         b.close()
+
+
+def _sections(counts):
+    """One soup section of each count, all with the identity instance."""
+    b = S._Builder()
+    for k, n in enumerate(counts):
+        S.soup(n, seed=20 + k, sigma=0.05, builder=b)
+    data = b.build(S.soup(1).camera, "sections")
+    data.instances = np.array([S.instance_of(np.eye(4), k) for k in range(len(counts))], S.INSTANCE_DTYPE)
+    return data
+
+
+def _moved_section(data, k, x):
+    """data's instances with section k moved by x along x."""
+    inst = data.instances.copy()
+    M = np.eye(4)
+    M[0, 3] = x
+    inst[k] = S.instance_of(M, k)
+    return inst
+
+
+@pytest.mark.parametrize("far", [1e13, 1e30, 3e38])
+@pytest.mark.parametrize("mode", ["REGEN_REBUILD", "REGEN_REFIT"])
+@pytest.mark.parametrize("graph", [False, True])
+def test_batch_launched_again_after_a_section_left_the_grid(solrt, ctx, graph, mode, far):
+    """A batch goes on with the nodes it was planned with: the sections that
+    stayed are still there when another one has moved beyond every 16-bit
+    grid."""
+    data = _sections((700, 50))
+    sc = solrt.SceneDescription(ctx, data, dynamic=True)
+    c = data.camera
+    cam = solrt.camera_look_at(c["eye"], c["center"], c["up"], c["vfov"], 1.0)
+    p = solrt.render_params(48, 48, spp=2, max_bounces=4, seed=9, miss_mode=solrt.MISS_GRADIENT,
+                            material_mode=solrt.MATERIAL_LAMBERT, rng_mode=solrt.RNG_PER_SAMPLE)
+    imgs = [solrt.Image(ctx, 48, 48) for _ in range(2)]
+    b = solrt.Batch(ctx, [(sc, imgs[0], cam, p)], graph=graph)
+    for inst in (data.instances, _moved_section(data, 1, far)):
+        sc.set_instances(inst)
+        sc.tlas_regenerate(getattr(solrt, mode))
+        for img in imgs:
+            img.clear()
+        b.launch()
+        solrt.Renderer(ctx).cmd_trace_rays(sc, cam, p, imgs[1])
+        ctx.synchronize()
+        got, want = (img.read()[0].view(np.uint32) for img in imgs)
+        assert np.array_equal(got, want)
+    b.close()
+    sc.close()
