@@ -518,13 +518,13 @@ __device__ __forceinline__ float q16_growth(float lx, float hx, float ly, float 
 
 // The traversal's 32-byte copy of BVH2 nodes and its header (the grid of the
 // root box nbox[0..1]); `growth` receives the sum of every child's, the most
-// each where an axis has no grid.
+// each where an axis has no grid or its cells are above 8 (copy_nodes_q16).
 __global__ void __launch_bounds__(256) k_q16_copy(const float4* __restrict__ nodes, const float4* __restrict__ nbox,
                                                   uint32_t ni, float4* __restrict__ out, float* __restrict__ growth) {
     __shared__ float s_g[3], s_c[3];
     __shared__ bool s_ok;
     if (threadIdx.x == 0) {
-        s_ok = q16_grid(nbox, true, s_g, s_c);
+        s_ok = q16_grid(nbox, true, s_g, s_c) && fmaxf(fmaxf(s_c[0], s_c[1]), s_c[2]) <= 8.0f;
         if (blockIdx.x == 0) {
             out[0] = make_float4(s_g[0], s_g[1], s_g[2], s_c[0]);
             out[1] = make_float4(s_c[1], s_c[2], __uint_as_float(s_ok ? 1u : 0u), 0.0f);
@@ -609,7 +609,10 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
 //   (1.61) 3.19 / 3.30, 61 times (4.2) 3.9 / 7.1.
 // So: from kSmallScene triangles on, up to a mean growth of 1.25. The mean is
 // over the children, not weighted by area, so that a small detailed object in a
-// large scene counts. `nbox` holds the exact internal-node boxes (root first); the
+// large scene counts. And cells up to 8 (coordinates up to 2^23, extents up to
+// 480,000): with larger ones the smallest direction component grows (q16_axis),
+// and rays with short axis-parallel directions would leave boxes that FP32 nodes
+// keep them in. `nbox` holds the exact internal-node boxes (root first); the
 // growth goes to `out` (which must start at 0), read by finish_nodes_q16.
 constexpr float kQ16MaxGrowth = 1.25f;
 solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox, BuildOut* out) {

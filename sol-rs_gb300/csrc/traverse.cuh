@@ -236,7 +236,8 @@ SOLRT_D float min3(float a, float b, float c) {
 // included) become +-2^-100 (sign kept) so that 1/d and o/d stay finite for
 // |o| < 2^27. Over t < 2^20 the tilt this gives a ray lying in a box plane is
 // below 2^-80, the absolute part of the face widening, so such a ray stays
-// inside the slab.
+// inside the slab; away from coordinate 0 the relative part keeps it there for
+// t up to about 2^79 (directions down to a length of 2^-79).
 SOLRT_D float box_dir(float v) { return fabsf(v) < 0x1p-100f ? copysignf(0x1p-100f, v) : v; }
 
 // 1 / v of a box-test direction component, to one unit in the last place: it
@@ -302,23 +303,44 @@ SOLRT_D void slab2_fma(const float4& n0, const float4& n1, const float4& n2, flo
 // a = (G - o) / d - 2^23 s; 2^23 + q is q placed in the mantissa of 2^23
 // (exact, one byte permute). The build quantises outward with two cells of
 // margin, which covers the rounding of a and s (see the grid rules there).
-// Direction components below 2^-80 are replaced by +-2^-80 for these tests
-// (2^23 s stays finite for cells up to 2^23).
-SOLRT_D float box_dir_q16(float v) { return fabsf(v) < 0x1p-80f ? copysignf(0x1p-80f, v) : v; }
 SOLRT_D float q16_lo(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7410u)); }
 SOLRT_D float q16_hi(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7432u)); }
+
+// s and a of one axis for a direction component of any size. A component below
+// the bound becomes plus or minus the bound, the smallest that keeps every
+// product finite: 2^-100 as box_dir's for cells up to 8 and |o| up to 2^26, so
+// that a short direction tilts no further out of its boxes here than through
+// FP32 nodes. Where s would lose bits to underflow the axis decides nothing
+// (NaN plane distances, which the slab test's minima and maxima pass over).
+SOLRT_D void q16_axis(float c, float g, float o, float d, float& s, float& a) {
+    const float least = fmaxf(fmaxf(0x1p-100f, c * 0x1p-103f), fmaxf(fabsf(o), fabsf(g)) * 0x1p-126f);
+    const float j = box_rcp(fabsf(d) < least ? copysignf(least, d) : d);
+    s = c * j;
+    a = fmaf(-8388608.0f, s, fmaf(g, j, -(o * j)));
+    if (fabsf(s) < 0x1p-110f) {
+        s = 0.0f;
+        a = __int_as_float(0x7fffffff);
+    }
+}
 
 SOLRT_D void q16_ray(const float4* header, float ox, float oy, float oz, float dx, float dy, float dz, float& sx,
                      float& sy, float& sz, float& ax, float& ay, float& az) {
     float4 g0, g1;
     ldg_2x4(header, g0, g1);
-    const float jx = box_rcp(box_dir_q16(dx)), jy = box_rcp(box_dir_q16(dy)), jz = box_rcp(box_dir_q16(dz));
-    sx = g0.w * jx;
-    sy = g1.x * jy;
-    sz = g1.y * jz;
-    ax = fmaf(-8388608.0f, sx, fmaf(g0.x, jx, -(ox * jx)));
-    ay = fmaf(-8388608.0f, sy, fmaf(g0.y, jy, -(oy * jy)));
-    az = fmaf(-8388608.0f, sz, fmaf(g0.z, jz, -(oz * jz)));
+    const float ux = fabsf(dx), uy = fabsf(dy), uz = fabsf(dz);
+    if (min3(ux, uy, uz) >= 0x1p-45f && max3(ux, uy, uz) <= 0x1p45f) {  // 2^23 c / d and o / d are ordinary numbers
+        const float jx = box_rcp(dx), jy = box_rcp(dy), jz = box_rcp(dz);
+        sx = g0.w * jx;
+        sy = g1.x * jy;
+        sz = g1.y * jz;
+        ax = fmaf(-8388608.0f, sx, fmaf(g0.x, jx, -(ox * jx)));
+        ay = fmaf(-8388608.0f, sy, fmaf(g0.y, jy, -(oy * jy)));
+        az = fmaf(-8388608.0f, sz, fmaf(g0.z, jz, -(oz * jz)));
+    } else {
+        q16_axis(g0.w, g0.x, ox, dx, sx, ax);
+        q16_axis(g1.x, g0.y, oy, dy, sy, ay);
+        q16_axis(g1.y, g0.z, oz, dz, sz, az);
+    }
 }
 
 // Both child boxes of a BVH2-q16 node (a, b: its two halves) against one

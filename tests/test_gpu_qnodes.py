@@ -102,6 +102,35 @@ def test_batch_mixing_both_node_formats(solrt, ctx):
         b.close()
 
 
+@pytest.mark.parametrize("scale,length", [(1.0, 1e-12), (1.0, 1e-18), (1.0, 1e-20), (1.0, 1e-21), (1.0, 1e-22),
+                                          (1.0, 1e-23), (1e6, 1e-20), (1.0, 1e14), (1.0, 1e25), (1.0, 1e33)])
+@pytest.mark.parametrize("kind", ["BVH2", "BVH2_Q16"])
+def test_short_and_long_axis_parallel_directions(solrt, oracle, ctx, kind, scale, length):
+    """A direction component of zero is traced as a tiny one; next to a short
+    direction that must not tilt the ray out of the boxes on its way. 1e6: a
+    scene whose grid has cells above 8."""
+    rng = np.random.default_rng(8)
+    d = _moved(2000, 0.0, scale)
+    tri = d.vertices["pos"][d.indices][:, :3].astype(np.float64).reshape(-1, 3, 3)
+    n = 1200
+    k = rng.integers(0, len(tri), n)
+    target = (tri[k] * rng.dirichlet((1, 1, 1), n)[:, :, None]).sum(1)
+    dirs = np.zeros((n, 3))
+    axis = rng.integers(0, 3, n)
+    dirs[np.arange(n), axis] = rng.choice([-1.0, 1.0], n)          # along an axis
+    dirs[n // 2:, :] += np.roll(dirs[n // 2:, :], 1, axis=1) * 0.7  # in a coordinate plane
+    rays = np.zeros(n, solrt.RAY_DTYPE)
+    rays["origin"] = target - dirs * rng.uniform(0.1, 1.5, (n, 1)) * scale
+    rays["dir"] = dirs * length
+    rays["tmax"] = 1e30
+    sc = solrt.SceneDescription(ctx, d, bvh=getattr(solrt, kind))
+    got = sc.trace_rays(rays)
+    want, _ = oracle.OracleScene(d).trace(rays, brute=True)
+    assert (want["prim"] != solrt.NO_HIT).mean() > 0.9
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    sc.close()
+
+
 def _sections(counts):
     """One soup section of each count, all with the identity instance."""
     b = S._Builder()
