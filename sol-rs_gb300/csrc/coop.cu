@@ -66,6 +66,8 @@ namespace {
 #define SOLRT_COOP_MINB 8
 #endif
 constexpr int kCoopBlock = SOLRT_COOP_BLOCK;
+static_assert(SOLRT_COOP_MINB * SOLRT_COOP_BLOCK <= (int)kMaxThreadsPerSm,
+              "more threads per SM than the contexts' traversal stacks are for");
 constexpr uint32_t kCoopSlots = stack_slots(32);  // traversal-stack entries in shared memory
 
 // Barrier state at the start of the batch's cooperative buffer (zeroed
@@ -573,7 +575,7 @@ solrt_status launch_kind(Context& ctx, const CoopArgs& args, bool nee) {
         return SOLRT_ERR_DEVICE;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ctx.sm_count * per_sm));
+    cfg.gridDim = dim3((unsigned)(ctx.sm_count * resident_blocks(per_sm, kCoopBlock)));
     cfg.blockDim = dim3(kCoopBlock);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = ctx.stream;

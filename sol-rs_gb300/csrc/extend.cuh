@@ -152,8 +152,7 @@ solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t uni
         const uint32_t most = 4u * 256u * (32u + kRayWords + state_words);
         SOLRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         SOLRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, (int)s.block, s.smem));
-        // (the stack memory of a context is for kMaxThreadsPerSm)
-        b = std::min(std::max(b, 1), (int)(kMaxThreadsPerSm / s.block));
+        b = resident_blocks(b, s.block);
         r.store(b, std::memory_order_relaxed);
     }
     const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;

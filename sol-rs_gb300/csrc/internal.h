@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/solrt.h"
+#include "launch_table.h"
 #include "traverse.cuh"
 
 namespace solrt {
@@ -206,12 +207,6 @@ struct TuneConfig {
     uint32_t smem = 32;        // shared-memory traversal stack: 16 or 32 (stack_slots entries)
     uint32_t pass_paths = 0;   // paths per batch pass (0 = the path capacity)
 };
-
-// Threads of the largest resident grid per SM, and the stack entries of each
-// kept in Context::deep_stack: those from the smallest number of shared slots
-// up.
-constexpr uint32_t kMaxThreadsPerSm = 1536;
-constexpr uint32_t kMinStackSlots = 12;
 
 // Traversal-stack entries per thread that a tuned shared-memory size keeps on
 // the SM. More than 16 buys nothing (rays of a 1M-triangle tree hold at most
