@@ -3,7 +3,6 @@
 #pragma once
 
 #include <algorithm>
-#include <atomic>
 
 #include "bvh2_2l.cuh"
 #include "bvh2_ww.cuh"
@@ -143,18 +142,16 @@ solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t uni
     s.block = ctx.tune.block;
     s.slots = kind_has_smem_stack<KIND>() ? stack_slots(ctx.tune.smem) : 0u;
     s.smem = 4u * s.block * (s.slots + kRayWords + state_words);
-    // resident blocks per SM of this kernel for each of the six shapes: a
-    // property of the compiled kernel, looked up once (0 = not yet)
-    static std::atomic<int> resident[6];
-    std::atomic<int>& r = resident[(s.block == 64 ? 0 : s.block == 128 ? 2 : 4) + (ctx.tune.smem == 16 ? 0 : 1)];
-    int b = r.load(std::memory_order_relaxed);
-    if (b == 0) {
+    static LaunchTable table;
+    const int shape = (s.block == 64 ? 0 : s.block == 128 ? 2 : 4) + (ctx.tune.smem == 16 ? 0 : 1);
+    const auto query = [&](int* fits) -> solrt_status {
         const uint32_t most = 4u * 256u * (32u + kRayWords + state_words);
         SOLRT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-        SOLRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, (int)s.block, s.smem));
-        b = resident_blocks(b, s.block);
-        r.store(b, std::memory_order_relaxed);
-    }
+        SOLRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(fits, kern, (int)s.block, s.smem));
+        return SOLRT_OK;
+    };
+    int b = 0;
+    SOLRT_TRY(table.blocks(ctx.device, shape, s.block, query, &b));
     const uint32_t full = (uint32_t)ctx.sm_count * (uint32_t)b;
     const uint32_t warps = full * (s.block / 32u);
     s.lanes = spread && units <= spread_units<KIND>() ? std::min(32u, std::max(1u, (units + warps - 1u) / warps)) : 32u;

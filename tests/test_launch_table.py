@@ -30,3 +30,25 @@ def test_cooperative_kernel_with_more_threads_is_refused(tmp_path):
                        "-x", "cu", "-c", os.path.join(build.CSRC, "coop.cu"), "-o", str(tmp_path / "coop.o")],
                        capture_output=True, text=True)
     assert r.returncode != 0 and "traversal stacks" in r.stderr
+
+
+def test_every_device_is_asked_for_once(tmp_path):
+    """Occupancy and kernel attributes are per device: a second device of the
+    process is looked up (and its attribute set) like the first, once per
+    shape; a failed lookup is tried again."""
+    out = _run(tmp_path, """
+    static LaunchTable t;
+    int asked = 0, b = 0;
+    const auto query = [&](int n, int status) { return [&asked, n, status](int* fits) { ++asked; *fits = n; return status; }; };
+    const auto get = [&](int dev, int shape, int n, int status) {
+        const int s = t.blocks(dev, shape, 128u, query(n, status), &b);
+        std::printf("%d,%d,%d ", s, s ? -1 : b, asked);
+    };
+    get(0, 2, 5, 0); get(0, 2, 9, 0);                    // one lookup
+    get(1, 2, 7, 0); get(1, 2, 9, 0); get(0, 2, 9, 0);   // the second device has its own
+    get(0, 3, 6, 0); get(1, 3, 8, 0);                    // and its own per shape
+    get(2, 0, 4, 3); get(2, 0, 4, 0); get(2, 0, 9, 0);   // an error is not kept
+    get(63, 5, 30, 0); get(64, 5, 4, 0); get(64, 5, 3, 0);  // clamped; past the table: asked each time
+    """)
+    assert out == ["0,5,1", "0,5,1", "0,7,2", "0,7,2", "0,5,2", "0,6,3", "0,8,4", "3,-1,5", "0,4,6", "0,4,6",
+                   "0,12,7", "0,4,8", "0,3,9"]
