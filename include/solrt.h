@@ -670,8 +670,11 @@ solrt_status solrt_trace_rays_device(solrt_context* ctx, solrt_scene* scene,
  * miss colour and gamma (see the tests); 8 = the bounded wait of the
  * cooperative batch's grid barrier: a cooperative grid in which one block
  * never arrives, each wait limited to in_f32[0] seconds (at most 10), its
- * error flags -> out_u32[0] (SOLRT_EFLAG_TIMEOUT when the waits gave up).
- * Synchronises. */
+ * error flags -> out_u32[0] (SOLRT_EFLAG_TIMEOUT when the waits gave up);
+ * 9 = lets the b[0]-th next call of a kind fail on the calling host thread,
+ * once (0: none): a[0] = 0 a device allocation, 1 a traversal launch; what was
+ * left of the previous count -> out_u32[0].
+ * Synchronises (0-8). */
 solrt_status solrt_debug_unit(solrt_context* ctx, uint32_t op, uint32_t n, const uint32_t* a,
                               const uint32_t* b, const float* in_f32, uint32_t* out_u32,
                               float* out_f32);

@@ -40,6 +40,15 @@ namespace solrt {
 
 namespace {
 thread_local std::string g_last_error;
+thread_local uint32_t g_fault[kFaultSites];
+}  // namespace
+
+bool host_fault(HostFault site) { return g_fault[site] != 0u && --g_fault[site] == 0u; }
+
+uint32_t set_host_fault(HostFault site, uint32_t nth) {
+    const uint32_t left = g_fault[site];
+    g_fault[site] = nth;
+    return left;
 }
 
 void set_error(const char* fmt, ...) {

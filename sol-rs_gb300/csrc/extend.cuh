@@ -139,6 +139,10 @@ struct LaunchShape {
 
 template <int KIND, auto kern>
 solrt_status launch_shape(const Context& ctx, uint32_t state_words, uint32_t units, bool spread, LaunchShape& s) {
+    if (host_fault(kFaultLaunch)) {
+        set_error("launch refused by a test");
+        return SOLRT_ERR_DEVICE;
+    }
     s.block = ctx.tune.block;
     s.slots = kind_has_smem_stack<KIND>() ? stack_slots(ctx.tune.smem) : 0u;
     s.smem = 4u * s.block * (s.slots + kRayWords + state_words);

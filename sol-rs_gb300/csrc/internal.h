@@ -16,6 +16,14 @@ namespace solrt {
 
 void set_error(const char* fmt, ...);
 
+// Calls that a test lets fail on the host (solrt_debug_unit op 9).
+enum HostFault : uint32_t { kFaultAlloc = 0, kFaultLaunch = 1, kFaultSites = 2 };
+// Whether the call at hand is the one that this thread was told to let fail.
+bool host_fault(HostFault site);
+// The `nth` call from now on fails, once (0: none). Returns what was left of
+// the count before.
+uint32_t set_host_fault(HostFault site, uint32_t nth);
+
 // Returns from the calling function with SOLRT_ERR_DEVICE on a CUDA error.
 #define SOLRT_CUDA(call)                                                              \
     do {                                                                              \
@@ -63,7 +71,7 @@ struct DeviceBuffer {
         if (n <= bytes && ptr) return SOLRT_OK;
         release();
         if (n == 0) return SOLRT_OK;
-        cudaError_t e = cudaMalloc(&ptr, n);
+        const cudaError_t e = host_fault(kFaultAlloc) ? cudaErrorMemoryAllocation : cudaMalloc(&ptr, n);
         if (e != cudaSuccess) {
             ptr = nullptr;
             set_error("cudaMalloc(%zu): %s", n, cudaGetErrorString(e));

@@ -694,13 +694,9 @@ DevJob make_job(const Scene& sc, uint32_t kind, const Image& img, const solrt_ca
     return J;
 }
 
-// One pass on the context stream: generate, (extend, shade) x bounces, then
-// its pixels (`resolve`: sums and finished images; else, for served jobs, the
-// sums alone). `single`: of a.job and a.item, else of the tables.
-solrt_status issue_pass(Context& ctx, uint32_t kind, PassArgs a, bool single, bool nee, bool resolve,
-                        bool record_timing) {
+solrt_status issue_stages(Context& ctx, uint32_t kind, PassArgs a, bool single, bool nee, bool resolve,
+                          bool record_timing) {
     cudaStream_t st = ctx.stream;
-    if (nee && !ctx.q_o[2].ptr) { set_error("shadow queue not allocated"); return SOLRT_ERR_INVALID; }
     a.capacity = ctx.capacity;
     a.count = ctx.queue_counts.as<unsigned int>();
     a.scount = a.count + SOLRT_MAX_BOUNCES + 2;
@@ -745,6 +741,23 @@ solrt_status issue_pass(Context& ctx, uint32_t kind, PassArgs a, bool single, bo
     ++ctx.launches;
     SOLRT_CUDA(cudaGetLastError());
     return SOLRT_OK;
+}
+
+// One pass on the context stream: generate, (extend, shade) x bounces, then
+// its pixels (`resolve`: sums and finished images; else, for served jobs, the
+// sums alone). `single`: of a.job and a.item, else of the tables.
+solrt_status issue_pass(Context& ctx, uint32_t kind, const PassArgs& a, bool single, bool nee, bool resolve,
+                        bool record_timing) {
+    if (nee && !ctx.q_o[2].ptr) { set_error("shadow queue not allocated"); return SOLRT_ERR_INVALID; }
+    const solrt_status s = issue_stages(ctx, kind, a, single, nee, resolve, record_timing);
+    if (s != SOLRT_OK) {
+        // the last launch of a pass zeroes the queue counts; one that ended
+        // before it leaves them set (not while the launches were only recorded)
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(ctx.stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
+            cudaMemsetAsync(ctx.queue_counts.ptr, 0, ctx.queue_counts.bytes, ctx.stream);
+    }
+    return s;
 }
 
 PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp) {
@@ -1371,6 +1384,14 @@ solrt_status debug_unit(Context& ctx, uint32_t op, uint32_t n, const uint32_t* a
             return SOLRT_ERR_INVALID;
         }
         return coop_wait_test(ctx, in_f32[0], out_u32);
+    }
+    if (op == 9) {  // the b[0]-th host call of site a[0] fails; what was left of the last count -> out_u32[0]
+        if (!a || !b || !out_u32 || a[0] >= kFaultSites) {
+            set_error("debug op 9 needs a site, a count and an output word");
+            return SOLRT_ERR_INVALID;
+        }
+        out_u32[0] = set_host_fault((HostFault)a[0], b[0]);
+        return SOLRT_OK;
     }
     if (op > 7) {
         set_error("unknown debug op %u", op);
