@@ -613,13 +613,17 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
 // 480,000): with larger ones the smallest direction component grows (q16_axis),
 // and rays with short axis-parallel directions would leave boxes that FP32 nodes
 // keep them in. `nbox` holds the exact internal-node boxes (root first); the
-// growth goes to `out` (which must start at 0), read by finish_nodes_q16.
+// growth goes to `out` (which must start at 0), read by finish_nodes_q16. A scene
+// for whose copy there is no memory keeps its 64-byte nodes.
 constexpr float kQ16MaxGrowth = 1.25f;
 solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox, BuildOut* out) {
     sc.use_qnodes = false;
     if (sc.tri_count < kSmallScene) return SOLRT_OK;
     const uint32_t ni = sc.info.node_count;
-    SOLRT_TRY(sc.qnodes.alloc(32ull * ((size_t)ni + 1)));
+    if (sc.qnodes.alloc(32ull * ((size_t)ni + 1)) != SOLRT_OK) {
+        cudaGetLastError();
+        return SOLRT_OK;
+    }
     k_q16_copy<<<blocks_for(ni, 256), 256, 0, ctx.stream>>>(sc.nodes.as<float4>(), nbox, ni, sc.qnodes.as<float4>(),
                                                            &out->growth);
     ++ctx.launches;
@@ -628,7 +632,7 @@ solrt_status copy_nodes_q16(Context& ctx, Scene& sc, const float4* nbox, BuildOu
 }
 
 void finish_nodes_q16(Scene& sc, const BuildOut& out) {
-    sc.use_qnodes = sc.info.kind == SOLRT_BVH2 && sc.tri_count >= kSmallScene &&
+    sc.use_qnodes = sc.info.kind == SOLRT_BVH2 && sc.tri_count >= kSmallScene && sc.qnodes.ptr &&
                     out.growth <= kQ16MaxGrowth * 2.0f * (float)sc.info.node_count;
 }
 

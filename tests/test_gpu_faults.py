@@ -75,3 +75,86 @@ def test_batch_after_a_failed_launch(solrt, ctx, graph):
     assert np.array_equal(img.read()[0].view(np.uint32), alone.read()[0].view(np.uint32))
     b.close()
     sc.close()
+
+
+def _rays(data, n=2000):
+    rng = np.random.default_rng(4)
+    rays = np.zeros(n, [("origin", "<f4", 3), ("tmin", "<f4"), ("dir", "<f4", 3), ("tmax", "<f4")])
+    rays["origin"] = rng.uniform(-0.2, 1.2, (n, 3))
+    d = rng.normal(size=(n, 3))
+    rays["dir"] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    rays["tmax"] = 1e4
+    return rays
+
+
+def test_every_allocation_of_a_build_may_fail(solrt, oracle):
+    """Without memory for the 32-byte copy of its nodes a BVH2 scene keeps the
+    64-byte ones; any other missing array is SOLRT_ERR_OOM, and the next
+    creation works."""
+    data = S.soup(1500, seed=3, sigma=0.05)
+    rays = _rays(data)
+    want, _ = oracle.OracleScene(data).trace(rays.view(solrt.RAY_DTYPE), brute=True)
+    sizes = {}
+    for nth in range(1, 100):
+        c = solrt.Context(0, path_capacity=1 << 16)
+        _let_fail(c, ALLOC, nth)
+        try:
+            sc = solrt.SceneDescription(c, data)
+        except solrt.SolrtError as e:
+            assert e.status == 2
+            assert _let_fail(c, ALLOC, 0) == 0
+            sc = solrt.SceneDescription(c, data)
+        else:
+            left = _let_fail(c, ALLOC, 0)
+            sizes[nth] = (left, sc.device_bytes())
+        assert np.array_equal(sc.trace_rays(rays.view(solrt.RAY_DTYPE)).view(np.uint32), want.view(np.uint32))
+        sc.close()
+        c.close()
+        if sizes.get(nth, (0, 0))[0]:
+            break
+    *without, last = sorted(sizes)  # last: no allocation failed
+    assert len(without) == 1 and sizes[without[0]] == (0, sizes[last][1] - 32 * 1500)
+
+
+def test_moving_scene_without_memory_for_the_copy(solrt, ctx):
+    """Refits and rebuilds of a scene that was created without the copy take it
+    once there is memory, and render the same either way."""
+    b = S._Builder()
+    for k in range(2):
+        S.soup(600, seed=7 + k, sigma=0.05, builder=b)
+    data = b.build(S.soup(1).camera, "two")
+    data.instances = np.array([S.instance_of(np.eye(4), k) for k in range(2)], S.INSTANCE_DTYPE)
+    plain = solrt.SceneDescription(ctx, data, dynamic=True)
+    full = plain.device_bytes()
+    cam = camera_of(data, 1.0)
+    p = solrt.render_params(40, 40, spp=2, max_bounces=3, seed=5, material_mode=solrt.MATERIAL_LAMBERT,
+                            rng_mode=solrt.RNG_PER_SAMPLE)
+    for nth in range(1, 100):
+        c = solrt.Context(0, path_capacity=1 << 16)
+        _let_fail(c, ALLOC, nth)
+        try:
+            sc = solrt.SceneDescription(c, data, dynamic=True)
+        except solrt.SolrtError:
+            sc = None
+        assert _let_fail(c, ALLOC, 0) == 0
+        if sc:
+            break
+        c.close()
+    assert sc.device_bytes() == full - 32 * 1200
+    want = solrt.Image(ctx, 40, 40)
+    solrt.Renderer(ctx).cmd_trace_rays(plain, cam, p, want)
+    img = solrt.Image(c, 40, 40)
+    for mode, refuse in ((solrt.REGEN_REFIT, True), (solrt.REGEN_REBUILD, False), (solrt.REGEN_REFIT, False)):
+        sc.set_instances(data.instances)
+        _let_fail(c, ALLOC, 1 if refuse else 0)
+        sc.tlas_regenerate(mode)
+        _let_fail(c, ALLOC, 0)
+        img.clear()
+        solrt.Renderer(c).cmd_trace_rays(sc, cam, p, img)
+        c.synchronize()
+        ctx.synchronize()
+        assert np.array_equal(img.read()[0].view(np.uint32), want.read()[0].view(np.uint32))
+    assert sc.device_bytes() == full
+    sc.close()
+    c.close()
+    plain.close()
