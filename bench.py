@@ -292,7 +292,7 @@ def precision_study(local, data, kw, cam, main_mrays, main_info, main_nodes, mai
     all_kinds = (("bvh2_fp32", solrt.BVH2, False), ("bvh2_treelet", solrt.BVH2, True), ("bvh2_q16", solrt.BVH2_Q16, False),
                  ("bvh4_q8", solrt.BVH4_Q8, False), ("bvh8_q8", solrt.BVH8_Q8, False),
                  ("bvh8_q8_sah", solrt.BVH8_Q8, True), ("bvh8_fp32", solrt.BVH8_F32, False))
-    with solrt.Context(local, enable_timing=True, path_capacity=capacity) as ctx, \
+    with solrt.Context(local, path_capacity=capacity) as ctx, \
             solrt.Context(local, enable_counters=True) as cctx:
         for name, kind, sah in all_kinds:
             if kinds is not None and name not in kinds:
@@ -925,7 +925,7 @@ def main():
         cimg.close()
         csc.close()
 
-    ctx = solrt.Context(local, enable_timing=True, path_capacity=args.capacity)
+    ctx = solrt.Context(local, path_capacity=args.capacity)
     ctx_capacity = ctx.capacity()
     spp_per_pass = max(1, min(kw["spp"], ctx_capacity // (W * H)))
     passes_per_step = -(-kw["spp"] // spp_per_pass)
@@ -1006,20 +1006,39 @@ def main():
             regen[name + "_ms"] = round(float(np.median(ts[1:])), 3)
         dyn.close()
 
+    # the stages of the same frames, in a context that times every launch
+    if args.kernel != "mega":
+        with solrt.Context(local, enable_timing=True, path_capacity=args.capacity) as tctx:
+            tsc = solrt.SceneDescription(tctx, data, bvh=bvh, sah=args.sah, keep_data=False)
+            timg = solrt.Image(tctx, W, H, kw["accum_mode"])
+            tr = solrt.Renderer(tctx)
+            for i in range(1 + args.steps):
+                if i == 1:
+                    tctx.synchronize()
+                    tctx.reset_stats()
+                tr.cmd_trace_rays(tsc, cam, solrt.render_params(**dict(kw, frame=args.warmup + i)), timg)
+            tctx.synchronize()
+            ts = tctx.stats()
+            timg.close()
+            tsc.close()
+    else:
+        ts = st
+
     # roofline of the extend kernel
     peak, peak_kind = peaks()
     b_seg = 32 + 16 + NODE_BYTES[info.kind] * nodes_per_seg + 48 * tris_per_seg
-    ext_s = st.extend_ms / 1000.0
+    ext_s = ts.extend_ms / 1000.0
+    stages_ms = ts.generate_ms + ts.extend_ms + ts.shade_ms + ts.accumulate_ms
     if args.kernel == "mega":  # traversal and shading in one launch: the whole render time
         ext_s = ms / 1000.0
     # extend launches also trace the shadow rays of --nee (same bytes per ray assumed)
-    achieved = ((st.segments + st.shadow_segments) * b_seg) / ext_s / 1e9 if ext_s > 0 else 0.0
+    achieved = ((ts.segments + ts.shadow_segments) * b_seg) / ext_s / 1e9 if ext_s > 0 else 0.0
     traffic = dram = None
     cap = EXTEND_CAPTURES.get((args.workload, "treelet" if args.sah else "lbvh"))
     if cap and info.kind == solrt.BVH2 and args.kernel != "mega" and not args.nee and ext_s > 0:
-        seg_per_launch = st.segments / max(st.extend_launches, 1)
+        seg_per_launch = ts.segments / max(ts.extend_launches, 1)
         traffic = round(cap["dram_bytes_per_segment"] * seg_per_launch)
-        dram_gbs = cap["dram_bytes_per_segment"] * st.segments / ext_s / 1e9
+        dram_gbs = cap["dram_bytes_per_segment"] * ts.segments / ext_s / 1e9
         dram = {"bytes_per_segment": cap["dram_bytes_per_segment"], "gbs": round(dram_gbs, 1),
                 "frac": round(dram_gbs / peak, 4), "source": cap["dram_source"],
                 "how": "ncu DRAM bytes per segment of this workload's extend launches x this run's segments / "
@@ -1035,12 +1054,12 @@ def main():
                 "kernel": "k_megakernel (traversal + shading, whole render time)" if args.kernel == "mega"
                           else "k_extend (BVH traversal)", "bytes_per_segment": round(b_seg, 1),
                 "nodes_per_segment": round(nodes_per_seg, 2), "tris_per_segment": round(tris_per_seg, 2),
-                "extend_ms_per_launch": round(st.extend_ms / max(st.extend_launches, 1), 4),
-                "stage_ms_per_step": {"generate": round(st.generate_ms / args.steps, 3),
-                                      "extend": round(st.extend_ms / args.steps, 3),
-                                      "shade": round(st.shade_ms / args.steps, 3),
-                                      "accumulate_finalize": round(st.accumulate_ms / args.steps, 3)},
-                "extend_share_of_step": round(st.extend_ms / ms, 4) if ms > 0 else None}
+                "extend_ms_per_launch": round(ts.extend_ms / max(ts.extend_launches, 1), 4),
+                "stage_ms_per_step": {"generate": round(ts.generate_ms / args.steps, 3),
+                                      "extend": round(ts.extend_ms / args.steps, 3),
+                                      "shade": round(ts.shade_ms / args.steps, 3),
+                                      "accumulate_finalize": round(ts.accumulate_ms / args.steps, 3)},
+                "extend_share_of_step": round(ts.extend_ms / stages_ms, 4) if stages_ms > 0 else None}
     if args.workload == "cornell":
         # a 32-triangle scene lives in L1 / L2: the HBM fraction says nothing,
         # so the same achieved bytes are set against the L2 copy bandwidth

@@ -261,7 +261,8 @@ typedef enum solrt_integrator {
 typedef enum solrt_kernel {
     /* generate / extend / shade stages over queues shared by all paths; frames
      * with few rays per bounce level run the same steps in one launch whose
-     * warps keep their paths to the end (same image) */
+     * warps keep their paths to the end (same image), unless the context
+     * counts visits or times stages */
     SOLRT_KERNEL_WAVEFRONT = 0,
     /* the reference's structure (pathtrace.rgen:39-104): one thread per pixel
      * loops over its samples and bounces; same image, the plain kernel that
@@ -333,7 +334,8 @@ typedef struct solrt_context_desc {
     uint32_t path_capacity;      /* paths in flight per pass; 0 = default (32M, 4.8 GB of queues) */
     uint32_t enable_counters;    /* 1 = count node visits / triangle tests */
     uint32_t block_size;         /* extend kernel block size; 0 = default */
-    uint32_t enable_timing;      /* 1 = CUDA-event timing of every extend / shade launch */
+    uint32_t enable_timing;      /* 1 = CUDA-event timing of every extend / shade launch (frames of
+                                    any size then run stage by stage) */
     uint32_t reserved[3];
 } solrt_context_desc;
 

@@ -793,7 +793,7 @@ PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp
 //   89, 102k: 136 / 153, 160k: 184 / 231; meshes 102k: 236 / 212, 160k: 282 /
 //   299 and 536 / 601.
 bool path_kernel_pays(const Context& ctx, const Scene& sc, const DevJob& J, uint64_t paths) {
-    if (ctx.counters) return false;  // node and triangle counts: wavefront only
+    if (ctx.counters || ctx.timing) return false;  // node and triangle counts, times per stage: wavefront only
     const uint64_t levels = J.max_bounces + 1ull;
     const uint64_t per_level = levels > 4 ? paths * 4 / levels : paths;
     const bool small = J.sc.tri_count < kSmallScene;
@@ -838,16 +838,12 @@ solrt_status issue_frame(Context& ctx, const Scene& sc, uint32_t kind, const Dev
             pa.deep = ctx.deep_stack.as<int>();
             pa.rad = ctx.rad.as<float4>();
             pa.stats = ctx.stats.as<DevStats>();
-            const int te = ctx.timing_begin(0);
             SOLRT_TRY(nee ? launch_paths_nee(ctx, kind, pa) : launch_paths(ctx, kind, pa));
-            ctx.timing_end(te);
             a.rad = pa.rad;
             a.count = a.scount = ctx.queue_counts.as<unsigned int>();
             PassArgs r = a;
             r.bounces = 0;
-            const int ta = ctx.timing_begin(3);
             k_resolve<true><<<cdiv(npix, 256), 256, 0, ctx.stream>>>(r);
-            ctx.timing_end(ta);
             ++ctx.launches;
             SOLRT_CUDA(cudaGetLastError());
         }

@@ -143,3 +143,29 @@ def test_rays_on_both_sides_of_the_spread_limit(solrt, oracle, ctx, bvh, n):
     want, _ = oracle.OracleScene(data, two_level=bvh == "bvh2t").trace(rays, brute=True)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
     sc.close()
+
+
+@pytest.mark.parametrize("mode", ["lambert", "nee"])
+def test_timing_contexts_time_every_stage(solrt, ctx, mode):
+    """A context that times its launches renders small frames stage by stage
+    too, so that the stages have their launches and times; same image."""
+    data = S.cornell()
+    kw = {k: getattr(solrt, v) if isinstance(v, str) else v for k, v in MODES[mode].items()}
+    cam = solrt.camera_look_at(*(data.camera[k] for k in ("eye", "center", "up", "vfov")), 1.0)
+    p = solrt.render_params(60, 60, spp=2, seed=3, **kw)
+    imgs = []
+    with solrt.Context(0, path_capacity=1 << 16, enable_timing=True) as timed:
+        for c in (timed, ctx):
+            sc, img = solrt.SceneDescription(c, data), solrt.Image(c, 60, 60)
+            c.reset_stats()
+            solrt.Renderer(c).cmd_trace_rays(sc, cam, p, img)
+            c.synchronize()
+            st = c.stats()
+            imgs.append(img.read()[0].view(np.uint32).copy())
+            if c is timed:
+                shadow = 5 if mode == "nee" else 0
+                assert (st.extend_launches, st.shade_launches) == (6 + shadow, 6 + shadow)
+                assert min(st.extend_ms, st.shade_ms, st.generate_ms, st.accumulate_ms) > 0.0
+            img.close()
+            sc.close()
+    assert np.array_equal(*imgs)
