@@ -786,21 +786,29 @@ PassArgs table_pass(const DevJob* jobs, const DevItem* items, const PassPlan& pp
 //   1472 (2000 triangles), 63k: 23902 / 18836 (150k), 111k: 30251 / 26188;
 //   next-event estimation (its light-tree walks hold up the other lanes): 25k:
 //   1853 / 907, 40k: 2086 / 1393;
-//   moving scenes, whose rebuild waits for the device before every frame, so
-//   that no other frame fills the ends of the launches: 415k: 2431 / 1998
-//   with the rebuild, 830k: 2786 / 2372;
 //   the wide kinds, whose refills find fewer lanes idle: Cornell box 68k: 102 /
 //   89, 102k: 136 / 153, 160k: 184 / 231; meshes 102k: 236 / 212, 160k: 282 /
-//   299 and 536 / 601.
+//   299 and 536 / 601; moving ones (262k triangles) 200k: 487 / 461, 400k: 675 /
+//   731, 829k: 1074 / 1210 with the camera alone moving, 1857 / 2044, 2046 /
+//   2256, 2401 / 2731 with the rebuild.
+// Moving binary scenes have the larger limit: a program that moves one scene
+// waits for each frame before it rebuilds for the next, so that no other frame
+// fills the ends of the launches, and there one frame gains more than three in
+// flight lose. Alone, with the rebuild: 8k triangles 829k: 671 / 496, 2949k:
+// 1021 / 854; 262k 829k: 1873 / 1486, 1474k: 2281 / 2034, 2949k: 3275 / 3258; 1M
+// 829k: 3068 / 2399, 2211k: 4563 / 4380, 2949k: 5326 / 5468. Three in flight: 8k
+// 829k: 336 / 373, 2949k: 697 / 731; 262k 829k: 1089 / 1223, 2949k: 2613 / 2996; 1M
+// 829k: 2102 / 2087, 2949k: 4547 / 5181; with the camera alone moving 8k 829k: 237 /
+// 206, 262k: 938 / 973, 1M: 1636 / 1590.
 bool path_kernel_pays(const Context& ctx, const Scene& sc, const DevJob& J, uint64_t paths) {
     if (ctx.counters || ctx.timing) return false;  // node and triangle counts, times per stage: wavefront only
     const uint64_t levels = J.max_bounces + 1ull;
     const uint64_t per_level = levels > 4 ? paths * 4 / levels : paths;
     const bool small = J.sc.tri_count < kSmallScene;
     if (J.integrator == SOLRT_INTEGRATOR_PATH_NEE) return per_level <= (small ? 73728 : 57344);
-    if (sc.dynamic && sc.info.kind != SOLRT_BVH2_TWO_LEVEL) return per_level <= 917504;
     const uint32_t k = sc.info.kind;
     if (k == SOLRT_BVH8_Q8 || k == SOLRT_BVH8_F32 || k == SOLRT_BVH4_Q8) return per_level <= (small ? 73728 : 114688);
+    if (sc.dynamic && k != SOLRT_BVH2_TWO_LEVEL) return per_level <= 917504;
     return per_level <= (small ? 180224 : 229376);
 }
 

@@ -169,3 +169,52 @@ def test_timing_contexts_time_every_stage(solrt, ctx, mode):
             img.close()
             sc.close()
     assert np.array_equal(*imgs)
+
+
+def _launches(solrt, ctx, sc, data, w, h, bounces):
+    """Kernels of one frame: the path kernel and the resolve, or two per bounce
+    level, the generate and the resolve."""
+    cam = solrt.camera_look_at(*(data.camera[k] for k in ("eye", "center", "up", "vfov")), w / h)
+    img = solrt.Image(ctx, w, h)
+    p = solrt.render_params(w, h, spp=1, max_bounces=bounces, seed=3, material_mode=solrt.MATERIAL_LAMBERT,
+                            rng_mode=solrt.RNG_PER_SAMPLE)
+    ctx.reset_stats()
+    solrt.Renderer(ctx).cmd_trace_rays(sc, cam, p, img)
+    ctx.synchronize()
+    n = ctx.stats().launches
+    img.close()
+    return int(n)
+
+
+@pytest.mark.parametrize("dynamic", [False, True])
+@pytest.mark.parametrize("kind", ["BVH8_Q8", "BVH4_Q8", "BVH8_F32"])
+def test_wide_kinds_have_their_limits_when_they_move_too(solrt, ctx, kind, dynamic):
+    for data, side in ((S.cornell(), (288, 256)), (S.soup(2000, seed=3, sigma=0.03), (512, 224))):
+        sc = solrt.SceneDescription(ctx, data, bvh=getattr(solrt, kind), dynamic=dynamic)
+        w, h = side  # 73,728 and 114,688 rays per level
+        assert _launches(solrt, ctx, sc, data, w, h, 3) == 2
+        assert _launches(solrt, ctx, sc, data, w + 1, h, 3) == 2 + 2 * 4
+        _both(solrt, ctx, sc, data, w, h, 1, "kahan", frames=1)
+        _both(solrt, ctx, sc, data, w + 1, h, 1, "kahan", frames=1)
+        sc.close()
+
+
+@pytest.mark.parametrize("w", [1024, 1025])
+def test_moving_scene_on_both_sides_of_its_limit(solrt, ctx, w):
+    """917,504 rays per level: the path kernel up to it, the stages above."""
+    data = S.soup(2000, seed=3, sigma=0.03)
+    sc = solrt.SceneDescription(ctx, data, dynamic=True)
+    sc.tlas_regenerate()
+    assert _launches(solrt, ctx, sc, data, w, 896, 3) == (2 if w == 1024 else 10)
+    _both(solrt, ctx, sc, data, w, 896, 1, "kahan", frames=1)
+    sc.close()
+
+
+@pytest.mark.parametrize("w", [512, 513])
+def test_per_pixel_streams_on_both_sides_of_the_limit(solrt, ctx, w):
+    """225,280 and 225,720 pixels over 5 levels: 180,224 and 180,576 rays per level."""
+    data = S.cornell()
+    sc = solrt.SceneDescription(ctx, data)
+    assert _launches(solrt, ctx, sc, data, w, 440, 4) == (2 if w == 512 else 12)
+    _both(solrt, ctx, sc, data, w, 440, 2, "kahan_stream", frames=1)
+    sc.close()
