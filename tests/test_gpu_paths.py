@@ -218,3 +218,32 @@ def test_per_pixel_streams_on_both_sides_of_the_limit(solrt, ctx, w):
     assert _launches(solrt, ctx, sc, data, w, 440, 4) == (2 if w == 512 else 12)
     _both(solrt, ctx, sc, data, w, 440, 2, "kahan_stream", frames=1)
     sc.close()
+
+
+@pytest.mark.parametrize("mode", ["lambert", "stream", "kahan", "kahan_stream", "nee", "nee_stream"])
+def test_stages_in_several_passes(solrt, ctx, mode):
+    """The frames of test_render_in_several_passes through the stages (a
+    counting context takes no path kernel): pixel chunks, several passes of
+    samples, and shadow rays with both."""
+    data = S.cornell()
+    kw = {k: getattr(solrt, v) if isinstance(v, str) else v for k, v in MODES[mode].items()}
+    cam = solrt.camera_look_at(*(data.camera[k] for k in ("eye", "center", "up", "vfov")), 1.0)
+    out = []
+    for cap in (0, 1000, 3000, 7000):
+        with (solrt.Context(0, path_capacity=cap, enable_counters=True) if cap
+              else solrt.Context(0, path_capacity=1 << 16)) as c:
+            sc = solrt.SceneDescription(c, data)
+            img = solrt.Image(c, 50, 50, kw.get("accum_mode", solrt.ACCUM_REF_MIX))
+            c.reset_stats()
+            for f in range(2):
+                p = solrt.render_params(50, 50, spp=5, seed=3, frame=f, **kw)
+                solrt.Renderer(c).cmd_trace_rays(sc, cam, p, img)
+            c.synchronize()
+            st = c.stats()
+            if cap:
+                assert st.launches > 2 * 2 * (kw["max_bounces"] + 1)
+            out.append((img.read()[0].view(np.uint32).copy(), st.segments, st.shadow_segments, st.shadow_unoccluded))
+            img.close()
+            sc.close()
+    for o in out[1:]:
+        assert np.array_equal(o[0], out[0][0]) and o[1:] == out[0][1:]
