@@ -675,7 +675,9 @@ solrt_status solrt_trace_rays_device(solrt_context* ctx, solrt_scene* scene,
  * error flags -> out_u32[0] (SOLRT_EFLAG_TIMEOUT when the waits gave up);
  * 9 = lets the b[0]-th next call of a kind fail on the calling host thread,
  * once (0: none): a[0] = 0 a device allocation, 1 a traversal launch; what was
- * left of the previous count -> out_u32[0].
+ * left of the previous count -> out_u32[0]; 10 = the solrt_bvh_kind of the nodes
+ * that the context's last traversal launch reads -> out_u32[0] (a BVH2 scene's
+ * may be its 32-byte copy, SOLRT_BVH2_Q16; per-pixel path kernels apart).
  * Synchronises (0-8). */
 solrt_status solrt_debug_unit(solrt_context* ctx, uint32_t op, uint32_t n, const uint32_t* a,
                               const uint32_t* b, const float* in_f32, uint32_t* out_u32,

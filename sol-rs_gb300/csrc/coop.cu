@@ -607,6 +607,7 @@ solrt_status launch_batch_coop(Context& ctx, uint32_t kind, const DevJob* jobs, 
                                const PassPlan* passes, uint32_t npasses, uint32_t ctr_stride, const uint32_t* job_pix,
                                uint32_t njobs, uint32_t total_pix, void* coop, bool nee) {
     SOLRT_CUDA(cudaMemsetAsync(coop, 0, coop_buffer_bytes(npasses, ctr_stride), ctx.stream));
+    ctx.last_kind = kind;
     CoopArgs a;
     a.jobs = jobs;
     a.items = items;

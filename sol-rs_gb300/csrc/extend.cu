@@ -90,6 +90,7 @@ bool extend_variant_ok(uint32_t block, uint32_t smem) {
 
 solrt_status launch_extend(Context& ctx, uint32_t kind, const DevScene* scene, const DevJob* jobs, const PathQueue& q,
                            float4* hits, const unsigned int* count, uint32_t most, DevStats* st, bool any_hit) {
+    ctx.last_kind = kind;
     const ExtendArgs a{scene ? trav_scene(*scene) : TravScene{}, scene ? nullptr : jobs, q, hits, count, 0, 32, any_hit,
                        ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
                        st ? st : ctx.stats.as<DevStats>()};

@@ -251,6 +251,7 @@ struct Context {
     uint32_t noise_w = 0, noise_h = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint64_t launches = 0;
+    uint32_t last_kind = 0;  // nodes that the last traversal launch reads (solrt_debug_unit op 10)
     // stage timing (enable_timing): event pairs recorded around launches
     bool timing = false;
     struct TimedLaunch {

@@ -231,6 +231,7 @@ solrt_status launch_paths_kind(Context& ctx, PathArgs a) {
 
 template <bool kNee>
 solrt_status launch_paths_any(Context& ctx, uint32_t kind, const PathArgs& a) {
+    ctx.last_kind = kind;
     switch (kind) {
         case SOLRT_BVH8_Q8: return launch_paths_kind<SOLRT_BVH8_Q8, kNee>(ctx, a);
         case SOLRT_BVH4_Q8: return launch_paths_kind<SOLRT_BVH4_Q8, kNee>(ctx, a);

@@ -1397,6 +1397,14 @@ solrt_status debug_unit(Context& ctx, uint32_t op, uint32_t n, const uint32_t* a
         out_u32[0] = set_host_fault((HostFault)a[0], b[0]);
         return SOLRT_OK;
     }
+    if (op == 10) {  // nodes that the last traversal launch of a queue, a ray array or a frame reads
+        if (!out_u32) {
+            set_error("debug op 10 needs an output word");
+            return SOLRT_ERR_INVALID;
+        }
+        out_u32[0] = ctx.last_kind;
+        return SOLRT_OK;
+    }
     if (op > 7) {
         set_error("unknown debug op %u", op);
         return SOLRT_ERR_INVALID;

@@ -289,6 +289,7 @@ bool sibling_plain(const Scene& sc, const solrt_render_params& p) {
 }
 
 solrt_status launch_sibling(Context& ctx, uint32_t kind, const DevJob& J, bool plain) {
+    ctx.last_kind = kind;
     const SiblingArgs a{J, J.width * J.height, 0, ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
                         ctx.stats.as<DevStats>()};
     switch (kind) {

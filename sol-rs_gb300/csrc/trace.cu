@@ -69,6 +69,7 @@ solrt_status launch_kind(Context& ctx, TraceArgs a) {
 solrt_status launch_trace_rays(Context& ctx, const Scene& sc, const solrt_ray* rays, uint32_t n, solrt_hit* hits) {
     if (n == 0) return SOLRT_OK;
     const DevScene d = sc.view();
+    ctx.last_kind = d.bvh_kind;
     const TraceArgs a{trav_scene(d), reinterpret_cast<const float4*>(rays), reinterpret_cast<float4*>(hits), n, 0, 32,
                       ctx.trace_work.as<unsigned int>(), ctx.deep_stack.as<int>(),
                       ctx.stats.as<DevStats>()};

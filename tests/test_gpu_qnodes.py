@@ -177,3 +177,81 @@ def test_batch_launched_again_after_a_section_left_the_grid(solrt, ctx, graph, m
         assert np.array_equal(got, want)
     b.close()
     sc.close()
+
+
+def _kind(ctx):
+    """Nodes that the context's last traversal launch read."""
+    out = np.zeros(1, np.uint32)
+    ctx.debug_unit(10, 1, out_u=out)
+    return int(out[0])
+
+
+def _with_infinity():
+    d = S.soup(1000, seed=3, sigma=0.05)
+    v = d.vertices.copy()
+    v["pos"][7, 1] = np.inf
+    return S.SceneData(v, d.indices, d.sections, d.materials, None, d.camera, "inf")
+
+
+@pytest.mark.parametrize("maker,copy", [
+    (lambda: S.soup(511, seed=1, sigma=0.05), False), (lambda: S.soup(512, seed=1, sigma=0.05), True),
+    (lambda: S.soup(3001, seed=2, sigma=0.03), True), (lambda: _stretched(2000, 3.0), True),
+    (lambda: _stretched(2000, 1e3), False), (lambda: _stretched(2000, 1e7), False),
+    (lambda: _moved(2000, 0.0, 1e-6), True), (lambda: _moved(2000, 0.0, 3e5), True),
+    (lambda: _moved(2000, 0.0, 1e6), False), (lambda: _moved(2000, 9e6, 1e4), False), (_with_infinity, False),
+    (lambda: S.tunnel(n_ang=64, n_ax=32, length=300.0), True),
+], ids=["511", "512", "3001", "far3", "far1e3", "far1e7", "tiny", "cells8", "cells32", "off9e6", "inf", "tunnel"])
+def test_which_scenes_traverse_the_copy(solrt, ctx, maker, copy):
+    """Rays and frames read the copy where the rules take it; debug frames keep
+    the 64-byte nodes."""
+    d = maker()
+    sc = solrt.SceneDescription(ctx, d)
+    want = solrt.BVH2_Q16 if copy else solrt.BVH2
+    sc.trace_rays(np.zeros(1, solrt.RAY_DTYPE))
+    assert _kind(ctx) == want
+    cam = solrt.camera_look_at((0.5, 0.5, -1.2), (0.5, 0.5, 0.5), (0.0, -1.0, 0.0), 45.0, 1.0)
+    img = solrt.Image(ctx, 16, 16)
+    for integrator, kind in ((solrt.INTEGRATOR_DEBUG, solrt.BVH2), (solrt.INTEGRATOR_PATH, want)):
+        solrt.Renderer(ctx).cmd_trace_rays(sc, cam, solrt.render_params(16, 16, spp=1, integrator=integrator), img)
+        assert _kind(ctx) == kind
+    img.close()
+    sc.close()
+
+
+@pytest.mark.parametrize("mode", ["REGEN_REBUILD", "REGEN_REFIT"])
+@pytest.mark.parametrize("how", [{}, dict(graph=True), dict(cooperative=True), dict(cooperative=True, graph=True)],
+                         ids=["launches", "graph", "coop", "coop_graph"])
+def test_batch_follows_a_scene_over_the_growth_limit(solrt, ctx, how, mode):
+    """A section moves away until the grid is too coarse for the others, and
+    back: the updated batch (its graph captured again) changes nodes each time
+    and renders what a lone frame does."""
+    data = _sections((700, 50))
+    sc = solrt.SceneDescription(ctx, data, dynamic=True)
+    small = solrt.SceneDescription(ctx, S.soup(600, seed=30, sigma=0.05))
+    c = data.camera
+    cam = solrt.camera_look_at(c["eye"], c["center"], c["up"], c["vfov"], 1.0)
+    p = solrt.render_params(48, 48, spp=2, max_bounces=4, seed=9, miss_mode=solrt.MISS_GRADIENT,
+                            material_mode=solrt.MATERIAL_LAMBERT, rng_mode=solrt.RNG_PER_SAMPLE)
+    jobs = [(s, solrt.Image(ctx, 48, 48), cam, p) for s in (sc, small)]
+    alone = solrt.Image(ctx, 48, 48)
+    b = solrt.Batch(ctx, jobs, **how)
+    b.launch()
+    for x, kind in ((3000.0, solrt.BVH2), (0.0, solrt.BVH2_Q16), (3000.0, solrt.BVH2), (1.0, solrt.BVH2_Q16)):
+        sc.set_instances(_moved_section(data, 1, x))
+        sc.tlas_regenerate(getattr(solrt, mode))
+        b.update(jobs)
+        for turn in range(2):
+            for job in jobs:
+                job[1].clear()
+            b.launch()
+            if not how.get("graph") or turn == 0:
+                assert _kind(ctx) == kind
+        for s, img, _, _ in jobs:
+            alone.clear()
+            solrt.Renderer(ctx).cmd_trace_rays(s, cam, p, alone)
+            ctx.synchronize()
+            assert _kind(ctx) == (kind if s is sc else solrt.BVH2_Q16)
+            assert np.array_equal(img.read()[0].view(np.uint32), alone.read()[0].view(np.uint32))
+    b.close()
+    small.close()
+    sc.close()
