@@ -92,7 +92,13 @@ struct solrt_server {
     std::vector<uint64_t> active;
     std::list<uint64_t> done_lru;                     // completed, unreleased; front = least recently used
     std::deque<uint64_t> finished;                    // done / failed / cancelled, not yet fetched (completion queue)
-    std::unordered_map<solrt_scene*, int> scene_refs;  // admitted (active or done) jobs per scene
+    // admitted (active or done) jobs per scene, and the bytes it counted with when
+    // the first came (a scene's own may change with its rebuilds)
+    struct SceneUse {
+        int jobs = 0;
+        uint64_t bytes = 0;
+    };
+    std::unordered_map<solrt_scene*, SceneUse> scene_refs;
     uint64_t bytes_in_use = 0;
     solrt_server_stats st{};
     solrt::TickBuffers tb;
@@ -132,8 +138,8 @@ void drop_job_memory(solrt_server* srv, ServerJob& j) {
         srv->bytes_in_use -= j.image_bytes;
     }
     auto it = srv->scene_refs.find(j.scene);
-    if (it != srv->scene_refs.end() && --it->second == 0) {
-        srv->bytes_in_use -= scene_bytes(j.scene);
+    if (it != srv->scene_refs.end() && --it->second.jobs == 0) {
+        srv->bytes_in_use -= it->second.bytes;
         srv->scene_refs.erase(it);
     }
 }
@@ -198,7 +204,8 @@ void admit(solrt_server* srv) {
         j.counted = true;
         j.image_bytes = image_bytes_of(j.p, rule);
         srv->bytes_in_use += j.image_bytes;
-        if (srv->scene_refs[j.scene]++ == 0) srv->bytes_in_use += scene_bytes(j.scene);
+        solrt_server::SceneUse& use = srv->scene_refs[j.scene];
+        if (use.jobs++ == 0) srv->bytes_in_use += use.bytes = scene_bytes(j.scene);
         j.state = kActive;
         j.t_admit = now_ns();
         srv->active.push_back(j.ticket);

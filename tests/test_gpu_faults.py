@@ -116,19 +116,8 @@ def test_every_allocation_of_a_build_may_fail(solrt, oracle):
     assert len(without) == 1 and sizes[without[0]] == (0, sizes[last][1] - 32 * 1500)
 
 
-def test_moving_scene_without_memory_for_the_copy(solrt, ctx):
-    """Refits and rebuilds of a scene that was created without the copy take it
-    once there is memory, and render the same either way."""
-    b = S._Builder()
-    for k in range(2):
-        S.soup(600, seed=7 + k, sigma=0.05, builder=b)
-    data = b.build(S.soup(1).camera, "two")
-    data.instances = np.array([S.instance_of(np.eye(4), k) for k in range(2)], S.INSTANCE_DTYPE)
-    plain = solrt.SceneDescription(ctx, data, dynamic=True)
-    full = plain.device_bytes()
-    cam = camera_of(data, 1.0)
-    p = solrt.render_params(40, 40, spp=2, max_bounces=3, seed=5, material_mode=solrt.MATERIAL_LAMBERT,
-                            rng_mode=solrt.RNG_PER_SAMPLE)
+def _without_copy(solrt, data):
+    """A context and a moving scene on it that had no memory for the copy."""
     for nth in range(1, 100):
         c = solrt.Context(0, path_capacity=1 << 16)
         _let_fail(c, ALLOC, nth)
@@ -138,8 +127,29 @@ def test_moving_scene_without_memory_for_the_copy(solrt, ctx):
             sc = None
         assert _let_fail(c, ALLOC, 0) == 0
         if sc:
-            break
+            return c, sc
         c.close()
+
+
+def _two_sections():
+    b = S._Builder()
+    for k in range(2):
+        S.soup(600, seed=7 + k, sigma=0.05, builder=b)
+    data = b.build(S.soup(1).camera, "two")
+    data.instances = np.array([S.instance_of(np.eye(4), k) for k in range(2)], S.INSTANCE_DTYPE)
+    return data
+
+
+def test_moving_scene_without_memory_for_the_copy(solrt, ctx):
+    """Refits and rebuilds of a scene that was created without the copy take it
+    once there is memory, and render the same either way."""
+    data = _two_sections()
+    plain = solrt.SceneDescription(ctx, data, dynamic=True)
+    full = plain.device_bytes()
+    cam = camera_of(data, 1.0)
+    p = solrt.render_params(40, 40, spp=2, max_bounces=3, seed=5, material_mode=solrt.MATERIAL_LAMBERT,
+                            rng_mode=solrt.RNG_PER_SAMPLE)
+    c, sc = _without_copy(solrt, data)
     assert sc.device_bytes() == full - 32 * 1200
     want = solrt.Image(ctx, 40, 40)
     solrt.Renderer(ctx).cmd_trace_rays(plain, cam, p, want)
@@ -158,3 +168,24 @@ def test_moving_scene_without_memory_for_the_copy(solrt, ctx):
     sc.close()
     c.close()
     plain.close()
+
+
+def test_server_frees_what_a_scene_counted_with(solrt):
+    """A served scene that grows by its copy between two jobs leaves no bytes
+    in use, and none below zero."""
+    data = _two_sections()
+    c, sc = _without_copy(solrt, data)
+    cam = camera_of(data, 1.0)
+    p = solrt.render_params(32, 32, spp=1, max_bounces=2, material_mode=solrt.MATERIAL_LAMBERT,
+                            rng_mode=solrt.RNG_PER_SAMPLE)
+    srv = solrt.Server(c)
+    small = sc.device_bytes()
+    t = srv.submit(sc, cam, p)
+    assert srv.wait(t, 60000).status == 0
+    sc.tlas_regenerate(solrt.REGEN_REFIT)
+    assert sc.device_bytes() > small
+    srv.release(t)
+    assert srv.stats().bytes_in_use == 0
+    srv.close()
+    sc.close()
+    c.close()
