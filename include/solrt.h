@@ -219,9 +219,9 @@ typedef struct solrt_render_params {
 } solrt_render_params;
 
 /* What one launch computes per pixel. DEBUG and AO are the reference's
- * sibling ray-tracing pipelines over the same acceleration structure; they
- * run one thread per pixel (their shaders' structure), ignore `kernel`, and
- * are not accepted by batches or the server. */
+ * sibling ray-tracing pipelines over the same acceleration structure; each
+ * frame is one launch. They ignore `kernel` and are not accepted by batches or
+ * the server. */
 typedef enum solrt_integrator {
     /* pathtrace.rgen / .rchit / .rmiss */
     SOLRT_INTEGRATOR_PATH = 0,
@@ -308,7 +308,7 @@ typedef struct solrt_stats {
     uint64_t extend_launches; /* launches timed into extend_ms */
     uint64_t shade_launches;  /* launches timed into shade_ms */
     double generate_ms;       /* camera-ray generation (enable_timing) */
-    double accumulate_ms;     /* per-pixel sums, frame begin / finalize (enable_timing) */
+    double accumulate_ms;     /* per-pixel sums and images (enable_timing) */
     uint64_t shadow_segments; /* shadow rays traced (SOLRT_INTEGRATOR_PATH_NEE) */
     uint64_t shadow_unoccluded; /* of them, those that reached their light */
 } solrt_stats;

@@ -688,7 +688,7 @@ __global__ void k_offset_refs(float4* __restrict__ nodes, uint32_t ni, uint32_t 
 // into tri_idx), and the topology and exact boxes the wide collapse and the
 // refit reuse. Its depth goes to out->depth (read_build_out).
 struct Lbvh {
-    uint32_t n = 0, ni = 0, depth = 0;
+    uint32_t n = 0, ni = 0;
     DeviceBuffer nodes, tri_wt, child, par_int, par_leaf, range, nbox, order;
 };
 

@@ -1,8 +1,8 @@
 // coop.cu — SOLRT_BATCH_COOPERATIVE: a whole batch step as one persistent
 // wavefront launch.
 //
-// The wavefront stages of pathtrace.cu (generate, extend, shade, accumulate,
-// finalize) normally run as one launch per stage and bounce, about 14 per
+// The wavefront stages of pathtrace.cu (generate, extend, shade, resolve)
+// normally run as one launch per stage and bounce, about 14 per
 // pass. Here one cooperative grid of (SMs x resident blocks) runs every pass
 // of the batch: the stages become phases of the same kernel, and the grid
 // meets at a grid-wide barrier where a stage needs the previous one's output
@@ -419,7 +419,7 @@ SOLRT_D StackMem coop_stack(const int* s_stack, int* deep) {
 }
 
 // The closest hits of the n rays of queue q (the extend kernel's loop for
-// the kind, 32 shared-memory stack slots for the binary kinds). Returns
+// the kind, kCoopSlots shared-memory stack slots for the binary kinds). Returns
 // (FP64 fallbacks, error flags).
 template <int KIND, bool kNee>
 SOLRT_COOP_EXTEND_ATTR uint2 coop_extend(const CoopIOT<kNee>& io, uint32_t n, unsigned int* work, int* deep) {

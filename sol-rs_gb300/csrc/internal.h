@@ -173,13 +173,13 @@ constexpr uint32_t kDepthMask = (1u << kDepthBits) - 1u;
 struct PassPlan {
     uint32_t item_begin, item_count;
     uint32_t paths, pixels;
-    uint32_t bounces;  // bounce levels of the pass (cooperative batches)
+    uint32_t bounces;  // bounce levels of the pass
     uint32_t nee = 0;  // a job of the pass uses SOLRT_INTEGRATOR_PATH_NEE
 };
 
 struct Context;
 
-// A planned batch (also a single render: a batch of one job).
+// A planned batch (also a render with the per-pixel kernel: a batch of one job).
 struct Batch {
     Context* ctx = nullptr;
     uint32_t flags = 0;
@@ -226,7 +226,7 @@ struct Context {
     // a reference; the context is freed when the last one goes, so objects
     // destroyed after solrt_context_destroy stay valid until then.
     int refs = 1;
-    Batch single;  // plan of the last solrt_render call
+    Batch single;  // plan of the last solrt_render call with the per-pixel kernel (SOLRT_KERNEL_MEGA)
     TuneConfig tune;
     int device = 0;
     int sm_count = 0;
@@ -256,7 +256,7 @@ struct Context {
     bool timing = false;
     struct TimedLaunch {
         cudaEvent_t start, end;
-        int stage;  // 0 extend, 1 shade, 2 generate, 3 begin / accumulate / finalize
+        int stage;  // 0 extend, 1 shade, 2 generate, 3 sums and images
     };
     std::vector<TimedLaunch> timed;
     size_t timed_used = 0;

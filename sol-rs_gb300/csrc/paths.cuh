@@ -4,18 +4,18 @@
 // samples and up to maxBounces+1 traceRayEXT calls, each resuming in the
 // closest-hit or miss shader (assets/glsl/pathtrace.rgen:39-104,
 // pathtrace.rchit:56-113, pathtrace.rmiss:8-21). Here a warp holds up to 32
-// paths in the traversal loop of the BVH kind; when at least half of its lanes
-// have finished their rays, those lanes shade their hits and go on with the
-// next ray of their path, or end it and take another one from the launch's
-// work counter (warp_feed). Path state that traversal does not touch waits in
-// shared memory.
+// paths in the traversal loop of the BVH kind; when enough of its lanes have
+// finished their rays (12 of 32, 24 where traversal is short or shading long:
+// PathArgs::refill), those lanes shade their hits and go on with the next ray of
+// their path, or end it and take another one from the launch's work counter
+// (warp_feed). Path state that traversal does not touch waits in shared memory.
 //
 // What it saves over the wavefront (pathtrace.cu) is the launches, two per
 // bounce level, and the end of each extend launch, which lasts as long as its
 // longest ray with few other rays left to trace. What it costs is shading with
 // part of a warp while the other lanes wait: on frames large enough to fill
-// the wavefront's launches it is a third slower (path_kernel_pays, below,
-// draws the line).
+// the wavefront's launches it is a third slower (path_kernel_pays in
+// pathtrace.cu draws the line).
 //
 // A unit of work is a path, or, for jobs with one random stream per pixel
 // (SOLRT_RNG_REF_STREAM), a pixel whose samples the lane traces one after

@@ -8,11 +8,16 @@
 // stages over structure-of-arrays queues in HBM:
 //
 //   generate  camera rays for the (pixel, sample) pairs of a pass (rgen:47-61)
-//   extend    closest hit per queued ray                           (trace.cu)
+//   extend    closest hit per queued ray                           (extend.cu)
 //   shade     miss / emissive / scatter; survivors are appended to the next
-//             queue with one atomic per warp (ballot compaction)   (rchit, rmiss)
-//   accumulate per-pixel sums of the pass's path radiance, in sample order
-//   finalize  mean, running mix with NaN/Inf guard, gamma, RGBA8   (rgen:86-103)
+//             queue (ballot compaction)                            (rchit, rmiss)
+//   resolve   per-pixel sums of the pass's path radiance, in sample order, and
+//             once a job's samples are complete its images: mean, running mix
+//             with NaN/Inf guard, gamma, RGBA8                     (rgen:86-103)
+//
+// Served jobs, whose samples come in over many ticks, take the last stage in two
+// (k_accumulate, k_finalize). Frames with few rays per bounce level run as one
+// launch instead (path_kernel_pays).
 //
 // A pass is a list of work items (job, pixel range, sample range) whose
 // paths fit the queues. Items of different jobs share a pass: each path
@@ -841,6 +846,7 @@ solrt_status issue_frame(Context& ctx, const Scene& sc, uint32_t kind, const Dev
             pa.item = a.item;
             pa.units = stream ? npix : a.paths;
             // fuller warps to shade where traversal is short or shading long
+            // (small BVH2 scenes trace and shade with whole warps either way)
             pa.refill = nee || J.sc.tri_count < kSmallScene ? 24 : kShadeRefill;
             pa.work = ctx.trace_work.as<unsigned int>();
             pa.deep = ctx.deep_stack.as<int>();
