@@ -610,7 +610,7 @@ solrt_status quantize_bvh2(Context& ctx, DeviceBuffer& nodes, const float4* nbox
 // So: from kSmallScene triangles on, up to a mean growth of 1.25. The mean is
 // over the children, not weighted by area, so that a small detailed object in a
 // large scene counts. And cells up to 8 (coordinates up to 2^23, extents up to
-// 480,000): with larger ones the smallest direction component grows (q16_axis),
+// 480,000): with larger ones the smallest direction component grows (q16_ray),
 // and rays with short axis-parallel directions would leave boxes that FP32 nodes
 // keep them in. `nbox` holds the exact internal-node boxes (root first); the
 // growth goes to `out` (which must start at 0), read by finish_nodes_q16. A scene
