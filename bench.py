@@ -41,35 +41,41 @@ METRIC = "Mrays/s at RMSE≤1e-3 vs FP64 oracle, batched vs plain on 1 GB300; p9
 UNIT = "Mrays/s"
 
 NODE_BYTES = {0: 64, 1: 80, 2: 64, 3: 224, 4: 32, 5: 64}
-# What ncu measured of the BVH2 extend kernel on the full-size workloads.
-# dram_bytes_per_segment: dram__bytes_read.sum + dram__bytes_write.sum over
-# all extend launches of one full wavefront pass, divided by the segments
-# the pass traced (profiles/extend_dram_soup1M_tunnel4M.md). limiter: the
-# counters of one `ncu --set full` launch (profiles/extend_soup1M_bvh2_full.md,
-# profiles/extend_soup1M_treelet_full.md, profiles/extend_tunnel_640x360_full.md).
-# All were captured with the 64-byte nodes, before the traversal's 32-byte
-# copies of them.
-# Keys: (workload, "lbvh" or "treelet" BVH2).
+# What ncu measured of the BVH2 extend kernel on the full-size workloads, on the
+# 32-byte node copies that it traverses. dram_bytes_per_segment:
+# dram__bytes_read.sum + dram__bytes_write.sum over all extend launches of one
+# full wavefront pass (soup 16 spp, tunnel 8 spp), divided by the segments the
+# pass traced. limiter: the counters of one `ncu --set full` launch, bounce level
+# 1 of a reduced frame (soup 4 spp, tunnel 640x360 at 8 spp). Keys: (workload,
+# "lbvh" or "treelet" BVH2).
+_DRAM_SOURCE = "ncu, all extend launches of one %d-spp frame"
+_LIMITER_SOURCE = "ncu --set full, bounce level 1 of %s"
+
+
+def _limiter(lsu, l1tex, issue, alu, threads, warps, l2, frame):
+    return {"issue_active_pct": issue, "alu_pipe_pct": alu, "l1tex_lsu_wavefronts_pct": lsu,
+            "l1tex_throughput_pct": l1tex, "threads_per_instruction": threads, "warps_active_pct": warps,
+            "l2_hit_pct": l2, "source": _LIMITER_SOURCE % frame}
+
+
 EXTEND_CAPTURES = {
-    ("soup", "lbvh"): {"dram_bytes_per_segment": 62.4, "dram_source": "profiles/extend_dram_soup1M_tunnel4M.md",
-             "limiter": {"l1tex_lsu_wavefronts_pct": 83.8, "l1tex_throughput_pct": 87.8, "issue_active_pct": 60.7,
-                         "threads_per_instruction": 14.27, "warps_active_pct": 48.0, "l2_hit_pct": 96.7,
-                         "dram_throughput_pct": 1.4, "source": "profiles/extend_soup1M_bvh2_full.md"}},
-    ("soup", "treelet"): {"dram_bytes_per_segment": 62.2, "dram_source": "profiles/extend_dram_soup1M_tunnel4M.md",
-                          "limiter": {"l1tex_lsu_wavefronts_pct": 85.2, "l1tex_throughput_pct": 87.9,
-                                      "issue_active_pct": 66.1, "threads_per_instruction": 14.83,
-                                      "warps_active_pct": 48.7, "l2_hit_pct": 94.2,
-                                      "source": "profiles/extend_soup1M_treelet_full.md"}},
-    ("tunnel", "treelet"): {"dram_bytes_per_segment": 78.0, "dram_source": "profiles/extend_dram_soup1M_tunnel4M.md",
-                            "limiter": {"l1tex_lsu_wavefronts_pct": 70.0, "l1tex_throughput_pct": 75.1,
-                                        "issue_active_pct": 65.2, "threads_per_instruction": 14.55,
-                                        "warps_active_pct": 46.7, "l2_hit_pct": 90.1,
-                                        "source": "profiles/extend_tunnel_640x360_full.md (treelet BVH2, bounce level 1)"}},
-    ("tunnel", "lbvh"): {"dram_bytes_per_segment": 78.8, "dram_source": "profiles/extend_dram_soup1M_tunnel4M.md",
-               "limiter": {"l1tex_lsu_wavefronts_pct": 71.9, "l1tex_throughput_pct": 77.7, "issue_active_pct": 65.0,
-                           "threads_per_instruction": 14.52, "warps_active_pct": 46.9, "l2_hit_pct": 91.7,
-                           "source": "profiles/extend_tunnel_640x360_full.md (bounce level 1)"}},
+    ("soup", "lbvh"): {"dram_bytes_per_segment": 51.4, "dram_source": _DRAM_SOURCE % 16,
+                       "limiter": _limiter(67.5, 70.2, 77.0, 67.0, 16.46, 61.0, 92.8, "a 4-spp frame")},
+    ("soup", "treelet"): {"dram_bytes_per_segment": 51.3, "dram_source": _DRAM_SOURCE % 16,
+                          "limiter": _limiter(66.3, 69.5, 76.7, 65.4, 16.42, 61.1, 92.2, "a 4-spp frame")},
+    ("tunnel", "treelet"): {"dram_bytes_per_segment": 60.2, "dram_source": _DRAM_SOURCE % 8,
+                            "limiter": _limiter(51.0, 59.5, 72.9, 59.9, 15.16, 58.8, 88.8, "a 640x360 frame")},
+    ("tunnel", "lbvh"): {"dram_bytes_per_segment": 60.6, "dram_source": _DRAM_SOURCE % 8,
+                         "limiter": _limiter(54.4, 61.5, 74.0, 62.5, 15.28, 59.0, 90.3, "a 640x360 frame")},
 }
+
+
+def traversed_kind(ctx):
+    """solrt_bvh_kind of the nodes that the context's last traversal launch
+    read: a BVH2 scene's may be its 32-byte copy."""
+    out = np.zeros(1, np.uint32)
+    ctx.debug_unit(10, 1, out_u=out)
+    return int(out[0])
 
 
 def workload(name):
@@ -265,7 +271,7 @@ def precision_study(local, data, kw, cam, main_mrays, main_info, main_nodes, mai
     hit records of 4M rays (every pixel-centre camera ray of the frame, then
     seeded rays from inside the scene's bounds) traced on the device by each
     kind and compared bit for bit with the oracle's CPU LBVH traversal on all
-    host cores (the checker), node bytes, visits per segment, Mrays/s of one
+    host cores, node bytes, visits per segment, Mrays/s of one
     frame and the FP64 fallback count of each."""
     import torch
     import oracle
@@ -337,7 +343,7 @@ def precision_study(local, data, kw, cam, main_mrays, main_info, main_nodes, mai
                 tris = cs.tri_tests / max(cs.segments, 1)
                 cimg.close()
                 csc.close()
-            nb = NODE_BYTES[info.kind]
+            nb = NODE_BYTES[traversed_kind(ctx)]
             out[name] = {"mrays_per_s": round(mr, 1) if mr else None, "node_bytes": int(info.node_bytes),
                          "node_count": int(info.node_count), "bytes_per_node": nb,
                          "nodes_per_segment": round(nodes, 2) if nodes is not None else None,
@@ -353,7 +359,7 @@ def precision_study(local, data, kw, cam, main_mrays, main_info, main_nodes, mai
 def rmse_vs_fp64(local, data, kw, cam, bvh, rows, frames=1, sah=False):
     """RMSE of the device RGBA32F image (after `frames` accumulated frames)
     against the FP64 oracle on identical RNG streams, over image rows
-    [rows[0], rows[1]) (the oracle is the checker). Also compares the same
+    [rows[0], rows[1]). Also compares the same
     rows with the FP32 oracle bit for bit."""
     import oracle
     solrt = importlib.import_module("sol-rs_gb300")
@@ -958,6 +964,8 @@ def main():
     barrier(pg)
     ms = e0.elapsed_time(e1)
     st = ctx.stats()
+    # the per-pixel kernel reads the scene's own nodes
+    node_kind = info.kind if args.kernel == "mega" else traversed_kind(ctx)
     clk = clocks.stop()
     ms_max = max_over_ranks(pg, ms)
     seg_total = sum_over_ranks(pg, float(st.segments))
@@ -1026,7 +1034,7 @@ def main():
 
     # roofline of the extend kernel
     peak, peak_kind = peaks()
-    b_seg = 32 + 16 + NODE_BYTES[info.kind] * nodes_per_seg + 48 * tris_per_seg
+    b_seg = 32 + 16 + NODE_BYTES[node_kind] * nodes_per_seg + 48 * tris_per_seg
     ext_s = ts.extend_ms / 1000.0
     stages_ms = ts.generate_ms + ts.extend_ms + ts.shade_ms + ts.accumulate_ms
     if args.kernel == "mega":  # traversal and shading in one launch: the whole render time
@@ -1047,8 +1055,7 @@ def main():
                 "frac": round(achieved / peak, 4), "traffic": traffic,
                 "frac_note": "achieved counts algorithmic bytes (node, triangle, ray and hit bytes of every visit) "
                              "with no cache reuse; L1 / L2 serve nearly all of them, so frac > 1 is not HBM "
-                             "traffic; BVH2 nodes count 64 bytes each, also where the traversal reads its 32-byte "
-                             "copy of them; dram and limiter were captured before those copies" if cap else None,
+                             "traffic: dram is what reaches HBM, limiter what binds" if cap else None,
                 "dram": dram, "limiter": cap["limiter"] if (cap and dram) else None,
                 "peak_source": peak_kind + " (MEASURED_PEAKS hbm_gbs)",
                 "kernel": "k_megakernel (traversal + shading, whole render time)" if args.kernel == "mega"
@@ -1068,7 +1075,7 @@ def main():
                           "peak_source": "measured here: 32 MB device-to-device copy, L2-resident, best of 20"}
 
     # RMSE of the device image against the FP64 oracle on the same RNG
-    # streams, over a central band of rows (the oracle is the checker); the
+    # streams, over a central band of rows; the
     # tunnel accumulates four frames (its sun-lit sky makes FP32 and FP64
     # paths that part ways differ by a lot for a few samples)
     rmse = None

@@ -1,7 +1,7 @@
 """ctypes binding of the CPU oracle (oracle.cpp). TEST INFRASTRUCTURE ONLY.
 
 Imported by the tests, the smoke check and the CPU-baseline leg of bench.py
-as the checker; never by the product. Parity status: the sampling and
+to check results; never by the product. Parity status: the sampling and
 postprocess functions and the whole path (pathtrace.rgen / .rchit / .rmiss)
 are pinned against the reference's own shaders compiled as C++
 (oracle/ref_glsl, ref_path_render below); unpinned only where the reference

@@ -1,7 +1,7 @@
 // oracle.cpp — CPU oracle of the solrt path tracer. TEST INFRASTRUCTURE ONLY.
 //
 // Loaded (through ctypes) by the tests, the smoke check and the CPU-baseline
-// leg of the benchmark, as the checker. Product code never links it.
+// leg of the benchmark, to check results. Product code never links it.
 //
 // Scalar C++17, templated on the real type R (float for bit-exact parity with
 // the device code, double for the converged FP64 reference images). Built

@@ -2,7 +2,7 @@
  * oracle.h — CPU oracle of the solrt path tracer. TEST INFRASTRUCTURE ONLY.
  *
  * Only the tests, the smoke check and the CPU-baseline leg of the benchmark
- * load this library, and only as the checker: no product code links it.
+ * load this library, and only to check results: no product code links it.
  *
  * It restates, in scalar C++ templated on the real type (float / double):
  *   - assets/glsl/sampling.glsl:18-96   tea, nextRand, fresnelDielectric,
